@@ -22,7 +22,7 @@ import torch
 from . import _lib
 from .schedule import (MixedGearM2LSchedule, gear_m2l_mixed_schedule, gear_m2l_mixed_schedule_device,
                        gear_m2l_schedule, gear_m2l_schedule_device, leaf_schedule, leaf_schedule_device,
-                       m2l_schedule, m2l_schedule_device, mixed_ladder, tc_m2l_schedule)
+                       m2l_schedule, m2l_schedule_device, m2l_unit_limit, mixed_ladder, tc_m2l_schedule)
 from .tree import Topology
 
 
@@ -297,7 +297,7 @@ class Pass:
     def __init__(self, dt: DeviceTopology, p: int, *, G: float = 1.0, eps2: float = 0.0,
                  m2l_mode: int = _lib.JB_M2L_FP32, p2p_mode: int = _lib.JB_P2P_FP32,
                  leaf_range: tuple[int, int] | None = None, m2l_unit_pairs: int | None = None,
-                 leaf_unit_sources: int = 4096, gear_unit_pairs: int = 128, gear_form: str = "mixed"):
+                 leaf_unit_sources: int = 4096, gear_unit_pairs: int | None = None, gear_form: str = "mixed"):
         if not (1 <= int(p) <= _lib.JB_MAX_ORDER):
             raise ValueError(f"max_order must be in [1, {_lib.JB_MAX_ORDER}], got {p}")
         if dt.topo.max_leaf_occupancy > _lib.JB_MAX_LEAF_OCCUPANCY:
@@ -314,8 +314,12 @@ class Pass:
         self.tc_layout = "units"
         self.tc_products = 1
         self.p2p_mode = int(p2p_mode)
-        # work-unit sizes (pairs per M2L unit, per gear unit; sources per leaf
-        # unit), measured at clustered N=4M, p=8
+        # work-unit sizes: pairs per M2L unit and per gear unit by the length of
+        # the far list (m2l_unit_limit), sources per leaf unit measured at
+        # clustered N=4M, p=8
+        npairs = dt.topo.num_far_pairs
+        if gear_unit_pairs is None:
+            gear_unit_pairs = m2l_unit_limit(npairs, mixed=True) if gear_form == "mixed" else 128
         self.gear_unit_pairs = int(gear_unit_pairs)
         # per-pair gears: "mixed" (one launch, jb_m2l_mixed) when the orders lie
         # on mixed_ladder(p), else (or "per_gear") one launch per gear
@@ -323,7 +327,7 @@ class Pass:
             raise ValueError(f"gear_form must be 'mixed' or 'per_gear', got {gear_form!r}")
         self.gear_form = gear_form
         if m2l_unit_pairs is None:  # the tensor-core form steps a group's units together: shorter units
-            m2l_unit_pairs = 64 if self.m2l_mode == _lib.JB_M2L_SPLIT_BF16 else 512
+            m2l_unit_pairs = 64 if self.m2l_mode == _lib.JB_M2L_SPLIT_BF16 else m2l_unit_limit(npairs)
         self.m2l_unit_pairs = int(m2l_unit_pairs)
         self.leaf_unit_sources = int(leaf_unit_sources)
         self.ws = Workspace.allocate(dt, self.p)
@@ -764,7 +768,8 @@ class Pass:
         if hasattr(self, "_adj_m2l"):
             msc = self._adj_m2l
         else:
-            msc = m2l_schedule_device(dt, max_pairs=512) if _on_gpu(dt) else m2l_schedule(t, max_pairs=512)
+            mp = m2l_unit_limit(t.num_far_pairs)
+            msc = m2l_schedule_device(dt, max_pairs=mp) if _on_gpu(dt) else m2l_schedule(t, max_pairs=mp)
             self._adj_m2l = msc
             up = lambda a: _up(a, dt.device)
             A["m2l_units"], A["m2l_split"] = up(msc.units), up(msc.split)

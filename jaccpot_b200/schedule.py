@@ -48,6 +48,34 @@ def _slots(n_per: np.ndarray) -> tuple[np.ndarray, np.ndarray]:
     return slot, slot[first]
 
 
+# Threads of the M2L kernels resident on a B200: 148 SMs x 4 blocks x 64.
+M2L_RESIDENT_THREADS = 148 * 4 * 64
+
+
+def m2l_unit_limit(num_pairs: int, mixed: bool = False) -> int:
+    """Pairs per M2L unit for a far list of ``num_pairs``.
+
+    A unit is one thread's serial chain (about 0.7 us a pair at order 4, 2.5 us
+    at order 8), so with few pairs a launch lasts as long as its longest unit
+    while most of the chip idles.  The limit is an even share of the pairs over
+    the resident threads, rounded up to a power of two.  Below 8 the partial
+    rows of split targets cost more than the shorter chains save; above 512
+    only the evenness of the launch's end changes, which the near field running
+    beside it hides (Plummer 1M p=6: the M2L alone 1008 us at 512 and 960 at
+    256, the step 2126 and 2134).  Measured (M2L with its split reduce, us, a
+    fixed 512 -> this): uniform 16k p=4 291 -> 40, Plummer 131k p=6 598 -> 147,
+    clustered 200k p=10 4888 -> 263, clustered 300k p=8 911 -> 222.
+    ``mixed``: units whose pairs have several orders end more unevenly (the
+    lanes of a warp wait for one another at every order), and half the share,
+    at most 64, is best (a fixed 128 -> this: clustered 100k 238 -> 74, 500k
+    422 -> 327, 2M 1384 -> 1229)."""
+    share, most = (2, 64) if mixed else (1, 512)
+    limit = 8
+    while limit < most and limit * M2L_RESIDENT_THREADS * share < num_pairs:
+        limit *= 2
+    return limit
+
+
 def m2l_schedule(topo: Topology, max_pairs: int = 64, targets: np.ndarray | None = None) -> M2LSchedule:
     off = topo.far_offsets
     counts = np.diff(off)
