@@ -473,6 +473,14 @@ JB_API int jb_leaf_eval_noalloc(int p, int p2p_mode, const float* pos4, int num_
                                 const float* centers, const float* locals, float G, float eps2, float* out_acc4,
                                 int num_slots, int num_split, const int* split, void* stream);
 
+/* Sorted slots of input-order target indices: slots[q] = inv_perm[targets[q]],
+ * n particles.  An index outside [0, n) takes slot 0 and sets the flag, which
+ * is copied to *bad_host (pinned, so that the copy is asynchronous): record an
+ * event after this call, queue jb_eval_targets, then wait for the event alone
+ * and look at the flag.                                                      */
+JB_API int jb_sort_targets(int64_t n, int64_t num_targets, const int64_t* targets, const int64_t* inv_perm,
+                           int* slots, int* bad_dev, int* bad_host, void* stream);
+
 /* Target subset (runtime/kernels/_evaluate.py:1941-2095): targets_sorted are
  * sorted-slot indices; out_acc4[q] in target order. */
 JB_API int jb_eval_targets(int p, const float* pos4, int num_internal, const int* node_ranges,

@@ -74,6 +74,18 @@ __global__ void k_gather_unsorted(int64_t n, const float4* __restrict__ acc4, co
   if (out_pot) out_pot[j] = a.w;
 }
 
+// Sorted slot of each target index; an index outside [0, n) takes slot 0 and
+// sets *bad, so whatever is queued behind reads in range.
+__global__ void k_sort_targets(int64_t n, int64_t num_targets, const int64_t* __restrict__ targets,
+                               const int64_t* __restrict__ inv_perm, int* __restrict__ slots, int* __restrict__ bad) {
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= num_targets) return;
+  const int64_t t = targets[q];
+  const bool ok = t >= 0 && t < n;
+  slots[q] = ok ? (int)inv_perm[t] : 0;
+  if (!ok) *bad = 1;
+}
+
 // ---------------------------------------------------------------------------
 // List validation (prepare time).
 // ---------------------------------------------------------------------------
@@ -494,6 +506,22 @@ JB_API int jb_gather_unsorted(int64_t n, const float* acc4, const int64_t* inv_p
   k_gather_unsorted<<<blocks_1d(n, 256), 256, 0, ST(stream)>>>(n, reinterpret_cast<const float4*>(acc4), inv_perm,
                                                                  out_acc, out_pot);
   return launch_status();
+}
+
+JB_API int jb_sort_targets(int64_t n, int64_t num_targets, const int64_t* targets, const int64_t* inv_perm, int* slots,
+                           int* bad_dev, int* bad_host, void* stream) {
+  if (n < 1 || num_targets < 0 || !bad_dev || !bad_host ||
+      (num_targets > 0 && (!targets || !inv_perm || !slots)))
+    return JB_ERR_ARG;
+  cudaError_t e = cudaMemsetAsync(bad_dev, 0, sizeof(int), ST(stream));
+  if (e != cudaSuccess) return cuda_status(e);
+  if (num_targets > 0) {
+    k_sort_targets<<<blocks_1d(num_targets, 256), 256, 0, ST(stream)>>>(n, num_targets, targets, inv_perm, slots,
+                                                                        bad_dev);
+    const int rc = launch_status();
+    if (rc) return rc;
+  }
+  return cuda_status(cudaMemcpyAsync(bad_host, bad_dev, sizeof(int), cudaMemcpyDeviceToHost, ST(stream)));
 }
 
 JB_API int jb_validate_lists(int num_nodes, int num_internal, const int* left, const int* right,

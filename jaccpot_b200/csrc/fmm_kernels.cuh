@@ -486,6 +486,7 @@ static __global__ void __launch_bounds__(256) k_m2l_reduce(int num_split, const 
   if (i >= num_split) return;
   const int4 sp = split[i];
   float a = 0.f;
+#pragma unroll 8
   for (int q = 0; q < sp.z; ++q) a += partials[(size_t)(sp.y + q) * CS + k];
   locals[(size_t)sp.x * CS + k] = a;
 }
@@ -1506,44 +1507,69 @@ static __global__ void __launch_bounds__(256) k_leaf_reduce(int num_split, const
 }
 
 // ---------------------------------------------------------------------------
-// Target subset: warp per target, lane per source leaf.
+// Target subset: far field (thread per target), then near field (warp per
+// target, added to it).  Two kernels, because the far field's harmonics take
+// a register array and one lane's time: with both in one warp-per-target
+// kernel 31 lanes waited for that lane and the registers halved the warps.
 // ---------------------------------------------------------------------------
 template <int P>
-__global__ void __launch_bounds__(128) k_eval_targets(const float4* __restrict__ pos4, int num_internal,
-                                                      const int2* __restrict__ ranges, const float4* __restrict__ centers,
-                                                      const float* __restrict__ locals, const int64_t* __restrict__ near_off,
-                                                      const int* __restrict__ near_src, const int* __restrict__ leaf_of,
-                                                      int64_t num_targets, const int* __restrict__ tsorted, float G,
-                                                      float eps2, float4* __restrict__ out) {
+__global__ void __launch_bounds__(128) k_targets_far(const float4* __restrict__ pos4, int num_internal,
+                                                     const float4* __restrict__ centers,
+                                                     const float* __restrict__ locals, const int* __restrict__ leaf_of,
+                                                     int64_t num_targets, const int* __restrict__ tsorted, float G,
+                                                     float4* __restrict__ out) {
   constexpr int C = csize(P), CS = cstride(P);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t q = (int64_t)blockIdx.x * 4 + warp;
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= num_targets) return;
+  const int i = tsorted[q];
+  const int node = num_internal + leaf_of[i];
+  const float4 ti = pos4[i], c = centers[node];
+  float U[C];
+  solid_harmonics<P>(c.x - ti.x, c.y - ti.y, c.z - ti.z, U);
+  float phi, g[3];
+  l2p_eval<P>(SmemF{locals + (size_t)node * CS}, U, &phi, g);
+  out[q] = make_float4(-G * g[0], -G * g[1], -G * g[2], -G * phi);
+}
+
+// The lanes look up 32 neighbour leaves at once (the target's own leaf
+// first); leaves that follow one another in memory join into runs, and the
+// warp reads each run's particles 32 at a time in consecutive 16-byte words.
+// With a leaf per lane instead, every load touched 32 cache lines and the L1
+// bounded the kernel: 65,536 targets of a Plummer sphere of 1M (order 6, leaf
+// 32, 1,900 sources each) took 387 us in one kernel, 330 us in these two.
+static __global__ void __launch_bounds__(256) k_targets_near(
+    const float4* __restrict__ pos4, int num_internal, const int2* __restrict__ ranges,
+    const int64_t* __restrict__ near_off, const int* __restrict__ near_src, const int* __restrict__ leaf_of,
+    int64_t num_targets, const int* __restrict__ tsorted, float G, float eps2, float4* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (q >= num_targets) return;
   const int i = tsorted[q];
   const int leaf = leaf_of[i];
-  const int node = num_internal + leaf;
   const float4 ti = pos4[i];
   float ax = 0.f, ay = 0.f, az = 0.f, aw = 0.f;
-  // lane k takes the k-th source leaf of each group of 32 (the target's own
-  // leaf first) and runs through its particles: the leaves' range lookups
-  // overlap instead of following one another
   const int64_t e0 = near_off[leaf], e1 = near_off[leaf + 1];
   for (int64_t eb = e0 - 1; eb < e1; eb += 32) {
     const int64_t e = eb + lane;
-    if (e >= e1) continue;
-    const int2 sr = (e < e0) ? ranges[node] : ranges[num_internal + near_src[e]];
-    for (int j = sr.x; j <= sr.y; ++j) {
-      const float4 s = pos4[j];
-      const float dx = ti.x - s.x, dy = ti.y - s.y, dz = ti.z - s.z;
-      const float d2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-      const float ir = rsqrt_ftz(d2);
-      const bool self = (j == i);
-      const float mir = self ? 0.f : s.w * ir;
-      const float w = self ? 0.f : mir * ir * ir;
-      ax = fmaf(w, dx, ax);
-      ay = fmaf(w, dy, ay);
-      az = fmaf(w, dz, az);
-      aw += mir;
+    int2 sr = make_int2(0, -1);  // past the list: a run of no particles
+    if (e < e1) sr = ranges[num_internal + (e < e0 ? leaf : near_src[e])];
+    const int before = __shfl_up_sync(0xffffffffu, sr.y, 1);
+    unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || sr.x != before + 1);
+    while (heads) {
+      const int h = __ffs(heads) - 1;
+      heads &= heads - 1;
+      const int last = __shfl_sync(0xffffffffu, sr.y, heads ? __ffs(heads) - 2 : 31);
+      for (int j = __shfl_sync(0xffffffffu, sr.x, h) + lane; j <= last; j += 32) {
+        const float4 s = pos4[j];
+        const float dx = ti.x - s.x, dy = ti.y - s.y, dz = ti.z - s.z;
+        const float ir = rsqrt_ftz(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2))));
+        const float mir = j == i ? 0.f : s.w * ir;
+        const float w = j == i ? 0.f : mir * ir * ir;
+        ax = fmaf(w, dx, ax);
+        ay = fmaf(w, dy, ay);
+        az = fmaf(w, dz, az);
+        aw += mir;
+      }
     }
   }
 #pragma unroll
@@ -1554,13 +1580,8 @@ __global__ void __launch_bounds__(128) k_eval_targets(const float4* __restrict__
     aw += __shfl_xor_sync(0xffffffffu, aw, o);
   }
   if (lane == 0) {
-    const float4 c = centers[node];
-    float U[C];
-    solid_harmonics<P>(c.x - ti.x, c.y - ti.y, c.z - ti.z, U);
-    const float* F = locals + (size_t)node * CS;
-    float phi, g[3];
-    l2p_eval<P>(SmemF{F}, U, &phi, g);
-    out[q] = make_float4(-G * ax - G * g[0], -G * ay - G * g[1], -G * az - G * g[2], -G * aw - G * phi);
+    const float4 f = out[q];
+    out[q] = make_float4(fmaf(-G, ax, f.x), fmaf(-G, ay, f.y), fmaf(-G, az, f.z), fmaf(-G, aw, f.w));
   }
 }
 
@@ -1748,10 +1769,14 @@ struct RunTargets {
                  const int64_t* near_off, const int* near_src, const int* leaf_of, int64_t nt, const int* ts, float G,
                  float eps2, float* out, cudaStream_t st) {
     if (nt <= 0) return JB_OK;
-    k_eval_targets<P><<<blocks_for(nt, 4), 128, 0, st>>>(
-        reinterpret_cast<const float4*>(pos4), num_internal, reinterpret_cast<const int2*>(ranges),
-        reinterpret_cast<const float4*>(centers), locals, near_off, near_src, leaf_of, nt, ts, G, eps2,
-        reinterpret_cast<float4*>(out));
+    k_targets_far<P><<<blocks_for(nt, 128), 128, 0, st>>>(
+        reinterpret_cast<const float4*>(pos4), num_internal, reinterpret_cast<const float4*>(centers), locals,
+        leaf_of, nt, ts, G, reinterpret_cast<float4*>(out));
+    const int rc = launch_status();
+    if (rc) return rc;
+    k_targets_near<<<blocks_for(nt, 8), 256, 0, st>>>(
+        reinterpret_cast<const float4*>(pos4), num_internal, reinterpret_cast<const int2*>(ranges), near_off, near_src,
+        leaf_of, nt, ts, G, eps2, reinterpret_cast<float4*>(out));
     return launch_status();
   }
 };

@@ -624,6 +624,28 @@ class Pass:
                                             _ptr(out), _stream_handle(stream)), "jb_eval_targets")
         return out
 
+    def evaluate_input_targets(self, targets: torch.Tensor) -> torch.Tensor:
+        """evaluate_targets for input-order indices (int64, on the device);
+        raises IndexError for one out of range.  The slots and the range check
+        are one kernel over the resident permutation, and the host waits for
+        the check alone, with the evaluation already queued behind it."""
+        dev, n, nt = self.dt.device, self.dt.topo.num_particles, int(targets.numel())
+        targets = targets.contiguous()
+        buf = torch.empty(nt + 1, device=dev, dtype=torch.int32)
+        bad = torch.empty(1, dtype=torch.int32, pin_memory=True)
+        _lib.check(self.lib.jb_sort_targets(n, nt, _ptr(targets), _ptr(self.dt.inv_perm), _ptr(buf),
+                                            buf.data_ptr() + 4 * nt, _ptr(bad), _stream_handle(None)),
+                   "jb_sort_targets")
+        checked = torch.cuda.Event()
+        checked.record()
+        try:
+            out = self.evaluate_targets(buf[:nt])
+        finally:
+            checked.synchronize()  # the flag's copy is done with its pinned word
+        if int(bad[0]):
+            raise IndexError("target_indices out of range")
+        return out
+
     def unsort(self, acc: torch.Tensor, pot: torch.Tensor | None, stream=None) -> None:
         n = self.dt.topo.num_particles
         _lib.check(self.lib.jb_gather_unsorted(n, _ptr(self.ws.acc4), _ptr(self.dt.inv_perm), _ptr(acc),

@@ -443,11 +443,7 @@ class FastMultipoleMethod:
             ps.unsort(acc, pot)
         else:
             ti = _to_torch(target_indices, dev, torch.int64).reshape(-1)
-            if ti.numel() and (int(ti.min()) < 0 or int(ti.max()) >= state.num_particles):
-                raise IndexError("target_indices out of range")
-            inv = torch.from_numpy(state.topology.inverse_permutation).to(dev)
-            ts = inv[ti].to(torch.int32)
-            out = ps.evaluate_targets(ts)
+            out = ps.evaluate_input_targets(ti)
             acc = out[:, :3].contiguous()
             pot = out[:, 3].contiguous() if return_potential else None
         self._counters["evaluate"] += 1
