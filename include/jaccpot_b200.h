@@ -105,7 +105,8 @@ enum {
   JB_TREE_NEAR_SOURCES = 11,    /* int32[num_near_pairs] (leaf indices) */
   JB_TREE_CENTERS_F64 = 12,     /* double[3*num_nodes], COM */
   JB_TREE_RADII_F64 = 13,       /* double[num_nodes], bounding radius about COM */
-  JB_TREE_FAR_GEARS = 14        /* int32[num_far_pairs]: gear of each far pair (jb_dtree_adaptive_walk only) */
+  JB_TREE_FAR_GEARS = 14,       /* int32[num_far_pairs]: gear of each far pair (jb_dtree_adaptive_walk only) */
+  JB_TREE_INVERSE_PERMUTATION = 15 /* int64[num_particles]: input index -> sorted slot (device trees only) */
 };
 
 /* Morton sort + radix tree with leaves of <= leaf_size particles + dual
@@ -139,6 +140,9 @@ JB_API int jb_dtree_info(const jb_dtree* t, jb_tree_info_t* info);
 JB_API const void* jb_dtree_field(const jb_dtree* t, int field);
 /* Synchronous device-to-host copy of a field (sizes as for jb_tree_copy). */
 JB_API int jb_dtree_copy(const jb_dtree* t, int field, void* dst);
+/* Copies count fields into device buffers dst[k] (sizes as for jb_tree_copy),
+ * in stream order. */
+JB_API int jb_dtree_export(const jb_dtree* t, int count, const int* fields, void* const* dst, void* stream);
 JB_API void jb_dtree_free(jb_dtree* t);
 
 /* Replaces the far and near lists of a device tree by those of the

@@ -53,6 +53,8 @@ TREE_FIELDS = {
     "radii_f64": (13, "float64"),
     "far_gears": (14, "int32"),
 }
+# fields only a device tree has
+DTREE_FIELDS = {**TREE_FIELDS, "inverse_permutation": (15, "int64")}
 
 
 class JBError(RuntimeError):
@@ -90,6 +92,7 @@ _SIGNATURES = {
     "jb_dtree_field": [_P, _I],
     "jb_dtree_copy": [_P, _I, _P],
     "jb_dtree_free": [_P],
+    "jb_dtree_export": [_P, _I, _P, _P, _P],
     "jb_dtree_adaptive_walk": [_P, _I, _P, _P, _D, _D, _D, _I, _P, _P],
     "jb_node_dehnen_power": [_I, _I, _P, _I, _P, _P],
     "jb_far_dehnen_gears": [_I64, _P, _P, _P, _P, _I, _P, _P, _D, _D, _I, _P, _P, _P],

@@ -8,14 +8,14 @@
 //   2. breadth-first radix split: a range of more than leaf_size particles is
 //      split at the highest differing code bit (duplicates at the midpoint);
 //      internal ids in BFS order, leaves renumbered in particle order
-//                                                -> one k_level_* pair per level;
+//                                                -> k_level_rank, k_level_emit per level;
 //   3. FP64 COM and bounding radius, leaves from their particles, internal
 //      nodes from their children, deepest level first -> k_leaf_com, k_internal_com;
 //   4. dual walk from (root, root): (A, A) opens into its children's three
 //      pairs; (A, B) is far when d^2 > 0 and (r_A + r_B)^2 <= theta^2 d^2,
 //      near when both are leaves, else the larger-radius internal node is
 //      split; far and near pairs are emitted in both directions
-//                                                -> breadth-first k_walk_*;
+//                                                -> breadth-first k_walk_step;
 //   5. target-major CSR with sources ascending   -> key radix sort + row counts.
 // The walk visits the same pairs as the host's depth-first recursion (every
 // decision depends on the pair alone); sorting the emitted pairs gives the
@@ -26,8 +26,9 @@
 // Work decomposition: thread per particle / range / node / pair; prefix sums
 // by a three-kernel tile scan; the sort is an LSD radix sort with 8-bit digits
 // whose scatter ranks keys by warp match masks in index order (stable).  The
-// only atomics are shared-memory digit counts, row counts and a max, all
-// order-independent, so every output is run-to-run identical.
+// atomics are shared-memory digit counts, row counts, a max and the walk's
+// append positions, whose order the sort of the (unique) keys removes, so
+// every output is run-to-run identical.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -155,26 +156,73 @@ __device__ __forceinline__ int split_point(const uint64_t* __restrict__ c, int s
   return lo;
 }
 
-__global__ void k_level_flags(const Pending* __restrict__ fr, int F, int leaf_size, int* __restrict__ flag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < F) flag[i] = (fr[i].e - fr[i].s + 1 > leaf_size) ? 1 : 0;
+// What level l of the split starts from: its frontier size and the internal
+// nodes and leaves above it.  Level l's kernels read slot l and fill slot
+// l + 1, so the host queues several levels before it looks at one.
+struct LevelState {
+  int F, int_base, leaf_base;
+};
+constexpr int kMaxSplitLevels = 128;  // 63 code bits, then halvings of equal codes: at most 63 + 31
+
+// rank[i] = the ranges before i in its tile of kScanTile that will be split.
+__global__ void __launch_bounds__(kScanThreads) k_level_rank(const Pending* __restrict__ fr,
+                                                             const LevelState* __restrict__ ls, int leaf_size,
+                                                             int* __restrict__ rank, int* __restrict__ tile_sums) {
+  __shared__ int warp_sums[32];
+  const int F = ls->F, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+  if (blockIdx.x * kScanTile >= F) return;
+  int v[kScanItems], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    v[k] = base + k < F && fr[base + k].e - fr[base + k].s + 1 > leaf_size;
+    sum += v[k];
+  }
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  int before = 0;
+  for (int k = 0; k < warp; ++k) before += warp_sums[k];
+  int run = before + incl - sum;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    if (base + k < F) rank[base + k] = run;
+    run += v[k];
+  }
+  if (threadIdx.x == kScanThreads - 1) tile_sums[blockIdx.x] = run;
 }
 
 struct LeafRec {
   int s, e, parent, side, level;
 };
 
-__global__ void k_level_emit(const Pending* __restrict__ fr, int F, const int* __restrict__ flag,
-                             const int* __restrict__ rank, int int_base, int leaf_base, int level,
-                             const uint64_t* __restrict__ codes, int* __restrict__ int_ranges, int* __restrict__ int_parent,
-                             int* __restrict__ int_level, int* __restrict__ left, int* __restrict__ right,
-                             Pending* __restrict__ next, LeafRec* __restrict__ leaves) {
+__global__ void __launch_bounds__(256) k_level_emit(const Pending* __restrict__ fr, LevelState* ls, int leaf_size,
+                                                    const int* __restrict__ rank, const int* __restrict__ tile_sums,
+                                                    int level, const uint64_t* __restrict__ codes,
+                                                    int* __restrict__ int_ranges, int* __restrict__ int_parent,
+                                                    int* __restrict__ int_level, int* __restrict__ left,
+                                                    int* __restrict__ right, Pending* __restrict__ next,
+                                                    LeafRec* __restrict__ leaves) {
+  const LevelState st = *ls;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= F) return;
+  static_assert(kScanTile % 256 == 0, "a block's ranges lie in one tile");
+  const int tile = (int)(blockIdx.x * blockDim.x) / kScanTile;
+  if (i == 0) {
+    int n_int = 0;
+    for (int t = 0; t * kScanTile < st.F; ++t) n_int += tile_sums[t];
+    ls[1] = LevelState{2 * n_int, st.int_base + n_int, st.leaf_base + st.F - n_int};
+  }
+  if (i >= st.F) return;
+  int r = rank[i];
+  for (int t = 0; t < tile; ++t) r += tile_sums[t];
   const Pending pd = fr[i];
-  const int r = rank[i];
-  if (flag[i]) {
-    const int id = int_base + r;
+  if (pd.e - pd.s + 1 > leaf_size) {
+    const int id = st.int_base + r;
     int_ranges[2 * id] = pd.s;
     int_ranges[2 * id + 1] = pd.e;
     int_parent[id] = pd.parent;
@@ -186,7 +234,7 @@ __global__ void k_level_emit(const Pending* __restrict__ fr, int F, const int* _
     next[2 * r] = Pending{pd.s, sp - 1, id, 0};
     next[2 * r + 1] = Pending{sp, pd.e, id, 1};
   } else {
-    leaves[leaf_base + (i - r)] = LeafRec{pd.s, pd.e, pd.parent, pd.side, level};
+    leaves[st.leaf_base + (i - r)] = LeafRec{pd.s, pd.e, pd.parent, pd.side, level};
   }
 }
 
@@ -214,9 +262,12 @@ __global__ void k_place_leaves(const LeafRec* __restrict__ lv, int L, const int*
   if (r.parent >= 0) (r.side == 0 ? left : right)[r.parent] = id;
 }
 
-__global__ void k_widen_perm(const int* __restrict__ v, int64_t n, int64_t* __restrict__ perm) {
+__global__ void k_widen_perm(const int* __restrict__ v, int64_t n, int64_t* __restrict__ perm,
+                             int64_t* __restrict__ inv) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) perm[i] = v[i];
+  if (i >= n) return;
+  perm[i] = v[i];
+  inv[v[i]] = i;
 }
 
 __global__ void k_max_occupancy(const int* __restrict__ ranges, int num_internal, int L, int* __restrict__ out) {
@@ -335,43 +386,6 @@ __device__ __forceinline__ int walk_decide(const WalkCtx& w, int a, int b) {
   return (!la && (lb || ra >= rb)) ? kSplitA : kSplitB;
 }
 
-__global__ void k_walk_count(const int2* __restrict__ fr, int F, WalkCtx w, I3* __restrict__ cnt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= F) return;
-  const int d = walk_decide(w, fr[i].x, fr[i].y);
-  cnt[i] = I3{d == kSelf ? 3 : (d >= kSplitA ? 2 : 0), d == kFar ? 2 : 0, d == kNear ? 2 : 0};
-}
-
-__global__ void k_walk_emit(const int2* __restrict__ fr, int F, WalkCtx w, const I3* __restrict__ off,
-                            int2* __restrict__ next, uint64_t* __restrict__ far_keys, int far_shift,
-                            uint64_t* __restrict__ near_keys, int near_shift) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= F) return;
-  const I3 o3 = off[i];
-  const int a = fr[i].x, b = fr[i].y;
-  const int d = walk_decide(w, a, b);
-  if (d == kSelf) {
-    const int l = w.left[a], r = w.right[a];
-    int2* o = next + o3.a;
-    o[0] = make_int2(l, l);
-    o[1] = make_int2(r, r);
-    o[2] = make_int2(l, r);
-  } else if (d == kSplitA) {
-    next[o3.a] = make_int2(w.left[a], b);
-    next[o3.a + 1] = make_int2(w.right[a], b);
-  } else if (d == kSplitB) {
-    next[o3.a] = make_int2(a, w.left[b]);
-    next[o3.a + 1] = make_int2(a, w.right[b]);
-  } else if (d == kFar) {
-    far_keys[o3.b] = ((uint64_t)a << far_shift) | (uint64_t)b;
-    far_keys[o3.b + 1] = ((uint64_t)b << far_shift) | (uint64_t)a;
-  } else if (d == kNear) {
-    const uint64_t la = (uint64_t)(a - w.num_internal), lb = (uint64_t)(b - w.num_internal);
-    near_keys[o3.c] = (la << near_shift) | lb;
-    near_keys[o3.c + 1] = (lb << near_shift) | la;
-  }
-}
-
 // Error-controlled acceptance of the far pair (target t <- source s), the
 // reference's Dehnen eq. (15)/(16a) policy (runtime/_adaptive_policy.py:
 // 267-376 dehnen_paper_pair_error_by_order, :2285-2338 the directional test):
@@ -433,40 +447,86 @@ __device__ __forceinline__ int adaptive_decide(const WalkCtx& w, int t, int s, i
   return (!lt && (ls || rt >= rs)) ? kSplitA : kSplitB;
 }
 
-__global__ void k_awalk_count(const int2* __restrict__ fr, int F, WalkCtx w, I3* __restrict__ cnt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= F) return;
-  int g = 0;
-  const int d = adaptive_decide(w, fr[i].x, fr[i].y, &g);
-  cnt[i] = I3{d == kSelf ? 4 : (d >= kSplitA ? 2 : 0), d == kFar ? 1 : 0, d == kNear ? 1 : 0};
-}
+// The walk's queue, in device memory: q[k] = node pairs of step k's frontier
+// (k <= kMaxWalkSteps), then the far and the near keys emitted so far.
+constexpr int kMaxWalkSteps = 510, kWalkFar = 511, kWalkNear = 512, kWalkWords = 513;
+constexpr int kWalkThreads = 256, kWalkBlocks = 148 * 8;
 
-__global__ void k_awalk_emit(const int2* __restrict__ fr, int F, WalkCtx w, const I3* __restrict__ off,
-                             int2* __restrict__ next, uint64_t* __restrict__ far_keys, int far_shift,
-                             uint64_t* __restrict__ near_keys, int near_shift) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= F) return;
-  const I3 o3 = off[i];
-  const int t = fr[i].x, s = fr[i].y;
-  int g = 0;
-  const int d = adaptive_decide(w, t, s, &g);
-  if (d == kSelf) {
-    const int l = w.left[t], r = w.right[t];
-    int2* o = next + o3.a;
-    o[0] = make_int2(l, l);
-    o[1] = make_int2(r, r);
-    o[2] = make_int2(l, r);
-    o[3] = make_int2(r, l);
-  } else if (d == kSplitA) {
-    next[o3.a] = make_int2(w.left[t], s);
-    next[o3.a + 1] = make_int2(w.right[t], s);
-  } else if (d == kSplitB) {
-    next[o3.a] = make_int2(t, w.left[s]);
-    next[o3.a + 1] = make_int2(t, w.right[s]);
-  } else if (d == kFar) {
-    far_keys[o3.b] = ((uint64_t)g << kGearShift) | ((uint64_t)t << far_shift) | (uint64_t)s;
-  } else if (d == kNear) {
-    near_keys[o3.c] = ((uint64_t)(t - w.num_internal) << near_shift) | (uint64_t)(s - w.num_internal);
+// One step of the walk: decides every pair of the frontier once and appends
+// its children, far and near keys behind what other blocks append (a block
+// takes its room with one atomic per list).  The order of a frontier or of
+// the keys does not matter: the keys are sorted afterwards, and each is
+// unique.  The frontier's size is read from the queue, so the host queues many
+// steps without looking; with a count, a scan and an emit per step, each
+// behind a read-back, the steps of a clustered walk took 25-30 us each.
+// Nothing is written past a buffer's end, but the counts go on, so that the
+// host sees what the lists need.
+template <bool ADAPTIVE>
+__global__ void __launch_bounds__(kWalkThreads) k_walk_step(const int2* __restrict__ fr, int2* __restrict__ next,
+                                                            int64_t cap_front, WalkCtx w,
+                                                            uint64_t* __restrict__ far_keys, int64_t cap_far,
+                                                            int far_shift, uint64_t* __restrict__ near_keys,
+                                                            int64_t cap_near, int near_shift, unsigned long long* q,
+                                                            int step) {
+  __shared__ unsigned warp_sum[kWalkThreads / 32];
+  __shared__ unsigned long long room[3];
+  const int64_t F = min((int64_t)q[step], cap_front);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t b0 = (int64_t)blockIdx.x * kWalkThreads; b0 < F; b0 += (int64_t)gridDim.x * kWalkThreads) {
+    const int64_t i = b0 + threadIdx.x;
+    int a = 0, b = 0, d = kNone, g = 0;
+    if (i < F) {
+      a = fr[i].x, b = fr[i].y;
+      d = ADAPTIVE ? adaptive_decide(w, a, b, &g) : walk_decide(w, a, b);
+    }
+    // children (at most 4 a thread), far and near keys (at most 2) as the
+    // three fields of one word: 11, 10 and 10 bits hold a block's sums
+    const unsigned ca = d == kSelf ? (ADAPTIVE ? 4 : 3) : (d >= kSplitA ? 2 : 0);
+    const unsigned cf = d == kFar ? (ADAPTIVE ? 1 : 2) : 0, cn = d == kNear ? (ADAPTIVE ? 1 : 2) : 0;
+    const unsigned mine = ca | cf << 11 | cn << 21;
+    unsigned incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    unsigned before = incl - mine, total = 0;
+#pragma unroll
+    for (int k = 0; k < kWalkThreads / 32; ++k) {
+      if (k < warp) before += warp_sum[k];
+      total += warp_sum[k];
+    }
+    if (threadIdx.x < 3) {
+      const unsigned c = threadIdx.x == 0 ? total & 2047u : threadIdx.x == 1 ? total >> 11 & 1023u : total >> 21;
+      unsigned long long* at = q + (threadIdx.x == 0 ? step + 1 : threadIdx.x == 1 ? kWalkFar : kWalkNear);
+      room[threadIdx.x] = c ? atomicAdd(at, (unsigned long long)c) : 0ull;
+    }
+    __syncthreads();
+    const int64_t oa = (int64_t)room[0] + (before & 2047u), of = (int64_t)room[1] + (before >> 11 & 1023u);
+    const int64_t on = (int64_t)room[2] + (before >> 21);
+    if (d == kSelf && oa + ca <= cap_front) {
+      const int l = w.left[a], r = w.right[a];
+      next[oa] = make_int2(l, l);
+      next[oa + 1] = make_int2(r, r);
+      next[oa + 2] = make_int2(l, r);
+      if (ADAPTIVE) next[oa + 3] = make_int2(r, l);
+    } else if (d == kSplitA && oa + 2 <= cap_front) {
+      next[oa] = make_int2(w.left[a], b);
+      next[oa + 1] = make_int2(w.right[a], b);
+    } else if (d == kSplitB && oa + 2 <= cap_front) {
+      next[oa] = make_int2(a, w.left[b]);
+      next[oa + 1] = make_int2(a, w.right[b]);
+    } else if (d == kFar && of + cf <= cap_far) {
+      far_keys[of] = ((uint64_t)g << kGearShift) | ((uint64_t)a << far_shift) | (uint64_t)b;
+      if (!ADAPTIVE) far_keys[of + 1] = ((uint64_t)b << far_shift) | (uint64_t)a;
+    } else if (d == kNear && on + cn <= cap_near) {
+      const uint64_t la = (uint64_t)(a - w.num_internal), lb = (uint64_t)(b - w.num_internal);
+      near_keys[on] = (la << near_shift) | lb;
+      if (!ADAPTIVE) near_keys[on + 1] = (lb << near_shift) | la;
+    }
+    __syncthreads();  // warp_sum and room are read
   }
 }
 
@@ -533,7 +593,7 @@ inline int bits_for(int64_t v) {  // bits to hold values in [0, v)
 // ---------------------------------------------------------------------------
 struct jb_dtree {
   jb_tree_info_t info{};
-  DBuf perm, ranges, left, right, parent, level, level_off, leaf_of, far_off, far_src, near_off, near_src, com, radius;
+  DBuf perm, inv, ranges, left, right, parent, level, level_off, leaf_of, far_off, far_src, near_off, near_src, com, radius;
   DBuf far_gear;  // gear index per far pair (CSR order) after jb_dtree_adaptive_walk
   int walk_kind = 0;  // 0: symmetric theta walk, 1: error-controlled target-centric walk
 };
@@ -546,59 +606,60 @@ namespace {
 int64_t walk_lists(jb_dtree& t, const WalkCtx& w, bool adaptive, int NN, int L, Scratch& s, int* d_total32,
                    cudaStream_t st) {
   const int far_shift = bits_for(NN), near_shift = bits_for(std::max(L, 1));
-  DBuf w0, w1, cnt3, off3, far_keys, near_keys;
+  DBuf w0, w1, queue, far_keys, near_keys;
   int64_t n_far = 0, n_near = 0;
   if (NN > 1) {
-    const int64_t cap = std::max<int64_t>(1 << 16, 4 * (int64_t)NN);
-    ck(w0.alloc(cap * sizeof(int2)));
-    ck(w1.alloc(cap * sizeof(int2)));
-    ck(cnt3.alloc(cap * sizeof(I3)));
-    ck(off3.alloc(cap * sizeof(I3)));
-    ck(far_keys.alloc((size_t)std::max<int64_t>(1 << 16, 256 * (int64_t)NN) * 8));
-    ck(near_keys.alloc((size_t)std::max<int64_t>(1 << 16, 256 * (int64_t)L) * 8));
-    I3* d_tot3 = reinterpret_cast<I3*>(d_total32);
+    // room for the widest frontier and the lists seen over the configurations
+    // (frontier below 40 pairs a node, far list below 256 a node); a walk that
+    // needs more is counted to its end, then run again with twice the room
+    int64_t cap_front = std::max<int64_t>(1 << 16, 64 * (int64_t)NN);
+    int64_t cap_far = std::max<int64_t>(1 << 16, 256 * (int64_t)NN), cap_near = std::max<int64_t>(1 << 16, 256 * (int64_t)L);
+    ck(queue.alloc(kWalkWords * 8));
     const int2 root = make_int2(0, 0);
-    ck(cudaMemcpyAsync(w0.p, &root, sizeof(root), cudaMemcpyHostToDevice, st));
-    DBuf* wc = &w0;
-    DBuf* wn = &w1;
-    int64_t Fw = 1;
-    while (Fw > 0) {
-      if ((size_t)Fw * sizeof(I3) > cnt3.bytes) {
-        ck(cnt3.alloc((size_t)Fw * 2 * sizeof(I3)));
-        ck(off3.alloc((size_t)Fw * 2 * sizeof(I3)));
+    std::vector<unsigned long long> q(kWalkWords);
+    for (bool again = true; again;) {
+      again = false;
+      if ((size_t)cap_front * sizeof(int2) > w0.bytes) {
+        ck(w0.alloc((size_t)cap_front * sizeof(int2)));
+        ck(w1.alloc((size_t)cap_front * sizeof(int2)));
       }
-      if (adaptive)
-        k_awalk_count<<<nblocks(Fw, 256), 256, 0, st>>>(wc->as<int2>(), (int)Fw, w, cnt3.as<I3>());
-      else
-        k_walk_count<<<nblocks(Fw, 256), 256, 0, st>>>(wc->as<int2>(), (int)Fw, w, cnt3.as<I3>());
-      ck_launch();
-      exclusive_scan<I3>(cnt3.as<I3>(), off3.as<I3>(), Fw, d_tot3, s, st);
-      const I3 tot = read_word(d_tot3, st);
-      // grow the next frontier and the key buffers as needed (stream-ordered)
-      ck(wn->grow((size_t)tot.a * 2 * sizeof(int2), 0, st));
-      const size_t need_far = (size_t)(n_far + tot.b) * 8, need_near = (size_t)(n_near + tot.c) * 8;
-      if (need_far > far_keys.bytes) ck(far_keys.grow(std::max(need_far, 2 * far_keys.bytes), (size_t)n_far * 8, st));
-      if (need_near > near_keys.bytes)
-        ck(near_keys.grow(std::max(need_near, 2 * near_keys.bytes), (size_t)n_near * 8, st));
-      if (adaptive)
-        k_awalk_emit<<<nblocks(Fw, 256), 256, 0, st>>>(wc->as<int2>(), (int)Fw, w, off3.as<I3>(), wn->as<int2>(),
-                                                       far_keys.as<uint64_t>() + n_far, far_shift,
-                                                       near_keys.as<uint64_t>() + n_near, near_shift);
-      else
-        k_walk_emit<<<nblocks(Fw, 256), 256, 0, st>>>(wc->as<int2>(), (int)Fw, w, off3.as<I3>(), wn->as<int2>(),
-                                                      far_keys.as<uint64_t>() + n_far, far_shift,
-                                                      near_keys.as<uint64_t>() + n_near, near_shift);
-      ck_launch();
-      n_far += tot.b;
-      n_near += tot.c;
-      Fw = tot.a;
-      std::swap(wc, wn);
+      if ((size_t)cap_far * 8 > far_keys.bytes) ck(far_keys.alloc((size_t)cap_far * 8));
+      if ((size_t)cap_near * 8 > near_keys.bytes) ck(near_keys.alloc((size_t)cap_near * 8));
+      std::fill(q.begin(), q.end(), 0ull);
+      q[0] = 1;
+      ck(cudaMemcpyAsync(queue.p, q.data(), kWalkWords * 8, cudaMemcpyHostToDevice, st));
+      ck(cudaMemcpyAsync(w0.p, &root, sizeof(root), cudaMemcpyHostToDevice, st));
+      int step = 0;
+      do {
+        if (step >= kMaxWalkSteps) throw Fail{JB_ERR_INDEX};  // no tree is that deep
+        const int stop = std::min(step + 12, (int)kMaxWalkSteps);
+        for (; step < stop; ++step) {
+          const int64_t most = step < 12 ? std::min<int64_t>(cap_front, (int64_t)1 << (2 * step)) : cap_front;
+          const unsigned nb = (unsigned)std::min<int64_t>(kWalkBlocks, nblocks(most, kWalkThreads));
+          const int2* cur = (step & 1) ? w1.as<int2>() : w0.as<int2>();
+          int2* nxt = (step & 1) ? w0.as<int2>() : w1.as<int2>();
+          auto kern = adaptive ? k_walk_step<true> : k_walk_step<false>;
+          kern<<<nb, kWalkThreads, 0, st>>>(cur, nxt, cap_front, w, far_keys.as<uint64_t>(), cap_far, far_shift,
+                                            near_keys.as<uint64_t>(), cap_near, near_shift,
+                                            queue.as<unsigned long long>(), step);
+          ck_launch();
+        }
+        ck(cudaMemcpyAsync(q.data(), queue.p, kWalkWords * 8, cudaMemcpyDeviceToHost, st));
+        ck(cudaStreamSynchronize(st));
+      } while (q[step] > 0);
+      n_far = (int64_t)q[kWalkFar];
+      n_near = (int64_t)q[kWalkNear];
+      const int64_t widest = (int64_t)*std::max_element(q.begin(), q.begin() + step + 1);
+      if (widest > cap_front || n_far > cap_far || n_near > cap_near) {
+        again = true;
+        if (widest > cap_front) cap_front = 2 * widest;
+        if (n_far > cap_far) cap_far = 2 * n_far;
+        if (n_near > cap_near) cap_near = 2 * n_near;
+      }
     }
   }
   w0.release();
   w1.release();
-  cnt3.release();
-  off3.release();
 
   auto to_csr = [&](DBuf& keys, int64_t m, int shift, int rows, DBuf& off, DBuf& col, DBuf* gears) {
     ck(off.alloc((size_t)(rows + 1) * 8));
@@ -682,24 +743,39 @@ void build(jb_dtree& t, int64_t n, const double* pos, const double* mass, int le
   }
   Pending* cur = fr0.as<Pending>();
   Pending* nxt = fr1.as<Pending>();
-  int F = 1, int_base = 0, leaf_base = 0, level = 0;
+  // Level l's frontier holds at most 2^l ranges and two per range of more than
+  // leaf_size particles; eight levels are queued, then one read-back.
+  const int64_t widest = std::max<int64_t>(2, 2 * (n / ((int64_t)leaf_size + 1)));
+  DBuf lstate, tile_sums;
+  ck(lstate.alloc((kMaxSplitLevels + 1) * sizeof(LevelState)));
+  ck(tile_sums.alloc((size_t)nblocks(widest, kScanTile) * 4));
+  std::vector<LevelState> ls(kMaxSplitLevels + 1);
+  ls[0] = LevelState{1, 0, 0};
+  ck(cudaMemcpyAsync(lstate.p, &ls[0], sizeof(LevelState), cudaMemcpyHostToDevice, st));
+  int level = 0;
+  do {
+    if (level >= kMaxSplitLevels) throw Fail{JB_ERR_INDEX};
+    const int first = level, stop = std::min(level + 8, (int)kMaxSplitLevels);
+    for (; level < stop; ++level) {
+      const int64_t most = level < 31 ? std::min<int64_t>(widest, (int64_t)1 << level) : widest;
+      LevelState* at = lstate.as<LevelState>() + level;
+      k_level_rank<<<nblocks(most, kScanTile), kScanThreads, 0, st>>>(cur, at, leaf_size, rank.as<int>(),
+                                                                      tile_sums.as<int>());
+      ck_launch();
+      k_level_emit<<<nblocks(most, 256), 256, 0, st>>>(cur, at, leaf_size, rank.as<int>(), tile_sums.as<int>(), level,
+                                                       codes, int_ranges.as<int>(), int_parent.as<int>(),
+                                                       int_level.as<int>(), left.as<int>(), right.as<int>(), nxt,
+                                                       leaves.as<LeafRec>());
+      ck_launch();
+      std::swap(cur, nxt);
+    }
+    ck(cudaMemcpyAsync(&ls[first + 1], lstate.as<LevelState>() + first + 1, (size_t)(level - first) * sizeof(LevelState),
+                       cudaMemcpyDeviceToHost, st));
+    ck(cudaStreamSynchronize(st));
+  } while (ls[level].F > 0);
   std::vector<int> level_off;
-  while (F > 0) {
-    level_off.push_back(int_base);
-    k_level_flags<<<nblocks(F, 256), 256, 0, st>>>(cur, F, leaf_size, flag.as<int>());
-    ck_launch();
-    exclusive_scan<int>(flag.as<int>(), rank.as<int>(), F, d_total32, s, st);
-    const int n_int = read_word(d_total32, st);
-    k_level_emit<<<nblocks(F, 256), 256, 0, st>>>(cur, F, flag.as<int>(), rank.as<int>(), int_base, leaf_base, level,
-                                                  codes, int_ranges.as<int>(), int_parent.as<int>(), int_level.as<int>(),
-                                                  left.as<int>(), right.as<int>(), nxt, leaves.as<LeafRec>());
-    ck_launch();
-    int_base += n_int;
-    leaf_base += F - n_int;
-    F = 2 * n_int;
-    std::swap(cur, nxt);
-    ++level;
-  }
+  for (int l = 0; l < level && ls[l].F > 0; ++l) level_off.push_back(ls[l].int_base);
+  const int int_base = ls[level].int_base, leaf_base = ls[level].leaf_base;
   const int NI = int_base, L = leaf_base, NN = NI + L;
   while (level_off.size() > 1 && level_off.back() == NI) level_off.pop_back();
   level_off.push_back(NI);
@@ -733,7 +809,8 @@ void build(jb_dtree& t, int64_t n, const double* pos, const double* mass, int le
   ck(t.level_off.alloc(level_off.size() * 4));
   ck(cudaMemcpyAsync(t.level_off.p, level_off.data(), level_off.size() * 4, cudaMemcpyHostToDevice, st));
   ck(t.perm.alloc((size_t)n * 8));
-  k_widen_perm<<<nblocks(n, 256), 256, 0, st>>>(sperm, n, t.perm.as<int64_t>());
+  ck(t.inv.alloc((size_t)n * 8));
+  k_widen_perm<<<nblocks(n, 256), 256, 0, st>>>(sperm, n, t.perm.as<int64_t>(), t.inv.as<int64_t>());
   ck_launch();
   ck(cudaMemsetAsync(d_total32, 0, 4, st));
   k_max_occupancy<<<nblocks(L, 256), 256, 0, st>>>(t.ranges.as<int>(), NI, L, d_total32);
@@ -791,6 +868,7 @@ void build(jb_dtree& t, int64_t n, const double* pos, const double* mass, int le
 const DBuf* field_buf(const jb_dtree* t, int field) {
   switch (field) {
     case JB_TREE_PERMUTATION: return &t->perm;
+    case JB_TREE_INVERSE_PERMUTATION: return &t->inv;
     case JB_TREE_NODE_RANGES: return &t->ranges;
     case JB_TREE_LEFT_CHILD: return &t->left;
     case JB_TREE_RIGHT_CHILD: return &t->right;
@@ -812,7 +890,8 @@ const DBuf* field_buf(const jb_dtree* t, int field) {
 size_t field_bytes(const jb_dtree* t, int field) {
   const jb_tree_info_t& i = t->info;
   switch (field) {
-    case JB_TREE_PERMUTATION: return (size_t)i.num_particles * 8;
+    case JB_TREE_PERMUTATION:
+    case JB_TREE_INVERSE_PERMUTATION: return (size_t)i.num_particles * 8;
     case JB_TREE_NODE_RANGES: return (size_t)i.num_nodes * 8;
     case JB_TREE_LEFT_CHILD:
     case JB_TREE_RIGHT_CHILD: return (size_t)i.num_internal * 4;
@@ -949,6 +1028,20 @@ JB_API int jb_dtree_copy(const jb_dtree* t, int field, void* dst) {
   const size_t bytes = field_bytes(t, field);
   if (bytes == 0) return JB_OK;
   return jb::cuda_status(cudaMemcpy(dst, b->p, bytes, cudaMemcpyDeviceToHost));
+}
+
+JB_API int jb_dtree_export(const jb_dtree* t, int count, const int* fields, void* const* dst, void* stream) {
+  if (!t || count < 0 || (count > 0 && (!fields || !dst))) return JB_ERR_ARG;
+  for (int k = 0; k < count; ++k) {
+    const DBuf* b = field_buf(t, fields[k]);
+    if (!b || !dst[k]) return JB_ERR_ARG;
+    const size_t bytes = field_bytes(t, fields[k]);
+    if (bytes == 0) continue;
+    const cudaError_t e =
+        cudaMemcpyAsync(dst[k], b->p, bytes, cudaMemcpyDeviceToDevice, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return jb::cuda_status(e);
+  }
+  return JB_OK;
 }
 
 JB_API void jb_dtree_free(jb_dtree* t) { delete t; }
