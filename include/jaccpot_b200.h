@@ -234,6 +234,12 @@ JB_API int jb_gear_mixed_schedule_device(int num_nodes, const int64_t* far_off, 
  * emits them); JB_ERR_INDEX when some pair has no reverse.  The host twin is
  * Topology.far_reverse_index in tree.py.  Synchronises the stream.           */
 JB_API int jb_far_reverse_index(int num_nodes, const int64_t* far_off, const int* far_src, int* rev, void* stream);
+/* Units of jb_l2l_leaves for the leaves [leaf_lo, leaf_hi): JB_SCHED_UNITS are
+ * (leaf node, first, end, -1) over JB_SCHED_RUNS, int32[num_runs], which holds
+ * each leaf's ancestors with far pairs, nearest first, leaf after leaf; units
+ * longest first (stable), leaves without such ancestors left out.           */
+JB_API int jb_l2l_schedule_device(int num_internal, int leaf_lo, int leaf_hi, const int* parent, const int64_t* far_off,
+                                  void* stream, jb_dsched** out);
 JB_API int jb_dsched_info(const jb_dsched* d, jb_sched_info_t* info);
 JB_API const void* jb_dsched_field(const jb_dsched* d, int field);
 JB_API void jb_dsched_free(jb_dsched* d);

@@ -93,6 +93,7 @@ _SIGNATURES = {
     "jb_dtree_copy": [_P, _I, _P],
     "jb_dtree_free": [_P],
     "jb_dtree_export": [_P, _I, _P, _P, _P],
+    "jb_l2l_schedule_device": [_I, _I, _I, _P, _P, _P, ctypes.POINTER(_P)],
     "jb_dtree_adaptive_walk": [_P, _I, _P, _P, _D, _D, _D, _I, _P, _P],
     "jb_node_dehnen_power": [_I, _I, _P, _I, _P, _P],
     "jb_far_dehnen_gears": [_I64, _P, _P, _P, _P, _I, _P, _P, _D, _D, _I, _P, _P, _P],

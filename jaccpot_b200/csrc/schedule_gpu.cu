@@ -906,6 +906,78 @@ const DBuf* sched_field(const jb_dsched* d, int field) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// Leaf-ancestor schedule (l2l_leaf_schedule).  Thread per leaf climbing to the
+// root, once to count its ancestors with far pairs and once to write them
+// behind a prefix sum: a chain of 20 to 45 dependent reads that stay in L2.
+// As tensor operations, one masked gather per tree level with its sizes read
+// back, the same took 1.4 of the 6.9 ms of a call on 16k new particles.
+// ---------------------------------------------------------------------------
+__global__ void k_anc_count(int num_internal, int lo, int hi, const int* __restrict__ parent,
+                            const int64_t* __restrict__ far_off, int* __restrict__ cnt, uint64_t* __restrict__ key,
+                            int* __restrict__ num_units) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool ok = lo + j < hi;
+  int c = 0;
+  if (ok) {
+    for (int a = parent[num_internal + lo + j]; a >= 0; a = parent[a]) c += far_off[a + 1] > far_off[a];
+    cnt[j] = c;
+    key[j] = (uint64_t)(255 - c);  // a tree has fewer than 128 levels
+  }
+  const unsigned have = __ballot_sync(kFull, ok && c > 0);
+  if ((threadIdx.x & 31) == 0 && have) atomicAdd(num_units, __popc(have));
+}
+
+__global__ void k_anc_fill(int num_internal, int lo, int hi, const int* __restrict__ parent,
+                           const int64_t* __restrict__ far_off, const int* __restrict__ off, int* __restrict__ anc) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (lo + j >= hi) return;
+  int at = off[j];
+  for (int a = parent[num_internal + lo + j]; a >= 0; a = parent[a])
+    if (far_off[a + 1] > far_off[a]) anc[at++] = a;
+}
+
+__global__ void k_anc_units(int num_internal, int lo, const int* __restrict__ order, int U, const int* __restrict__ off,
+                            const int* __restrict__ cnt, int4* __restrict__ units) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= U) return;
+  const int j = order[u];
+  units[u] = make_int4(num_internal + lo + j, off[j], off[j] + cnt[j], -1);
+}
+
+void build_l2l(jb_dsched& d, int num_internal, int lo, int hi, const int* parent, const int64_t* far_off,
+               cudaStream_t st) {
+  const int NL = hi - lo;
+  if (NL <= 0) return;
+  Scratch s;
+  ck(s.total.alloc(64));
+  int* d_tot = tot32(s);  // ancestors in all, units
+  DBuf cnt, off, k0, k1, v0, v1;
+  for (DBuf* b : {&cnt, &off, &v0, &v1}) ck(b->alloc((size_t)NL * 4));
+  for (DBuf* b : {&k0, &k1}) ck(b->alloc((size_t)NL * 8));
+  ck(cudaMemsetAsync(d_tot, 0, 8, st));
+  k_anc_count<<<nblocks(NL, 128), 128, 0, st>>>(num_internal, lo, hi, parent, far_off, cnt.as<int>(),
+                                                k0.as<uint64_t>(), d_tot + 1);
+  ck_launch();
+  exclusive_scan<int>(cnt.as<int>(), off.as<int>(), NL, d_tot, s, st);
+  int tot[2];
+  ck(cudaMemcpyAsync(tot, d_tot, sizeof(tot), cudaMemcpyDeviceToHost, st));
+  k_iota<<<nblocks(NL, 256), 256, 0, st>>>(v0.as<int>(), NL);
+  ck_launch();
+  radix_sort(k0.as<uint64_t>(), v0.as<int>(), k1.as<uint64_t>(), v1.as<int>(), NL, 8, s, st);
+  ck(cudaStreamSynchronize(st));
+  d.info.num_runs = tot[0];
+  d.info.num_units = tot[1];
+  if (tot[1] == 0) return;
+  ck(d.runs.alloc((size_t)tot[0] * 4));
+  k_anc_fill<<<nblocks(NL, 128), 128, 0, st>>>(num_internal, lo, hi, parent, far_off, off.as<int>(), d.runs.as<int>());
+  ck_launch();
+  ck(d.units.alloc((size_t)tot[1] * 16));
+  k_anc_units<<<nblocks(tot[1], 256), 256, 0, st>>>(num_internal, lo, v0.as<int>(), tot[1], off.as<int>(), cnt.as<int>(),
+                                                    d.units.as<int4>());
+  ck_launch();
+}
+
 template <typename F>
 int run_builder(jb_dsched** out, cudaStream_t st, F&& fn) {
   if (!out) return JB_ERR_ARG;
@@ -949,6 +1021,14 @@ JB_API int jb_leaf_schedule_device(int num_internal, int num_leaves, const int* 
   return run_builder(out, st, [&](jb_dsched& d) {
     build_leaf(d, num_internal, node_ranges, near_off, near_src, leaf_lo, leaf_hi, max_sources, st);
   });
+}
+
+JB_API int jb_l2l_schedule_device(int num_internal, int leaf_lo, int leaf_hi, const int* parent, const int64_t* far_off,
+                                  void* stream, jb_dsched** out) {
+  if (num_internal < 0 || leaf_lo < 0 || leaf_hi < leaf_lo || !parent || !far_off) return JB_ERR_ARG;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  return run_builder(out, st,
+                     [&](jb_dsched& d) { build_l2l(d, num_internal, leaf_lo, leaf_hi, parent, far_off, st); });
 }
 
 JB_API int jb_gear_schedule_device(int num_nodes, const int64_t* far_off, const int* far_src, const int* gears,

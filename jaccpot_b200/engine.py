@@ -21,7 +21,7 @@ import torch
 
 from . import _lib
 from .schedule import (MixedGearM2LSchedule, gear_m2l_mixed_schedule, gear_m2l_mixed_schedule_device,
-                       gear_m2l_schedule, gear_m2l_schedule_device, leaf_schedule, leaf_schedule_device,
+                       _run_device, gear_m2l_schedule, gear_m2l_schedule_device, leaf_schedule, leaf_schedule_device,
                        m2l_schedule, m2l_schedule_device, m2l_unit_limit, mixed_ladder, tc_m2l_schedule)
 from .tree import Topology
 
@@ -58,6 +58,7 @@ class DeviceTopology:
         self.node_ranges = up(topo.node_ranges.reshape(-1), torch.int32)
         self.left = up(topo.left_child if topo.num_internal else np.zeros(1, np.int32), torch.int32)
         self.right = up(topo.right_child if topo.num_internal else np.zeros(1, np.int32), torch.int32)
+        self.parent = up(topo.parent, torch.int32)
         self.far_off = up(topo.far_offsets, torch.int64)
         self.far_src = up(topo.far_sources if topo.num_far_pairs else np.zeros(1, np.int32), torch.int32)
         # per-far-pair gear tags of an error-controlled walk (None: one order)
@@ -184,36 +185,17 @@ def l2l_leaf_schedule(topo: Topology, leaf_range: tuple[int, int]):
 
 
 def l2l_leaf_schedule_device(dt: "DeviceTopology", leaf_range: tuple[int, int]):
-    """l2l_leaf_schedule on the device (torch operations over the resident
-    far offsets and the uploaded parents): the same arrays, as device
-    tensors."""
-    t, dev = dt.topo, dt.device
-    ni = t.num_internal
+    """l2l_leaf_schedule on the device (jb_l2l_schedule_device): the same
+    arrays, as device tensors."""
     lo, hi = leaf_range
-    parent = torch.from_numpy(np.asarray(t.parent).astype(np.int64)).to(dev)
-    has_far = (dt.far_off[1:] - dt.far_off[:-1]) > 0
-    leaves = torch.arange(ni + lo, ni + hi, device=dev, dtype=torch.int64)
-    idx = torch.arange(leaves.numel(), device=dev, dtype=torch.int64)
-    cur = parent[leaves]
-    rows, cols = [], []
-    while cur.numel():
-        ok = cur >= 0
-        idx, cur = idx[ok], cur[ok]
-        m = has_far[cur]
-        rows.append(idx[m])
-        cols.append(cur[m])
-        cur = parent[cur]
-    z = torch.zeros(0, dtype=torch.int64, device=dev)
-    rows = torch.cat(rows) if rows else z
-    cols = torch.cat(cols) if cols else z
-    order = torch.sort(rows, stable=True).indices  # nearest ancestor first within a leaf
-    rows, cols = rows[order], cols[order]
-    cnt = torch.bincount(rows, minlength=leaves.numel())
-    off = torch.cat([torch.zeros(1, dtype=torch.int64, device=dev), torch.cumsum(cnt, 0)])
-    have = torch.nonzero(cnt).flatten()
-    have = have[torch.sort(-cnt[have], stable=True).indices]
-    units = torch.stack([leaves[have], off[have], off[have + 1], torch.full_like(have, -1)], dim=1)
-    return units.to(torch.int32).contiguous(), cols.to(torch.int32).contiguous()
+    info, field, free = _run_device("jb_l2l_schedule_device", [dt.topo.num_internal, int(lo), int(hi), _ptr(dt.parent),
+                                                               _ptr(dt.far_off)], dt.device)
+    try:
+        units = field(_lib.JB_SCHED_UNITS, (info.num_units, 4), np.int32)
+        anc = field(_lib.JB_SCHED_RUNS, (info.num_runs,), np.int32)
+    finally:
+        free()
+    return units, anc
 
 
 def _restrict_gears(gs, targets, num_nodes: int, dev):
