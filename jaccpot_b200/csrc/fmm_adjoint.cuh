@@ -311,51 +311,72 @@ template <int P>
 struct RunAdj {
   static int leaf_far(const float* pos4, const float* w4, int num_nodes, int num_internal, const int* ranges,
                       const float* centers, const float* locals, float G, float* xm4, float* lbar, float* cbar4,
-                      cudaStream_t st) {
-    const int L = num_nodes - num_internal;
-    if (L <= 0) return JB_OK;
-    const size_t sm = sizeof(float) * kWarpsPerBlock * (32 * (csize(P) + 1) + cstride(P));
-    cudaFuncSetAttribute(k_adj_leaf_far<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_adj_leaf_far<P><<<blocks_for(L, kWarpsPerBlock), 32 * kWarpsPerBlock, sm, st>>>(
-        reinterpret_cast<const float4*>(pos4), reinterpret_cast<const float4*>(w4), num_nodes, num_internal,
-        reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(centers), locals, G,
-        reinterpret_cast<float4*>(xm4), lbar, reinterpret_cast<float4*>(cbar4));
-    return launch_status();
-  }
+                      cudaStream_t st);
   static int l2l_level(int first, int last, const int* left, const int* right, const float* centers,
-                       const float* locals, float* lbar, float* cbar4, cudaStream_t st) {
-    if (last <= first) return JB_OK;
-    k_adj_l2l_level<P><<<blocks_for(last - first, 128), 128, 0, st>>>(
-        first, last, left, right, reinterpret_cast<const float4*>(centers), locals, lbar,
-        reinterpret_cast<float4*>(cbar4));
-    return launch_status();
-  }
+                       const float* locals, float* lbar, float* cbar4, cudaStream_t st);
   static int m2l_pairs(int64_t num_pairs, const int* pair_tgt, const int* far_src, const float* mult,
-                       const float* lbar, const float* centers, float* g4, cudaStream_t st) {
-    if (num_pairs <= 0) return JB_OK;
-    k_adj_m2l_pairs<P><<<blocks_for(num_pairs, 128), 128, 0, st>>>(
-        num_pairs, pair_tgt, far_src, mult, lbar, reinterpret_cast<const float4*>(centers),
-        reinterpret_cast<float4*>(g4));
-    return launch_status();
-  }
+                       const float* lbar, const float* centers, float* g4, cudaStream_t st);
   static int m2m_level(int first, int last, const int* left, const int* right, const float* centers,
-                       const float* mult, float* mbar, float* cbar4, cudaStream_t st) {
-    if (last <= first) return JB_OK;
-    k_adj_m2m_level<P><<<blocks_for(last - first, 128), 128, 0, st>>>(
-        first, last, left, right, reinterpret_cast<const float4*>(centers), mult, mbar,
-        reinterpret_cast<float4*>(cbar4));
-    return launch_status();
-  }
+                       const float* mult, float* mbar, float* cbar4, cudaStream_t st);
   static int p2m(const float* pos4, int num_nodes, int num_internal, const int* ranges, const float* centers,
-                 const float* mbar, const float* cbar4, float* xm4, cudaStream_t st) {
-    const int L = num_nodes - num_internal;
-    if (L <= 0) return JB_OK;
-    k_adj_p2m<P><<<blocks_for(L, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, st>>>(
-        reinterpret_cast<const float4*>(pos4), num_nodes, num_internal, reinterpret_cast<const int2*>(ranges),
-        reinterpret_cast<const float4*>(centers), mbar, reinterpret_cast<const float4*>(cbar4),
-        reinterpret_cast<float4*>(xm4));
-    return launch_status();
-  }
+                 const float* mbar, const float* cbar4, float* xm4, cudaStream_t st);
 };
+
+template <int P>
+int RunAdj<P>::leaf_far(const float* pos4, const float* w4, int num_nodes, int num_internal, const int* ranges,
+                      const float* centers, const float* locals, float G, float* xm4, float* lbar, float* cbar4,
+                      cudaStream_t st) {
+  const int L = num_nodes - num_internal;
+  if (L <= 0) return JB_OK;
+  const size_t sm = sizeof(float) * kWarpsPerBlock * (32 * (csize(P) + 1) + cstride(P));
+  cudaFuncSetAttribute(k_adj_leaf_far<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_adj_leaf_far<P><<<blocks_for(L, kWarpsPerBlock), 32 * kWarpsPerBlock, sm, st>>>(
+      reinterpret_cast<const float4*>(pos4), reinterpret_cast<const float4*>(w4), num_nodes, num_internal,
+      reinterpret_cast<const int2*>(ranges), reinterpret_cast<const float4*>(centers), locals, G,
+      reinterpret_cast<float4*>(xm4), lbar, reinterpret_cast<float4*>(cbar4));
+  return launch_status();
+}
+
+template <int P>
+int RunAdj<P>::l2l_level(int first, int last, const int* left, const int* right, const float* centers,
+                       const float* locals, float* lbar, float* cbar4, cudaStream_t st) {
+  if (last <= first) return JB_OK;
+  k_adj_l2l_level<P><<<blocks_for(last - first, 128), 128, 0, st>>>(
+      first, last, left, right, reinterpret_cast<const float4*>(centers), locals, lbar,
+      reinterpret_cast<float4*>(cbar4));
+  return launch_status();
+}
+
+template <int P>
+int RunAdj<P>::m2l_pairs(int64_t num_pairs, const int* pair_tgt, const int* far_src, const float* mult,
+                       const float* lbar, const float* centers, float* g4, cudaStream_t st) {
+  if (num_pairs <= 0) return JB_OK;
+  k_adj_m2l_pairs<P><<<blocks_for(num_pairs, 128), 128, 0, st>>>(
+      num_pairs, pair_tgt, far_src, mult, lbar, reinterpret_cast<const float4*>(centers),
+      reinterpret_cast<float4*>(g4));
+  return launch_status();
+}
+
+template <int P>
+int RunAdj<P>::m2m_level(int first, int last, const int* left, const int* right, const float* centers,
+                       const float* mult, float* mbar, float* cbar4, cudaStream_t st) {
+  if (last <= first) return JB_OK;
+  k_adj_m2m_level<P><<<blocks_for(last - first, 128), 128, 0, st>>>(
+      first, last, left, right, reinterpret_cast<const float4*>(centers), mult, mbar,
+      reinterpret_cast<float4*>(cbar4));
+  return launch_status();
+}
+
+template <int P>
+int RunAdj<P>::p2m(const float* pos4, int num_nodes, int num_internal, const int* ranges, const float* centers,
+                 const float* mbar, const float* cbar4, float* xm4, cudaStream_t st) {
+  const int L = num_nodes - num_internal;
+  if (L <= 0) return JB_OK;
+  k_adj_p2m<P><<<blocks_for(L, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, st>>>(
+      reinterpret_cast<const float4*>(pos4), num_nodes, num_internal, reinterpret_cast<const int2*>(ranges),
+      reinterpret_cast<const float4*>(centers), mbar, reinterpret_cast<const float4*>(cbar4),
+      reinterpret_cast<float4*>(xm4));
+  return launch_status();
+}
 
 }  // namespace jb

@@ -1590,196 +1590,239 @@ static inline unsigned blocks_for(int64_t n, int per) { return (unsigned)((n + p
 template <int P>
 struct RunP2M {
   static int run(const float* pos4, int num_nodes, int num_internal, const int* ranges, float* centers, float* mult,
-                 cudaStream_t st) {
-    const int L = num_nodes - num_internal;
-    if (L <= 0) return JB_OK;
-    const size_t sm = sizeof(float) * kWarpsPerBlock * 32 * (csize(P) + 1);
-    cudaFuncSetAttribute(k_p2m<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_p2m<P><<<blocks_for(L, kWarpsPerBlock), 32 * kWarpsPerBlock, sm, st>>>(
-        reinterpret_cast<const float4*>(pos4), num_nodes, num_internal, reinterpret_cast<const int2*>(ranges),
-        reinterpret_cast<float4*>(centers), mult);
-    return launch_status();
-  }
+                 cudaStream_t st);
 };
+
+template <int P>
+int RunP2M<P>::run(const float* pos4, int num_nodes, int num_internal, const int* ranges, float* centers, float* mult,
+                 cudaStream_t st) {
+  const int L = num_nodes - num_internal;
+  if (L <= 0) return JB_OK;
+  const size_t sm = sizeof(float) * kWarpsPerBlock * 32 * (csize(P) + 1);
+  cudaFuncSetAttribute(k_p2m<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_p2m<P><<<blocks_for(L, kWarpsPerBlock), 32 * kWarpsPerBlock, sm, st>>>(
+      reinterpret_cast<const float4*>(pos4), num_nodes, num_internal, reinterpret_cast<const int2*>(ranges),
+      reinterpret_cast<float4*>(centers), mult);
+  return launch_status();
+}
 
 template <int P>
 struct RunM2M {
   static int run(int first, int last, const int* left, const int* right, const int* ranges, float* centers,
-                 float* mult, cudaStream_t st) {
-    if (last <= first) return JB_OK;
-    if (last - first <= g_split_max_parents[0]) {
-      k_m2m_level_split<P><<<blocks_for(2 * (int64_t)(last - first), kSplitItems), 128, 0, st>>>(
-          first, last, left, right, reinterpret_cast<const int2*>(ranges), reinterpret_cast<float4*>(centers), mult);
-    } else {
-      k_m2m_level<P><<<blocks_for(2 * (int64_t)(last - first), 128), 128, 0, st>>>(
-          first, last, left, right, reinterpret_cast<const int2*>(ranges), reinterpret_cast<float4*>(centers), mult);
-    }
-    return launch_status();
-  }
+                 float* mult, cudaStream_t st);
 };
+
+template <int P>
+int RunM2M<P>::run(int first, int last, const int* left, const int* right, const int* ranges, float* centers,
+                 float* mult, cudaStream_t st) {
+  if (last <= first) return JB_OK;
+  if (last - first <= g_split_max_parents[0]) {
+    k_m2m_level_split<P><<<blocks_for(2 * (int64_t)(last - first), kSplitItems), 128, 0, st>>>(
+        first, last, left, right, reinterpret_cast<const int2*>(ranges), reinterpret_cast<float4*>(centers), mult);
+  } else {
+    k_m2m_level<P><<<blocks_for(2 * (int64_t)(last - first), 128), 128, 0, st>>>(
+        first, last, left, right, reinterpret_cast<const int2*>(ranges), reinterpret_cast<float4*>(centers), mult);
+  }
+  return launch_status();
+}
 
 template <int P>
 struct RunM2L {
   static int run(int num_units, const int* units, const float* mult, const float* centers, const int* far_src,
                  float* locals, float* partials, int num_split, const int* split, cudaStream_t st, bool neg = false,
-                 int rs = 0, const float* far_w = nullptr) {
-    if (rs <= 0) rs = cstride(P);
-    if (num_units > 0) {
-      const bool coop = g_m2l_coop != 0;
-      const size_t sm = sizeof(float4) * kM2LThreads * row4(P) + (coop ? sizeof(int) * kM2LThreads : 0);
-      auto kern = coop ? (far_w ? k_m2l_units_coop<P, false, true>
-                                : (neg ? k_m2l_units_coop<P, true> : k_m2l_units_coop<P, false>))
-                       : (far_w ? k_m2l_units<P, false, true> : (neg ? k_m2l_units<P, true> : k_m2l_units<P, false>));
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      kern<<<blocks_for(num_units, kM2LThreads), kM2LThreads, sm, st>>>(
-          num_units, reinterpret_cast<const int4*>(units), mult, reinterpret_cast<const float4*>(centers), far_src,
-          locals, partials, rs, far_w);
-      const int rc = launch_status();
-      if (rc) return rc;
-    }
-    if (num_split > 0) {
-      k_m2l_reduce<<<blocks_for((int64_t)num_split * rs, 256), 256, 0, st>>>(
-          num_split, reinterpret_cast<const int4*>(split), partials, locals, rs);
-      return launch_status();
-    }
-    return JB_OK;
-  }
+                 int rs = 0, const float* far_w = nullptr);
 };
+
+template <int P>
+int RunM2L<P>::run(int num_units, const int* units, const float* mult, const float* centers, const int* far_src,
+                 float* locals, float* partials, int num_split, const int* split, cudaStream_t st, bool neg,
+                 int rs, const float* far_w) {
+  if (rs <= 0) rs = cstride(P);
+  if (num_units > 0) {
+    const bool coop = g_m2l_coop != 0;
+    const size_t sm = sizeof(float4) * kM2LThreads * row4(P) + (coop ? sizeof(int) * kM2LThreads : 0);
+    auto kern = coop ? (far_w ? k_m2l_units_coop<P, false, true>
+                              : (neg ? k_m2l_units_coop<P, true> : k_m2l_units_coop<P, false>))
+                     : (far_w ? k_m2l_units<P, false, true> : (neg ? k_m2l_units<P, true> : k_m2l_units<P, false>));
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    kern<<<blocks_for(num_units, kM2LThreads), kM2LThreads, sm, st>>>(
+        num_units, reinterpret_cast<const int4*>(units), mult, reinterpret_cast<const float4*>(centers), far_src,
+        locals, partials, rs, far_w);
+    const int rc = launch_status();
+    if (rc) return rc;
+  }
+  if (num_split > 0) {
+    k_m2l_reduce<<<blocks_for((int64_t)num_split * rs, 256), 256, 0, st>>>(
+        num_split, reinterpret_cast<const int4*>(split), partials, locals, rs);
+    return launch_status();
+  }
+  return JB_OK;
+}
 
 template <int P>
 struct RunM2LMixed {
   static int run(int num_units, const int* units, const int* bounds, const float* mult, const float* centers,
-                 const int* far_src, float* locals, float* partials, int num_split, const int* split, cudaStream_t st) {
-    const int rs = cstride(P);
-    if (num_units > 0) {
-      const size_t sm = sizeof(float4) * kM2LThreads * row4(P);
-      cudaFuncSetAttribute(k_m2l_mixed<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-      k_m2l_mixed<P><<<blocks_for(num_units, kM2LThreads), kM2LThreads, sm, st>>>(
-          num_units, reinterpret_cast<const int4*>(units), reinterpret_cast<const int4*>(bounds), mult,
-          reinterpret_cast<const float4*>(centers), far_src, locals, partials, rs);
-      const int rc = launch_status();
-      if (rc) return rc;
-    }
-    if (num_split > 0) {
-      k_m2l_reduce<<<blocks_for((int64_t)num_split * rs, 256), 256, 0, st>>>(
-          num_split, reinterpret_cast<const int4*>(split), partials, locals, rs);
-      return launch_status();
-    }
-    return JB_OK;
-  }
+                 const int* far_src, float* locals, float* partials, int num_split, const int* split, cudaStream_t st);
 };
+
+template <int P>
+int RunM2LMixed<P>::run(int num_units, const int* units, const int* bounds, const float* mult, const float* centers,
+                 const int* far_src, float* locals, float* partials, int num_split, const int* split, cudaStream_t st) {
+  const int rs = cstride(P);
+  if (num_units > 0) {
+    const size_t sm = sizeof(float4) * kM2LThreads * row4(P);
+    cudaFuncSetAttribute(k_m2l_mixed<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_m2l_mixed<P><<<blocks_for(num_units, kM2LThreads), kM2LThreads, sm, st>>>(
+        num_units, reinterpret_cast<const int4*>(units), reinterpret_cast<const int4*>(bounds), mult,
+        reinterpret_cast<const float4*>(centers), far_src, locals, partials, rs);
+    const int rc = launch_status();
+    if (rc) return rc;
+  }
+  if (num_split > 0) {
+    k_m2l_reduce<<<blocks_for((int64_t)num_split * rs, 256), 256, 0, st>>>(
+        num_split, reinterpret_cast<const int4*>(split), partials, locals, rs);
+    return launch_status();
+  }
+  return JB_OK;
+}
 
 template <int P>
 struct RunL2L {
   static int run(int first, int last, const int* left, const int* right, const float* centers, float* locals,
-                 cudaStream_t st) {
-    if (last <= first) return JB_OK;
-    if (last - first <= g_split_max_parents[1]) {
-      k_l2l_level_split<P><<<blocks_for(2 * (int64_t)(last - first), kSplitItems), 128, 0, st>>>(
-          first, last, left, right, reinterpret_cast<const float4*>(centers), locals);
-    } else {
-      k_l2l_level<P><<<blocks_for(2 * (int64_t)(last - first), 128), 128, 0, st>>>(
-          first, last, left, right, reinterpret_cast<const float4*>(centers), locals);
-    }
-    return launch_status();
-  }
+                 cudaStream_t st);
 };
+
+template <int P>
+int RunL2L<P>::run(int first, int last, const int* left, const int* right, const float* centers, float* locals,
+                 cudaStream_t st) {
+  if (last <= first) return JB_OK;
+  if (last - first <= g_split_max_parents[1]) {
+    k_l2l_level_split<P><<<blocks_for(2 * (int64_t)(last - first), kSplitItems), 128, 0, st>>>(
+        first, last, left, right, reinterpret_cast<const float4*>(centers), locals);
+  } else {
+    k_l2l_level<P><<<blocks_for(2 * (int64_t)(last - first), 128), 128, 0, st>>>(
+        first, last, left, right, reinterpret_cast<const float4*>(centers), locals);
+  }
+  return launch_status();
+}
 
 template <int P>
 struct RunL2LLeaves {
   static int run(int num_units, const int* units, const int* anc, const float* centers, float* locals,
-                 cudaStream_t st) {
-    if (num_units <= 0) return JB_OK;
-    const size_t sm = sizeof(float4) * kM2LThreads * row4(P) + sizeof(int) * kM2LThreads;
-    cudaFuncSetAttribute(k_l2l_leaves<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_l2l_leaves<P><<<blocks_for(num_units, kM2LThreads), kM2LThreads, sm, st>>>(
-        num_units, reinterpret_cast<const int4*>(units), anc, reinterpret_cast<const float4*>(centers), locals);
-    return launch_status();
-  }
+                 cudaStream_t st);
 };
+
+template <int P>
+int RunL2LLeaves<P>::run(int num_units, const int* units, const int* anc, const float* centers, float* locals,
+                 cudaStream_t st) {
+  if (num_units <= 0) return JB_OK;
+  const size_t sm = sizeof(float4) * kM2LThreads * row4(P) + sizeof(int) * kM2LThreads;
+  cudaFuncSetAttribute(k_l2l_leaves<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_l2l_leaves<P><<<blocks_for(num_units, kM2LThreads), kM2LThreads, sm, st>>>(
+      num_units, reinterpret_cast<const int4*>(units), anc, reinterpret_cast<const float4*>(centers), locals);
+  return launch_status();
+}
 
 template <int P>
 struct RunLeafEval {
   template <bool K, bool PT>
   static void go(unsigned nb, cudaStream_t st, const float4* pos4, int num_internal, int num_units, const int4* units,
                  const int2* aux, const int2* runs, const int2* ranges, float G, float eps2, float4* out,
-                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err) {
-    if (rung)
-      k_leaf_units<K, PT, true><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
-                                                                    ranges, G, eps2, out, partial, max_slots, err,
-                                                                    rung, lw, nlw);
-    else if (flat) {
-      // 23.5 KB of shared memory per block: ask for the carveout that holds
-      // the eight blocks per SM the launch bounds allow.
-      static const cudaError_t carve = cudaFuncSetAttribute(
-          k_leaf_units_flat<K, PT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-      (void)carve;
-      k_leaf_units_flat<K, PT><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
-                                                                   ranges, G, eps2, out, partial, max_slots, err);
-    }
-    else
-      k_leaf_units<K, PT><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs, ranges,
-                                                              G, eps2, out, partial, max_slots, err);
-  }
+                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err);
   static int run(int mode, const float* pos4, int num_internal, int num_units, const int* units, const int* aux,
                  const int* runs, const int* ranges, const float* centers, const float* locals, float G, float eps2,
                  float* out, float* partial, int num_split, const int* split, cudaStream_t st,
                  const int* rung = nullptr, const float* lw = nullptr, int nlw = 1, bool flat = false,
-                 int max_slots = 0x7fffffff, int* err = nullptr) {
-    if (num_units > 0) {
-      const unsigned nb = blocks_for(num_units, kWarpsPerBlock);
-      auto a0 = reinterpret_cast<const float4*>(pos4);
-      auto a1 = reinterpret_cast<const int4*>(units);
-      auto a2 = reinterpret_cast<const int2*>(aux);
-      auto a3 = reinterpret_cast<const int2*>(runs);
-      auto a4 = reinterpret_cast<const int2*>(ranges);
-      auto o = reinterpret_cast<float4*>(out);
-      auto pt = reinterpret_cast<float4*>(partial);
-      const bool far_only = (mode & JB_P2P_FAR_ONLY) != 0, far_after = (mode & JB_P2P_FAR_AFTER) != 0;
-      const bool zero = (mode & (JB_P2P_NEAR_ONLY | JB_P2P_NEAR_FIRST)) != 0;
-      k_leaf_l2p<P><<<nb, 32 * kWarpsPerBlock, 0, st>>>(a0, num_internal, num_units, a1, a2, a4,
-                                                        reinterpret_cast<const float4*>(centers), locals, G, o,
-                                                        zero ? kL2PZero : far_after ? kL2PAdd : kL2PWrite);
-      int rc = launch_status();
-      if (rc) return rc;
-      if (far_only) return JB_OK;
-      if (!far_after) {  // FAR_AFTER: the near field is already in out (and partials)
-        const bool kahan = (mode & JB_P2P_KAHAN) != 0, pot = (mode & JB_P2P_POTENTIAL) != 0;
-        if (kahan && pot) go<true, true>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
-        else if (kahan) go<true, false>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
-        else if (pot) go<false, true>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
-        else go<false, false>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
-        rc = launch_status();
-        if (rc) return rc;
-      }
-    }
-    if (num_split > 0 && !(mode & JB_P2P_NEAR_FIRST)) {  // NEAR_FIRST: summed by the FAR_AFTER call
-      k_leaf_reduce<true><<<blocks_for((int64_t)num_split * kMaxLeaf, 256), 256, 0, st>>>(
-          num_split, reinterpret_cast<const int4*>(split), num_internal, reinterpret_cast<const int2*>(ranges),
-          reinterpret_cast<const float4*>(partial), reinterpret_cast<float4*>(out), max_slots, err);
-      return launch_status();
-    }
-    return JB_OK;
-  }
+                 int max_slots = 0x7fffffff, int* err = nullptr);
 };
+
+template <int P>
+template <bool K, bool PT>
+void RunLeafEval<P>::go(unsigned nb, cudaStream_t st, const float4* pos4, int num_internal, int num_units, const int4* units,
+                 const int2* aux, const int2* runs, const int2* ranges, float G, float eps2, float4* out,
+                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err) {
+  if (rung)
+    k_leaf_units<K, PT, true><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
+                                                                  ranges, G, eps2, out, partial, max_slots, err,
+                                                                  rung, lw, nlw);
+  else if (flat) {
+    // 23.5 KB of shared memory per block: ask for the carveout that holds
+    // the eight blocks per SM the launch bounds allow.
+    static const cudaError_t carve = cudaFuncSetAttribute(
+        k_leaf_units_flat<K, PT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    (void)carve;
+    k_leaf_units_flat<K, PT><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
+                                                                 ranges, G, eps2, out, partial, max_slots, err);
+  }
+  else
+    k_leaf_units<K, PT><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs, ranges,
+                                                            G, eps2, out, partial, max_slots, err);
+}
+
+template <int P>
+int RunLeafEval<P>::run(int mode, const float* pos4, int num_internal, int num_units, const int* units, const int* aux,
+                 const int* runs, const int* ranges, const float* centers, const float* locals, float G, float eps2,
+                 float* out, float* partial, int num_split, const int* split, cudaStream_t st,
+                 const int* rung, const float* lw, int nlw, bool flat,
+                 int max_slots, int* err) {
+  if (num_units > 0) {
+    const unsigned nb = blocks_for(num_units, kWarpsPerBlock);
+    auto a0 = reinterpret_cast<const float4*>(pos4);
+    auto a1 = reinterpret_cast<const int4*>(units);
+    auto a2 = reinterpret_cast<const int2*>(aux);
+    auto a3 = reinterpret_cast<const int2*>(runs);
+    auto a4 = reinterpret_cast<const int2*>(ranges);
+    auto o = reinterpret_cast<float4*>(out);
+    auto pt = reinterpret_cast<float4*>(partial);
+    const bool far_only = (mode & JB_P2P_FAR_ONLY) != 0, far_after = (mode & JB_P2P_FAR_AFTER) != 0;
+    const bool zero = (mode & (JB_P2P_NEAR_ONLY | JB_P2P_NEAR_FIRST)) != 0;
+    k_leaf_l2p<P><<<nb, 32 * kWarpsPerBlock, 0, st>>>(a0, num_internal, num_units, a1, a2, a4,
+                                                      reinterpret_cast<const float4*>(centers), locals, G, o,
+                                                      zero ? kL2PZero : far_after ? kL2PAdd : kL2PWrite);
+    int rc = launch_status();
+    if (rc) return rc;
+    if (far_only) return JB_OK;
+    if (!far_after) {  // FAR_AFTER: the near field is already in out (and partials)
+      const bool kahan = (mode & JB_P2P_KAHAN) != 0, pot = (mode & JB_P2P_POTENTIAL) != 0;
+      if (kahan && pot) go<true, true>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
+      else if (kahan) go<true, false>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
+      else if (pot) go<false, true>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
+      else go<false, false>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
+      rc = launch_status();
+      if (rc) return rc;
+    }
+  }
+  if (num_split > 0 && !(mode & JB_P2P_NEAR_FIRST)) {  // NEAR_FIRST: summed by the FAR_AFTER call
+    k_leaf_reduce<true><<<blocks_for((int64_t)num_split * kMaxLeaf, 256), 256, 0, st>>>(
+        num_split, reinterpret_cast<const int4*>(split), num_internal, reinterpret_cast<const int2*>(ranges),
+        reinterpret_cast<const float4*>(partial), reinterpret_cast<float4*>(out), max_slots, err);
+    return launch_status();
+  }
+  return JB_OK;
+}
 
 template <int P>
 struct RunTargets {
   static int run(const float* pos4, int num_internal, const int* ranges, const float* centers, const float* locals,
                  const int64_t* near_off, const int* near_src, const int* leaf_of, int64_t nt, const int* ts, float G,
-                 float eps2, float* out, cudaStream_t st) {
-    if (nt <= 0) return JB_OK;
-    k_targets_far<P><<<blocks_for(nt, 128), 128, 0, st>>>(
-        reinterpret_cast<const float4*>(pos4), num_internal, reinterpret_cast<const float4*>(centers), locals,
-        leaf_of, nt, ts, G, reinterpret_cast<float4*>(out));
-    const int rc = launch_status();
-    if (rc) return rc;
-    k_targets_near<<<blocks_for(nt, 8), 256, 0, st>>>(
-        reinterpret_cast<const float4*>(pos4), num_internal, reinterpret_cast<const int2*>(ranges), near_off, near_src,
-        leaf_of, nt, ts, G, eps2, reinterpret_cast<float4*>(out));
-    return launch_status();
-  }
+                 float eps2, float* out, cudaStream_t st);
 };
+
+template <int P>
+int RunTargets<P>::run(const float* pos4, int num_internal, const int* ranges, const float* centers, const float* locals,
+                 const int64_t* near_off, const int* near_src, const int* leaf_of, int64_t nt, const int* ts, float G,
+                 float eps2, float* out, cudaStream_t st) {
+  if (nt <= 0) return JB_OK;
+  k_targets_far<P><<<blocks_for(nt, 128), 128, 0, st>>>(
+      reinterpret_cast<const float4*>(pos4), num_internal, reinterpret_cast<const float4*>(centers), locals,
+      leaf_of, nt, ts, G, reinterpret_cast<float4*>(out));
+  const int rc = launch_status();
+  if (rc) return rc;
+  k_targets_near<<<blocks_for(nt, 8), 256, 0, st>>>(
+      reinterpret_cast<const float4*>(pos4), num_internal, reinterpret_cast<const int2*>(ranges), near_off, near_src,
+      leaf_of, nt, ts, G, eps2, reinterpret_cast<float4*>(out));
+  return launch_status();
+}
 
 }  // namespace jb
 
