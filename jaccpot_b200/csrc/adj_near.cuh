@@ -1,0 +1,235 @@
+#pragma once
+// Near-field adjoint, warp per leaf unit.  For the pair (k, l), d = x_k - x_l,
+// q = (|d|^2 + eps^2)^-1/2:
+//   dL/dx_k += G [ -m_l q^3 w_k + m_k q^3 w_l + 3 q^5 (m_l (w_k.d) - m_k (w_l.d)) d ]
+//   dL/dm_k += G q^3 (w_l . d)
+// which needs l in near(k) <=> k in near(l) (the lists are symmetric).
+//
+// Per target the pair sums are S = sum q^3 m_l, V = sum q^3 w_l, A = sum q^5
+// (m_l (w_k.d) - m_k (w_l.d)) d and D = sum q^3 (w_l.d), so w_k and m_k enter
+// once a target: 26 FP32 operations and one rsqrt a pair where the terms
+// written out took 43, and the sources come two to an instruction
+// (f32x2), staged per coordinate as in k_leaf_units_flat.  The kernel is bound
+// by FP32 issue and by the seven 16-byte broadcast loads per four sources.
+// At a Plummer sphere of 1M (leaf 32, 2.0e9 pairs): 4.02 ms with one lane per
+// target and scalar pairs.
+#include "fmm_kernels.cuh"
+
+namespace jb {
+
+constexpr int kAdjChunk = 32;             // sources per chunk (item)
+constexpr int kAdjSlot = kAdjChunk + 4;   // slot stride: the slots one load reads use distinct banks
+
+// Four ring slots of sources per coordinate (x, y, z, m, w), the targets and
+// their sums.
+struct alignas(16) AdjStage {
+  float v[7][4][kAdjSlot];
+  float4 tp[32], tw[32];
+  float4 sv[32], ad[32];  // (S, V) and (A, D)
+};
+
+struct AdjSums {
+  float4 sv, ad;
+};
+
+// One target against NS staged sources (a multiple of 4) at position o of
+// slot sl; SELF: source self_j is the target.
+template <bool SELF>
+__device__ __forceinline__ AdjSums adj_chunk(const AdjStage& st, int sl, int o, int ns, float4 t, float4 w, int self_j,
+                                             float eps2) {
+  const f32x2 TX = f2(t.x, t.x), TY = f2(t.y, t.y), TZ = f2(t.z, t.z), E2 = f2(eps2, eps2);
+  const f32x2 WX = f2(w.x, w.x), WY = f2(w.y, w.y), WZ = f2(w.z, w.z), NM = f2(-t.w, -t.w);
+  f32x2 S = f2(0.f, 0.f), VX = S, VY = S, VZ = S, AX = S, AY = S, AZ = S, D = S;
+  auto pair2 = [&](f32x2 sx, f32x2 sy, f32x2 sz, f32x2 sm, f32x2 wx, f32x2 wy, f32x2 wz, int j0) {
+    const f32x2 dx = f2_sub(TX, sx), dy = f2_sub(TY, sy), dz = f2_sub(TZ, sz);
+    const f32x2 d2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, E2)));
+    float a, b;
+    f2_split(d2, a, b);
+    float qa = rsqrt_ftz(a), qb = rsqrt_ftz(b);
+    if (SELF) {
+      qa = j0 == self_j ? 0.f : qa;
+      qb = j0 + 1 == self_j ? 0.f : qb;
+    }
+    const f32x2 q = f2(qa, qb), q2 = f2_mul(q, q), q3 = f2_mul(q2, q);
+    S = f2_fma(q3, sm, S);
+    VX = f2_fma(q3, wx, VX);
+    VY = f2_fma(q3, wy, VY);
+    VZ = f2_fma(q3, wz, VZ);
+    const f32x2 wkd = f2_fma(WX, dx, f2_fma(WY, dy, f2_mul(WZ, dz)));
+    const f32x2 wld = f2_fma(wx, dx, f2_fma(wy, dy, f2_mul(wz, dz)));
+    const f32x2 c = f2_mul(f2_mul(q3, q2), f2_fma(NM, wld, f2_mul(sm, wkd)));
+    AX = f2_fma(c, dx, AX);
+    AY = f2_fma(c, dy, AY);
+    AZ = f2_fma(c, dz, AZ);
+    D = f2_fma(q3, wld, D);
+  };
+  const ulonglong2* X[7];
+#pragma unroll
+  for (int k = 0; k < 7; ++k) X[k] = reinterpret_cast<const ulonglong2*>(&st.v[k][sl][o]);
+#pragma unroll 4
+  for (int i = 0; i < ns / 4; ++i) {
+    const ulonglong2 x = X[0][i], y = X[1][i], z = X[2][i], m = X[3][i], wx = X[4][i], wy = X[5][i], wz = X[6][i];
+    pair2(x.x, y.x, z.x, m.x, wx.x, wy.x, wz.x, 4 * i);
+    pair2(x.y, y.y, z.y, m.y, wx.y, wy.y, wz.y, 4 * i + 2);
+  }
+  auto sum = [](f32x2 v) {
+    float lo, hi;
+    f2_split(v, lo, hi);
+    return lo + hi;
+  };
+  return AdjSums{make_float4(sum(S), sum(VX), sum(VY), sum(VZ)), make_float4(sum(AX), sum(AY), sum(AZ), sum(D))};
+}
+
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+  return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
+__device__ __forceinline__ float4 shfl_down4(float4 v, int o) {
+  return make_float4(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o),
+                     __shfl_down_sync(0xffffffffu, v.z, o), __shfl_down_sync(0xffffffffu, v.w, o));
+}
+
+__device__ __forceinline__ void adj_stage(AdjStage& s, int sl, int q, float4 p, float4 w) {
+  s.v[0][sl][q] = p.x;
+  s.v[1][sl][q] = p.y;
+  s.v[2][sl][q] = p.z;
+  s.v[3][sl][q] = p.w;
+  s.v[4][sl][q] = w.x;
+  s.v[5][sl][q] = w.y;
+  s.v[6][sl][q] = w.z;
+}
+
+// The targets rg (at most 32, of the leaf lr) against the unit's sources.
+// The chunk-major walk of leaf_unit_flat: item f = c * nt + t is target t
+// against chunk c, 32 items a step, so every lane works.  A step of 17 to 32
+// targets spans at most three chunks, and four ring slots hold them.  Fewer
+// targets are taken G = 2 or 4 times, copy h of a target against the h-th part
+// of each chunk, one chunk a step.
+template <int G>
+__device__ __forceinline__ void adj_unit(const float4* __restrict__ pos4, const float4* __restrict__ w4, int2 rg,
+                                         int4 U, int2 aux, const int2* __restrict__ runs, AdjStage& S, int lane,
+                                         float G_, float eps2, float4* __restrict__ out, float4* __restrict__ partial,
+                                         int2 lr, int row) {
+  constexpr int CH = kAdjChunk, PART = CH / G;
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int nt = rg.y - rg.x + 1, items = nt * G;
+  const bool tgt = lane < nt;
+  S.tp[lane] = tgt ? pos4[rg.x + lane] : zero4;
+  S.tw[lane] = tgt ? w4[rg.x + lane] : zero4;
+  S.sv[lane] = zero4;
+  S.ad[lane] = zero4;
+  __syncwarp();
+  // adds the items' sums, G lanes to a target, in lane order
+  auto add_items = [&](AdjSums v, int nl) {
+#pragma unroll
+    for (int h = 1; h < G; ++h) {
+      const float4 a = shfl_down4(v.sv, h), b = shfl_down4(v.ad, h);
+      if (lane % G == 0) v.sv = add4(v.sv, a), v.ad = add4(v.ad, b);
+    }
+    if (lane % G == 0 && lane < nl) {
+      S.sv[lane / G] = add4(S.sv[lane / G], v.sv);
+      S.ad[lane / G] = add4(S.ad[lane / G], v.ad);
+    }
+  };
+  if (aux.y & 1) {  // the leaf itself, 32 at a time, the diagonal excluded
+    for (int b = lr.x; b <= lr.y; b += 32) {
+      const bool ok = b + lane <= lr.y;
+      __syncwarp();  // the previous chunk's reads are done
+      adj_stage(S, 0, lane, ok ? pos4[b + lane] : JB_PAD4, ok ? w4[b + lane] : zero4);
+      __syncwarp();
+      const int t = min(lane / G, nt - 1), h = lane % G;
+      add_items(adj_chunk<true>(S, 0, h * PART, PART, S.tp[t], S.tw[t], rg.x + t - b - h * PART, eps2), items);
+    }
+  }
+  const int nsrc = U.w;
+  if (nsrc > 0) {
+    const int C = (nsrc + CH - 1) / CH;
+    int r = U.y, rbase = 0;
+    int2 run = runs[r];
+    float4 np, nw;  // the next chunk's source of this lane, in flight
+    auto fetch = [&](int f) {
+      while (f >= rbase + run.y && r + 1 < U.z) {
+        rbase += run.y;
+        ++r;
+        run = runs[r];
+      }
+      np = f < nsrc ? pos4[run.x + (f - rbase)] : JB_PAD4;
+      nw = f < nsrc ? w4[run.x + (f - rbase)] : zero4;
+    };
+    fetch(lane);
+    if (G > 1) {  // one chunk a step, all its items at once
+      for (int c = 0; c < C; ++c) {
+        __syncwarp();
+        adj_stage(S, c & 1, lane, np, nw);
+        if (c + 1 < C) fetch((c + 1) * CH + lane);
+        __syncwarp();
+        const int t = min(lane / G, nt - 1), h = lane % G;
+        add_items(adj_chunk<false>(S, c & 1, h * PART, PART, S.tp[t], S.tw[t], -1, eps2), items);
+      }
+    } else {
+      const int total = nt * C;
+      int staged = 0;
+      int c = (lane >= nt) ? 1 : 0, t = lane - c * nt;  // item f = lane
+      for (int base = 0; base < total; base += 32) {
+        const int need = min(__shfl_sync(0xffffffffu, c, 31), C - 1);
+        __syncwarp();  // the previous step's reads and adds are done
+        while (staged <= need) {
+          adj_stage(S, staged & 3, lane, np, nw);
+          if (++staged < C) fetch(staged * CH + lane);
+        }
+        __syncwarp();
+        const AdjSums v = adj_chunk<false>(S, c & 3, 0, CH, S.tp[t], S.tw[t], -1, eps2);
+        const float4 sv2 = shfl_down4(v.sv, nt), ad2 = shfl_down4(v.ad, nt);
+        if (tgt && base + lane < total) {
+          float4 a = add4(S.sv[t], v.sv), b = add4(S.ad[t], v.ad);
+          if (lane + nt < 32 && base + lane + nt < total) {  // lane + nt holds (t, c + 1)
+            a = add4(a, sv2);
+            b = add4(b, ad2);
+          }
+          S.sv[t] = a;
+          S.ad[t] = b;
+        }
+        t += 32 - nt;  // item f + 32
+        c += 1;
+        if (t >= nt) {
+          t -= nt;
+          c += 1;
+        }
+      }
+    }
+  }
+  __syncwarp();
+  if (tgt) {
+    const float4 sv = S.sv[lane], ad = S.ad[lane], w = S.tw[lane];
+    const float m = S.tp[lane].w;
+    const float4 res = make_float4(G_ * (m * sv.y - sv.x * w.x + 3.f * ad.x), G_ * (m * sv.z - sv.x * w.y + 3.f * ad.y),
+                                   G_ * (m * sv.w - sv.x * w.z + 3.f * ad.z), G_ * ad.w);
+    if (aux.x < 0) out[rg.x + lane] = res;
+    else partial[(size_t)aux.x * kMaxLeaf + row + lane] = res;
+  }
+}
+
+static __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_adj_near(
+    const float4* __restrict__ pos4, const float4* __restrict__ w4, int num_internal, int num_units,
+    const int4* __restrict__ units, const int2* __restrict__ aux, const int2* __restrict__ runs,
+    const int2* __restrict__ ranges, float G, float eps2, float4* __restrict__ out, float4* __restrict__ partial) {
+  __shared__ AdjStage sA[kWarpsPerBlock];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int u = blockIdx.x * kWarpsPerBlock + warp;
+  if (u >= num_units) return;
+  const int4 U = units[u];
+  const int2 ax = aux[u];
+  const int2 rg = ranges[num_internal + U.x];
+  const int n = rg.y - rg.x + 1;
+  if (n > kMaxLeaf) return;  // a split leaf's partial row holds kMaxLeaf targets (jb_validate_leaves)
+  for (int row = 0; row < n; row += 32) {  // a leaf of more than 32 particles in two passes
+    const int2 rt = make_int2(rg.x + row, min(rg.y, rg.x + row + 31));
+    const int nt = rt.y - rt.x + 1;
+    if (row > 0) __syncwarp();  // the first pass's reads of the stage are done
+    if (nt <= 8) adj_unit<4>(pos4, w4, rt, U, ax, runs, sA[warp], lane, G, eps2, out, partial, rg, row);
+    else if (nt <= 16) adj_unit<2>(pos4, w4, rt, U, ax, runs, sA[warp], lane, G, eps2, out, partial, rg, row);
+    else adj_unit<1>(pos4, w4, rt, U, ax, runs, sA[warp], lane, G, eps2, out, partial, rg, row);
+  }
+}
+
+}  // namespace jb

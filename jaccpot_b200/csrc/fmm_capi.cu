@@ -1,5 +1,6 @@
 // C-ABI entry points (include/jaccpot_b200.h) and the order-independent kernels.
 #include "device_symbol.cuh"
+#include "adj_near.cuh"
 #include "fmm_adjoint.cuh"
 
 #include <cooperative_groups.h>
@@ -312,96 +313,6 @@ __global__ void k_probe(int iters, int use_mufu, float* out) {
 #pragma unroll
   for (int k = 0; k < 8; ++k) s += a[k];
   if (s == 12345.678f) out[threadIdx.x] = s;  // keeps the chains live
-}
-
-// ---------------------------------------------------------------------------
-// Near field: warp per leaf unit, lane = target particle.  For the pair
-// (k, l), d = x_k - x_l, q = (|d|^2 + eps^2)^-1/2:
-//   dL/dx_k += G [ -m_l q^3 w_k + m_k q^3 w_l + 3 q^5 (m_l (w_k.d) - m_k (w_l.d)) d ]
-//   dL/dm_k += G q^3 (w_l . d)
-// which needs l in near(k) <=> k in near(l) (the lists are symmetric).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void adj_near_pair(float4 tk, float4 wk, float4 s, float4 ws, float eps2, bool skip,
-                                              float* a) {
-  const float dx = tk.x - s.x, dy = tk.y - s.y, dz = tk.z - s.z;
-  const float d2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-  const float q = skip ? 0.f : rsqrt_ftz(d2);
-  const float q3 = q * q * q;
-  const float q5 = q3 * q * q;
-  const float wkd = wk.x * dx + wk.y * dy + wk.z * dz;
-  const float wld = ws.x * dx + ws.y * dy + ws.z * dz;
-  const float c = 3.f * q5 * (s.w * wkd - tk.w * wld);
-  const float aml = -s.w * q3, amk = tk.w * q3;
-  a[0] += aml * wk.x + amk * ws.x + c * dx;
-  a[1] += aml * wk.y + amk * ws.y + c * dy;
-  a[2] += aml * wk.z + amk * ws.z + c * dz;
-  a[3] += q3 * wld;
-}
-
-static __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_adj_near(
-    const float4* __restrict__ pos4, const float4* __restrict__ w4, int num_internal, int num_units,
-    const int4* __restrict__ units, const int2* __restrict__ aux, const int2* __restrict__ runs,
-    const int2* __restrict__ ranges, float G, float eps2, float4* __restrict__ out, float4* __restrict__ partial) {
-  __shared__ float4 sP[kWarpsPerBlock][32];
-  __shared__ float4 sW[kWarpsPerBlock][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int u = blockIdx.x * kWarpsPerBlock + warp;
-  if (u >= num_units) return;
-  const int4 U = units[u];
-  const int2 ax = aux[u];
-  const int2 rg = ranges[num_internal + U.x];
-  const int nt = rg.y - rg.x + 1;
-  if (nt > kMaxLeaf) return;  // a split leaf's partial row holds kMaxLeaf targets (jb_validate_leaves)
-  float a[4] = {0.f, 0.f, 0.f, 0.f};
-  // targets beyond 32 particles take further passes
-  for (int t0 = 0; t0 < nt; t0 += 32) {
-    const int tl = t0 + lane;
-    const bool active = tl < nt;
-    const float4 tk = active ? pos4[rg.x + tl] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 wk = active ? w4[rg.x + tl] : make_float4(0.f, 0.f, 0.f, 0.f);
-    a[0] = a[1] = a[2] = a[3] = 0.f;
-    if (ax.y & 1) {
-      for (int s0 = 0; s0 < nt; s0 += 32) {
-        const int j = s0 + lane;
-        sP[warp][lane] = (j < nt) ? pos4[rg.x + j] : JB_PAD4;
-        sW[warp][lane] = (j < nt) ? w4[rg.x + j] : make_float4(0.f, 0.f, 0.f, 0.f);
-        __syncwarp();
-#pragma unroll 8
-        for (int q = 0; q < 32; ++q)
-          adj_near_pair(tk, wk, sP[warp][q], sW[warp][q], eps2, (s0 + q == tl) || (s0 + q >= nt), a);
-        __syncwarp();
-      }
-    }
-    const int nsrc = U.w;
-    int r = U.y, rbase = 0;
-    int2 run = (U.z > U.y) ? runs[r] : make_int2(0, 0);
-    auto fetch = [&](int f, float4& p, float4& w) {  // source f of the unit (padding past the end)
-      while (f >= rbase + run.y && r + 1 < U.z) {
-        rbase += run.y;
-        ++r;
-        run = runs[r];
-      }
-      const bool ok = f < nsrc;
-      p = ok ? pos4[run.x + (f - rbase)] : JB_PAD4;
-      w = ok ? w4[run.x + (f - rbase)] : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    float4 qp = JB_PAD4, qw = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (nsrc > 0) fetch(lane, qp, qw);
-    for (int base = 0; base < nsrc; base += 32) {
-      sP[warp][lane] = qp;
-      sW[warp][lane] = qw;
-      __syncwarp();
-      if (base + 32 < nsrc) fetch(base + 32 + lane, qp, qw);  // the next chunk, while this one is used
-#pragma unroll 8
-      for (int q = 0; q < 32; ++q) adj_near_pair(tk, wk, sP[warp][q], sW[warp][q], eps2, base + q >= nsrc, a);
-      __syncwarp();
-    }
-    if (active) {
-      const float4 res = make_float4(G * a[0], G * a[1], G * a[2], G * a[3]);
-      if (ax.x < 0) out[rg.x + tl] = res;
-      else partial[(size_t)ax.x * kMaxLeaf + tl] = res;
-    }
-  }
 }
 
 // M2L centre-gradient gather, thread per node u: for every pair e = (u <- v)
