@@ -237,7 +237,9 @@ JB_API int jb_far_reverse_index(int num_nodes, const int64_t* far_off, const int
 /* Units of jb_l2l_leaves for the leaves [leaf_lo, leaf_hi): JB_SCHED_UNITS are
  * (leaf node, first, end, -1) over JB_SCHED_RUNS, int32[num_runs], which holds
  * each leaf's ancestors with far pairs, nearest first, leaf after leaf; units
- * longest first (stable), leaves without such ancestors left out.           */
+ * longest first (stable), leaves without such ancestors left out.
+ * num_targets is the lowest-numbered of all those ancestors (num_internal when
+ * there is none): the sweep by levels starts at its level.                  */
 JB_API int jb_l2l_schedule_device(int num_internal, int leaf_lo, int leaf_hi, const int* parent, const int64_t* far_off,
                                   void* stream, jb_dsched** out);
 JB_API int jb_dsched_info(const jb_dsched* d, jb_sched_info_t* info);

@@ -14,6 +14,7 @@ _HERE = Path(__file__).resolve().parent
 LIB_PATH = _HERE / "_lib" / "libjaccpot_b200.so"
 
 JB_OK = 0
+JB_ERR_INDEX = 4
 ERRORS = {
     1: "invalid argument",
     2: "unsupported expansion order",

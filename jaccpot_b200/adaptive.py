@@ -42,7 +42,11 @@ class AdaptivePrepared:
     eps: float
     theta_max: float
     prepass_far_pairs: int
-    prepass_near_interactions: int
+    prepass_near: torch.Tensor  # int64 scalar on the device
+
+    @property
+    def prepass_near_interactions(self) -> int:
+        return int(self.prepass_near)
 
 
 def node_force_scale(ps: engine.Pass, acc4: torch.Tensor | None = None) -> torch.Tensor:
@@ -107,7 +111,7 @@ def prepare(positions, masses, *, leaf_size: int, orders, eps: float, theta_max:
             acc4[:, 0] = a[dt0.perm]
         fscale = node_force_scale(pre, acc4)
         power = node_dehnen_power(pre)
-        pre_far, pre_near = topo0.num_far_pairs, topo0.near_pair_interactions()
+        pre_far, pre_near = topo0.num_far_pairs, pre.near_pair_interactions()
         del pre, dt0
         dtree.adaptive_walk(power, fscale, G=G, eps=eps, theta_max=theta_max, gear_orders=orders)
         topo = dtree.topology()
@@ -115,7 +119,7 @@ def prepare(positions, masses, *, leaf_size: int, orders, eps: float, theta_max:
     dt.validate()
     ps = engine.Pass(dt, p_top, G=G, eps2=eps2, m2l_mode=m2l_mode, p2p_mode=p2p_mode, **pass_kw)
     if len(orders) > 1 and topo.num_far_pairs:
-        ps.set_gears(torch.from_numpy(topo.far_gears).to(dev), orders)
+        ps.set_gears(topo.device_arrays["far_gears"], orders)
     return AdaptivePrepared(topology=topo, device_topology=dt, pass_=ps, orders=orders, eps=float(eps),
                             theta_max=float(theta_max), prepass_far_pairs=pre_far,
-                            prepass_near_interactions=pre_near)
+                            prepass_near=pre_near)

@@ -915,17 +915,25 @@ const DBuf* sched_field(const jb_dsched* d, int field) {
 // ---------------------------------------------------------------------------
 __global__ void k_anc_count(int num_internal, int lo, int hi, const int* __restrict__ parent,
                             const int64_t* __restrict__ far_off, int* __restrict__ cnt, uint64_t* __restrict__ key,
-                            int* __restrict__ num_units) {
+                            int* __restrict__ num_units, int* __restrict__ lowest) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   const bool ok = lo + j < hi;
-  int c = 0;
+  int c = 0, top = num_internal;
   if (ok) {
-    for (int a = parent[num_internal + lo + j]; a >= 0; a = parent[a]) c += far_off[a + 1] > far_off[a];
+    for (int a = parent[num_internal + lo + j]; a >= 0; a = parent[a])
+      if (far_off[a + 1] > far_off[a]) {
+        ++c;
+        top = a;  // ids fall towards the root
+      }
     cnt[j] = c;
     key[j] = (uint64_t)(255 - c);  // a tree has fewer than 128 levels
   }
   const unsigned have = __ballot_sync(kFull, ok && c > 0);
-  if ((threadIdx.x & 31) == 0 && have) atomicAdd(num_units, __popc(have));
+  top = __reduce_min_sync(kFull, top);
+  if ((threadIdx.x & 31) == 0 && have) {
+    atomicAdd(num_units, __popc(have));
+    atomicMin(lowest, top);
+  }
 }
 
 __global__ void k_anc_fill(int num_internal, int lo, int hi, const int* __restrict__ parent,
@@ -951,16 +959,17 @@ void build_l2l(jb_dsched& d, int num_internal, int lo, int hi, const int* parent
   if (NL <= 0) return;
   Scratch s;
   ck(s.total.alloc(64));
-  int* d_tot = tot32(s);  // ancestors in all, units
+  int* d_tot = tot32(s);  // ancestors in all, units, lowest ancestor
   DBuf cnt, off, k0, k1, v0, v1;
   for (DBuf* b : {&cnt, &off, &v0, &v1}) ck(b->alloc((size_t)NL * 4));
   for (DBuf* b : {&k0, &k1}) ck(b->alloc((size_t)NL * 8));
   ck(cudaMemsetAsync(d_tot, 0, 8, st));
+  ck(cudaMemcpyAsync(d_tot + 2, &num_internal, 4, cudaMemcpyHostToDevice, st));
   k_anc_count<<<nblocks(NL, 128), 128, 0, st>>>(num_internal, lo, hi, parent, far_off, cnt.as<int>(),
-                                                k0.as<uint64_t>(), d_tot + 1);
+                                                k0.as<uint64_t>(), d_tot + 1, d_tot + 2);
   ck_launch();
   exclusive_scan<int>(cnt.as<int>(), off.as<int>(), NL, d_tot, s, st);
-  int tot[2];
+  int tot[3];
   ck(cudaMemcpyAsync(tot, d_tot, sizeof(tot), cudaMemcpyDeviceToHost, st));
   k_iota<<<nblocks(NL, 256), 256, 0, st>>>(v0.as<int>(), NL);
   ck_launch();
@@ -968,6 +977,7 @@ void build_l2l(jb_dsched& d, int num_internal, int lo, int hi, const int* parent
   ck(cudaStreamSynchronize(st));
   d.info.num_runs = tot[0];
   d.info.num_units = tot[1];
+  d.info.num_targets = tot[2];
   if (tot[1] == 0) return;
   ck(d.runs.alloc((size_t)tot[0] * 4));
   k_anc_fill<<<nblocks(NL, 128), 128, 0, st>>>(num_internal, lo, hi, parent, far_off, off.as<int>(), d.runs.as<int>());

@@ -23,7 +23,7 @@ from . import _lib
 from .schedule import (MixedGearM2LSchedule, gear_m2l_mixed_schedule, gear_m2l_mixed_schedule_device,
                        _run_device, gear_m2l_schedule, gear_m2l_schedule_device, leaf_schedule, leaf_schedule_device,
                        m2l_schedule, m2l_schedule_device, m2l_unit_limit, mixed_ladder, tc_m2l_schedule)
-from .tree import Topology
+from .tree import DeviceBuiltTopology, Topology
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -54,28 +54,80 @@ class DeviceTopology:
             raise ValueError("DeviceTopology needs a CUDA device (there is no CPU path)")
         self.topo = topo
         self.device = dev
-        up = lambda a, dt: torch.from_numpy(np.ascontiguousarray(a)).to(device=dev, dtype=dt)
-        self.node_ranges = up(topo.node_ranges.reshape(-1), torch.int32)
-        self.left = up(topo.left_child if topo.num_internal else np.zeros(1, np.int32), torch.int32)
-        self.right = up(topo.right_child if topo.num_internal else np.zeros(1, np.int32), torch.int32)
-        self.parent = up(topo.parent, torch.int32)
-        self.far_off = up(topo.far_offsets, torch.int64)
-        self.far_src = up(topo.far_sources if topo.num_far_pairs else np.zeros(1, np.int32), torch.int32)
+        # arrays of a tree built on this device are taken as they are, others
+        # are uploaded (a dummy word when empty, so no pointer is null)
+        built = topo.device_array if isinstance(topo, DeviceBuiltTopology) else (lambda name: None)
+        self.as_built = True  # every array as the device builder left it
+        here = torch.device(dev.type, torch.cuda.current_device() if dev.index is None else dev.index)
+
+        def up(name, dt, empty=False):
+            t = built(name)
+            if t is not None and t.device == here:
+                return t
+            self.as_built = False
+            a = np.zeros(1) if empty else np.ascontiguousarray(getattr(topo, name)).reshape(-1)
+            return torch.from_numpy(a).to(device=dev, dtype=dt)
+
+        no_internal, no_far = not topo.num_internal, not topo.num_far_pairs
+        self.node_ranges = up("node_ranges", torch.int32)
+        self.left = up("left_child", torch.int32, no_internal)
+        self.right = up("right_child", torch.int32, no_internal)
+        self.parent = up("parent", torch.int32)
+        self.far_off = up("far_offsets", torch.int64)
+        self.far_src = up("far_sources", torch.int32, no_far)
         # per-far-pair gear tags of an error-controlled walk (None: one order)
         self.far_gear = None
-        self.near_off = up(topo.near_offsets, torch.int64)
-        self.near_src = up(topo.near_leaves if topo.num_near_pairs else np.zeros(1, np.int32), torch.int32)
-        self.leaf_of = up(topo.leaf_of_particle, torch.int32)
-        self.perm = up(topo.permutation, torch.int64)
-        self.inv_perm = up(topo.inverse_permutation, torch.int64)
-        self.m2l_targets = up(topo.m2l_targets if topo.m2l_targets.size else np.zeros(1, np.int32), torch.int32)
-        self.num_m2l_targets = int(topo.m2l_targets.size)
+        self.near_off = up("near_offsets", torch.int64)
+        self.near_src = up("near_leaves", torch.int32, not topo.num_near_pairs)
+        self.leaf_of = up("leaf_of_particle", torch.int32)
+        self.perm = up("permutation", torch.int64)
+        self.inv_perm = up("inverse_permutation", torch.int64)
         self.level_offsets = [int(x) for x in topo.level_offsets]
-        # the L2L levels above the shallowest internal far target move zeros
-        # (every local there is zero): the sweep starts at that level
-        ni = topo.num_internal
-        tgt = np.nonzero(np.diff(np.asarray(topo.far_offsets))[:ni] > 0)[0]
-        self.l2l_first_level = int(np.asarray(topo.node_level)[tgt].min()) if tgt.size else int(topo.num_levels)
+        self._l2l_first = None
+
+    @property
+    def l2l_first_level(self) -> int:
+        """The shallowest level with an internal far target: the L2L levels above
+        it move zeros (every local there is zero), so the level-by-level sweep
+        starts there."""
+        if self._l2l_first is None:
+            ni = self.topo.num_internal
+            has = torch.nonzero(self.far_off[1:ni + 1] > self.far_off[:ni])[:1]
+            self.set_lowest_far_target(int(has[0]) if has.numel() else ni)
+        return self._l2l_first
+
+    def set_lowest_far_target(self, node: int) -> None:
+        """The lowest-numbered internal node with far pairs (the number of
+        internal nodes when there is none); ids rise with the level."""
+        levels = np.asarray(self.level_offsets[1:])
+        self._l2l_first = int(np.searchsorted(levels, node, side="right"))
+
+    @l2l_first_level.setter
+    def l2l_first_level(self, level: int) -> None:
+        self._l2l_first = int(level)
+
+    def far_pair_targets(self) -> torch.Tensor:
+        """int32 on the device: the target node of every far pair (a zero when
+        there is none)."""
+        n = self.topo.num_far_pairs
+        if not n:
+            return torch.zeros(1, dtype=torch.int32, device=self.device)
+        nodes = torch.arange(self.topo.num_nodes, dtype=torch.int32, device=self.device)
+        return torch.repeat_interleave(nodes, self.far_off[1:] - self.far_off[:-1], output_size=n)
+
+    def near_lists_symmetric(self) -> bool:
+        """True when leaf B is in A's neighbour list exactly when A is in B's
+        (jb_far_reverse_index over the near lists, whose rows ascend)."""
+        n = self.topo.num_near_pairs
+        if not n:
+            return True
+        rev = torch.empty(n, dtype=torch.int32, device=self.device)
+        rc = _lib.lib().jb_far_reverse_index(self.topo.num_leaves, _ptr(self.near_off), _ptr(self.near_src), _ptr(rev),
+                                             torch.cuda.current_stream(self.device).cuda_stream)
+        if rc == _lib.JB_ERR_INDEX:  # not symmetric, or rows of a caller's own that do not ascend
+            return self.topo.near_lists_symmetric()
+        _lib.check(rc, "jb_far_reverse_index(near)")
+        return True
 
     def far_reverse_index(self) -> torch.Tensor:
         """int32[num_far] on the device: the reverse pair (s <- t) of every far
@@ -95,6 +147,8 @@ class DeviceTopology:
     def validate(self) -> None:
         """Device-side range check of every list entry (jb_validate_lists)."""
         t = self.topo
+        if self.as_built and t.max_leaf_occupancy <= _lib.JB_MAX_LEAF_OCCUPANCY:
+            return  # the device builder's own lists, never outside this process's GPU
         bad = torch.zeros(1, dtype=torch.int32, device=self.device)
         _lib.check(_lib.lib().jb_validate_lists(
             t.num_nodes, t.num_internal, _ptr(self.left), _ptr(self.right), _ptr(self.far_off),
@@ -195,6 +249,8 @@ def l2l_leaf_schedule_device(dt: "DeviceTopology", leaf_range: tuple[int, int]):
         anc = field(_lib.JB_SCHED_RUNS, (info.num_runs,), np.int32)
     finally:
         free()
+    if (lo, hi) == (0, dt.topo.num_leaves):
+        dt.set_lowest_far_target(int(info.num_targets))
     return units, anc
 
 
@@ -372,6 +428,16 @@ class Pass:
         for name in ("_tc", "_tc_status", "_adj", "_adj_sched", "_adj_m2l", "_far_stream"):
             q.__dict__.pop(name, None)
         return q
+
+    def near_pair_interactions(self) -> torch.Tensor:
+        """int64 scalar on the device: the particle-particle interactions of the
+        near field (Topology.near_pair_interactions) of a whole-tree pass, from
+        its units' source counts."""
+        ni = self.dt.topo.num_internal
+        span = self.dt.node_ranges.view(-1, 2)[ni:]
+        count = (span[:, 1] - span[:, 0] + 1).long()
+        units = torch.as_tensor(self.leaf_sched.units).to(self.dt.device).long()
+        return (count[units[:, 0]] * units[:, 3]).sum() + (count * (count - 1)).sum()
 
     # -- stages -------------------------------------------------------------
     def load_particles(self, positions: torch.Tensor, masses: torch.Tensor, stream=None) -> None:
@@ -717,11 +783,11 @@ class Pass:
                 "mbar": torch.empty((t.num_nodes, cs), **f32),
                 "cbar4": torch.empty((t.num_nodes, 4), **f32),
                 "g4": torch.empty((max(t.num_far_pairs, 1), 4), **f32),
-                "pair_tgt": torch.from_numpy(t.far_pair_targets() if t.num_far_pairs else np.zeros(1, np.int32)).to(dev),
+                "pair_tgt": self.dt.far_pair_targets(),
                 "rev": (self.dt.far_reverse_index() if _on_gpu(self.dt) and t.num_far_pairs else
                         torch.from_numpy(t.far_reverse_index() if t.num_far_pairs else np.zeros(1, np.int32)).to(dev)),
             }
-            if not t.near_lists_symmetric():
+            if not (self.dt.near_lists_symmetric() if _on_gpu(self.dt) else t.near_lists_symmetric()):
                 raise ValueError("the near-field adjoint needs symmetric neighbour lists")
             # full near list of every leaf (the forward schedule may be a leaf range)
             self._adj_sched = (leaf_schedule_device(self.dt, max_sources=4096) if _on_gpu(self.dt)

@@ -84,8 +84,9 @@ class GearContext:
         t = ps.dt.topo
         dev = ps.dt.device
         self.ps = ps
-        self.radii = torch.from_numpy(t.radii_f64.astype(np.float32)).to(dev)
-        self.pair_tgt = torch.from_numpy(t.far_pair_targets() if t.num_far_pairs else np.zeros(1, np.int32)).to(dev)
+        radii = t.device_array("radii_f64") if isinstance(t, tree.DeviceBuiltTopology) else None
+        self.radii = (torch.from_numpy(t.radii_f64).to(dev) if radii is None else radii.to(dev)).float()
+        self.pair_tgt = ps.dt.far_pair_targets()
         self.node_feat = torch.empty((t.num_nodes, 8), device=dev, dtype=torch.float32)
         self.scale = torch.empty((t.num_nodes,), device=dev, dtype=torch.float32)
         self.h_levels = np.ascontiguousarray(t.level_offsets.astype(np.int32))

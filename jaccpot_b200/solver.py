@@ -22,7 +22,7 @@ import torch
 
 from . import _lib
 from .engine import DeviceTopology, Pass
-from .tree import Topology, build_topology
+from .tree import DeviceBuiltTopology, Topology, build_topology
 
 # Preset defaults: (theta, leaf_size hint); solver.py:27-118 + config.py presets.
 _PRESETS = {"fast": 0.6, "balanced": 0.6, "accurate": 0.5, "large_n_gpu": 0.6}
@@ -250,9 +250,10 @@ class FastMultipoleMethod:
         if runtime_overrides_override is not None:
             raise ValueError("runtime_overrides_override is not provided")
         th = self.theta if theta is None else float(theta)
-        pos_np = positions.detach().cpu().numpy() if isinstance(positions, torch.Tensor) else np.asarray(positions)
-        mass_np = masses.detach().cpu().numpy() if isinstance(masses, torch.Tensor) else np.asarray(masses)
-        if pos_np.ndim != 2 or pos_np.shape[1] != 3 or mass_np.shape != (pos_np.shape[0],):
+        positions = positions.detach() if isinstance(positions, torch.Tensor) else np.asarray(positions)
+        masses = masses.detach() if isinstance(masses, torch.Tensor) else np.asarray(masses)
+        n = positions.shape[0] if positions.ndim == 2 else -1
+        if tuple(positions.shape) != (n, 3) or tuple(masses.shape) != (n,):
             raise ValueError("positions must be (N, 3) and masses (N,)")
         self._counters["prepare_state"] += 1
         if self.adaptive_error_model == "dehnen_paper":
@@ -261,9 +262,8 @@ class FastMultipoleMethod:
             raise ValueError("force_scale_nodes applies to adaptive_error_model='dehnen_paper'")
         # tree + lists on the GPU when the solver runs there (the same arrays
         # as the host build, bit for bit), else on the host
-        topo = build_topology(positions if isinstance(positions, torch.Tensor) else pos_np,
-                              masses if isinstance(masses, torch.Tensor) else mass_np, leaf_size=int(leaf_size),
-                              theta=th, device=self.device if self.device.type == "cuda" else None)
+        topo = build_topology(positions, masses, leaf_size=int(leaf_size), theta=th,
+                              device=self.device if self.device.type == "cuda" else None)
         return self._prepare_from_topology(topo, positions, masses, int(max_order), th, int(leaf_size))
 
     def _prepare_adaptive(self, positions, masses, leaf_size: int, max_order: int, th: float,
@@ -391,8 +391,11 @@ class FastMultipoleMethod:
                 stats["miss_topology"] += 1
                 topo = nt.topology()
             else:
-                centers = nt.field("centers_f64").reshape(-1, 3).cpu().numpy()
-                radii = nt.field("radii_f64").cpu().numpy()
+                if isinstance(t, DeviceBuiltTopology):
+                    moved = t.with_geometry(nt.field("centers_f64").clone(), nt.field("radii_f64").clone())
+                else:
+                    moved = replace(t, centers_f64=nt.field("centers_f64").reshape(-1, 3).cpu().numpy(),
+                                    radii_f64=nt.field("radii_f64").cpu().numpy())
         if not same:
             return self._prepare_from_topology(topo, positions, masses, order, th, leaf)
         stats["hits"] += 1
@@ -406,8 +409,7 @@ class FastMultipoleMethod:
             _gears.apply_gears(ps, model)
         ps.upward()
         ps.downward()
-        new = FMMPreparedState(topology=replace(t, centers_f64=centers, radii_f64=radii), device_topology=dt,
-                               pass_=ps, max_order=st.max_order, theta=st.theta, leaf_size=st.leaf_size,
+        new = FMMPreparedState(topology=moved, device_topology=dt, pass_=ps, max_order=st.max_order, theta=st.theta, leaf_size=st.leaf_size,
                                num_particles=st.num_particles,
                                input_dtype=positions.dtype if hasattr(positions, "dtype") else np.float64)
         self._last_state = new

@@ -9,6 +9,7 @@ jaccpot/runtime/fmm_state.py:870-897 for the state that carries them.
 
 from __future__ import annotations
 
+import copy
 import ctypes
 from dataclasses import dataclass, field
 
@@ -93,9 +94,92 @@ class Topology:
         return int((per_edge_t * src_cnt).sum() + (leaf_cnt * (leaf_cnt - 1)).sum())
 
 
+class _OnFirstRead:
+    """A DeviceBuiltTopology field that Topology gives a default: the instance's
+    own value, else the one brought from the device."""
+
+    def __set_name__(self, owner, name):
+        self.name = name
+
+    def __get__(self, obj, owner=None):
+        return None if obj is None else obj._host(self.name)
+
+    def __set__(self, obj, value):
+        obj.__dict__[self.name] = value
+
+
+class DeviceBuiltTopology(Topology):
+    """A Topology whose arrays are on the GPU (``device_arrays``, torch tensors
+    that own their memory) and come to the host one by one, when they are first
+    read as numpy arrays; from then on the host's array is the field.  An
+    evaluation needs only the sizes and the level offsets there: at clustered
+    1M the copies down and up again were 35 of the 52 ms that the GPU was busy
+    in a call on new particles, and most of the host's 140 ms."""
+
+    m2l_targets = _OnFirstRead()
+    far_gears = _OnFirstRead()
+    gear_orders = None
+
+    @staticmethod
+    def of(n: int, info, arrays: dict, level_offsets: np.ndarray, leaf_size: int, theta: float,
+           gear_orders=None) -> "DeviceBuiltTopology":
+        t = object.__new__(DeviceBuiltTopology)
+        t.num_particles = n
+        for name in ("num_nodes", "num_internal", "num_leaves", "num_levels", "max_leaf_occupancy"):
+            setattr(t, name, int(getattr(info, name)))
+        t.leaf_size, t.theta = int(leaf_size), float(theta)
+        t.level_offsets = level_offsets
+        t.gear_orders = None if gear_orders is None else tuple(int(o) for o in gear_orders)
+        t.device_arrays = arrays
+        t._sizes = _field_sizes(n, info)
+        return t
+
+    @property
+    def num_far_pairs(self) -> int:
+        return int(self.far_sources.shape[0]) if "far_sources" in self.__dict__ else self._sizes["far_sources"]
+
+    @property
+    def num_near_pairs(self) -> int:
+        return int(self.near_leaves.shape[0]) if "near_leaves" in self.__dict__ else self._sizes["near_leaves"]
+
+    def device_array(self, name: str):
+        """The field's tensor, with at least one element; None when the field has
+        been read on the host, whose array then counts."""
+        return None if name in self.__dict__ else self.__dict__.get("device_arrays", {}).get(name)
+
+    def with_geometry(self, centers_f64, radii_f64) -> "DeviceBuiltTopology":
+        """The same tree and lists with other centres and radii (device tensors)."""
+        t = copy.copy(self)
+        for name in ("centers_f64", "radii_f64"):
+            t.__dict__.pop(name, None)
+        t.device_arrays = dict(self.device_arrays, centers_f64=centers_f64, radii_f64=radii_f64)
+        return t
+
+    def _host(self, name: str):
+        d = self.__dict__
+        if name not in d:
+            if name == "m2l_targets":
+                d[name] = _m2l_targets(self.far_offsets)
+            elif name not in d.get("device_arrays", {}):  # far_gears without an error-controlled walk
+                return None
+            else:
+                a = d["device_arrays"][name][:self._sizes[name]].cpu().numpy()
+                d[name] = a.reshape({"node_ranges": (-1, 2), "centers_f64": (-1, 3)}.get(name, (-1,)))
+        return d[name]
+
+    def __getattr__(self, name: str):  # a field that the instance does not hold yet
+        if name in _LAZY_FIELDS and "device_arrays" in self.__dict__:
+            return self._host(name)
+        raise AttributeError(name)
+
+
+_LAZY_FIELDS = frozenset(_lib.DTREE_FIELDS) - {"level_offsets", "far_gears"}
+
+
 def _field_sizes(n: int, info) -> dict:
     return {
         "permutation": n,
+        "inverse_permutation": n,
         "node_ranges": 2 * info.num_nodes,
         "left_child": info.num_internal,
         "right_child": info.num_internal,
@@ -113,11 +197,11 @@ def _field_sizes(n: int, info) -> dict:
     }
 
 
-def _copy_fields(copy_fn, handle, n: int, info, with_gears: bool = False) -> dict:
+def _copy_fields(copy_fn, handle, n: int, info) -> dict:
     sizes = _field_sizes(n, info)
     arrs = {}
     for name, (fid, dt) in _lib.TREE_FIELDS.items():
-        if name == "far_gears" and not with_gears:
+        if name == "far_gears":  # error-controlled walks run on the GPU only
             continue
         a = np.empty(max(sizes[name], 1), dtype=dt)
         _lib.check(copy_fn(handle, fid, a.ctypes.data), f"tree field copy ({name})")
@@ -125,13 +209,17 @@ def _copy_fields(copy_fn, handle, n: int, info, with_gears: bool = False) -> dic
     return arrs
 
 
-def _topology(n: int, info, arrs: dict, leaf_size: int, theta: float, gear_orders=None) -> Topology:
+def _m2l_targets(far_offsets: np.ndarray) -> np.ndarray:
+    """int32: the nodes with at least one far pair, longest list first (stable)."""
+    counts = np.diff(far_offsets)
+    tg = np.nonzero(counts)[0]
+    return tg[np.argsort(-counts[tg], kind="stable")].astype(np.int32)
+
+
+def _topology(n: int, info, arrs: dict, leaf_size: int, theta: float) -> Topology:
     perm = arrs["permutation"]
     inv = np.empty_like(perm)
     inv[perm] = np.arange(n, dtype=np.int64)
-    counts = np.diff(arrs["far_offsets"])
-    tg = np.nonzero(counts)[0]
-    order = np.argsort(-counts[tg], kind="stable")
     return Topology(
         num_particles=n,
         num_nodes=info.num_nodes,
@@ -156,9 +244,7 @@ def _topology(n: int, info, arrs: dict, leaf_size: int, theta: float, gear_order
         near_leaves=arrs["near_leaves"],
         centers_f64=arrs["centers_f64"].reshape(-1, 3),
         radii_f64=arrs["radii_f64"],
-        m2l_targets=tg[order].astype(np.int32),
-        far_gears=arrs.get("far_gears"),
-        gear_orders=None if gear_orders is None else tuple(int(o) for o in gear_orders),
+        m2l_targets=_m2l_targets(arrs["far_offsets"]),
     )
 
 
@@ -168,8 +254,9 @@ def build_topology(positions, masses, *, leaf_size: int = 16, theta: float = 0.6
     a CUDA device."""
     if device is not None and str(device).startswith("cuda"):
         return build_topology_device(positions, masses, leaf_size=leaf_size, theta=theta, device=device)
-    pos = np.ascontiguousarray(np.asarray(positions, dtype=np.float64).reshape(-1, 3))
-    mass = np.ascontiguousarray(np.asarray(masses, dtype=np.float64).reshape(-1))
+    host = lambda a: a.detach().cpu().numpy() if hasattr(a, "detach") else a
+    pos = np.ascontiguousarray(np.asarray(host(positions), dtype=np.float64).reshape(-1, 3))
+    mass = np.ascontiguousarray(np.asarray(host(masses), dtype=np.float64).reshape(-1))
     n = pos.shape[0]
     if mass.shape[0] != n:
         raise ValueError("positions and masses disagree in length")
@@ -184,6 +271,12 @@ def build_topology(positions, masses, *, leaf_size: int = 16, theta: float = 0.6
     finally:
         lb.jb_tree_free(h)
     return _topology(n, info, arrs, leaf_size, theta)
+
+
+def _torch_dtype(dtype):
+    import torch
+
+    return {"int32": torch.int32, "int64": torch.int64, "float64": torch.float64}[np.dtype(dtype).name]
 
 
 def device_view(ptr, shape, dtype, device):
@@ -207,8 +300,8 @@ class DeviceTree:
     """Owner of a ``jb_tree_build_device`` handle: the tree and lists of a
     particle set, resident on the GPU.  ``field(name)`` is a zero-copy torch
     view of one array (valid while the handle lives); ``topology()`` copies
-    everything back into a :class:`Topology`.  Use as a context manager or
-    call ``free()``."""
+    everything into tensors of its own, as a :class:`DeviceBuiltTopology`.
+    Use as a context manager or call ``free()``."""
 
     def __init__(self, positions, masses, *, leaf_size: int = 16, theta: float = 0.6, device="cuda"):
         import torch
@@ -252,12 +345,36 @@ class DeviceTree:
         self.gear_orders = tuple(int(o) for o in orders)
 
     def field(self, name: str):
-        fid, dt = _lib.TREE_FIELDS[name]
+        fid, dt = _lib.DTREE_FIELDS[name]
         return device_view(self._lb.jb_dtree_field(self._h, fid), (self.sizes[name],), dt, self.device)
 
-    def topology(self) -> Topology:
-        arrs = _copy_fields(self._lb.jb_dtree_copy, self._h, self.n, self.info, with_gears=self.gear_orders is not None)
-        return _topology(self.n, self.info, arrs, self.leaf_size, self.theta, self.gear_orders)
+    def topology(self) -> DeviceBuiltTopology:
+        """Tree and lists in one device buffer that the topology owns (copied
+        in stream order, one call); only the level offsets come to the host."""
+        torch = self._torch
+        names = [f for f in _lib.DTREE_FIELDS if f != "far_gears" or self.gear_orders is not None]
+        at, spans = 0, {}
+        for f in names:
+            dtype = np.dtype(_lib.DTREE_FIELDS[f][1])
+            count = max(self.sizes[f], 1)  # an empty field keeps a word, so that its pointer is never null
+            spans[f] = (at, count, dtype)
+            at += (count * dtype.itemsize + 255) & ~255
+        buf = torch.empty(at, dtype=torch.uint8, device=self.device)
+        base = buf.data_ptr()
+        ids = np.array([_lib.DTREE_FIELDS[f][0] for f in names], dtype=np.int32)
+        dst = np.array([base + spans[f][0] for f in names], dtype=np.uint64)
+        stream = torch.cuda.current_stream(self.device).cuda_stream
+        _lib.check(self._lb.jb_dtree_export(self._h, len(names), ids.ctypes.data, dst.ctypes.data, stream),
+                   "jb_dtree_export")
+        arrays = {f: buf[o:o + c * d.itemsize].view(_torch_dtype(d)) for f, (o, c, d) in spans.items()}
+        for f in names:
+            if self.sizes[f] == 0:
+                arrays[f].zero_()
+        offsets = np.empty(self.info.num_levels + 1, dtype=np.int32)
+        _lib.check(self._lb.jb_dtree_copy(self._h, _lib.DTREE_FIELDS["level_offsets"][0], offsets.ctypes.data),
+                   "tree field copy (level_offsets)")
+        return DeviceBuiltTopology.of(self.n, self.info, arrays, offsets, self.leaf_size, self.theta,
+                                      self.gear_orders)
 
     def free(self) -> None:
         if self._h:
@@ -279,8 +396,7 @@ class DeviceTree:
 
 def build_topology_device(positions, masses, *, leaf_size: int = 16, theta: float = 0.6, device="cuda") -> Topology:
     """The tree and lists built on the GPU by ``jb_tree_build_device``
-    (csrc/tree_gpu.cu) from float64 copies of the inputs on ``device``; the
-    arrays are copied back into the same :class:`Topology` the host build
-    returns."""
+    (csrc/tree_gpu.cu) from float64 copies of the inputs on ``device``: the
+    host build's :class:`Topology`, its arrays copied to the host when read."""
     with DeviceTree(positions, masses, leaf_size=leaf_size, theta=theta, device=device) as dtree:
         return dtree.topology()
