@@ -242,6 +242,15 @@ JB_API int jb_far_reverse_index(int num_nodes, const int64_t* far_off, const int
  * there is none): the sweep by levels starts at its level.                  */
 JB_API int jb_l2l_schedule_device(int num_internal, int leaf_lo, int leaf_hi, const int* parent, const int64_t* far_off,
                                   void* stream, jb_dsched** out);
+/* Items of jb_m2m_hops: JB_SCHED_AUX holds int32[num_units][2] (node, source;
+ * -1 where a place is empty), hop k's in [hop_offsets[k], hop_offsets[k + 1]),
+ * both multiples of 32.  The lowest single_levels (0 to 16) heights above the
+ * leaves have a hop each, the others one for four.  hop_offsets is host memory
+ * for JB_MAX_M2M_HOPS + 1 values, *num_hops the hops used.                  */
+#define JB_MAX_M2M_HOPS 64
+JB_API int jb_m2m_schedule_device(int num_nodes, int num_internal, const int* parent, const int* left,
+                                  const int* right, int single_levels, int64_t* hop_offsets, int* num_hops,
+                                  void* stream, jb_dsched** out);
 JB_API int jb_dsched_info(const jb_dsched* d, jb_sched_info_t* info);
 JB_API const void* jb_dsched_field(const jb_dsched* d, int field);
 JB_API void jb_dsched_free(jb_dsched* d);
@@ -326,6 +335,12 @@ JB_API int jb_p2m(int p, const float* pos4, int num_nodes, int num_internal, con
  * aggregate_m2m_real_by_level, upward/real_tree_expansions.py:216-364). */
 JB_API int jb_m2m_level(int p, int first, int last, const int* left, const int* right, const int* node_ranges,
                         float* centers, float* mult, void* stream);
+
+/* Upward sweep after jb_p2m over the items of jb_m2m_schedule_device: what
+ * jb_m2m_level gives level by level, deepest first (to FP32 rounding: a node
+ * takes its sources four levels down at once).  hop_offsets: host memory.   */
+JB_API int jb_m2m_hops(int p, int num_hops, const int64_t* hop_offsets, const int* items, const int* node_ranges,
+                       float* centers, float* mult, void* stream);
 
 /* Far field (M2L + accumulation) over work units.  units is int4[num_units]:
  * (target node, first pair, end pair, slot) with pairs indexing far_src (the

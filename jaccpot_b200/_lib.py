@@ -32,6 +32,7 @@ JB_P2P_NEAR_FIRST, JB_P2P_FAR_AFTER = 16, 32
 JB_LEAF_EVAL_NOALLOC_MAX_SLOTS = 16384
 JB_MAX_LEAF_OCCUPANCY = 64
 JB_MIXED_GEAR_SEGMENTS = 4
+JB_MAX_M2M_HOPS = 64
 JB_LEAF_ERR_OCCUPANCY, JB_LEAF_ERR_SLOT = 1, 2
 (JB_SCHED_UNITS, JB_SCHED_AUX, JB_SCHED_RUNS, JB_SCHED_SPLIT, JB_SCHED_FAR_SOURCES, JB_SCHED_GEAR_OFFSETS,
  JB_SCHED_TARGETS, JB_SCHED_PAIRS_PER_GEAR) = range(8)
@@ -94,6 +95,8 @@ _SIGNATURES = {
     "jb_dtree_copy": [_P, _I, _P],
     "jb_dtree_free": [_P],
     "jb_dtree_export": [_P, _I, _P, _P, _P],
+    "jb_m2m_schedule_device": [_I, _I, _P, _P, _P, _I, _P, ctypes.POINTER(_I), _P, ctypes.POINTER(_P)],
+    "jb_m2m_hops": [_I, _I, _P, _P, _P, _P, _P, _P],
     "jb_l2l_schedule_device": [_I, _I, _I, _P, _P, _P, ctypes.POINTER(_P)],
     "jb_dtree_adaptive_walk": [_P, _I, _P, _P, _D, _D, _D, _I, _P, _P],
     "jb_node_dehnen_power": [_I, _I, _P, _I, _P, _P],

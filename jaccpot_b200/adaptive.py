@@ -112,11 +112,13 @@ def prepare(positions, masses, *, leaf_size: int, orders, eps: float, theta_max:
         fscale = node_force_scale(pre, acc4)
         power = node_dehnen_power(pre)
         pre_far, pre_near = topo0.num_far_pairs, pre.near_pair_interactions()
+        hops = dt0.m2m_hops() if pre.m2m_hops else None  # of the tree, which both lists share
         del pre, dt0
         dtree.adaptive_walk(power, fscale, G=G, eps=eps, theta_max=theta_max, gear_orders=orders)
         topo = dtree.topology()
     dt = engine.DeviceTopology(topo, dev)
     dt.validate()
+    dt.share_m2m_hops(hops)
     ps = engine.Pass(dt, p_top, G=G, eps2=eps2, m2l_mode=m2l_mode, p2p_mode=p2p_mode, **pass_kw)
     if len(orders) > 1 and topo.num_far_pairs:
         ps.set_gears(topo.device_arrays["far_gears"], orders)

@@ -501,6 +501,14 @@ JB_API int jb_m2m_level(int p, int first, int last, const int* left, const int* 
   return dispatch<RunM2M>(p, first, last, left, right, node_ranges, centers, mult, ST(stream));
 }
 
+JB_API int jb_m2m_hops(int p, int num_hops, const int64_t* hop_offsets, const int* items, const int* node_ranges,
+                       float* centers, float* mult, void* stream) {
+  if (num_hops < 0 || num_hops > JB_MAX_M2M_HOPS ||
+      (num_hops > 0 && (!hop_offsets || !items || !node_ranges || !centers || !mult)))
+    return JB_ERR_ARG;
+  return dispatch<RunM2MHops>(p, num_hops, hop_offsets, items, node_ranges, centers, mult, ST(stream));
+}
+
 JB_API int jb_m2l(int p, int mode, int num_units, const int* units, const float* mult, const float* centers,
                   const int* far_src, float* locals, float* partials, int num_split, const int* split,
                   void* stream) {

@@ -769,6 +769,125 @@ __global__ void __launch_bounds__(128) k_m2m_level_split(int first, int last, co
   }
 }
 
+// ---------------------------------------------------------------------------
+// M2M by hops of four levels (jb_m2m_schedule_device): a node is formed at once
+// from its up to 16 descendants four levels below.  M2M to a farther ancestor
+// is as exact as M2M to the parent, so the result is that of the sweep by
+// levels; there are 1.1 to 2.2 times as many translations, in a third of the
+// launches.  The levels of a small tree are bound by their number, not their
+// work (25 to 40 of 2 to 5 us each, nearly all of it launch, cold code and one
+// chain): Plummer 65k p=6 91 -> 45 us with the P2M, clustered 10k p=4 80 -> 33.
+// Block and warps as in k_m2m_level_split: lane = item (node,
+// source), a warp per degree set; the items of a node are aligned to their
+// number (2 to 16), so that butterflies over the lanes with the same node add
+// them, and its first lane writes it.  The node's centre is the sources' centre
+// of mass.  ADJ: rows move from source to node by M2M(c_node - c_source) about
+// given centres (the adjoint of the L2L).
+// ---------------------------------------------------------------------------
+template <int P, unsigned MASK, bool ADJ>
+__device__ __forceinline__ void m2m_hop_warp(const int2* __restrict__ items, const int2* __restrict__ ranges,
+                                             float4* __restrict__ centers, float* __restrict__ rows, float* xr,
+                                             bool first_warp) {
+  constexpr int C = csize(P), CS = cstride(P);
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int2 it = items[(size_t)blockIdx.x * kSplitItems + lane];
+  const int dst = it.x, src = it.y;
+  const float4 cs = src >= 0 ? centers[src] : make_float4(0.f, 0.f, 0.f, 0.f);
+  float v[C];
+  const float* row = rows + (size_t)(src >= 0 ? src : 0) * CS;
+  ForDeg<P, MASK>::run([&](auto lc) {
+    constexpr int L = decltype(lc)::value;
+#pragma unroll
+    for (int m = -L; m <= L; ++m) v[shi(L, m)] = src >= 0 ? row[shi(L, m)] : 0.f;
+  });
+  const int before = __shfl_up_sync(kAll, dst, 1);
+  const bool head = dst >= 0 && (lane == 0 || before != dst);
+  bool same[4];  // the lane 1, 2, 4, 8 places over holds the same node
+  unsigned any[4];
+#pragma unroll
+  for (int o = 0; o < 4; ++o) {
+    same[o] = __shfl_xor_sync(kAll, dst, 1 << o) == dst && dst >= 0;
+    any[o] = __ballot_sync(kAll, same[o]);
+  }
+  auto gather = [&](float x) {
+#pragma unroll
+    for (int o = 0; o < 4; ++o)
+      if (any[o]) {
+        const float y = __shfl_xor_sync(kAll, x, 1 << o);
+        x += same[o] ? y : 0.f;
+      }
+    return x;
+  };
+  float4 c;
+  if (ADJ) {
+    c = dst >= 0 ? centers[dst] : cs;
+  } else {
+    // offsets from the node's first source, so that the sums round at the
+    // node's size and not at its distance from the origin
+    const int first = 31 - __clz(__ballot_sync(kAll, head) & (kAll >> (31 - lane)));
+    const float ox = __shfl_sync(kAll, cs.x, first & 31), oy = __shfl_sync(kAll, cs.y, first & 31),
+                oz = __shfl_sync(kAll, cs.z, first & 31);
+    const float x = cs.x - ox, y = cs.y - oy, z = cs.z - oz;
+    const float m = gather(cs.w);
+    c = make_float4(gather(cs.w * x), gather(cs.w * y), gather(cs.w * z), m);
+    float inv = m > 0.f ? 1.f / m : 0.f;
+    if (__any_sync(kAll, !(m > 0.f))) {  // no mass below: the mean particle position (k_m2m_level)
+      const float k = src >= 0 ? (float)(ranges[src].y - ranges[src].x + 1) : 0.f;
+      const float n = gather(k), nx = gather(k * x), ny = gather(k * y), nz = gather(k * z);
+      if (!(m > 0.f)) {
+        c = make_float4(nx, ny, nz, 0.f);
+        inv = n > 0.f ? 1.f / n : 0.f;
+      }
+    }
+    c = make_float4(fmaf(c.x, inv, ox), fmaf(c.y, inv, oy), fmaf(c.z, inv, oz), c.w);
+  }
+  const float sg = ADJ ? -1.f : 1.f;
+  split_translate<P, MASK, true>(v, sg * (cs.x - c.x), sg * (cs.y - c.y), sg * (cs.z - c.z), xr);
+  float* out = rows + (size_t)(dst >= 0 ? dst : 0) * CS;
+  ForDeg<P, MASK>::run([&](auto lc) {
+    constexpr int L = decltype(lc)::value;
+#pragma unroll
+    for (int m = -L; m <= L; ++m) {
+      const float x = gather(v[shi(L, m)]);
+      if (head) out[shi(L, m)] = x;
+    }
+  });
+  if (head && first_warp) {
+    if (!ADJ) centers[dst] = c;
+#pragma unroll
+    for (int k = C; k < CS; ++k) out[k] = 0.f;
+  }
+}
+
+template <int P, bool ADJ>
+__global__ void __launch_bounds__(128) k_m2m_hop(const int2* __restrict__ items, const int2* __restrict__ ranges,
+                                                 float4* __restrict__ centers, float* __restrict__ rows) {
+  __shared__ float xs[kSplitItems * xrow(P)];
+  float* xr = xs + (threadIdx.x & 31) * xrow(P);
+  switch (threadIdx.x >> 5) {
+    case 0: m2m_hop_warp<P, kDegSet(P, 0), ADJ>(items, ranges, centers, rows, xr, true); break;
+    case 1: m2m_hop_warp<P, kDegSet(P, 1), ADJ>(items, ranges, centers, rows, xr, false); break;
+    case 2: m2m_hop_warp<P, kDegSet(P, 2), ADJ>(items, ranges, centers, rows, xr, false); break;
+    default: m2m_hop_warp<P, kDegSet(P, 3), ADJ>(items, ranges, centers, rows, xr, false); break;
+  }
+}
+
+template <int P, bool ADJ>
+int launch_hops(int num_hops, const int64_t* off, const int* items, const int* ranges, const float* centers, float* rows,
+                cudaStream_t st) {
+  for (int h = 0; h < num_hops; ++h) {
+    const int64_t n = off[h + 1] - off[h];
+    if (n <= 0) continue;
+    k_m2m_hop<P, ADJ><<<(unsigned)(n / kSplitItems), 128, 0, st>>>(
+        reinterpret_cast<const int2*>(items) + off[h], reinterpret_cast<const int2*>(ranges),
+        reinterpret_cast<float4*>(const_cast<float*>(centers)), rows);
+    const int rc = launch_status();
+    if (rc) return rc;
+  }
+  return JB_OK;
+}
+
 template <int P, unsigned MASK>
 __device__ __forceinline__ void l2l_split_warp(int first, int last, const int* __restrict__ left,
                                                const int* __restrict__ right, const float4* __restrict__ centers,
@@ -1627,6 +1746,18 @@ int RunM2M<P>::run(int first, int last, const int* left, const int* right, const
 }
 
 template <int P>
+struct RunM2MHops {
+  static int run(int num_hops, const int64_t* off, const int* items, const int* ranges, float* centers, float* mult,
+                 cudaStream_t st);
+};
+
+template <int P>
+int RunM2MHops<P>::run(int num_hops, const int64_t* off, const int* items, const int* ranges, float* centers,
+                       float* mult, cudaStream_t st) {
+  return launch_hops<P, false>(num_hops, off, items, ranges, centers, mult, st);
+}
+
+template <int P>
 struct RunM2L {
   static int run(int num_units, const int* units, const float* mult, const float* centers, const int* far_src,
                  float* locals, float* partials, int num_split, const int* split, cudaStream_t st, bool neg = false,
@@ -1830,6 +1961,7 @@ int RunTargets<P>::run(const float* pos4, int num_internal, const int* ranges, c
 #define JB_DECLARE_ORDER(PP)                 \
   extern template struct jb::RunP2M<PP>;      \
   extern template struct jb::RunM2M<PP>;      \
+  extern template struct jb::RunM2MHops<PP>;  \
   extern template struct jb::RunM2L<PP>;      \
   extern template struct jb::RunM2LMixed<PP>; \
   extern template struct jb::RunL2L<PP>;      \

@@ -7,6 +7,7 @@
 
 template struct jb::RunP2M<JB_ORDER>;
 template struct jb::RunM2M<JB_ORDER>;
+template struct jb::RunM2MHops<JB_ORDER>;
 template struct jb::RunM2L<JB_ORDER>;
 template struct jb::RunM2LMixed<JB_ORDER>;
 template struct jb::RunL2L<JB_ORDER>;

@@ -988,6 +988,144 @@ void build_l2l(jb_dsched& d, int num_internal, int lo, int hi, const int* parent
   ck_launch();
 }
 
+// ---------------------------------------------------------------------------
+// M2M hops.  The heights (leaves 0) are cut into bands, the lowest `singles`
+// of one height, the others of kHopLevels.  A node is formed in its band's hop
+// from its descendants below the band whose parents are in it: at most
+// 2^kHopLevels of them, all finished by the hops before.  A hop's items (node, source) are padded to 2, 4, 8 or 16 per
+// node and laid out largest first, so that a node's items are aligned to their
+// number and never cross the 32 items that a block of the sweep takes.
+// ---------------------------------------------------------------------------
+constexpr int kHopLevels = 4, kHopMost = 1 << kHopLevels;
+constexpr int kHopClasses = kHopLevels;  // padded sizes kHopMost, ..., 4, 2
+
+struct HopBands {
+  int singles;
+  __device__ __forceinline__ int hop(int h) const { return h <= singles ? h - 1 : singles + (h - singles - 1) / kHopLevels; }
+  // the greatest height below h's band
+  __device__ __forceinline__ int below(int h) const {
+    return h <= singles ? h - 1 : singles + (h - singles - 1) / kHopLevels * kHopLevels;
+  }
+};
+
+// Thread per leaf climbing: the second child to arrive knows both heights.
+__global__ void k_node_heights(int num_internal, int num_nodes, const int* __restrict__ parent, int* height,
+                               int* arrived) {
+  int node = num_internal + blockIdx.x * blockDim.x + threadIdx.x;
+  if (node >= num_nodes) return;
+  height[node] = 0;
+  for (int h = 0;;) {
+    node = parent[node];
+    if (node < 0) return;
+    atomicMax(height + node, h + 1);
+    __threadfence();  // this child's height before its arrival
+    if (atomicAdd(arrived + node, 1) == 0) return;
+    __threadfence();
+    h = atomicMax(height + node, 0);
+  }
+}
+
+// Calls f(source) for the sources of internal node i, left to right.
+template <typename F>
+__device__ __forceinline__ void hop_sources(int i, const int* __restrict__ left, const int* __restrict__ right,
+                                            const int* __restrict__ height, HopBands bands, F&& f) {
+  const int limit = bands.below(height[i]);
+  int stack[kHopLevels + 2], top = 0;
+  stack[top++] = i;
+  while (top > 0) {
+    const int x = stack[--top];
+    if (x != i && height[x] <= limit) {
+      f(x);
+      continue;
+    }
+    stack[top++] = right[x];
+    stack[top++] = left[x];
+  }
+}
+
+__global__ void k_hop_keys(int num_internal, const int* __restrict__ left, const int* __restrict__ right,
+                           const int* __restrict__ height, HopBands bands, uint64_t* __restrict__ key,
+                           int* __restrict__ idx, int* __restrict__ bins) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= num_internal) return;
+  int n = 0;
+  hop_sources(i, left, right, height, bands, [&](int) { ++n; });
+  int cls = 0;  // padded size kHopMost >> cls
+  while ((kHopMost >> (cls + 1)) >= n) ++cls;
+  const int k = bands.hop(height[i]) * kHopClasses + cls;  // heights below 128, at most 16 singles: under 192 keys
+  key[i] = (uint64_t)k;
+  idx[i] = i;
+  atomicAdd(bins + k, 1);
+}
+
+constexpr int kHopKeys = 256;
+struct HopLayout {
+  int first[kHopKeys];  // place of the key's first node in key order
+  int item[kHopKeys];   // its first item
+};
+
+__global__ void k_hop_items(int num_internal, const uint64_t* __restrict__ key, const int* __restrict__ idx, HopLayout h,
+                            const int* __restrict__ left, const int* __restrict__ right,
+                            const int* __restrict__ height, HopBands bands, int2* __restrict__ items) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= num_internal) return;
+  const int k = (int)key[r], i = idx[r], size = kHopMost >> (k % kHopClasses);
+  int2* at = items + h.item[k] + (r - h.first[k]) * size;
+  int n = 0;
+  hop_sources(i, left, right, height, bands, [&](int x) { at[n++] = make_int2(i, x); });
+  for (; n < size; ++n) at[n] = make_int2(i, -1);
+}
+
+void build_m2m(jb_dsched& d, int num_nodes, int num_internal, const int* parent, const int* left, const int* right,
+               int singles, int64_t* hop_offsets, int* num_hops, cudaStream_t st) {
+  const HopBands bands{singles};
+  *num_hops = 0;
+  hop_offsets[0] = 0;
+  if (num_internal == 0) return;
+  Scratch s;
+  DBuf height, arrived, k0, k1, v0, v1;
+  ck(height.alloc((size_t)num_nodes * 4));
+  ck(arrived.alloc(((size_t)num_internal + kHopKeys) * 4));  // and the key counts
+  int* bins = arrived.as<int>() + num_internal;
+  for (DBuf* b : {&k0, &k1}) ck(b->alloc((size_t)num_internal * 8));
+  for (DBuf* b : {&v0, &v1}) ck(b->alloc((size_t)num_internal * 4));
+  ck(cudaMemsetAsync(height.p, 0, (size_t)num_nodes * 4, st));
+  ck(cudaMemsetAsync(arrived.p, 0, ((size_t)num_internal + kHopKeys) * 4, st));
+  k_node_heights<<<nblocks(num_nodes - num_internal, 128), 128, 0, st>>>(num_internal, num_nodes, parent,
+                                                                         height.as<int>(), arrived.as<int>());
+  ck_launch();
+  k_hop_keys<<<nblocks(num_internal, 128), 128, 0, st>>>(num_internal, left, right, height.as<int>(), bands,
+                                                         k0.as<uint64_t>(),                                                         v0.as<int>(), bins);
+  ck_launch();
+  int count[kHopKeys];
+  ck(cudaMemcpyAsync(count, bins, sizeof(count), cudaMemcpyDeviceToHost, st));
+  radix_sort(k0.as<uint64_t>(), v0.as<int>(), k1.as<uint64_t>(), v1.as<int>(), num_internal, 8, s, st);
+  ck(cudaStreamSynchronize(st));
+  HopLayout h{};
+  int nodes = 0, hops = 0;
+  int64_t items = 0;
+  for (int k = 0; k < kHopKeys && nodes < num_internal; ++k) {
+    if (k % kHopClasses == 0 && k > 0) {
+      items = (items + 31) / 32 * 32;
+      hop_offsets[hops = k / kHopClasses] = items;
+    }
+    h.first[k] = nodes;
+    h.item[k] = (int)items;
+    nodes += count[k];
+    items += (int64_t)count[k] * (kHopMost >> (k % kHopClasses));
+  }
+  items = (items + 31) / 32 * 32;
+  hop_offsets[++hops] = items;
+  *num_hops = hops;
+  if (items > (int64_t)0x7fffffff) throw Fail{JB_ERR_ARG};
+  ck(d.aux.alloc((size_t)items * sizeof(int2)));
+  ck(cudaMemsetAsync(d.aux.p, 0xff, (size_t)items * sizeof(int2), st));
+  k_hop_items<<<nblocks(num_internal, 128), 128, 0, st>>>(num_internal, k0.as<uint64_t>(), v0.as<int>(), h, left, right,
+                                                          height.as<int>(), bands, d.aux.as<int2>());
+  ck_launch();
+  d.info.num_units = items;
+}
+
 template <typename F>
 int run_builder(jb_dsched** out, cudaStream_t st, F&& fn) {
   if (!out) return JB_ERR_ARG;
@@ -1039,6 +1177,18 @@ JB_API int jb_l2l_schedule_device(int num_internal, int leaf_lo, int leaf_hi, co
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   return run_builder(out, st,
                      [&](jb_dsched& d) { build_l2l(d, num_internal, leaf_lo, leaf_hi, parent, far_off, st); });
+}
+
+JB_API int jb_m2m_schedule_device(int num_nodes, int num_internal, const int* parent, const int* left,
+                                  const int* right, int single_levels, int64_t* hop_offsets, int* num_hops,
+                                  void* stream, jb_dsched** out) {
+  if (single_levels < 0 || single_levels > 16 || num_internal < 0 || num_nodes <= num_internal || !hop_offsets || !num_hops ||
+      (num_internal > 0 && (!parent || !left || !right)))
+    return JB_ERR_ARG;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  return run_builder(out, st, [&](jb_dsched& d) {
+    build_m2m(d, num_nodes, num_internal, parent, left, right, single_levels, hop_offsets, num_hops, st);
+  });
 }
 
 JB_API int jb_gear_schedule_device(int num_nodes, const int64_t* far_off, const int* far_src, const int* gears,

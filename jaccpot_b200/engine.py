@@ -21,8 +21,8 @@ import torch
 
 from . import _lib
 from .schedule import (MixedGearM2LSchedule, gear_m2l_mixed_schedule, gear_m2l_mixed_schedule_device,
-                       _run_device, gear_m2l_schedule, gear_m2l_schedule_device, leaf_schedule, leaf_schedule_device,
-                       m2l_schedule, m2l_schedule_device, m2l_unit_limit, mixed_ladder, tc_m2l_schedule)
+                       _run_device, m2m_single_levels, gear_m2l_schedule, gear_m2l_schedule_device, leaf_schedule, leaf_schedule_device,
+                       m2l_schedule, m2l_schedule_device, m2l_unit_limit, M2M_HOPS_MAX_INTERNAL, mixed_ladder, tc_m2l_schedule)
 from .tree import DeviceBuiltTopology, Topology
 
 
@@ -84,6 +84,7 @@ class DeviceTopology:
         self.inv_perm = up("inverse_permutation", torch.int64)
         self.level_offsets = [int(x) for x in topo.level_offsets]
         self._l2l_first = None
+        self._hops = None
 
     @property
     def l2l_first_level(self) -> int:
@@ -105,6 +106,29 @@ class DeviceTopology:
     @l2l_first_level.setter
     def l2l_first_level(self, level: int) -> None:
         self._l2l_first = int(level)
+
+    def m2m_hops(self):
+        """(items int32[.., 2], hop offsets int64 on the host) of jb_m2m_hops for
+        this tree, built on first use (at the construction of a Pass whose upward
+        sweep takes the hops, or with the adjoint's buffers)."""
+        if self._hops is None:
+            t = self.topo
+            offsets = np.zeros(_lib.JB_MAX_M2M_HOPS + 1, dtype=np.int64)
+            hops = ctypes.c_int(0)
+            info, field, free = _run_device("jb_m2m_schedule_device",
+                                            [t.num_nodes, t.num_internal, _ptr(self.parent), _ptr(self.left),
+                                             _ptr(self.right), m2m_single_levels(t.num_internal), offsets.ctypes.data,
+                                             ctypes.byref(hops)], self.device)
+            try:
+                items = field(_lib.JB_SCHED_AUX, (info.num_units, 2), np.int32)
+            finally:
+                free()
+            self._hops = (items, offsets[:hops.value + 1].copy())
+        return self._hops
+
+    def share_m2m_hops(self, hops) -> None:
+        """Takes m2m_hops() of another topology over the same tree (None: builds its own)."""
+        self._hops = hops
 
     def far_pair_targets(self) -> torch.Tensor:
         """int32 on the device: the target node of every far pair (a zero when
@@ -410,6 +434,10 @@ class Pass:
         self.num_l2l_units = int(units.shape[0])
         self.d_l2l_units = up(units)
         self.d_l2l_anc = up(anc)
+        # the M2M by hops of several levels, or level by level on a large tree
+        self.m2m_hops = _on_gpu(dt) and t.num_internal <= M2M_HOPS_MAX_INTERNAL
+        if self.m2m_hops:
+            dt.m2m_hops()
         # run(): the near field on the caller's stream while the upward sweep,
         # M2L and L2L run on a high-priority stream of the pass (same bits)
         self.overlap = True
@@ -454,11 +482,16 @@ class Pass:
         t, dt, ws, s = self.dt.topo, self.dt, self.ws, _stream_handle(stream)
         _lib.check(self.lib.jb_p2m(self.p, _ptr(ws.pos4), t.num_nodes, t.num_internal, _ptr(dt.node_ranges),
                                    _ptr(ws.centers), _ptr(ws.mult), s), "jb_p2m")
-        lo = dt.level_offsets
-        for lev in range(t.num_levels - 1, -1, -1):
-            _lib.check(self.lib.jb_m2m_level(self.p, lo[lev], lo[lev + 1], _ptr(dt.left), _ptr(dt.right),
-                                             _ptr(dt.node_ranges), _ptr(ws.centers), _ptr(ws.mult), s),
-                       "jb_m2m_level")
+        if not self.m2m_hops:
+            lo = dt.level_offsets
+            for lev in range(t.num_levels - 1, -1, -1):
+                _lib.check(self.lib.jb_m2m_level(self.p, lo[lev], lo[lev + 1], _ptr(dt.left), _ptr(dt.right),
+                                                 _ptr(dt.node_ranges), _ptr(ws.centers), _ptr(ws.mult), s),
+                           "jb_m2m_level")
+            return
+        items, offsets = dt.m2m_hops()
+        _lib.check(self.lib.jb_m2m_hops(self.p, len(offsets) - 1, offsets.ctypes.data, _ptr(items),
+                                        _ptr(dt.node_ranges), _ptr(ws.centers), _ptr(ws.mult), s), "jb_m2m_hops")
 
     def set_gears(self, gears, orders) -> None:
         """Per-far-pair expansion orders: gears[e] indexes `orders` for pair e
@@ -863,7 +896,7 @@ class Pass:
                                          _ptr(grad_mass), s), "jb_gather_unsorted(grad)")
 
     def launches_per_run(self) -> int:
-        """This library's kernel launches in one run(): P2M, one M2M per level,
+        """This library's kernel launches in one run(): P2M, one M2M per hop or level,
         the M2L (one launch per non-empty gear with gears) and its split
         reduce, one L2L per level from the first with a non-zero local, the
         leaf L2P + P2P and their split reduce."""
@@ -876,4 +909,5 @@ class Pass:
         else:
             m2l = 1 + int(self.m2l_sched.split.shape[0] > 0)
         l2l = t.num_levels - self.dt.l2l_first_level
-        return (1 + t.num_levels + m2l + l2l + 2 + int(self.leaf_sched.split.shape[0] > 0))
+        m2m = int((np.diff(self.dt.m2m_hops()[1]) > 0).sum()) if self.m2m_hops else t.num_levels
+        return (1 + m2m + m2l + l2l + 2 + int(self.leaf_sched.split.shape[0] > 0))

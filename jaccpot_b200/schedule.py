@@ -76,6 +76,28 @@ def m2l_unit_limit(num_pairs: int, mixed: bool = False) -> int:
     return limit
 
 
+# Trees of up to this many internal nodes take the M2M by hops in the forward
+# pass, larger ones level by level.  The hops cost fewer launches but more
+# translations; alone they are faster at every size (Plummer 65k p=6 91 -> 45
+# us with the P2M, clustered 500k p=8 208 -> 143, 4M 604 -> 553), but a large
+# tree's sweep runs beside the near field, where the work counts and the
+# launches do not (step: 500k, 25k nodes, 1402 -> 1395 us replayed and 1213 ->
+# 1152 launched one by one; 1M, 48k nodes, 2082 -> 2088; 4M 7535 -> 7609).
+M2M_HOPS_MAX_INTERNAL = 32768
+
+
+def m2m_single_levels(num_internal: int) -> int:
+    """The lowest heights that get a hop of their own: those of more than about
+    1,024 nodes (a height holds about 0.6 of the one below, the lowest 0.4 of
+    all), where four levels in one hop would double the translations and the
+    launches are filled anyway.  (Clustered 500k p=8, step: 1416 us with none,
+    1395 with 5; Plummer 65k p=6, upward: 43 us with none, 45 with 1 or 2.)"""
+    n, s = 0.4 * num_internal, 0
+    while n > 1024 and s < 16:
+        n, s = 0.6 * n, s + 1
+    return s
+
+
 def m2l_schedule(topo: Topology, max_pairs: int = 64, targets: np.ndarray | None = None) -> M2LSchedule:
     off = topo.far_offsets
     counts = np.diff(off)
