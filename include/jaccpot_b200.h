@@ -435,6 +435,11 @@ JB_API int jb_l2l_level(int p, int first, int last, const int* left, const int* 
 JB_API int jb_l2l_leaves(int p, int num_units, const int* units, const int* anc, const float* centers,
                          float* locals, void* stream);
 
+/* jb_l2l_leaves with the sums added to leaf_rows (num_leaves rows that hold the
+ * leaves' own M2L sums) instead of the leaves' rows of locals.              */
+JB_API int jb_l2l_leaves_to(int p, int num_units, const int* units, const int* anc, const float* centers,
+                            const float* locals, int num_internal, float* leaf_rows, void* stream);
+
 /* Leaf evaluation over work units: L2P of each leaf's local at its particles
  * (runtime/kernels/_evaluate.py:2106-2484, evaluate_local_real_with_grad) plus
  * the near field over the self leaf and the leaf's neighbour list
@@ -541,7 +546,12 @@ JB_API int jb_gather_unsorted(int64_t n, const float* acc4, const int64_t* inv_p
 /*   jb_adj_near, jb_adj_leaf_far, jb_adj_l2l_level (deepest level first),  */
 /*   jb_adj_m2l, jb_adj_m2l_centers, jb_adj_m2m_level (root first),         */
 /*   jb_adj_p2m.  cbar4 (num_nodes float4) and mbar (num_nodes x stride)    */
-/*   start at zero; w4 is the sorted float4 cotangent (w, 0);               */
+/*   start at zero.  Or, in a third of the launches and with a near field    */
+/*   that can run beside the rest, from locals that hold each node's own M2L */
+/*   sum: jb_adj_near; jb_adj_leaf_far (cbar4 NULL, xm4 a buffer of its own, */
+/*   the leaves' complete locals from jb_l2l_leaves_to), jb_adj_l2l_hops,    */
+/*   jb_adj_m2l, jb_adj_far_nodes, jb_adj_leaves; jb_adj_particles.  mbar and */
+/*   chain4 start at zero; w4 is the sorted float4 cotangent (w, 0);         */
 /*   xm4[i] = (dL/dx, dL/dy, dL/dz, dL/dm) sorted.  Needs symmetric near and */
 /*   far lists (jb_tree_build emits both directions).  Orders 1..9.         */
 /* ------------------------------------------------------------------------ */
@@ -551,7 +561,8 @@ JB_API int jb_gather_unsorted(int64_t n, const float* acc4, const int64_t* inv_p
 JB_API int jb_adj_near(const float* pos4, const float* w4, int num_internal, int num_units, const int* units,
                        const int* aux, const int* runs, const int* node_ranges, float G, float eps2, float* out_xm4,
                        float* partials, int num_split, const int* split, void* stream);
-/* L2P VJP: lbar[leaf] = dL/dlocal, adds the particle and leaf-centre terms. */
+/* L2P VJP: lbar[leaf] = dL/dlocal, adds the particle and leaf-centre terms;
+ * with cbar4 NULL, sets xm4 to the particle terms alone.                    */
 JB_API int jb_adj_leaf_far(int p, const float* pos4, const float* w4, int num_nodes, int num_internal,
                            const int* node_ranges, const float* centers, const float* locals, float G, float* xm4,
                            float* lbar, float* cbar4, void* stream);
@@ -573,6 +584,25 @@ JB_API int jb_adj_m2l_centers(int p, int num_nodes, int64_t num_pairs, const int
  * upward/real_tree_expansions.py:216-364 and the COM of :439). */
 JB_API int jb_adj_m2m_level(int p, int first, int last, const int* left, const int* right, const float* centers,
                             const float* mult, float* mbar, float* cbar4, void* stream);
+/* L2L VJP of all levels: lbar of every internal node from the leaves', over
+ * the items of jb_m2m_schedule_device.                                      */
+JB_API int jb_adj_l2l_hops(int p, int num_hops, const int64_t* hop_offsets, const int* items, const float* centers,
+                           float* lbar, void* stream);
+/* cbar4 of every node (set): the M2L's displacement terms (g4: scratch of
+ * num_pairs float4) and Lbar . D L - M . D Mbar with the node's own M2L sums. */
+JB_API int jb_adj_far_nodes(int p, int num_nodes, int64_t num_pairs, const int* pair_tgt, const int* far_src,
+                            const int64_t* far_off, const int* rev, const float* mult, const float* lbar,
+                            const float* locals, const float* mbar, const float* centers, float* g4, float* cbar4,
+                            void* stream);
+/* M2M VJP straight to the leaves, over the units of jb_l2l_schedule_device:
+ * adds each leaf's ancestors into its mbar row; chain4[leaf] (num_nodes rows)
+ * is the chain of the centres of mass.                                      */
+JB_API int jb_adj_leaves(int p, int num_units, const int* units, const int* anc, const int* parent,
+                         const float* centers, const float* cbar4, float* mbar, float* chain4, void* stream);
+/* P2M + COM VJP after jb_adj_leaves: adds far4 and the particle terms to xm4. */
+JB_API int jb_adj_particles(int p, const float* pos4, int num_nodes, int num_internal, const int* node_ranges,
+                            const float* centers, const float* mbar, const float* cbar4, const float* chain4,
+                            const float* far4, float* xm4, void* stream);
 /* P2M + leaf COM VJP (transpose of real_tree_expansions.py:89-213); adds into xm4. */
 JB_API int jb_adj_p2m(int p, const float* pos4, int num_nodes, int num_internal, const int* node_ranges,
                       const float* centers, const float* mbar, const float* cbar4, float* xm4, void* stream);

@@ -6,8 +6,9 @@ whose backward is the hand-written adjoint kernels (``Pass.vjp``) -- the torch
 counterpart of the reference's ``jax.custom_vjp`` around
 ``differentiable_accelerations`` (runtime/fmm_evaluate.py:542-731, :1175-1250).
 
-Memory policy: the forward's node coefficients (centres, multipoles, locals:
-num_nodes x (2 stride + 4) floats) are kept for the backward when they fit in
+Memory policy: the forward's coefficients (centres, multipoles, every node's own
+locals and the leaves' complete ones: num_nodes x (2 stride + 4) and num_leaves x
+stride floats) are kept for the backward when they fit in
 ``keep_bytes``; above that the backward recomputes them from the saved inputs.
 """
 
@@ -25,14 +26,14 @@ class FMMAccelerations(torch.autograd.Function):
     def forward(ctx, positions: torch.Tensor, masses: torch.Tensor, pass_: Pass, keep_bytes: int = DEFAULT_KEEP_BYTES):
         n = pass_.dt.topo.num_particles
         pass_.load_particles(positions.detach(), masses.detach())
-        pass_.run(cascade=True)  # the backward reads every node's complete local
+        pass_.run(own=True)  # the backward reads every node's own M2L sum
         acc = torch.empty((n, 3), device=pass_.dt.device, dtype=torch.float32)
         pass_.unsort(acc, None)
         ws = pass_.ws
-        coeff_bytes = 4 * (ws.centers.numel() + ws.mult.numel() + ws.locals.numel())
+        coeffs = (ws.centers, ws.mult, ws.locals, pass_.leaf_rows())
         ctx.kept = None
-        if coeff_bytes <= keep_bytes:
-            ctx.kept = (ws.centers.clone(), ws.mult.clone(), ws.locals.clone())
+        if 4 * sum(c.numel() for c in coeffs) <= keep_bytes:
+            ctx.kept = tuple(c.clone() for c in coeffs)
         ctx.pass_ = pass_
         ctx.save_for_backward(positions.detach(), masses.detach())
         return acc.to(positions.dtype)
@@ -44,9 +45,9 @@ class FMMAccelerations(torch.autograd.Function):
         n = ps.dt.topo.num_particles
         ps.load_particles(positions, masses)
         if ctx.kept is not None:
-            ps.ws.centers.copy_(ctx.kept[0])
-            ps.ws.mult.copy_(ctx.kept[1])
-            ps.ws.locals.copy_(ctx.kept[2])
+            for into, kept in zip((ps.ws.centers, ps.ws.mult, ps.ws.locals, ps.leaf_rows()), ctx.kept):
+                into.copy_(kept)
+            ps.own_locals = True
         gx = torch.empty((n, 3), device=ps.dt.device, dtype=torch.float32)
         gm = torch.empty((n,), device=ps.dt.device, dtype=torch.float32)
         ps.vjp(grad_acc.contiguous(), gx, gm, recompute=ctx.kept is None)

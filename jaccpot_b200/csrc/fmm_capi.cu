@@ -634,7 +634,18 @@ JB_API int jb_m2l_mixed(int p_max, int num_units, const int* units, const int* b
 JB_API int jb_l2l_leaves(int p, int num_units, const int* units, const int* anc, const float* centers,
                          float* locals, void* stream) {
   if (num_units < 0 || (num_units > 0 && (!units || !anc || !centers || !locals))) return JB_ERR_ARG;
-  return dispatch<RunL2LLeaves>(p, num_units, units, anc, centers, locals, ST(stream));
+  return dispatch<RunL2LLeaves>(p, num_units, units, anc, centers, locals, locals, ST(stream));
+}
+
+JB_API int jb_l2l_leaves_to(int p, int num_units, const int* units, const int* anc, const float* centers,
+                            const float* locals, int num_internal, float* leaf_rows, void* stream) {
+  if (num_units < 0 || num_internal < 0 ||
+      (num_units > 0 && (!units || !anc || !centers || !locals || !leaf_rows)))
+    return JB_ERR_ARG;
+  const int cs = jb_coeff_stride(p);
+  if (cs <= 0) return JB_ERR_ORDER;
+  return dispatch<RunL2LLeaves>(p, num_units, units, anc, centers, locals, leaf_rows - (ptrdiff_t)num_internal * cs,
+                                ST(stream));
 }
 
 JB_API int jb_l2l_level(int p, int first, int last, const int* left, const int* right, const float* centers,
@@ -724,7 +735,7 @@ JB_API int jb_adj_near(const float* pos4, const float* w4, int num_internal, int
 JB_API int jb_adj_leaf_far(int p, const float* pos4, const float* w4, int num_nodes, int num_internal,
                            const int* node_ranges, const float* centers, const float* locals, float G, float* xm4,
                            float* lbar, float* cbar4, void* stream) {
-  if (!pos4 || !w4 || !node_ranges || !centers || !locals || !xm4 || !lbar || !cbar4 || num_nodes < 1 ||
+  if (!pos4 || !w4 || !node_ranges || !centers || !locals || !xm4 || !lbar || num_nodes < 1 ||
       num_internal < 0 || num_internal >= num_nodes)
     return JB_ERR_ARG;
   return dispatch_adj(p, [&](auto R) {
@@ -767,6 +778,49 @@ JB_API int jb_adj_m2l_centers(int p, int num_nodes, int64_t num_pairs, const int
   k_adj_m2l_gather<<<blocks_1d(num_nodes, 128), 128, 0, ST(stream)>>>(
       num_nodes, far_off, rev, reinterpret_cast<const float4*>(g4), reinterpret_cast<float4*>(cbar4));
   return launch_status();
+}
+
+JB_API int jb_adj_l2l_hops(int p, int num_hops, const int64_t* hop_offsets, const int* items, const float* centers,
+                           float* lbar, void* stream) {
+  if (num_hops < 0 || num_hops > JB_MAX_M2M_HOPS || (num_hops > 0 && (!hop_offsets || !items || !centers || !lbar)))
+    return JB_ERR_ARG;
+  return dispatch_adj(p, [&](auto R) {
+    return decltype(R)::l2l_hops(num_hops, hop_offsets, items, centers, lbar, ST(stream));
+  });
+}
+
+JB_API int jb_adj_far_nodes(int p, int num_nodes, int64_t num_pairs, const int* pair_tgt, const int* far_src,
+                            const int64_t* far_off, const int* rev, const float* mult, const float* lbar,
+                            const float* locals, const float* mbar, const float* centers, float* g4, float* cbar4,
+                            void* stream) {
+  if (num_nodes < 1 || num_pairs < 0 || !far_off || !cbar4 || !mult || !lbar || !locals || !mbar ||
+      (num_pairs > 0 && (!pair_tgt || !far_src || !rev || !centers || !g4)))
+    return JB_ERR_ARG;
+  return dispatch_adj(p, [&](auto R) {
+    const int rc = decltype(R)::m2l_pairs(num_pairs, pair_tgt, far_src, mult, lbar, centers, g4, ST(stream));
+    return rc ? rc : decltype(R)::nodes(num_nodes, far_off, rev, g4, mult, lbar, locals, mbar, cbar4, ST(stream));
+  });
+}
+
+JB_API int jb_adj_leaves(int p, int num_units, const int* units, const int* anc, const int* parent,
+                         const float* centers, const float* cbar4, float* mbar, float* chain4, void* stream) {
+  if (num_units < 0 || (num_units > 0 && (!units || !anc || !parent || !centers || !cbar4 || !mbar || !chain4)))
+    return JB_ERR_ARG;
+  return dispatch_adj(p, [&](auto R) {
+    return decltype(R)::leaves(num_units, units, anc, parent, centers, cbar4, mbar, chain4, ST(stream));
+  });
+}
+
+JB_API int jb_adj_particles(int p, const float* pos4, int num_nodes, int num_internal, const int* node_ranges,
+                            const float* centers, const float* mbar, const float* cbar4, const float* chain4,
+                            const float* far4, float* xm4, void* stream) {
+  if (!pos4 || !node_ranges || !centers || !mbar || !cbar4 || !chain4 || !far4 || !xm4 || num_nodes < 1 ||
+      num_internal < 0 || num_internal >= num_nodes)
+    return JB_ERR_ARG;
+  return dispatch_adj(p, [&](auto R) {
+    return decltype(R)::particles(pos4, num_nodes, num_internal, node_ranges, centers, mbar, cbar4, chain4, far4, xm4,
+                                  ST(stream));
+  });
 }
 
 JB_API int jb_adj_m2m_level(int p, int first, int last, const int* left, const int* right, const float* centers,

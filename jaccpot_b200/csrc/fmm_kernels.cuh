@@ -412,11 +412,21 @@ __global__ void __launch_bounds__(kM2LThreads, 4) k_m2l_units_coop(int num_units
 // warp's ancestor rows fetched together as in k_m2l_units_coop.  One launch
 // with every leaf's chain in parallel, where the cascade runs one dependent
 // launch per level.
-template <int P>
+//
+// Results go to rows out + leaf * stride, which hold the leaves' own sums
+// before (out = locals: in place).  ADJ is the same sweep of the M2M's
+// adjoint: L2L(c_leaf - c_a) of each ancestor's row, and per leaf the chain of
+// the centres of mass, chain4[leaf] = (sum_a cbar_a / mu_a, sum_a (c_leaf - c_a)
+// . cbar_a / mu_a); below a node without mass, whose centre the masses do not
+// move, that node stands for the leaf in the last sum.
+template <int P, bool ADJ>
 __global__ void __launch_bounds__(kM2LThreads, 4) k_l2l_leaves(int num_units, const int4* __restrict__ units,
                                                                const int* __restrict__ anc,
                                                                const float4* __restrict__ centers,
-                                                               float* __restrict__ locals) {
+                                                               const float* locals, float* out,
+                                                               const float4* __restrict__ cbar4,
+                                                               float4* __restrict__ chain4,
+                                                               const int* __restrict__ parent) {
   constexpr int C = csize(P), CS = cstride(P), R4 = row4(P), NW = CS / 4;
   extern __shared__ float4 m2l_smem[];
   const int lane = threadIdx.x & 31;
@@ -441,6 +451,10 @@ __global__ void __launch_bounds__(kM2LThreads, 4) k_l2l_leaves(int num_units, co
     ca = centers[s0];
     ca1 = centers[s1];
   }
+  float4 chain = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 cm = cl;  // what the masses move: the highest node up from the leaf that has no mass, else the leaf
+  if (ADJ && ok)
+    for (int q = leaf, up; !(cm.w > 0.f) && (up = parent[q]) >= 0 && !(centers[up].w > 0.f); q = up) cm = centers[up];
   warp_rows_fetch<NW, R4>(wrows, ids, lane, s0, locals, CS);
   for (int it = 0; it < nmax; ++it) {
     const bool act = it < n;
@@ -461,7 +475,18 @@ __global__ void __launch_bounds__(kM2LThreads, 4) k_l2l_leaves(int num_units, co
     warp_rows_fetch<NW, R4>(wrows, ids, lane, act && it + 1 < n ? s1 : -1, locals, CS);
     if (act) {
       const int s2 = (it + 2 < n) ? __ldg(anc + e0 + it + 2) : s1;
-      l2l_pair<P>(v, ca.x - cl.x, ca.y - cl.y, ca.z - cl.z);
+      if (ADJ) {
+        const float4 cb = cbar4[anc[e0 + it]];
+        const float inv = ca.w > 0.f ? 1.f / ca.w : 0.f;
+        const float bx = cb.x * inv, by = cb.y * inv, bz = cb.z * inv;
+        chain.x += bx;
+        chain.y += by;
+        chain.z += bz;
+        chain.w += (cm.x - ca.x) * bx + (cm.y - ca.y) * by + (cm.z - ca.z) * bz;
+        l2l_pair<P>(v, cl.x - ca.x, cl.y - ca.y, cl.z - ca.z);
+      } else {
+        l2l_pair<P>(v, ca.x - cl.x, ca.y - cl.y, ca.z - cl.z);
+      }
 #pragma unroll
       for (int k = 0; k < C; ++k) acc[k] += v[k];
       ca = ca1;
@@ -471,9 +496,10 @@ __global__ void __launch_bounds__(kM2LThreads, 4) k_l2l_leaves(int num_units, co
   }
   cp_async_wait_all();
   if (!ok || n == 0) return;
-  float* dst = locals + (size_t)leaf * CS;
+  float* dst = out + (ptrdiff_t)leaf * CS;
 #pragma unroll
   for (int k = 0; k < C; ++k) dst[k] += acc[k];
+  if (ADJ) chain4[leaf] = chain;
 }
 
 // Sums the partial rows of targets whose list was split: split[i] =
@@ -1837,21 +1863,28 @@ int RunL2L<P>::run(int first, int last, const int* left, const int* right, const
   return launch_status();
 }
 
+template <int P, bool ADJ>
+int launch_l2l_leaves(int num_units, const int* units, const int* anc, const float* centers, const float* locals,
+                      float* out, const float* cbar4, float* chain4, const int* parent, cudaStream_t st) {
+  if (num_units <= 0) return JB_OK;
+  const size_t sm = sizeof(float4) * kM2LThreads * row4(P) + sizeof(int) * kM2LThreads;
+  cudaFuncSetAttribute(k_l2l_leaves<P, ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k_l2l_leaves<P, ADJ><<<blocks_for(num_units, kM2LThreads), kM2LThreads, sm, st>>>(
+      num_units, reinterpret_cast<const int4*>(units), anc, reinterpret_cast<const float4*>(centers), locals, out,
+      reinterpret_cast<const float4*>(cbar4), reinterpret_cast<float4*>(chain4), parent);
+  return launch_status();
+}
+
 template <int P>
 struct RunL2LLeaves {
-  static int run(int num_units, const int* units, const int* anc, const float* centers, float* locals,
+  static int run(int num_units, const int* units, const int* anc, const float* centers, const float* locals, float* out,
                  cudaStream_t st);
 };
 
 template <int P>
-int RunL2LLeaves<P>::run(int num_units, const int* units, const int* anc, const float* centers, float* locals,
-                 cudaStream_t st) {
-  if (num_units <= 0) return JB_OK;
-  const size_t sm = sizeof(float4) * kM2LThreads * row4(P) + sizeof(int) * kM2LThreads;
-  cudaFuncSetAttribute(k_l2l_leaves<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_l2l_leaves<P><<<blocks_for(num_units, kM2LThreads), kM2LThreads, sm, st>>>(
-      num_units, reinterpret_cast<const int4*>(units), anc, reinterpret_cast<const float4*>(centers), locals);
-  return launch_status();
+int RunL2LLeaves<P>::run(int num_units, const int* units, const int* anc, const float* centers, const float* locals,
+                         float* out, cudaStream_t st) {
+  return launch_l2l_leaves<P, false>(num_units, units, anc, centers, locals, out, nullptr, nullptr, nullptr, st);
 }
 
 template <int P>

@@ -393,6 +393,7 @@ class Pass:
         self.m2l_unit_pairs = int(m2l_unit_pairs)
         self.leaf_unit_sources = int(leaf_unit_sources)
         self.ws = Workspace.allocate(dt, self.p)
+        self.own_locals = False  # ws.locals holds the M2L's own sums, leaf_rows() the leaves' complete locals
         self.lib = _lib.lib()
         t = dt.topo
         self.leaf_range = (0, t.num_leaves) if leaf_range is None else (int(leaf_range[0]), int(leaf_range[1]))
@@ -453,8 +454,9 @@ class Pass:
         q.leaf_partials = torch.empty_like(self.leaf_partials)
         if getattr(self, "gear_sched", None) is not None:
             q.gear_partials = torch.empty_like(self.gear_partials)
-        for name in ("_tc", "_tc_status", "_adj", "_adj_sched", "_adj_m2l", "_far_stream"):
+        for name in ("_tc", "_tc_status", "_adj", "_far_stream", "_leaf_rows"):
             q.__dict__.pop(name, None)
+        q.own_locals = False
         return q
 
     def near_pair_interactions(self) -> torch.Tensor:
@@ -536,6 +538,7 @@ class Pass:
 
     def m2l(self, stream=None) -> None:
         ws, s, sc = self.ws, _stream_handle(stream), self.m2l_sched
+        self.own_locals = False
         _zero(ws.locals, stream)
         if self.m2l_mode == _lib.JB_M2L_SPLIT_BF16:
             self._m2l_split(s, stream)
@@ -566,6 +569,7 @@ class Pass:
         w = far_w.to(device=self.dt.device, dtype=torch.float32).contiguous()
         if w.numel() != self.dt.topo.num_far_pairs:
             raise ValueError("one weight per far pair is required")
+        self.own_locals = False
         _zero(ws.locals, stream)
         _lib.check(self.lib.jb_m2l_weighted(self.p, int(sc.units.shape[0]), _ptr(self.d_m2l_units), _ptr(ws.mult),
                                             _ptr(ws.centers), _ptr(self.dt.far_src), _ptr(w) if w.numel() else None,
@@ -585,8 +589,8 @@ class Pass:
         _lib.check(self.lib.jb_leaf_eval_weighted(self.p, mode, _ptr(ws.pos4), _ptr(r), int(lw.numel()), _ptr(lw),
                                                   t.num_internal, int(sc.units.shape[0]), _ptr(self.d_leaf_units),
                                                   _ptr(self.d_leaf_aux), _ptr(self.d_leaf_runs),
-                                                  _ptr(dt.node_ranges), _ptr(ws.centers), _ptr(ws.locals), self.G,
-                                                  self.eps2, _ptr(ws.acc4), _ptr(self.leaf_partials),
+                                                  _ptr(dt.node_ranges), _ptr(ws.centers), self._leaf_locals_ptr(),
+                                                  self.G, self.eps2, _ptr(ws.acc4), _ptr(self.leaf_partials),
                                                   int(sc.split.shape[0]), _ptr(self.d_leaf_split),
                                                   _stream_handle(stream)), "jb_leaf_eval_weighted")
         return ws.acc4
@@ -667,6 +671,34 @@ class Pass:
             _lib.check(self.lib.jb_l2l_level(self.p, lo[lev], lo[lev + 1], _ptr(dt.left), _ptr(dt.right),
                                              _ptr(ws.centers), _ptr(ws.locals), s), "jb_l2l_level")
 
+    def l2l_to_rows(self, stream=None) -> None:
+        """The downward sweep into leaf_rows(), with ws.locals left as the M2L's
+        own sums at every node -- what the adjoint reads."""
+        t, dt, ws, s = self.dt.topo, self.dt, self.ws, _stream_handle(stream)
+        rows = self.leaf_rows()
+        if stream is None:
+            rows.copy_(ws.locals[t.num_internal:])
+        else:
+            with torch.cuda.stream(stream):
+                rows.copy_(ws.locals[t.num_internal:])
+        _lib.check(self.lib.jb_l2l_leaves_to(self.p, self.num_l2l_units, _ptr(self.d_l2l_units), _ptr(self.d_l2l_anc),
+                                             _ptr(ws.centers), _ptr(ws.locals), t.num_internal, _ptr(rows), s),
+                   "jb_l2l_leaves_to")
+        self.own_locals = True
+
+    def leaf_rows(self) -> torch.Tensor:
+        """(leaves, stride): the leaves' complete locals beside ws.locals."""
+        if getattr(self, "_leaf_rows", None) is None:
+            self._leaf_rows = torch.empty((self.dt.topo.num_leaves, self.ws.stride), device=self.dt.device,
+                                          dtype=torch.float32)
+        return self._leaf_rows
+
+    def _leaf_locals_ptr(self) -> int:
+        """Base address for the kernels that read leaf rows by node id."""
+        if not self.own_locals:
+            return _ptr(self.ws.locals)
+        return _ptr(self.leaf_rows()) - 4 * self.ws.stride * self.dt.topo.num_internal
+
     _PARTS = {"near": _lib.JB_P2P_NEAR_ONLY, "far": _lib.JB_P2P_FAR_ONLY,
               "near_first": _lib.JB_P2P_NEAR_FIRST, "far_after": _lib.JB_P2P_FAR_AFTER}
 
@@ -686,7 +718,7 @@ class Pass:
             mode |= self._PARTS[part]
         _lib.check(self.lib.jb_leaf_eval(self.p, mode, _ptr(ws.pos4), t.num_internal, int(sc.units.shape[0]),
                                          _ptr(self.d_leaf_units), _ptr(self.d_leaf_aux), _ptr(self.d_leaf_runs),
-                                         _ptr(dt.node_ranges), _ptr(ws.centers), _ptr(ws.locals), self.G,
+                                         _ptr(dt.node_ranges), _ptr(ws.centers), self._leaf_locals_ptr(), self.G,
                                          self.eps2, _ptr(acc4), _ptr(self.leaf_partials),
                                          int(sc.split.shape[0]), _ptr(self.d_leaf_split),
                                          _stream_handle(stream)), "jb_leaf_eval")
@@ -700,7 +732,7 @@ class Pass:
         if out is None:
             out = torch.empty((nt, 4), device=dt.device, dtype=torch.float32)
         _lib.check(self.lib.jb_eval_targets(self.p, _ptr(ws.pos4), t.num_internal, _ptr(dt.node_ranges),
-                                            _ptr(ws.centers), _ptr(ws.locals), _ptr(dt.near_off),
+                                            _ptr(ws.centers), self._leaf_locals_ptr(), _ptr(dt.near_off),
                                             _ptr(dt.near_src), _ptr(dt.leaf_of), nt, _ptr(ts), self.G, self.eps2,
                                             _ptr(out), _stream_handle(stream)), "jb_eval_targets")
         return out
@@ -732,9 +764,12 @@ class Pass:
         _lib.check(self.lib.jb_gather_unsorted(n, _ptr(self.ws.acc4), _ptr(self.dt.inv_perm), _ptr(acc),
                                                _ptr(pot), _stream_handle(stream)), "jb_gather_unsorted")
 
-    def downward(self, stream=None, cascade: bool = False) -> None:
+    def downward(self, stream=None, cascade: bool = False, own: bool = False) -> None:
         self.m2l(stream)
-        self.l2l(stream, cascade=cascade)
+        if own:
+            self.l2l_to_rows(stream)
+        else:
+            self.l2l(stream, cascade=cascade)
 
     def far_stream(self) -> torch.cuda.Stream:
         """The high-priority stream run(overlap=True) puts the far-field chain
@@ -746,23 +781,24 @@ class Pass:
         return self._far_stream
 
     def run(self, stream=None, cascade: bool = False, potential: bool = False,
-            overlap: bool | None = None) -> torch.Tensor:
+            overlap: bool | None = None, own: bool = False) -> torch.Tensor:
         """Whole pass on the particles already in ws.pos4; returns sorted acc4
-        (cascade: the level-by-level downward sweep, see l2l).  overlap
+        (cascade: the level-by-level downward sweep, see l2l; own: leave every
+        node's own M2L sum in ws.locals, see l2l_to_rows).  overlap
         (default self.overlap): the near field runs on `stream` while the
         upward sweep, M2L and L2L run on far_stream(), joined before the L2P
         and the sum of split leaves; the result has the same bits as the
         one-stream order (at 4M, p = 8: 7.89 -> 7.64 ms a step)."""
         if not (self.overlap if overlap is None else overlap):
             self.upward(stream)
-            self.downward(stream, cascade=cascade)
+            self.downward(stream, cascade=cascade, own=own)
             return self.evaluate(stream, potential=potential)
         main = stream if stream is not None else torch.cuda.current_stream(self.dt.device)
         far = self.far_stream()
         far.wait_stream(main)  # the particles are loaded
         self.evaluate(main, potential=potential, part="near_first")
         self.upward(far)
-        self.downward(far, cascade=cascade)
+        self.downward(far, cascade=cascade, own=own)
         main.wait_stream(far)
         return self.evaluate(main, potential=potential, part="far_after")
 
@@ -806,31 +842,42 @@ class Pass:
     # -- adjoint --------------------------------------------------------------
     def _adj_buffers(self):
         if getattr(self, "_adj", None) is None:
-            t, dev, cs = self.dt.topo, self.dt.device, self.ws.stride
+            dt, t, dev, cs = self.dt, self.dt.topo, self.dt.device, self.ws.stride
+            # a tree built here by the theta walk lists every pair both ways
+            mutual = dt.as_built and t.gear_orders is None
+            if not (mutual or dt.near_lists_symmetric()):
+                raise ValueError("the near-field adjoint needs symmetric neighbour lists")
             f32 = dict(device=dev, dtype=torch.float32)
-            self._adj = {
+            dt.m2m_hops()
+            A = {
                 "w4": torch.empty((t.num_particles, 4), **f32),
                 "zeros": torch.zeros((t.num_particles,), **f32),
                 "xm4": torch.empty((t.num_particles, 4), **f32),
+                "far4": torch.empty((t.num_particles, 4), **f32),
                 "lbar": torch.empty((t.num_nodes, cs), **f32),
                 "mbar": torch.empty((t.num_nodes, cs), **f32),
                 "cbar4": torch.empty((t.num_nodes, 4), **f32),
+                "chain4": torch.empty((t.num_nodes, 4), **f32),
                 "g4": torch.empty((max(t.num_far_pairs, 1), 4), **f32),
-                "pair_tgt": self.dt.far_pair_targets(),
-                "rev": (self.dt.far_reverse_index() if _on_gpu(self.dt) and t.num_far_pairs else
-                        torch.from_numpy(t.far_reverse_index() if t.num_far_pairs else np.zeros(1, np.int32)).to(dev)),
+                "pair_tgt": dt.far_pair_targets(),
+                "rev": (dt.far_reverse_index() if t.num_far_pairs else torch.zeros(1, dtype=torch.int32, device=dev)),
             }
-            if not (self.dt.near_lists_symmetric() if _on_gpu(self.dt) else t.near_lists_symmetric()):
-                raise ValueError("the near-field adjoint needs symmetric neighbour lists")
-            # full near list of every leaf (the forward schedule may be a leaf range)
-            self._adj_sched = (leaf_schedule_device(self.dt, max_sources=4096) if _on_gpu(self.dt)
-                               else leaf_schedule(t, max_sources=4096))
-            up = lambda a: _up(a, dev)
-            self._adj["units"] = up(self._adj_sched.units)
-            self._adj["aux"] = up(self._adj_sched.aux)
-            self._adj["runs"] = up(self._adj_sched.runs)
-            self._adj["split"] = up(self._adj_sched.split)
-            self._adj["partials"] = torch.empty((max(self._adj_sched.num_slots, 1) * _lib.JB_MAX_LEAF_OCCUPANCY, 4), **f32)
+            # the forward's schedules (its leaf units of another size are rebuilt)
+            if self.leaf_unit_sources == 4096:
+                A["sched"], names = self.leaf_sched, ("d_leaf_units", "d_leaf_aux", "d_leaf_runs", "d_leaf_split")
+                A["units"], A["aux"], A["runs"], A["split"] = (getattr(self, n) for n in names)
+            else:
+                sc = A["sched"] = leaf_schedule_device(dt, max_sources=4096)
+                A["units"], A["aux"], A["runs"], A["split"] = (_up(x, dev) for x in (sc.units, sc.aux, sc.runs, sc.split))
+            A["partials"] = torch.empty((max(A["sched"].num_slots, 1) * _lib.JB_MAX_LEAF_OCCUPANCY, 4), **f32)
+            mp = m2l_unit_limit(t.num_far_pairs)
+            if self.m2l_unit_pairs == mp:
+                A["m2l"], A["m2l_units"], A["m2l_split"] = self.m2l_sched, self.d_m2l_units, self.d_m2l_split
+            else:
+                sc = A["m2l"] = m2l_schedule_device(dt, max_pairs=mp)
+                A["m2l_units"], A["m2l_split"] = _up(sc.units, dev), _up(sc.split, dev)
+            A["m2l_partials"] = torch.empty((max(A["m2l"].num_slots, 1), cs), **f32)
+            self._adj = A
         return self._adj
 
     def vjp(self, w: torch.Tensor, grad_pos: torch.Tensor, grad_mass: torch.Tensor, stream=None,
@@ -839,59 +886,55 @@ class Pass:
         currently loaded (acc = the pass's accelerations, input order), written
         into grad_pos (N,3) and grad_mass (N,).  recompute=True reruns the
         upward and downward sweeps first (multipoles / locals are not kept from
-        the forward call); False reuses the coefficients already in the
-        workspace."""
+        the forward call); False reuses the coefficients in the workspace when
+        they are those of run(own=True) (own_locals).  With self.overlap the
+        near field's adjoint runs on `stream` beside the rest on far_stream()."""
         if self.p > 9:
             raise ValueError("the adjoint is built for expansion orders <= 9")
         if self.leaf_range != (0, self.dt.topo.num_leaves):
             raise ValueError("the adjoint runs on the whole leaf range")
-        t, dt, ws, lb, s = self.dt.topo, self.dt, self.ws, self.lib, _stream_handle(stream)
+        t, dt, ws, lb = self.dt.topo, self.dt, self.ws, self.lib
         A = self._adj_buffers()
-        sc = self._adj_sched
-        if recompute:  # the reverse sweeps read every node's complete local
-            self.upward(stream)
-            self.downward(stream, cascade=True)
+        main = stream if stream is not None else torch.cuda.current_stream(dt.device)
+        far = self.far_stream() if self.overlap else main
+        s, fs = main.cuda_stream, far.cuda_stream
         w = w.to(device=dt.device, dtype=torch.float32).contiguous()
         _lib.check(lb.jb_gather_sorted(t.num_particles, _ptr(w), _ptr(A["zeros"]), _ptr(dt.perm), _ptr(A["w4"]), s),
                    "jb_gather_sorted(w)")
-        _zero(A["cbar4"], stream)
-        _zero(A["mbar"], stream)
+        if far is not main:
+            far.wait_stream(main)
+        sc = A["sched"]
         _lib.check(lb.jb_adj_near(_ptr(ws.pos4), _ptr(A["w4"]), t.num_internal, int(sc.units.shape[0]),
                                   _ptr(A["units"]), _ptr(A["aux"]), _ptr(A["runs"]), _ptr(dt.node_ranges), self.G,
                                   self.eps2, _ptr(A["xm4"]), _ptr(A["partials"]), int(sc.split.shape[0]),
                                   _ptr(A["split"]), s), "jb_adj_near")
+        if recompute or not self.own_locals:
+            self.upward(far)
+            self.downward(far, own=True)
+        _zero(A["mbar"], far)
+        _zero(A["chain4"], far)
         _lib.check(lb.jb_adj_leaf_far(self.p, _ptr(ws.pos4), _ptr(A["w4"]), t.num_nodes, t.num_internal,
-                                      _ptr(dt.node_ranges), _ptr(ws.centers), _ptr(ws.locals), self.G,
-                                      _ptr(A["xm4"]), _ptr(A["lbar"]), _ptr(A["cbar4"]), s), "jb_adj_leaf_far")
-        lo = dt.level_offsets
-        for lev in range(t.num_levels - 1, -1, -1):
-            _lib.check(lb.jb_adj_l2l_level(self.p, lo[lev], lo[lev + 1], _ptr(dt.left), _ptr(dt.right),
-                                           _ptr(ws.centers), _ptr(ws.locals), _ptr(A["lbar"]), _ptr(A["cbar4"]), s),
-                       "jb_adj_l2l_level")
-        if hasattr(self, "_adj_m2l"):
-            msc = self._adj_m2l
-        else:
-            mp = m2l_unit_limit(t.num_far_pairs)
-            msc = m2l_schedule_device(dt, max_pairs=mp) if _on_gpu(dt) else m2l_schedule(t, max_pairs=mp)
-            self._adj_m2l = msc
-            up = lambda a: _up(a, dt.device)
-            A["m2l_units"], A["m2l_split"] = up(msc.units), up(msc.split)
-            A["m2l_partials"] = torch.empty((max(msc.num_slots, 1), ws.stride), device=dt.device,
-                                            dtype=torch.float32)
+                                      _ptr(dt.node_ranges), _ptr(ws.centers), self._leaf_locals_ptr(), self.G,
+                                      _ptr(A["far4"]), _ptr(A["lbar"]), None, fs), "jb_adj_leaf_far")
+        items, offsets = dt.m2m_hops()
+        _lib.check(lb.jb_adj_l2l_hops(self.p, len(offsets) - 1, offsets.ctypes.data, _ptr(items), _ptr(ws.centers),
+                                      _ptr(A["lbar"]), fs), "jb_adj_l2l_hops")
+        msc = A["m2l"]
         _lib.check(lb.jb_adj_m2l(self.p, int(msc.units.shape[0]), _ptr(A["m2l_units"]), _ptr(A["lbar"]),
                                  _ptr(ws.centers), _ptr(dt.far_src), _ptr(A["mbar"]), _ptr(A["m2l_partials"]),
-                                 int(msc.split.shape[0]), _ptr(A["m2l_split"]), s), "jb_adj_m2l")
-        _lib.check(lb.jb_adj_m2l_centers(self.p, t.num_nodes, t.num_far_pairs, _ptr(A["pair_tgt"]),
-                                         _ptr(dt.far_src), _ptr(dt.far_off), _ptr(A["rev"]), _ptr(ws.mult),
-                                         _ptr(A["lbar"]), _ptr(ws.centers), _ptr(A["g4"]), _ptr(A["cbar4"]), s),
-                   "jb_adj_m2l_centers")
-        for lev in range(t.num_levels):
-            _lib.check(lb.jb_adj_m2m_level(self.p, lo[lev], lo[lev + 1], _ptr(dt.left), _ptr(dt.right),
-                                           _ptr(ws.centers), _ptr(ws.mult), _ptr(A["mbar"]), _ptr(A["cbar4"]), s),
-                       "jb_adj_m2m_level")
-        _lib.check(lb.jb_adj_p2m(self.p, _ptr(ws.pos4), t.num_nodes, t.num_internal, _ptr(dt.node_ranges),
-                                 _ptr(ws.centers), _ptr(A["mbar"]), _ptr(A["cbar4"]), _ptr(A["xm4"]), s),
-                   "jb_adj_p2m")
+                                 int(msc.split.shape[0]), _ptr(A["m2l_split"]), fs), "jb_adj_m2l")
+        _lib.check(lb.jb_adj_far_nodes(self.p, t.num_nodes, t.num_far_pairs, _ptr(A["pair_tgt"]), _ptr(dt.far_src),
+                                       _ptr(dt.far_off), _ptr(A["rev"]), _ptr(ws.mult), _ptr(A["lbar"]),
+                                       _ptr(ws.locals), _ptr(A["mbar"]), _ptr(ws.centers), _ptr(A["g4"]),
+                                       _ptr(A["cbar4"]), fs), "jb_adj_far_nodes")
+        _lib.check(lb.jb_adj_leaves(self.p, self.num_l2l_units, _ptr(self.d_l2l_units), _ptr(self.d_l2l_anc),
+                                    _ptr(dt.parent), _ptr(ws.centers), _ptr(A["cbar4"]), _ptr(A["mbar"]),
+                                    _ptr(A["chain4"]), fs), "jb_adj_leaves")
+        if far is not main:
+            main.wait_stream(far)
+        _lib.check(lb.jb_adj_particles(self.p, _ptr(ws.pos4), t.num_nodes, t.num_internal, _ptr(dt.node_ranges),
+                                       _ptr(ws.centers), _ptr(A["mbar"]), _ptr(A["cbar4"]), _ptr(A["chain4"]),
+                                       _ptr(A["far4"]), _ptr(A["xm4"]), s), "jb_adj_particles")
         _lib.check(lb.jb_gather_unsorted(t.num_particles, _ptr(A["xm4"]), _ptr(dt.inv_perm), _ptr(grad_pos),
                                          _ptr(grad_mass), s), "jb_gather_unsorted(grad)")
 
