@@ -1047,6 +1047,7 @@ struct NearAcc {
 };
 
 #define JB_PAD4 make_float4(1e18f, 1e18f, 1e18f, 0.f)
+#define JB_ZERO4 make_float4(0.f, 0.f, 0.f, 0.f)
 
 // Packed FP32x2 arithmetic (sm_100 add/sub/mul/fma .f32x2): one instruction
 // for two lanes of work, so the near-field loop handles two sources per step
@@ -1185,10 +1186,8 @@ template <int G, bool KAHAN, bool POT, bool W, bool FTZ>
 __device__ __forceinline__ void leaf_unit(const float4* __restrict__ pos4, int2 rg, int4 U, int2 aux,
                                           const int2* __restrict__ runs, NearStage& sP, int lane, float G_,
                                           float eps2, float4* __restrict__ out, float4* __restrict__ partial,
-                                          int max_slots, int* err, const int* __restrict__ rung = nullptr,
-                                          const float* tbl = nullptr, int nlw = 1, int2 lr = make_int2(0, -1),
-                                          int row = 0) {
-  if (lr.y < lr.x) lr = rg;
+                                          int max_slots, int* err, bool fresh, const int* __restrict__ rung,
+                                          const float* tbl, int nlw, int2 lr, int row) {
   const int tl = lane / G, h = lane % G;
   const int nt = rg.y - rg.x + 1;
   const bool active = tl < nt;
@@ -1245,8 +1244,7 @@ __device__ __forceinline__ void leaf_unit(const float4* __restrict__ pos4, int2 
   const float4 res = near_scaled(G_, v);
   if (active && h == 0) {
     if (aux.x < 0) {
-      const float4 f = out[rg.x + tl];  // the far field k_leaf_l2p wrote
-      out[rg.x + tl] = add_rn(f, res);
+      out[rg.x + tl] = add_rn(fresh ? JB_ZERO4 : out[rg.x + tl], res);  // to the far field k_leaf_l2p wrote
     } else if (aux.x < max_slots) {
       partial[(size_t)aux.x * kMaxLeaf + row + tl] = res;
     } else {
@@ -1255,8 +1253,18 @@ __device__ __forceinline__ void leaf_unit(const float4* __restrict__ pos4, int2 
   }
 }
 
+// A near field that starts from nothing: the first unit of a split leaf zeroes
+// the leaf's rows, which only the far field and the sum of the partial rows
+// write (whole leaves are written by their one unit).
+__device__ __forceinline__ void zero_split_leaf(int2 aux, int2 rg, int lane, float4* __restrict__ out) {
+  if (aux.x < 0 || !(aux.y & 1)) return;
+  for (int i = rg.x + lane; i <= rg.y; i += 32) out[i] = JB_ZERO4;
+}
+
 // Near field (P2P) of the work units, added to the far field already in out
-// (whole leaves) or written to the partial rows (split leaves).
+// (whole leaves) or written to the partial rows (split leaves).  fresh: out
+// holds nothing yet (JB_P2P_NEAR_ONLY, JB_P2P_NEAR_FIRST) and is only written:
+// a launch that zeroed it first, and a read of it, less.
 //
 // W: the block-step weighted form of the mutual lane -- every pair scaled by
 // lw[max(rung_i, rung_j)] (rung: per sorted particle, lw: nlw <= 32 weights).
@@ -1265,7 +1273,7 @@ template <bool KAHAN, bool POT, bool W = false, bool FTZ = true>
 static __global__ void __launch_bounds__(32 * kWarpsPerBlock, POT ? 6 : 8) k_leaf_units(
     const float4* __restrict__ pos4, int num_internal, int num_units, const int4* __restrict__ units,
     const int2* __restrict__ aux, const int2* __restrict__ runs, const int2* __restrict__ ranges, float G,
-    float eps2, float4* __restrict__ out, float4* __restrict__ partial, int max_slots, int* err,
+    float eps2, float4* __restrict__ out, float4* __restrict__ partial, int max_slots, int* err, bool fresh,
     const int* __restrict__ rung = nullptr, const float* __restrict__ lw = nullptr, int nlw = 1) {
   __shared__ NearStage sP[kWarpsPerBlock];
   __shared__ float tbl[32];
@@ -1284,19 +1292,20 @@ static __global__ void __launch_bounds__(32 * kWarpsPerBlock, POT ? 6 : 8) k_lea
     if (lane == 0) leaf_error(err, JB_LEAF_ERR_OCCUPANCY);
     return;
   }
+  if (fresh) zero_split_leaf(ax, rg, lane, out);
   for (int row = 0; row < ntl; row += 32) {  // a leaf of more than 32 particles in two passes
     const int2 rt = make_int2(rg.x + row, min(rg.y, rg.x + row + 31));
     const int nt = rt.y - rt.x + 1;
     if (row > 0) __syncwarp();  // the first pass's reads of the stage are done
     if (nt <= 8)
       leaf_unit<4, KAHAN, POT, W, FTZ>(pos4, rt, U, ax, runs, sP[warp], lane, G, eps2, out, partial, max_slots, err,
-                                       rung, tbl, nlw, rg, row);
+                                       fresh, rung, tbl, nlw, rg, row);
     else if (nt <= 16)
       leaf_unit<2, KAHAN, POT, W, FTZ>(pos4, rt, U, ax, runs, sP[warp], lane, G, eps2, out, partial, max_slots, err,
-                                       rung, tbl, nlw, rg, row);
+                                       fresh, rung, tbl, nlw, rg, row);
     else
       leaf_unit<1, KAHAN, POT, W, FTZ>(pos4, rt, U, ax, runs, sP[warp], lane, G, eps2, out, partial, max_slots, err,
-                                       rung, tbl, nlw, rg, row);
+                                       fresh, rung, tbl, nlw, rg, row);
   }
 }
 
@@ -1411,7 +1420,7 @@ template <bool KAHAN, bool POT>
 __device__ __forceinline__ void leaf_unit_flat(const float4* __restrict__ pos4, int2 rg, int4 U, int2 aux,
                                                const int2* __restrict__ runs, FlatStage& S, int lane, float G_,
                                                float eps2, float4* __restrict__ out, float4* __restrict__ partial,
-                                               int max_slots, int* err, int2 lr, int row) {
+                                               int max_slots, int* err, bool fresh, int2 lr, int row) {
   constexpr int CH = kFlatChunk;
   const int nt = rg.y - rg.x + 1;  // 17..32 targets (the leaf lr, or one of its halves)
   const bool tgt = lane < nt;
@@ -1533,8 +1542,7 @@ __device__ __forceinline__ void leaf_unit_flat(const float4* __restrict__ pos4, 
     for (int i = 0; i < 4; ++i) v[i] = (POT || i < 3) ? a.value(i) : 0.f;
     const float4 res = near_scaled(G_, v);
     if (aux.x < 0) {
-      const float4 f = out[rg.x + lane];  // the far field k_leaf_l2p wrote
-      out[rg.x + lane] = add_rn(f, res);
+      out[rg.x + lane] = add_rn(fresh ? JB_ZERO4 : out[rg.x + lane], res);  // to the far field k_leaf_l2p wrote
     } else if (aux.x < max_slots) {
       partial[(size_t)aux.x * kMaxLeaf + row + lane] = res;
     } else {
@@ -1550,7 +1558,7 @@ template <bool KAHAN, bool POT>
 static __global__ void __launch_bounds__(32 * kWarpsPerBlock, POT ? 6 : 8) k_leaf_units_flat(
     const float4* __restrict__ pos4, int num_internal, int num_units, const int4* __restrict__ units,
     const int2* __restrict__ aux, const int2* __restrict__ runs, const int2* __restrict__ ranges, float G,
-    float eps2, float4* __restrict__ out, float4* __restrict__ partial, int max_slots, int* err) {
+    float eps2, float4* __restrict__ out, float4* __restrict__ partial, int max_slots, int* err, bool fresh) {
   __shared__ WarpStage sW[kWarpsPerBlock];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int u = blockIdx.x * kWarpsPerBlock + warp;
@@ -1563,19 +1571,20 @@ static __global__ void __launch_bounds__(32 * kWarpsPerBlock, POT ? 6 : 8) k_lea
     if (lane == 0) leaf_error(err, JB_LEAF_ERR_OCCUPANCY);
     return;
   }
+  if (fresh) zero_split_leaf(ax, rg, lane, out);
   for (int row = 0; row < ntl; row += 32) {  // a leaf of more than 32 particles in two passes
     const int2 rt = make_int2(rg.x + row, min(rg.y, rg.x + row + 31));
     const int nt = rt.y - rt.x + 1;
     if (row > 0) __syncwarp();  // the first pass's reads of the stage are done
     if (nt <= 8)
       leaf_unit<4, KAHAN, POT, false, true>(pos4, rt, U, ax, runs, sW[warp].n, lane, G, eps2, out, partial,
-                                            max_slots, err, nullptr, nullptr, 1, rg, row);
+                                            max_slots, err, fresh, nullptr, nullptr, 1, rg, row);
     else if (nt <= 16)
       leaf_unit<2, KAHAN, POT, false, true>(pos4, rt, U, ax, runs, sW[warp].n, lane, G, eps2, out, partial,
-                                            max_slots, err, nullptr, nullptr, 1, rg, row);
+                                            max_slots, err, fresh, nullptr, nullptr, 1, rg, row);
     else
-      leaf_unit_flat<KAHAN, POT>(pos4, rt, U, ax, runs, sW[warp].f, lane, G, eps2, out, partial, max_slots, err, rg,
-                                 row);
+      leaf_unit_flat<KAHAN, POT>(pos4, rt, U, ax, runs, sW[warp].f, lane, G, eps2, out, partial, max_slots, err, fresh,
+                                 rg, row);
   }
 }
 
@@ -1584,11 +1593,10 @@ static __global__ void __launch_bounds__(32 * kWarpsPerBlock, POT ? 6 : 8) k_lea
 // out = -G (grad phi, phi); runs before k_leaf_units, which adds the near
 // field.  Kept out of the near-field kernel so that kernel's register count
 // is set by the P2P loop alone (about half, and twice the resident warps).
-// mode kL2PZero: write zeros instead (the near field alone, JB_P2P_NEAR_ONLY
-// and JB_P2P_NEAR_FIRST); kL2PAdd: add the far field to what out holds (the
-// near field a JB_P2P_NEAR_FIRST launch wrote), with the rounding of the
-// near-field kernel's own add.
-enum { kL2PWrite = 0, kL2PZero = 1, kL2PAdd = 2 };
+// mode kL2PAdd: add the far field to what out holds (the near field a
+// JB_P2P_NEAR_FIRST launch wrote), with the rounding of the near-field kernel's
+// own add.
+enum { kL2PWrite = 0, kL2PAdd = 1 };
 template <int P>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_leaf_l2p(
     const float4* __restrict__ pos4, int num_internal, int num_units, const int4* __restrict__ units,
@@ -1602,10 +1610,6 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_leaf_l2p(
   const int node = num_internal + units[u].x;
   const int2 rg = ranges[node];
   if (rg.y - rg.x + 1 > kMaxLeaf) return;  // refused by the near-field kernel, which flags it
-  if (mode == kL2PZero) {  // near field alone: the sums start from zero
-    for (int i = rg.x + lane; i <= rg.y; i += 32) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    return;
-  }
   // the first particle and the centre are fetched alongside the local's staging
   const float4 c = centers[node];
   const float4 t0 = (rg.x + lane <= rg.y) ? pos4[rg.x + lane] : c;
@@ -1892,7 +1896,7 @@ struct RunLeafEval {
   template <bool K, bool PT>
   static void go(unsigned nb, cudaStream_t st, const float4* pos4, int num_internal, int num_units, const int4* units,
                  const int2* aux, const int2* runs, const int2* ranges, float G, float eps2, float4* out,
-                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err);
+                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err, bool fresh);
   static int run(int mode, const float* pos4, int num_internal, int num_units, const int* units, const int* aux,
                  const int* runs, const int* ranges, const float* centers, const float* locals, float G, float eps2,
                  float* out, float* partial, int num_split, const int* split, cudaStream_t st,
@@ -1904,10 +1908,10 @@ template <int P>
 template <bool K, bool PT>
 void RunLeafEval<P>::go(unsigned nb, cudaStream_t st, const float4* pos4, int num_internal, int num_units, const int4* units,
                  const int2* aux, const int2* runs, const int2* ranges, float G, float eps2, float4* out,
-                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err) {
+                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err, bool fresh) {
   if (rung)
     k_leaf_units<K, PT, true><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
-                                                                  ranges, G, eps2, out, partial, max_slots, err,
+                                                                  ranges, G, eps2, out, partial, max_slots, err, fresh,
                                                                   rung, lw, nlw);
   else if (flat) {
     // 23.5 KB of shared memory per block: ask for the carveout that holds
@@ -1916,11 +1920,11 @@ void RunLeafEval<P>::go(unsigned nb, cudaStream_t st, const float4* pos4, int nu
         k_leaf_units_flat<K, PT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     (void)carve;
     k_leaf_units_flat<K, PT><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
-                                                                 ranges, G, eps2, out, partial, max_slots, err);
+                                                                 ranges, G, eps2, out, partial, max_slots, err, fresh);
   }
   else
     k_leaf_units<K, PT><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs, ranges,
-                                                            G, eps2, out, partial, max_slots, err);
+                                                            G, eps2, out, partial, max_slots, err, fresh);
 }
 
 template <int P>
@@ -1939,19 +1943,22 @@ int RunLeafEval<P>::run(int mode, const float* pos4, int num_internal, int num_u
     auto o = reinterpret_cast<float4*>(out);
     auto pt = reinterpret_cast<float4*>(partial);
     const bool far_only = (mode & JB_P2P_FAR_ONLY) != 0, far_after = (mode & JB_P2P_FAR_AFTER) != 0;
-    const bool zero = (mode & (JB_P2P_NEAR_ONLY | JB_P2P_NEAR_FIRST)) != 0;
-    k_leaf_l2p<P><<<nb, 32 * kWarpsPerBlock, 0, st>>>(a0, num_internal, num_units, a1, a2, a4,
-                                                      reinterpret_cast<const float4*>(centers), locals, G, o,
-                                                      zero ? kL2PZero : far_after ? kL2PAdd : kL2PWrite);
-    int rc = launch_status();
-    if (rc) return rc;
+    const bool fresh = (mode & (JB_P2P_NEAR_ONLY | JB_P2P_NEAR_FIRST)) != 0;
+    int rc = JB_OK;
+    if (!fresh) {
+      k_leaf_l2p<P><<<nb, 32 * kWarpsPerBlock, 0, st>>>(a0, num_internal, num_units, a1, a2, a4,
+                                                        reinterpret_cast<const float4*>(centers), locals, G, o,
+                                                        far_after ? kL2PAdd : kL2PWrite);
+      rc = launch_status();
+      if (rc) return rc;
+    }
     if (far_only) return JB_OK;
     if (!far_after) {  // FAR_AFTER: the near field is already in out (and partials)
       const bool kahan = (mode & JB_P2P_KAHAN) != 0, pot = (mode & JB_P2P_POTENTIAL) != 0;
-      if (kahan && pot) go<true, true>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
-      else if (kahan) go<true, false>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
-      else if (pot) go<false, true>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
-      else go<false, false>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
+      if (kahan && pot) go<true, true>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err, fresh);
+      else if (kahan) go<true, false>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err, fresh);
+      else if (pot) go<false, true>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err, fresh);
+      else go<false, false>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err, fresh);
       rc = launch_status();
       if (rc) return rc;
     }
