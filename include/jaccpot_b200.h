@@ -458,6 +458,14 @@ JB_API int jb_l2l_leaves_to(int p, int num_units, const int* units, const int* a
  * particles (check once with jb_validate_leaves; a unit breaking it writes
  * nothing and sets JB_LEAF_ERR_OCCUPANCY), and partials holds
  * JB_MAX_LEAF_OCCUPANCY float4 per slot for every slot in aux / split. */
+/* Weights of jb_m2l_weighted for block steps: far_w[e] = level_weights[max of
+ * the two nodes' rungs, clamped to the table], a node's rung being the finest
+ * (largest) of its particles' (rung per sorted particle).  scratch is
+ * int32[num_nodes + num_internal].                                          */
+JB_API int jb_far_level_weights(int num_nodes, int num_internal, const int* node_ranges, const int* parent,
+                                const int* rung, const int64_t* far_off, const int* far_src, int num_level_weights,
+                                const float* level_weights, int* scratch, float* far_w, void* stream);
+
 /* jb_leaf_eval with every particle pair scaled by
  * level_weights[max(rung_i, rung_j)] (rung: int32 per SORTED particle,
  * clamped to [0, num_level_weights); num_level_weights <= 32; device

@@ -336,6 +336,44 @@ __global__ void k_adj_m2l_gather(int num_nodes, const int64_t* __restrict__ far_
   cbar4[u] = c;
 }
 
+// ---------------------------------------------------------------------------
+// Block-step weights of the far pairs (mutual lane): a node's rung is the finest
+// of its particles', a pair's weight level_weights[max of the two, clamped].
+// ---------------------------------------------------------------------------
+// Thread per leaf climbing: the second child to arrive carries the maximum on.
+__global__ void k_node_rungs(int num_internal, int num_nodes, const int2* __restrict__ ranges,
+                             const int* __restrict__ parent, const int* __restrict__ rung, int* node_rung,
+                             int* arrived) {
+  int node = num_internal + blockIdx.x * blockDim.x + threadIdx.x;
+  if (node >= num_nodes) return;
+  const int2 rg = ranges[node];
+  int r = -1;
+  for (int i = rg.x; i <= rg.y; ++i) r = max(r, rung[i]);
+  node_rung[node] = r;
+  for (;;) {
+    node = parent[node];
+    if (node < 0) return;
+    atomicMax(node_rung + node, r);
+    __threadfence();  // this child's rung before its arrival
+    if (atomicAdd(arrived + node, 1) == 0) return;
+    __threadfence();
+    r = atomicMax(node_rung + node, -1);
+  }
+}
+
+// Warp per target node.
+__global__ void __launch_bounds__(128) k_far_level_weights(int num_nodes, const int64_t* __restrict__ far_off,
+                                                           const int* __restrict__ far_src,
+                                                           const int* __restrict__ node_rung, int num_weights,
+                                                           const float* __restrict__ level_weights,
+                                                           float* __restrict__ far_w) {
+  const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= num_nodes) return;
+  const int rt = node_rung[t];
+  for (int64_t e = far_off[t] + lane; e < far_off[t + 1]; e += 32)
+    far_w[e] = level_weights[min(max(max(rt, node_rung[far_src[e]]), 0), num_weights - 1)];
+}
+
 static inline unsigned blocks_1d(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
 
 }  // namespace jb
@@ -654,6 +692,26 @@ JB_API int jb_l2l_level(int p, int first, int last, const int* left, const int* 
   return dispatch<RunL2L>(p, first, last, left, right, centers, locals, ST(stream));
 }
 
+JB_API int jb_far_level_weights(int num_nodes, int num_internal, const int* node_ranges, const int* parent,
+                                const int* rung, const int64_t* far_off, const int* far_src, int num_level_weights,
+                                const float* level_weights, int* scratch, float* far_w, void* stream) {
+  if (num_nodes < 1 || num_internal < 0 || num_internal >= num_nodes || !node_ranges || !parent || !rung || !far_off ||
+      !far_src || num_level_weights < 1 || !level_weights || !scratch || !far_w)
+    return JB_ERR_ARG;
+  int* arrived = scratch + num_nodes;
+  cudaError_t e = cudaMemsetAsync(scratch, 0xff, sizeof(int) * (size_t)num_nodes, ST(stream));  // rung -1
+  if (e == cudaSuccess && num_internal > 0)
+    e = cudaMemsetAsync(arrived, 0, sizeof(int) * (size_t)num_internal, ST(stream));
+  if (e != cudaSuccess) return cuda_status(e);
+  k_node_rungs<<<blocks_1d(num_nodes - num_internal, 128), 128, 0, ST(stream)>>>(
+      num_internal, num_nodes, reinterpret_cast<const int2*>(node_ranges), parent, rung, scratch, arrived);
+  const int rc = launch_status();
+  if (rc) return rc;
+  k_far_level_weights<<<blocks_1d(num_nodes, 4), 128, 0, ST(stream)>>>(num_nodes, far_off, far_src, scratch,
+                                                                       num_level_weights, level_weights, far_w);
+  return launch_status();
+}
+
 JB_API int jb_leaf_eval_weighted(int p, int p2p_mode, const float* pos4, const int* rung, int num_level_weights,
                                  const float* level_weights, int num_internal, int num_units, const int* units,
                                  const int* aux, const int* runs, const int* node_ranges, const float* centers,
@@ -664,8 +722,9 @@ JB_API int jb_leaf_eval_weighted(int p, int p2p_mode, const float* pos4, const i
       (num_units > 0 && (!pos4 || !units || !aux || !runs || !node_ranges || !centers || !locals || !out_acc4)) ||
       (num_split > 0 && (!split || !partials || !out_acc4 || !node_ranges)))
     return JB_ERR_ARG;
-  if (p2p_mode & ~(JB_P2P_KAHAN | JB_P2P_POTENTIAL | JB_P2P_FAR_ONLY | JB_P2P_NEAR_ONLY)) return JB_ERR_ARG;
-  if ((p2p_mode & JB_P2P_FAR_ONLY) && (p2p_mode & JB_P2P_NEAR_ONLY)) return JB_ERR_ARG;
+  constexpr int parts = JB_P2P_FAR_ONLY | JB_P2P_NEAR_ONLY | JB_P2P_NEAR_FIRST | JB_P2P_FAR_AFTER;
+  if (p2p_mode & ~(JB_P2P_KAHAN | JB_P2P_POTENTIAL | parts)) return JB_ERR_ARG;
+  if (__builtin_popcount(p2p_mode & parts) > 1) return JB_ERR_ARG;  // at most one of the four
   int* err = nullptr;
   const int rc = leaf_error_word(&err);
   if (rc != JB_OK) return rc;

@@ -454,7 +454,7 @@ class Pass:
         q.leaf_partials = torch.empty_like(self.leaf_partials)
         if getattr(self, "gear_sched", None) is not None:
             q.gear_partials = torch.empty_like(self.gear_partials)
-        for name in ("_tc", "_tc_status", "_adj", "_far_stream", "_leaf_rows"):
+        for name in ("_tc", "_tc_status", "_adj", "_far_stream", "_leaf_rows", "_weights"):
             q.__dict__.pop(name, None)
         q.own_locals = False
         return q
@@ -576,6 +576,40 @@ class Pass:
                                             _ptr(ws.locals), _ptr(self.m2l_partials), int(sc.split.shape[0]),
                                             _ptr(self.d_m2l_split), s), "jb_m2l_weighted")
 
+    def far_level_weights(self, rung_sorted: torch.Tensor, level_weights: torch.Tensor, stream=None) -> torch.Tensor:
+        """float32 per CSR far entry: level_weights at the finer of the two
+        nodes' rungs (a node's rung is its particles' finest), the same for both
+        directions of a pair (force.py:885, :920 there)."""
+        t, dt = self.dt.topo, self.dt
+        f = self._weight_buffers()
+        _lib.check(self.lib.jb_far_level_weights(t.num_nodes, t.num_internal, _ptr(dt.node_ranges), _ptr(dt.parent),
+                                                 _ptr(rung_sorted), _ptr(dt.far_off), _ptr(dt.far_src),
+                                                 int(level_weights.numel()), _ptr(level_weights), _ptr(f["scratch"]),
+                                                 _ptr(f["far_w"]), _stream_handle(stream)), "jb_far_level_weights")
+        return f["far_w"][:t.num_far_pairs]
+
+    def _weight_buffers(self) -> dict:
+        if getattr(self, "_weights", None) is None:
+            t, dev = self.dt.topo, self.dt.device
+            self._weights = {"scratch": torch.empty(t.num_nodes + t.num_internal, device=dev, dtype=torch.int32),
+                             "far_w": torch.empty(max(t.num_far_pairs, 1), device=dev, dtype=torch.float32)}
+        return self._weights
+
+    def run_weighted(self, rung_sorted: torch.Tensor, level_weights: torch.Tensor) -> torch.Tensor:
+        """run() with every pair scaled by its level's weight: the near field on
+        the current stream beside the far-field chain on far_stream()."""
+        main = torch.cuda.current_stream(self.dt.device)
+        far = self.far_stream() if self.overlap else main
+        if far is not main:
+            far.wait_stream(main)
+        self.evaluate_weighted(rung_sorted, level_weights, main, part="near_first")
+        self.upward(far)
+        self.m2l_weighted(self.far_level_weights(rung_sorted, level_weights, far), far)
+        self.l2l(far)
+        if far is not main:
+            main.wait_stream(far)
+        return self.evaluate_weighted(rung_sorted, level_weights, main, part="far_after")
+
     def evaluate_weighted(self, rung_sorted: torch.Tensor, level_weights: torch.Tensor, stream=None,
                           part: str | None = None) -> torch.Tensor:
         """evaluate() with every near pair scaled by
@@ -585,7 +619,7 @@ class Pass:
         lw = level_weights.to(device=dt.device, dtype=torch.float32).contiguous()
         mode = self.p2p_mode
         if part is not None:
-            mode |= {"near": _lib.JB_P2P_NEAR_ONLY, "far": _lib.JB_P2P_FAR_ONLY}[part]
+            mode |= self._PARTS[part]
         _lib.check(self.lib.jb_leaf_eval_weighted(self.p, mode, _ptr(ws.pos4), _ptr(r), int(lw.numel()), _ptr(lw),
                                                   t.num_internal, int(sc.units.shape[0]), _ptr(self.d_leaf_units),
                                                   _ptr(self.d_leaf_aux), _ptr(self.d_leaf_runs),

@@ -169,33 +169,6 @@ def _unsort(sorted_rows: torch.Tensor, perm: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def _node_rungs(dt: DeviceTopology, rung_sorted: torch.Tensor) -> torch.Tensor:
-    """Rung of every node: the finest (largest) rung of its particles, leaves
-    first, then up the levels (force.py:885 _cell_rungs there)."""
-    t = dt.topo
-    node = torch.full((t.num_nodes,), -1, dtype=torch.int32, device=rung_sorted.device)
-    leaf = torch.full((t.num_leaves,), -1, dtype=torch.int32, device=rung_sorted.device)
-    leaf = leaf.scatter_reduce(0, dt.leaf_of.long(), rung_sorted, reduce="amax", include_self=True)
-    node[t.num_internal:] = leaf
-    left, right, lo = dt.left.long(), dt.right.long(), dt.level_offsets
-    for lev in range(t.num_levels - 1, -1, -1):
-        a, b = lo[lev], lo[lev + 1]
-        if b > a:
-            node[a:b] = torch.maximum(node[left[a:b]], node[right[a:b]])
-    return node
-
-
-def _far_pair_weights(dt: DeviceTopology, node_rung: torch.Tensor, lw: torch.Tensor) -> torch.Tensor:
-    """Weight of every directed far entry: lw[max(rung_a, rung_b)], the same
-    for both directions of a pair (force.py:920 there)."""
-    t = dt.topo
-    counts = (dt.far_off[1:] - dt.far_off[:-1]).long()
-    tgt = torch.repeat_interleave(torch.arange(t.num_nodes, device=lw.device), counts)
-    src = dt.far_src[: t.num_far_pairs].long()
-    lev = torch.maximum(node_rung[tgt], node_rung[src]).clamp(0, lw.numel() - 1).long()
-    return lw[lev]
-
-
 def mutual_weighted_accelerations(state: MutualFMMState, positions, masses, *, rung=None, level_weights=None,
                                   return_parts: bool = False):
     """sum_k level_weights[k] * a_k in one traversal (force.py:985 there):
@@ -215,31 +188,36 @@ def mutual_weighted_accelerations(state: MutualFMMState, positions, masses, *, r
     mass = torch.as_tensor(masses).to(device=dev, dtype=torch.float32)
     perm = dt.perm
     ps.load_particles(pos, mass)
-    ps.upward()
-    if rung is None:
-        ps.m2l()
-        ps.l2l()
-        ev = lambda part=None: ps.evaluate(part=part)
-    else:
+    lw = None
+    if rung is not None:
         lw = torch.as_tensor(np.asarray(level_weights, dtype=np.float32) if not isinstance(level_weights, torch.Tensor)
                              else level_weights).to(device=dev, dtype=torch.float32).reshape(-1)
         if not 1 <= lw.numel() <= 32:
             raise ValueError("between 1 and 32 level weights")
         r_sorted = torch.as_tensor(rung).to(device=dev, dtype=torch.int32).reshape(-1)[perm].contiguous()
-        ps.m2l_weighted(_far_pair_weights(dt, _node_rungs(dt, r_sorted), lw))
-        ps.l2l()
-        ev = lambda part=None: ps.evaluate_weighted(r_sorted, lw, part=part)
-    m_sorted = mass[perm]
-    if return_parts:
-        near_a = ev("near")[:, :3].clone()
-        far_a = ev("far")[:, :3].clone()
-        acc = near_a + far_a
+    if not return_parts:
+        if lw is None:
+            ps.run()
+        else:
+            ps.run_weighted(r_sorted, lw)
+        out = torch.empty((state.topology.num_particles, 3), device=dev, dtype=torch.float32)
+        ps.unsort(out, None)
+        out = torch.where(mass[:, None] > 0, out, 0.0)
+        return out.cpu().numpy() if want_np else out
+    ps.upward()
+    if lw is None:
+        ps.downward()
+        ev = lambda part: ps.evaluate(part=part)
     else:
-        acc = ev()[:, :3].clone()
+        ps.m2l_weighted(ps.far_level_weights(r_sorted, lw))
+        ps.l2l()
+        ev = lambda part: ps.evaluate_weighted(r_sorted, lw, part=part)
+    m_sorted = mass[perm]
+    near_a = ev("near")[:, :3].clone()
+    far_a = ev("far")[:, :3].clone()
+    acc = near_a + far_a
     acc = torch.where(m_sorted[:, None] > 0, acc, torch.zeros_like(acc))
     out = _unsort(acc, perm)
-    if not return_parts:
-        return out.cpu().numpy() if want_np else out
     near_f = _unsort(m_sorted[:, None] * near_a, perm)
     far_f = _unsort(m_sorted[:, None] * far_a, perm)
     if want_np:
