@@ -66,15 +66,24 @@ __global__ void k_row_counts(const int64_t* __restrict__ off, int rows, int64_t*
 
 __global__ void k_max64(const int64_t* __restrict__ v, int64_t n, unsigned long long* __restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) atomicMax(out, (unsigned long long)v[i]);
+  unsigned long long m = i < n ? (unsigned long long)v[i] : 0ull;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(kFull, m, o));
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);  // one per warp: 64 us at 95k nodes with one per thread
 }
 
-// Expands CSR offsets into the row of every entry (thread per row).
+// Expands CSR offsets into the row of every entry (warp per row).
 __global__ void k_expand_rows(const int64_t* __restrict__ off, int r0, int r1, int64_t base, int* __restrict__ row) {
-  const int r = r0 + blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = r0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (r >= r1) return;
-  for (int64_t e = off[r]; e < off[r + 1]; ++e) row[e - base] = r;
+  for (int64_t e = off[r] + (threadIdx.x & 31); e < off[r + 1]; e += 32) row[e - base] = r;
 }
+
+// The result words as one read-back takes them.
+struct Totals {
+  int64_t w64[4];
+  int w32[8];
+};
 
 int* tot32(Scratch& s) { return reinterpret_cast<int*>(s.total.as<int64_t>() + 4); }
 
@@ -88,7 +97,8 @@ __global__ void k_count_keys(const int64_t* __restrict__ cnt, int n, int64_t max
 
 __global__ void k_count_nonempty(const int64_t* __restrict__ cnt, int n, int* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && cnt[i] > 0) atomicAdd(out, 1);
+  const unsigned have = __ballot_sync(kFull, i < n && cnt[i] > 0);
+  if ((threadIdx.x & 31) == 0 && have) atomicAdd(out, __popc(have));
 }
 
 __global__ void k_flag_nonempty(const int* __restrict__ tg, int n, const int64_t* __restrict__ cnt, int* __restrict__ flag) {
@@ -161,16 +171,15 @@ void build_m2l(jb_dsched& d, int num_nodes, const int64_t* far_off, int max_pair
       ck_launch();
     }
   } else if (num_nodes > 0) {  // every node with far pairs, longest list first (stable)
-    DBuf mx, key0, key1, v1;
-    ck(mx.alloc(8));
-    ck(cudaMemsetAsync(mx.p, 0, 8, st));
-    k_max64<<<nblocks(num_nodes, 256), 256, 0, st>>>(cnt.as<int64_t>(), num_nodes, mx.as<unsigned long long>());
+    DBuf key0, key1, v1;
+    ck(cudaMemsetAsync(s.total.p, 0, 64, st));
+    k_max64<<<nblocks(num_nodes, 256), 256, 0, st>>>(cnt.as<int64_t>(), num_nodes, s.total.as<unsigned long long>());
     ck_launch();
-    ck(cudaMemsetAsync(d_tot, 0, 4, st));
     k_count_nonempty<<<nblocks(num_nodes, 256), 256, 0, st>>>(cnt.as<int64_t>(), num_nodes, d_tot);
     ck_launch();
-    const int64_t maxc = (int64_t)read_word(mx.as<unsigned long long>(), st);
-    T = read_word(d_tot, st);
+    const Totals got = read_word(s.total.as<Totals>(), st);
+    const int64_t maxc = got.w64[0];
+    T = got.w32[0];
     ck(key0.alloc((size_t)num_nodes * 8));
     ck(key1.alloc((size_t)num_nodes * 8));
     ck(tg.alloc((size_t)num_nodes * 4));
@@ -224,7 +233,6 @@ void build_m2l(jb_dsched& d, int num_nodes, const int64_t* far_off, int max_pair
   k_m2l_split<<<nblocks(T, 256), 256, 0, st>>>(tg.as<int>(), T, nu.as<int>(), multi.as<int>(), split_pos.as<int>(),
                                                slot_base.as<int>(), d.split.as<int4>());
   ck_launch();
-  ck(cudaStreamSynchronize(st));
 }
 
 // ---------------------------------------------------------------------------
@@ -336,11 +344,6 @@ __global__ void k_place_lone(const int64_t* __restrict__ near_off, int lo, int h
   work[pos] = leaf_count(ranges, num_internal, j);
 }
 
-__global__ void k_max32(const int* __restrict__ v, int n, int* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) atomicMax(out, v[i]);
-}
-
 __global__ void k_work_keys(const int* __restrict__ work, int n, int maxw, uint64_t* __restrict__ key) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) key[i] = (uint64_t)(maxw - work[i]);
@@ -357,7 +360,9 @@ __global__ void k_leaf_max_occ(const int* __restrict__ ranges, int num_internal,
   const int j = lo + blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= hi) return;
   const int n = num_internal + j;
-  atomicMax(occ, ranges[2 * n + 1] - ranges[2 * n] + 1);
+  const unsigned peers = __activemask();
+  const int m = __reduce_max_sync(peers, ranges[2 * n + 1] - ranges[2 * n] + 1);
+  if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicMax(occ, m);
 }
 
 void build_leaf(jb_dsched& d, int num_internal, const int* ranges, const int64_t* near_off, const int* near_src, int lo,
@@ -368,16 +373,16 @@ void build_leaf(jb_dsched& d, int num_internal, const int* ranges, const int64_t
   int64_t* d_tot64 = s.total.as<int64_t>();
   const int NL = hi - lo;
   // the leaf kernels hold at most kMaxLeafOcc targets per leaf: refuse more
+  ck(cudaMemsetAsync(s.total.p, 0, 64, st));
   if (NL > 0) {
-    ck(cudaMemsetAsync(d_tot, 0, sizeof(int), st));
     k_leaf_max_occ<<<nblocks(NL, 256), 256, 0, st>>>(ranges, num_internal, lo, hi, d_tot);
     ck_launch();
-    if (read_word(d_tot, st) > kMaxLeafOcc) throw Fail{JB_ERR_ARG};
   }
-  int64_t ends[2] = {0, 0};
-  ck(cudaMemcpyAsync(&ends[0], near_off + lo, 8, cudaMemcpyDeviceToHost, st));
-  ck(cudaMemcpyAsync(&ends[1], near_off + hi, 8, cudaMemcpyDeviceToHost, st));
-  ck(cudaStreamSynchronize(st));
+  ck(cudaMemcpyAsync(d_tot64, near_off + lo, 8, cudaMemcpyDeviceToDevice, st));
+  ck(cudaMemcpyAsync(d_tot64 + 1, near_off + hi, 8, cudaMemcpyDeviceToDevice, st));
+  const Totals head = read_word(s.total.as<Totals>(), st);
+  if (head.w32[0] > kMaxLeafOcc) throw Fail{JB_ERR_ARG};
+  const int64_t* ends = head.w64;
   const int64_t e0 = ends[0], E = ends[1] - ends[0];
   DBuf tgt, w, cs, uil, brk, rpos, rfirst, runs_raw, run_tgt, run_uil, ubrk, upos, ufirst, eu, n_per, first_u;
   int R = 0, Ue = 0;
@@ -393,7 +398,7 @@ void build_leaf(jb_dsched& d, int num_internal, const int* ranges, const int64_t
     ck(uil.alloc(e * 4));
     ck(brk.alloc(e * 4));
     ck(rpos.alloc(e * 4));
-    k_expand_rows<<<nblocks(NL, 128), 128, 0, st>>>(near_off, lo, hi, e0, tgt.as<int>());
+    k_expand_rows<<<nblocks(NL, 4), 128, 0, st>>>(near_off, lo, hi, e0, tgt.as<int>());
     ck_launch();
     k_edge_w<<<nblocks(E, 256), 256, 0, st>>>(near_src, e0, E, ranges, num_internal, w.as<int64_t>());
     ck_launch();
@@ -402,8 +407,9 @@ void build_leaf(jb_dsched& d, int num_internal, const int* ranges, const int64_t
                                                 max_sources, uil.as<int>(), brk.as<int>());
     ck_launch();
     exclusive_scan<int>(brk.as<int>(), rpos.as<int>(), E, d_tot, s, st);
-    total_w = read_word(d_tot64, st);
-    R = read_word(d_tot, st);
+    const Totals got = read_word(s.total.as<Totals>(), st);
+    total_w = got.w64[0];
+    R = got.w32[0];
     ck(rfirst.alloc((size_t)R * 4));
     k_mark<<<nblocks(E, 256), 256, 0, st>>>(brk.as<int>(), rpos.as<int>(), E, rfirst.as<int>());
     ck_launch();
@@ -453,7 +459,7 @@ void build_leaf(jb_dsched& d, int num_internal, const int* ranges, const int64_t
   d.info.num_units = U;
   d.info.num_slots = tot[1];
   d.info.num_split = S;
-  DBuf cu, ca, work, mx, k0, k1, idx0, idx1;
+  DBuf cu, ca, work, k0, k1, idx0, idx1;
   ck(cu.alloc((size_t)U * 16));
   ck(ca.alloc((size_t)U * 8));
   ck(work.alloc((size_t)U * 4));
@@ -466,11 +472,9 @@ void build_leaf(jb_dsched& d, int num_internal, const int* ranges, const int64_t
   k_place_lone<<<nblocks(NL, 256), 256, 0, st>>>(near_off, lo, hi, base.as<int>(), ranges, num_internal, cu.as<int4>(),
                                                  ca.as<int2>(), work.as<int>());
   ck_launch();
-  ck(mx.alloc(4));
-  ck(cudaMemsetAsync(mx.p, 0, 4, st));
-  k_max32<<<nblocks(U, 256), 256, 0, st>>>(work.as<int>(), U, mx.as<int>());
-  ck_launch();
-  const int maxw = read_word(mx.as<int>(), st);
+  // no unit holds more: its sources end with the leaf that crosses
+  // max_sources, and the first has the leaf itself
+  const int maxw = (int)std::min<int64_t>((int64_t)max_sources + 2 * kMaxLeafOcc, 0x7fffffff);
   ck(k0.alloc((size_t)U * 8));
   ck(k1.alloc((size_t)U * 8));
   ck(idx0.alloc((size_t)U * 4));
@@ -491,7 +495,6 @@ void build_leaf(jb_dsched& d, int num_internal, const int* ranges, const int64_t
   k_leaf_split<<<nblocks(NL, 256), 256, 0, st>>>(NL, lo, n_per.as<int>(), spos.as<int>(), slot_base.as<int>(),
                                                  d.split.as<int4>());
   ck_launch();
-  ck(cudaStreamSynchronize(st));
 }
 
 // ---------------------------------------------------------------------------
@@ -610,7 +613,7 @@ void build_gears(jb_dsched& d, int num_nodes, const int64_t* far_off, const int*
   }
   DBuf row, k0, k1, v0, v1, brk, spos, sfirst, nu, unit_off;
   ck(row.alloc((size_t)P * 4));
-  k_expand_rows<<<nblocks(num_nodes, 128), 128, 0, st>>>(far_off, 0, num_nodes, 0, row.as<int>());
+  k_expand_rows<<<nblocks(num_nodes, 4), 128, 0, st>>>(far_off, 0, num_nodes, 0, row.as<int>());
   ck_launch();
   ck(k0.alloc((size_t)P * 8));
   ck(k1.alloc((size_t)P * 8));
@@ -802,7 +805,7 @@ void build_gears_mixed(jb_dsched& d, int num_nodes, const int64_t* far_off, cons
   }
   DBuf row, k0, k1, v0, v1;
   ck(row.alloc((size_t)P * 4));
-  k_expand_rows<<<nblocks(num_nodes, 128), 128, 0, st>>>(far_off, 0, num_nodes, 0, row.as<int>());
+  k_expand_rows<<<nblocks(num_nodes, 4), 128, 0, st>>>(far_off, 0, num_nodes, 0, row.as<int>());
   ck_launch();
   ck(k0.alloc((size_t)P * 8));
   ck(k1.alloc((size_t)P * 8));

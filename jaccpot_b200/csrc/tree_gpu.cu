@@ -274,7 +274,9 @@ __global__ void k_max_occupancy(const int* __restrict__ ranges, int num_internal
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= L) return;
   const int id = num_internal + j;
-  atomicMax(out, ranges[2 * id + 1] - ranges[2 * id] + 1);
+  const unsigned peers = __activemask();
+  const int m = __reduce_max_sync(peers, ranges[2 * id + 1] - ranges[2 * id] + 1);
+  if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicMax(out, m);  // one per warp
 }
 
 // ---------------------------------------------------------------------------
