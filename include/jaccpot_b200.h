@@ -253,6 +253,8 @@ JB_API int jb_m2m_schedule_device(int num_nodes, int num_internal, const int* pa
                                   void* stream, jb_dsched** out);
 JB_API int jb_dsched_info(const jb_dsched* d, jb_sched_info_t* info);
 JB_API const void* jb_dsched_field(const jb_dsched* d, int field);
+/* Copies the first `bytes` bytes of a field into a device buffer, in stream order. */
+JB_API int jb_dsched_export(const jb_dsched* d, int field, void* dst, int64_t bytes, void* stream);
 JB_API void jb_dsched_free(jb_dsched* d);
 
 /* ------------------------------------------------------------------------ */

@@ -119,6 +119,7 @@ _SIGNATURES = {
     "jb_dsched_info": [_P, _P],
     "jb_dsched_field": [_P, _I],
     "jb_dsched_free": [_P],
+    "jb_dsched_export": [_P, _I, _P, _I64, _P],
     "jb_coeff_stride": [_I],
     "jb_last_cuda_error": [],
     "jb_gather_sorted": [_I64, _P, _P, _P, _P, _P],
@@ -192,6 +193,17 @@ def check(status: int, what: str) -> None:
         if status == 3:
             msg += ": " + (lib().jb_last_cuda_error() or b"").decode()
         raise JBError(f"{what} failed: {msg}")
+
+
+def stream_handle(device=None) -> int:
+    """torch's current stream on `device` (default: the current device) as the
+    pointer the library takes.  torch.cuda.current_stream builds a stream object
+    and looks the device up several times on the way (5 us a call, 12 to 25
+    calls a pass or prepare)."""
+    import torch
+
+    index = None if device is None else torch.device(device).index
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice() if index is None else index)
 
 
 def coeff_stride(p: int) -> int:

@@ -58,7 +58,7 @@ def node_force_scale(ps: engine.Pass, acc4: torch.Tensor | None = None) -> torch
     a4 = ps.ws.acc4 if acc4 is None else acc4
     _lib.check(_lib.lib().jb_node_force_scale(t.num_nodes, t.num_internal, _ptr(dt.left), _ptr(dt.right),
                                               lo.ctypes.data, t.num_levels, _ptr(dt.node_ranges), _ptr(a4),
-                                              _ptr(out), torch.cuda.current_stream(dt.device).cuda_stream),
+                                              _ptr(out), _lib.stream_handle(dt.device)),
                "jb_node_force_scale")
     return out
 
@@ -70,7 +70,7 @@ def node_dehnen_power(ps: engine.Pass, p: int | None = None) -> torch.Tensor:
     t = ps.dt.topo
     out = torch.empty((t.num_nodes, p + 1), device=ps.dt.device, dtype=torch.float64)
     _lib.check(_lib.lib().jb_node_dehnen_power(p, t.num_nodes, _ptr(ps.ws.mult), ps.ws.stride, _ptr(out),
-                                               torch.cuda.current_stream(ps.dt.device).cuda_stream),
+                                               _lib.stream_handle(ps.dt.device)),
                "jb_node_dehnen_power")
     return out
 

@@ -1254,6 +1254,15 @@ JB_API const void* jb_dsched_field(const jb_dsched* d, int field) {
   return b ? b->p : nullptr;
 }
 
+JB_API int jb_dsched_export(const jb_dsched* d, int field, void* dst, int64_t bytes, void* stream) {
+  if (!d || bytes < 0) return JB_ERR_ARG;
+  if (bytes == 0) return JB_OK;
+  const DBuf* b = sched_field(d, field);
+  if (!b || !dst || (size_t)bytes > b->bytes) return JB_ERR_ARG;
+  return jb::cuda_status(
+      cudaMemcpyAsync(dst, b->p, (size_t)bytes, cudaMemcpyDeviceToDevice, reinterpret_cast<cudaStream_t>(stream)));
+}
+
 JB_API void jb_dsched_free(jb_dsched* d) { delete d; }
 
 }  // extern "C"

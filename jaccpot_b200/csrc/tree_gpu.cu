@@ -99,12 +99,16 @@ __global__ void __launch_bounds__(256) k_bbox_partial(const double* __restrict__
   if (threadIdx.x < 6) part[6 * blockIdx.x + threadIdx.x] = sm[threadIdx.x][0];
 }
 
+// Warp per bound (one block of six): minima and maxima have no order.
 __global__ void k_bbox_final(const double* __restrict__ part, int nblk, double* __restrict__ bb) {
-  if (threadIdx.x >= 6) return;
-  const int k = threadIdx.x;
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double v = part[k];
-  for (int b = 1; b < nblk; ++b) v = (k < 3) ? fmin(v, part[6 * b + k]) : fmax(v, part[6 * b + k]);
-  bb[k] = v;
+  for (int b = lane; b < nblk; b += 32) v = (k < 3) ? fmin(v, part[6 * b + k]) : fmax(v, part[6 * b + k]);
+  for (int o = 16; o > 0; o >>= 1) {
+    const double u = __shfl_xor_sync(kFull, v, o);
+    v = (k < 3) ? fmin(v, u) : fmax(v, u);
+  }
+  if (lane == 0) bb[k] = v;
 }
 
 __device__ __forceinline__ uint64_t spread21(uint64_t v) {
@@ -715,7 +719,7 @@ void build(jb_dtree& t, int64_t n, const double* pos, const double* mass, int le
   ck(bb.alloc(6 * sizeof(double)));
   k_bbox_partial<<<nb_bb, 256, 0, st>>>(pos, n, part.as<double>());
   ck_launch();
-  k_bbox_final<<<1, 32, 0, st>>>(part.as<double>(), nb_bb, bb.as<double>());
+  k_bbox_final<<<1, 192, 0, st>>>(part.as<double>(), nb_bb, bb.as<double>());
   ck_launch();
   ck(k0.alloc((size_t)n * 8));
   ck(k1.alloc((size_t)n * 8));

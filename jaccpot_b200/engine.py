@@ -41,8 +41,7 @@ def _zero(t: torch.Tensor, stream: torch.cuda.Stream | None) -> None:
 
 
 def _stream_handle(stream: torch.cuda.Stream | None) -> int:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    return _lib.stream_handle() if stream is None else stream.cuda_stream
 
 
 class DeviceTopology:
@@ -147,7 +146,7 @@ class DeviceTopology:
             return True
         rev = torch.empty(n, dtype=torch.int32, device=self.device)
         rc = _lib.lib().jb_far_reverse_index(self.topo.num_leaves, _ptr(self.near_off), _ptr(self.near_src), _ptr(rev),
-                                             torch.cuda.current_stream(self.device).cuda_stream)
+                                             _lib.stream_handle(self.device))
         if rc == _lib.JB_ERR_INDEX:  # not symmetric, or rows of a caller's own that do not ascend
             return self.topo.near_lists_symmetric()
         _lib.check(rc, "jb_far_reverse_index(near)")
@@ -162,7 +161,7 @@ class DeviceTopology:
             rev = torch.empty(max(n, 1), dtype=torch.int32, device=self.device)
             _lib.check(_lib.lib().jb_far_reverse_index(self.topo.num_nodes, self.far_off.data_ptr(),
                                                        self.far_src.data_ptr(), rev.data_ptr(),
-                                                       torch.cuda.current_stream(self.device).cuda_stream),
+                                                       _lib.stream_handle(self.device)),
                        "jb_far_reverse_index")
             rev = rev[:n]
             self._far_rev = rev
@@ -896,13 +895,8 @@ class Pass:
                 "pair_tgt": dt.far_pair_targets(),
                 "rev": (dt.far_reverse_index() if t.num_far_pairs else torch.zeros(1, dtype=torch.int32, device=dev)),
             }
-            # the forward's schedules (its leaf units of another size are rebuilt)
-            if self.leaf_unit_sources == 4096:
-                A["sched"], names = self.leaf_sched, ("d_leaf_units", "d_leaf_aux", "d_leaf_runs", "d_leaf_split")
-                A["units"], A["aux"], A["runs"], A["split"] = (getattr(self, n) for n in names)
-            else:
-                sc = A["sched"] = leaf_schedule_device(dt, max_sources=4096)
-                A["units"], A["aux"], A["runs"], A["split"] = (_up(x, dev) for x in (sc.units, sc.aux, sc.runs, sc.split))
+            A["sched"], names = self.leaf_sched, ("d_leaf_units", "d_leaf_aux", "d_leaf_runs", "d_leaf_split")
+            A["units"], A["aux"], A["runs"], A["split"] = (getattr(self, n) for n in names)
             A["partials"] = torch.empty((max(A["sched"].num_slots, 1) * _lib.JB_MAX_LEAF_OCCUPANCY, 4), **f32)
             mp = m2l_unit_limit(t.num_far_pairs)
             if self.m2l_unit_pairs == mp:

@@ -403,20 +403,22 @@ def _run_device(fn_name: str, args: list, device):
     import torch
 
     from . import _lib
-    from .tree import device_view
 
     global _SchedInfo
     if _SchedInfo is None:
         _SchedInfo = _sched_info_cls()
     lb = _lib.lib()
     h = ctypes.c_void_p()
-    stream = torch.cuda.current_stream(device).cuda_stream
+    stream = _lib.stream_handle(device)
     _lib.check(getattr(lb, fn_name)(*args, stream, ctypes.byref(h)), fn_name)
     info = _SchedInfo()
     _lib.check(lb.jb_dsched_info(h, ctypes.byref(info)), "jb_dsched_info")
 
     def field(fid: int, shape, dtype):
-        return device_view(lb.jb_dsched_field(h, fid), shape, dtype, device).clone()
+        out = torch.empty(shape, dtype=torch.int64 if dtype is np.int64 else torch.int32, device=device)
+        _lib.check(lb.jb_dsched_export(h, fid, out.data_ptr(), out.numel() * out.element_size(), stream),
+                   "jb_dsched_export")
+        return out
 
     return info, field, (lambda: lb.jb_dsched_free(h))
 

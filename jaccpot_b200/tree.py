@@ -276,7 +276,13 @@ def build_topology(positions, masses, *, leaf_size: int = 16, theta: float = 0.6
 def _torch_dtype(dtype):
     import torch
 
-    return {"int32": torch.int32, "int64": torch.int64, "float64": torch.float64}[np.dtype(dtype).name]
+    return {"i4": torch.int32, "i8": torch.int64, "f8": torch.float64}[dtype.str[1:]]
+
+
+class _View:
+    def __init__(self, ptr, shape, typestr):
+        self.__cuda_array_interface__ = {"shape": shape, "typestr": typestr, "data": (int(ptr), False), "version": 3,
+                                         "strides": None}
 
 
 def device_view(ptr, shape, dtype, device):
@@ -289,11 +295,7 @@ def device_view(ptr, shape, dtype, device):
     if int(np.prod(shape)) == 0:
         return torch.zeros(shape, dtype=torch.from_numpy(np.zeros(0, dtype)).dtype, device=device)
 
-    class _View:
-        __cuda_array_interface__ = {"shape": shape, "typestr": dtype.str, "data": (int(ptr), False), "version": 3,
-                                    "strides": None}
-
-    return torch.as_tensor(_View(), device=device)
+    return torch.as_tensor(_View(ptr, shape, dtype.str), device=device)
 
 
 class DeviceTree:
@@ -315,7 +317,7 @@ class DeviceTree:
         self.n, self.leaf_size, self.theta, self.device = int(n), int(leaf_size), float(theta), pos.device
         self._lb = _lib.lib()
         self._h = ctypes.c_void_p()
-        stream = torch.cuda.current_stream(pos.device).cuda_stream
+        stream = _lib.stream_handle(pos.device)
         _lib.check(self._lb.jb_tree_build_device(n, pos.data_ptr(), mass.data_ptr(), self.leaf_size, self.theta,
                                                  stream, ctypes.byref(self._h)), "jb_tree_build_device")
         self.info = _lib.TreeInfo()
@@ -336,7 +338,7 @@ class DeviceTree:
         fs = force_scale.to(device=self.device, dtype=torch.float32).contiguous()
         if pw.dim() != 2 or pw.shape[0] != self.info.num_nodes or fs.shape != (self.info.num_nodes,):
             raise ValueError("power must be (num_nodes, P+1) and force_scale (num_nodes,)")
-        stream = torch.cuda.current_stream(self.device).cuda_stream
+        stream = _lib.stream_handle(self.device)
         _lib.check(self._lb.jb_dtree_adaptive_walk(self._h, int(pw.shape[1]), pw.data_ptr(), fs.data_ptr(),
                                                    float(G), float(eps), float(theta_max), int(orders.size),
                                                    orders.ctypes.data, stream), "jb_dtree_adaptive_walk")
@@ -363,7 +365,7 @@ class DeviceTree:
         base = buf.data_ptr()
         ids = np.array([_lib.DTREE_FIELDS[f][0] for f in names], dtype=np.int32)
         dst = np.array([base + spans[f][0] for f in names], dtype=np.uint64)
-        stream = torch.cuda.current_stream(self.device).cuda_stream
+        stream = _lib.stream_handle(self.device)
         _lib.check(self._lb.jb_dtree_export(self._h, len(names), ids.ctypes.data, dst.ctypes.data, stream),
                    "jb_dtree_export")
         arrays = {f: buf[o:o + c * d.itemsize].view(_torch_dtype(d)) for f, (o, c, d) in spans.items()}
