@@ -16,7 +16,8 @@ at the top gear on it (its accelerations give the per-node force scale, the
 smallest |a| under each node -- the "min" reduction the reference switches to
 with dehnen_paper, _adaptive_policy.py:402; its multipoles give Dehnen's
 per-degree powers), then the error-controlled walk on the same tree.  The
-returned pass runs every far pair at its gear (``Pass.set_gears``).
+returned pass runs every far pair at its gear (``Pass.set_gears``), and holds the
+prepass's particles, centres and multipoles: its upward sweep is done.
 """
 
 from __future__ import annotations
@@ -113,6 +114,8 @@ def prepare(positions, masses, *, leaf_size: int, orders, eps: float, theta_max:
         power = node_dehnen_power(pre)
         pre_far, pre_near = topo0.num_far_pairs, pre.near_pair_interactions()
         hops = dt0.m2m_hops() if pre.m2m_hops else None  # of the tree, which both lists share
+        # particles, centres and multipoles are the tree's, whatever the lists
+        tree_ws = (pre.ws.pos4, pre.ws.centers, pre.ws.mult)
         del pre, dt0
         dtree.adaptive_walk(power, fscale, G=G, eps=eps, theta_max=theta_max, gear_orders=orders)
         topo = dtree.topology()
@@ -120,6 +123,7 @@ def prepare(positions, masses, *, leaf_size: int, orders, eps: float, theta_max:
     dt.validate()
     dt.share_m2m_hops(hops)
     ps = engine.Pass(dt, p_top, G=G, eps2=eps2, m2l_mode=m2l_mode, p2p_mode=p2p_mode, **pass_kw)
+    ps.ws.pos4, ps.ws.centers, ps.ws.mult = tree_ws
     if len(orders) > 1 and topo.num_far_pairs:
         ps.set_gears(topo.device_arrays["far_gears"], orders)
     return AdaptivePrepared(topology=topo, device_topology=dt, pass_=ps, orders=orders, eps=float(eps),

@@ -814,23 +814,26 @@ class Pass:
         return self._far_stream
 
     def run(self, stream=None, cascade: bool = False, potential: bool = False,
-            overlap: bool | None = None, own: bool = False) -> torch.Tensor:
+            overlap: bool | None = None, own: bool = False, upward: bool = True) -> torch.Tensor:
         """Whole pass on the particles already in ws.pos4; returns sorted acc4
         (cascade: the level-by-level downward sweep, see l2l; own: leave every
-        node's own M2L sum in ws.locals, see l2l_to_rows).  overlap
+        node's own M2L sum in ws.locals, see l2l_to_rows; upward=False: the
+        centres and multipoles are already there).  overlap
         (default self.overlap): the near field runs on `stream` while the
         upward sweep, M2L and L2L run on far_stream(), joined before the L2P
         and the sum of split leaves; the result has the same bits as the
         one-stream order (at 4M, p = 8: 7.89 -> 7.64 ms a step)."""
         if not (self.overlap if overlap is None else overlap):
-            self.upward(stream)
+            if upward:
+                self.upward(stream)
             self.downward(stream, cascade=cascade, own=own)
             return self.evaluate(stream, potential=potential)
         main = stream if stream is not None else torch.cuda.current_stream(self.dt.device)
         far = self.far_stream()
         far.wait_stream(main)  # the particles are loaded
         self.evaluate(main, potential=potential, part="near_first")
-        self.upward(far)
+        if upward:
+            self.upward(far)
         self.downward(far, cascade=cascade, own=own)
         main.wait_stream(far)
         return self.evaluate(main, potential=potential, part="far_after")

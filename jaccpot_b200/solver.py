@@ -249,6 +249,18 @@ class FastMultipoleMethod:
             raise ValueError(f"unknown cache_policy {cache_policy!r}")
         if runtime_overrides_override is not None:
             raise ValueError("runtime_overrides_override is not provided")
+        return self._prepare(positions, masses, leaf_size, max_order, theta, force_scale_nodes)
+
+    def _sweeps_with_near_field(self) -> bool:
+        """Whether a call that prepares and evaluates leaves the sweeps to the
+        evaluation, which runs them beside the near field (Pass.run).  The
+        tensor-core M2L's status is checked by the prepare, so it keeps them."""
+        return self.m2l_mode == _lib.JB_M2L_FP32
+
+    def _prepare(self, positions, masses, leaf_size, max_order, theta, force_scale_nodes=None,
+                 sweep: bool = True) -> FMMPreparedState:
+        """prepare_state; sweep=False leaves the state without its sweeps, for
+        _evaluate_whole(sweep=True) to run."""
         th = self.theta if theta is None else float(theta)
         positions = positions.detach() if isinstance(positions, torch.Tensor) else np.asarray(positions)
         masses = masses.detach() if isinstance(masses, torch.Tensor) else np.asarray(masses)
@@ -257,17 +269,18 @@ class FastMultipoleMethod:
             raise ValueError("positions must be (N, 3) and masses (N,)")
         self._counters["prepare_state"] += 1
         if self.adaptive_error_model == "dehnen_paper":
-            return self._prepare_adaptive(positions, masses, int(leaf_size), int(max_order), th, force_scale_nodes)
+            return self._prepare_adaptive(positions, masses, int(leaf_size), int(max_order), th, force_scale_nodes,
+                                          sweep)
         if force_scale_nodes is not None:
             raise ValueError("force_scale_nodes applies to adaptive_error_model='dehnen_paper'")
         # tree + lists on the GPU when the solver runs there (the same arrays
         # as the host build, bit for bit), else on the host
         topo = build_topology(positions, masses, leaf_size=int(leaf_size), theta=th,
                               device=self.device if self.device.type == "cuda" else None)
-        return self._prepare_from_topology(topo, positions, masses, int(max_order), th, int(leaf_size))
+        return self._prepare_from_topology(topo, positions, masses, int(max_order), th, int(leaf_size), sweep)
 
     def _prepare_adaptive(self, positions, masses, leaf_size: int, max_order: int, th: float,
-                          force_scale=None) -> FMMPreparedState:
+                          force_scale=None, sweep: bool = True) -> FMMPreparedState:
         """Error-controlled walk (jaccpot_b200.adaptive): the reference's
         adaptive_error_model="dehnen_paper" lane with adaptive_eps,
         mac_theta_max and p_gears (runtime/_adaptive_policy.py:2216)."""
@@ -298,11 +311,10 @@ class FastMultipoleMethod:
                                  eps2=self.softening ** 2, device=self.device, m2l_mode=self.m2l_mode,
                                  p2p_mode=self.p2p_mode, force_scale=force_scale)
         self._counters["adaptive_prepares"] += 1
-        ps = prep.pass_
-        ps.load_particles(pos, mass)
-        ps.upward()
-        ps.downward()
-        ps.check_tc_status()
+        ps = prep.pass_  # its particles are loaded and its upward sweep done
+        if sweep:
+            ps.downward()
+            ps.check_tc_status()
         st = FMMPreparedState(topology=prep.topology, device_topology=prep.device_topology, pass_=ps,
                               max_order=int(max_order), theta=th, leaf_size=int(leaf_size),
                               num_particles=int(prep.topology.num_particles),
@@ -312,7 +324,7 @@ class FastMultipoleMethod:
         return st
 
     def _prepare_from_topology(self, topo: Topology, positions, masses, max_order: int, th: float,
-                               leaf_size: int) -> FMMPreparedState:
+                               leaf_size: int, sweep: bool = True) -> FMMPreparedState:
         dt = DeviceTopology(topo, self.device)
         dt.validate()
         ps = Pass(dt, int(max_order), G=self.G, eps2=self.softening ** 2, m2l_mode=self.m2l_mode,
@@ -327,9 +339,10 @@ class FastMultipoleMethod:
             if self.p_gears is not None and tuple(self.p_gears) != tuple(model.orders):
                 raise ValueError(f"the gear model is trained for p_gears={model.orders}")
             _gears.apply_gears(ps, model)
-        ps.upward()
-        ps.downward()
-        ps.check_tc_status()
+        if sweep:
+            ps.upward()
+            ps.downward()
+            ps.check_tc_status()
         st = FMMPreparedState(topology=topo, device_topology=dt, pass_=ps, max_order=int(max_order), theta=th,
                               leaf_size=int(leaf_size), num_particles=int(topo.num_particles),
                               input_dtype=positions.dtype if hasattr(positions, "dtype") else np.float64)
@@ -355,6 +368,11 @@ class FastMultipoleMethod:
         ``refresh_stats`` counts attempts, hits and the reason of each miss.
         ``bounds`` and ``fused_device_mode`` are accepted for signature
         compatibility (the state is always device resident)."""
+        return self._refresh(prepared_state, positions, masses, leaf_size, max_order, theta)
+
+    def _refresh(self, prepared_state: FMMPreparedState, positions, masses, leaf_size=None, max_order=None, theta=None,
+                 sweep: bool = True) -> FMMPreparedState:
+        """refresh_prepared_state; sweep as _prepare's."""
         from dataclasses import replace
 
         from .tree import DeviceTree
@@ -368,12 +386,12 @@ class FastMultipoleMethod:
         th = st.theta if theta is None else float(theta)
         if (leaf, order, th) != (st.leaf_size, st.max_order, st.theta) or self.device.type != "cuda":
             stats["miss_config"] += 1
-            return self.prepare_state(positions, masses, bounds=bounds, leaf_size=leaf, max_order=order, theta=th)
+            return self._prepare(positions, masses, leaf, order, th, sweep=sweep)
         if "adaptive" in st.scratch:
             # the error-controlled lists depend on the multipoles and the force
             # scale, not on the tree alone: a new walk every time
             stats["miss_adaptive"] = stats.get("miss_adaptive", 0) + 1
-            return self.prepare_state(positions, masses, bounds=bounds, leaf_size=leaf, max_order=order, theta=th)
+            return self._prepare(positions, masses, leaf, order, th, sweep=sweep)
         dt = st.device_topology
         t = st.topology
         with DeviceTree(positions, masses, leaf_size=leaf, theta=th, device=self.device) as nt:
@@ -397,7 +415,7 @@ class FastMultipoleMethod:
                     moved = replace(t, centers_f64=nt.field("centers_f64").reshape(-1, 3).cpu().numpy(),
                                     radii_f64=nt.field("radii_f64").cpu().numpy())
         if not same:
-            return self._prepare_from_topology(topo, positions, masses, order, th, leaf)
+            return self._prepare_from_topology(topo, positions, masses, order, th, leaf, sweep)
         stats["hits"] += 1
         ps = st.pass_.fork()
         ps.load_particles(_to_torch(positions, self.device, torch.float32),
@@ -407,8 +425,9 @@ class FastMultipoleMethod:
 
             model = self.gear_model if self.gear_model is not None else _gears.GearModel.load()
             _gears.apply_gears(ps, model)
-        ps.upward()
-        ps.downward()
+        if sweep:
+            ps.upward()
+            ps.downward()
         new = FMMPreparedState(topology=moved, device_topology=dt, pass_=ps, max_order=st.max_order, theta=st.theta, leaf_size=st.leaf_size,
                                num_particles=st.num_particles,
                                input_dtype=positions.dtype if hasattr(positions, "dtype") else np.float64)
@@ -421,13 +440,12 @@ class FastMultipoleMethod:
         """Prepare when ``prepared_state`` is None, refresh it otherwise, then
         evaluate every particle (solver.py:1664 there): a time-stepping loop
         calls this unconditionally.  Returns (state, accelerations)."""
+        late = self._sweeps_with_near_field()
         if prepared_state is None:
-            st = self.prepare_state(positions, masses, bounds=bounds, leaf_size=leaf_size, max_order=max_order,
-                                    theta=theta)
+            st = self._prepare(positions, masses, leaf_size, max_order, theta, sweep=not late)
         else:
-            st = self.refresh_prepared_state(prepared_state, positions, masses, bounds=bounds,
-                                             leaf_size=leaf_size, max_order=max_order, theta=theta)
-        return st, self.evaluate_prepared_state(st, as_numpy=not isinstance(positions, torch.Tensor))
+            st = self._refresh(prepared_state, positions, masses, leaf_size, max_order, theta, sweep=not late)
+        return st, self._evaluate_whole(st, False, not isinstance(positions, torch.Tensor), sweep=late)
 
     # ----------------------------------------------------------------- evaluate
     def evaluate_prepared_state(self, state: FMMPreparedState, *, target_indices=None,
@@ -435,30 +453,40 @@ class FastMultipoleMethod:
                                 max_acc_derivative_order: int = 0, as_numpy: Optional[bool] = None):
         if max_acc_derivative_order:
             raise ValueError("acceleration derivative towers are not provided")
-        ps = state.pass_
-        dev = state.device_topology.device
         want_np = as_numpy if as_numpy is not None else not isinstance(target_indices, torch.Tensor)
         if target_indices is None:
-            ps.evaluate(potential=return_potential)
-            acc = torch.empty((state.num_particles, 3), device=dev, dtype=torch.float32)
-            pot = torch.empty((state.num_particles,), device=dev, dtype=torch.float32) if return_potential else None
-            ps.unsort(acc, pot)
-        else:
-            ti = _to_torch(target_indices, dev, torch.int64).reshape(-1)
-            out = ps.evaluate_input_targets(ti)
-            acc = out[:, :3].contiguous()
-            pot = out[:, 3].contiguous() if return_potential else None
+            return self._evaluate_whole(state, return_potential, want_np)
+        ti = _to_torch(target_indices, state.device_topology.device, torch.int64).reshape(-1)
+        out = state.pass_.evaluate_input_targets(ti)
+        acc = out[:, :3].contiguous()
+        pot = out[:, 3].contiguous() if return_potential else None
         self._counters["evaluate"] += 1
-        if target_indices is None:
-            self._monitor_check(state)
-        if (target_indices is None and self.adaptive_error_model == "dehnen_paper"
-                and self.mac_force_scale_mode in ("prev", "paper_cached")):
-            # the next error-controlled prepare takes its force scale from here
-            self._force_scale_cache = torch.linalg.vector_norm(acc, dim=1)
+        return self._results(acc, pot, want_np)
+
+    @staticmethod
+    def _results(acc, pot, want_np: bool):
         if want_np:
             acc = acc.cpu().numpy()
             pot = pot.cpu().numpy() if pot is not None else None
-        return (acc, pot) if return_potential else acc
+        return acc if pot is None else (acc, pot)
+
+    def _evaluate_whole(self, state: FMMPreparedState, return_potential: bool, want_np: bool, sweep: bool = False):
+        """Every particle of the state; sweep: its sweeps are still to run (the
+        upward one is done for an error-controlled state)."""
+        ps, dev = state.pass_, state.device_topology.device
+        if sweep:
+            ps.run(potential=return_potential, upward="adaptive" not in state.scratch)
+        else:
+            ps.evaluate(potential=return_potential)
+        acc = torch.empty((state.num_particles, 3), device=dev, dtype=torch.float32)
+        pot = torch.empty((state.num_particles,), device=dev, dtype=torch.float32) if return_potential else None
+        ps.unsort(acc, pot)
+        self._counters["evaluate"] += 1
+        self._monitor_check(state)
+        if self.adaptive_error_model == "dehnen_paper" and self.mac_force_scale_mode in ("prev", "paper_cached"):
+            # the next error-controlled prepare takes its force scale from here
+            self._force_scale_cache = torch.linalg.vector_norm(acc, dim=1)
+        return self._results(acc, pot, want_np)
 
     def differentiable_accelerations(self, state: FMMPreparedState, positions, masses, *, target_indices=None,
                                      jit_traversal: bool = False, grad_plan=None, grad_config=None, out=None):
@@ -550,6 +578,9 @@ class FastMultipoleMethod:
                                     theta=theta)
             self._reuse = {"state": st, "calls": 1, "key": key}
             self._counters["reuse_rebuilds"] += 1
+        elif target_indices is None and self._sweeps_with_near_field():
+            st = self._prepare(positions, masses, leaf_size, max_order, theta, sweep=False)
+            return self._evaluate_whole(st, return_potential, as_np, sweep=True)
         else:
             st = self.prepare_state(positions, masses, bounds=bounds, leaf_size=leaf_size, max_order=max_order,
                                     theta=theta)
@@ -694,8 +725,13 @@ class FastMultipoleMethod:
         m = _to_torch(masses, self.device, torch.float32)
         x, v = S[:, 0], S[:, 1]
 
+        late = self._sweeps_with_near_field()
+
+        def refreshed(st):
+            return self._refresh(st, x, m, leaf_size, max_order, theta, sweep=not late)
+
         def accel(st):
-            a = self.evaluate_prepared_state(st, as_numpy=False)
+            a = self._evaluate_whole(st, False, False, sweep=late)
             if add_external:
                 a = a + _to_torch(external_acceleration_fn(x), self.device, torch.float32)
             return a
@@ -708,14 +744,14 @@ class FastMultipoleMethod:
             if add_external:
                 a = a + _to_torch(external_acceleration_fn(x), self.device, torch.float32)
         else:
-            st = self.refresh_prepared_state(st, x, m, leaf_size=leaf_size, max_order=max_order, theta=theta)
+            st = refreshed(st)
             a = accel(st)
         hist = [] if return_history else None
         h = float(dt)
         for i in range(int(num_steps)):
             v.add_(a, alpha=0.5 * h)
             x.add_(v, alpha=h)
-            st = self.refresh_prepared_state(st, x, m, leaf_size=leaf_size, max_order=max_order, theta=theta)
+            st = refreshed(st)
             a = accel(st)
             v.add_(a, alpha=0.5 * h)
             if hist is not None:
