@@ -1680,19 +1680,26 @@ __global__ void __launch_bounds__(128) k_targets_far(const float4* __restrict__ 
   out[q] = make_float4(-G * g[0], -G * g[1], -G * g[2], -G * phi);
 }
 
-// The lanes look up 32 neighbour leaves at once (the target's own leaf
-// first); leaves that follow one another in memory join into runs, and the
-// warp reads each run's particles 32 at a time in consecutive 16-byte words.
-// With a leaf per lane instead, every load touched 32 cache lines and the L1
-// bounded the kernel: 65,536 targets of a Plummer sphere of 1M (order 6, leaf
-// 32, 1,900 sources each) took 387 us in one kernel, 330 us in these two.
-static __global__ void __launch_bounds__(256) k_targets_near(
+// The lanes look up 32 neighbour leaves at once (the target's own leaf first);
+// leaves that follow one another in memory join into runs, whose particle
+// counts are summed up in shared memory.  The warp then walks the group's
+// particles 32 at a time, each lane finding its particle's run with a cursor
+// that only advances, four particles in flight per lane.  The kernel is bound
+// by issue (70% of the slots).  A call with 65,536 targets of a Plummer sphere
+// of 1M (order 6, leaf 32, 1,900 sources each): a leaf per lane, 32 cache lines
+// to a load, 387 us of kernel; runs read in turn, one load in flight, 378 us the
+// whole call; a cursor over the leaves themselves 330; over the runs 262.
+constexpr int kTargetWarps = 8;
+static __global__ void __launch_bounds__(32 * kTargetWarps) k_targets_near(
     const float4* __restrict__ pos4, int num_internal, const int2* __restrict__ ranges,
     const int64_t* __restrict__ near_off, const int* __restrict__ near_src, const int* __restrict__ leaf_of,
     int64_t num_targets, const int* __restrict__ tsorted, float G, float eps2, float4* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  __shared__ int s_end[kTargetWarps][32], s_base[kTargetWarps][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t q = (int64_t)blockIdx.x * kTargetWarps + warp;
   if (q >= num_targets) return;
+  int* end = s_end[warp];    // particles of the group's runs up to and with run k
+  int* base = s_base[warp];  // run k's first particle less the particles before it
   const int i = tsorted[q];
   const int leaf = leaf_of[i];
   const float4 ti = pos4[i];
@@ -1700,20 +1707,44 @@ static __global__ void __launch_bounds__(256) k_targets_near(
   const int64_t e0 = near_off[leaf], e1 = near_off[leaf + 1];
   for (int64_t eb = e0 - 1; eb < e1; eb += 32) {
     const int64_t e = eb + lane;
-    int2 sr = make_int2(0, -1);  // past the list: a run of no particles
+    int2 sr = make_int2(0, -1);  // past the list: no particles
     if (e < e1) sr = ranges[num_internal + (e < e0 ? leaf : near_src[e])];
+    const int count = sr.y - sr.x + 1;
+    int incl = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
     const int before = __shfl_up_sync(0xffffffffu, sr.y, 1);
-    unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || sr.x != before + 1);
-    while (heads) {
-      const int h = __ffs(heads) - 1;
-      heads &= heads - 1;
-      const int last = __shfl_sync(0xffffffffu, sr.y, heads ? __ffs(heads) - 2 : 31);
-      for (int j = __shfl_sync(0xffffffffu, sr.x, h) + lane; j <= last; j += 32) {
-        const float4 s = pos4[j];
-        const float dx = ti.x - s.x, dy = ti.y - s.y, dz = ti.z - s.z;
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || sr.x != before + 1);
+    const int run = __popc(heads << (31 - lane)) - 1;  // heads up to and with this lane
+    __syncwarp();  // the previous group's runs are read
+    if (heads >> lane & 1u) base[run] = sr.x - (incl - count);
+    if (lane == 31 || (heads >> (lane + 1) & 1u)) end[run] = incl;
+    __syncwarp();
+    int r = 0, r_end = end[0], r_base = base[0];
+    for (int f = lane; f < total; f += 128) {
+      int j[4];
+      float4 s[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int fu = min(f + 32 * u, total - 1);
+        while (fu >= r_end) {  // ends: fu < total, the last run's end
+          ++r;
+          r_end = end[r];
+          r_base = base[r];
+        }
+        j[u] = f + 32 * u < total ? r_base + fu : i;  // the target itself adds nothing
+        s[u] = pos4[j[u]];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float dx = ti.x - s[u].x, dy = ti.y - s[u].y, dz = ti.z - s[u].z;
         const float ir = rsqrt_ftz(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2))));
-        const float mir = j == i ? 0.f : s.w * ir;
-        const float w = j == i ? 0.f : mir * ir * ir;
+        const float mir = j[u] == i ? 0.f : s[u].w * ir;
+        const float w = j[u] == i ? 0.f : mir * ir * ir;
         ax = fmaf(w, dx, ax);
         ay = fmaf(w, dy, ay);
         az = fmaf(w, dz, az);
@@ -1989,7 +2020,7 @@ int RunTargets<P>::run(const float* pos4, int num_internal, const int* ranges, c
       leaf_of, nt, ts, G, reinterpret_cast<float4*>(out));
   const int rc = launch_status();
   if (rc) return rc;
-  k_targets_near<<<blocks_for(nt, 8), 256, 0, st>>>(
+  k_targets_near<<<blocks_for(nt, kTargetWarps), 32 * kTargetWarps, 0, st>>>(
       reinterpret_cast<const float4*>(pos4), num_internal, reinterpret_cast<const int2*>(ranges), near_off, near_src,
       leaf_of, nt, ts, G, eps2, reinterpret_cast<float4*>(out));
   return launch_status();
