@@ -1182,12 +1182,15 @@ __device__ __forceinline__ void near_chunk(const NearStage& st, float4 ti, int h
 // The targets rg (at most 32: the leaf, or one of its two halves) of the
 // leaf whose particles are lr; row: where this pass's targets start in the
 // leaf's partial row (0 or 32).
-template <int G, bool KAHAN, bool POT, bool W, bool FTZ>
+template <int G, bool KAHAN, bool POT, bool W, bool FTZ, bool FRESH>
 __device__ __forceinline__ void leaf_unit(const float4* __restrict__ pos4, int2 rg, int4 U, int2 aux,
                                           const int2* __restrict__ runs, NearStage& sP, int lane, float G_,
                                           float eps2, float4* __restrict__ out, float4* __restrict__ partial,
-                                          int max_slots, int* err, bool fresh, const int* __restrict__ rung,
+                                          int max_slots, int* err, const int* __restrict__ rung,
                                           const float* tbl, int nlw, int2 lr, int row) {
+  // every caller passes the leaf; without this line ptxas spills 12 to 28 bytes
+  // in the loops of k_leaf_units_flat (evaluate at 200k: 810 -> 815 us)
+  if (lr.y < lr.x) lr = rg;
   const int tl = lane / G, h = lane % G;
   const int nt = rg.y - rg.x + 1;
   const bool active = tl < nt;
@@ -1244,7 +1247,9 @@ __device__ __forceinline__ void leaf_unit(const float4* __restrict__ pos4, int2 
   const float4 res = near_scaled(G_, v);
   if (active && h == 0) {
     if (aux.x < 0) {
-      out[rg.x + tl] = add_rn(fresh ? JB_ZERO4 : out[rg.x + tl], res);  // to the far field k_leaf_l2p wrote
+      float4 f = JB_ZERO4;
+      if constexpr (!FRESH) f = out[rg.x + tl];  // the far field k_leaf_l2p wrote
+      out[rg.x + tl] = add_rn(f, res);
     } else if (aux.x < max_slots) {
       partial[(size_t)aux.x * kMaxLeaf + row + tl] = res;
     } else {
@@ -1262,18 +1267,18 @@ __device__ __forceinline__ void zero_split_leaf(int2 aux, int2 rg, int lane, flo
 }
 
 // Near field (P2P) of the work units, added to the far field already in out
-// (whole leaves) or written to the partial rows (split leaves).  fresh: out
+// (whole leaves) or written to the partial rows (split leaves).  FRESH: out
 // holds nothing yet (JB_P2P_NEAR_ONLY, JB_P2P_NEAR_FIRST) and is only written:
 // a launch that zeroed it first, and a read of it, less.
 //
 // W: the block-step weighted form of the mutual lane -- every pair scaled by
 // lw[max(rung_i, rung_j)] (rung: per sorted particle, lw: nlw <= 32 weights).
 // FTZ: 1/r from rsqrt_ftz (the pass's forms all use it; false gives rsqrtf).
-template <bool KAHAN, bool POT, bool W = false, bool FTZ = true>
+template <bool KAHAN, bool POT, bool FRESH, bool W = false, bool FTZ = true>
 static __global__ void __launch_bounds__(32 * kWarpsPerBlock, POT ? 6 : 8) k_leaf_units(
     const float4* __restrict__ pos4, int num_internal, int num_units, const int4* __restrict__ units,
     const int2* __restrict__ aux, const int2* __restrict__ runs, const int2* __restrict__ ranges, float G,
-    float eps2, float4* __restrict__ out, float4* __restrict__ partial, int max_slots, int* err, bool fresh,
+    float eps2, float4* __restrict__ out, float4* __restrict__ partial, int max_slots, int* err,
     const int* __restrict__ rung = nullptr, const float* __restrict__ lw = nullptr, int nlw = 1) {
   __shared__ NearStage sP[kWarpsPerBlock];
   __shared__ float tbl[32];
@@ -1292,20 +1297,20 @@ static __global__ void __launch_bounds__(32 * kWarpsPerBlock, POT ? 6 : 8) k_lea
     if (lane == 0) leaf_error(err, JB_LEAF_ERR_OCCUPANCY);
     return;
   }
-  if (fresh) zero_split_leaf(ax, rg, lane, out);
+  if (FRESH) zero_split_leaf(ax, rg, lane, out);
   for (int row = 0; row < ntl; row += 32) {  // a leaf of more than 32 particles in two passes
     const int2 rt = make_int2(rg.x + row, min(rg.y, rg.x + row + 31));
     const int nt = rt.y - rt.x + 1;
     if (row > 0) __syncwarp();  // the first pass's reads of the stage are done
     if (nt <= 8)
-      leaf_unit<4, KAHAN, POT, W, FTZ>(pos4, rt, U, ax, runs, sP[warp], lane, G, eps2, out, partial, max_slots, err,
-                                       fresh, rung, tbl, nlw, rg, row);
+      leaf_unit<4, KAHAN, POT, W, FTZ, FRESH>(pos4, rt, U, ax, runs, sP[warp], lane, G, eps2, out, partial, max_slots, err,
+                                       rung, tbl, nlw, rg, row);
     else if (nt <= 16)
-      leaf_unit<2, KAHAN, POT, W, FTZ>(pos4, rt, U, ax, runs, sP[warp], lane, G, eps2, out, partial, max_slots, err,
-                                       fresh, rung, tbl, nlw, rg, row);
+      leaf_unit<2, KAHAN, POT, W, FTZ, FRESH>(pos4, rt, U, ax, runs, sP[warp], lane, G, eps2, out, partial, max_slots, err,
+                                       rung, tbl, nlw, rg, row);
     else
-      leaf_unit<1, KAHAN, POT, W, FTZ>(pos4, rt, U, ax, runs, sP[warp], lane, G, eps2, out, partial, max_slots, err,
-                                       fresh, rung, tbl, nlw, rg, row);
+      leaf_unit<1, KAHAN, POT, W, FTZ, FRESH>(pos4, rt, U, ax, runs, sP[warp], lane, G, eps2, out, partial, max_slots, err,
+                                       rung, tbl, nlw, rg, row);
   }
 }
 
@@ -1416,11 +1421,11 @@ __device__ __forceinline__ void flat_add(FlatStage& S, int t, float4 v) {
   if (KAHAN) S.c[t] = make_float4(a.c[0], a.c[1], a.c[2], a.c[3]);
 }
 
-template <bool KAHAN, bool POT>
+template <bool KAHAN, bool POT, bool FRESH>
 __device__ __forceinline__ void leaf_unit_flat(const float4* __restrict__ pos4, int2 rg, int4 U, int2 aux,
                                                const int2* __restrict__ runs, FlatStage& S, int lane, float G_,
                                                float eps2, float4* __restrict__ out, float4* __restrict__ partial,
-                                               int max_slots, int* err, bool fresh, int2 lr, int row) {
+                                               int max_slots, int* err, int2 lr, int row) {
   constexpr int CH = kFlatChunk;
   const int nt = rg.y - rg.x + 1;  // 17..32 targets (the leaf lr, or one of its halves)
   const bool tgt = lane < nt;
@@ -1542,7 +1547,9 @@ __device__ __forceinline__ void leaf_unit_flat(const float4* __restrict__ pos4, 
     for (int i = 0; i < 4; ++i) v[i] = (POT || i < 3) ? a.value(i) : 0.f;
     const float4 res = near_scaled(G_, v);
     if (aux.x < 0) {
-      out[rg.x + lane] = add_rn(fresh ? JB_ZERO4 : out[rg.x + lane], res);  // to the far field k_leaf_l2p wrote
+      float4 f = JB_ZERO4;
+      if constexpr (!FRESH) f = out[rg.x + lane];  // the far field k_leaf_l2p wrote
+      out[rg.x + lane] = add_rn(f, res);
     } else if (aux.x < max_slots) {
       partial[(size_t)aux.x * kMaxLeaf + row + lane] = res;
     } else {
@@ -1554,11 +1561,11 @@ __device__ __forceinline__ void leaf_unit_flat(const float4* __restrict__ pos4, 
 // k_leaf_units with the chunk-major form for leaves of more than 16
 // particles (the lane-group forms below that) and rsqrt_ftz.  Same results
 // for squared distances in the normal FP32 range.
-template <bool KAHAN, bool POT>
+template <bool KAHAN, bool POT, bool FRESH>
 static __global__ void __launch_bounds__(32 * kWarpsPerBlock, POT ? 6 : 8) k_leaf_units_flat(
     const float4* __restrict__ pos4, int num_internal, int num_units, const int4* __restrict__ units,
     const int2* __restrict__ aux, const int2* __restrict__ runs, const int2* __restrict__ ranges, float G,
-    float eps2, float4* __restrict__ out, float4* __restrict__ partial, int max_slots, int* err, bool fresh) {
+    float eps2, float4* __restrict__ out, float4* __restrict__ partial, int max_slots, int* err) {
   __shared__ WarpStage sW[kWarpsPerBlock];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int u = blockIdx.x * kWarpsPerBlock + warp;
@@ -1571,20 +1578,20 @@ static __global__ void __launch_bounds__(32 * kWarpsPerBlock, POT ? 6 : 8) k_lea
     if (lane == 0) leaf_error(err, JB_LEAF_ERR_OCCUPANCY);
     return;
   }
-  if (fresh) zero_split_leaf(ax, rg, lane, out);
+  if (FRESH) zero_split_leaf(ax, rg, lane, out);
   for (int row = 0; row < ntl; row += 32) {  // a leaf of more than 32 particles in two passes
     const int2 rt = make_int2(rg.x + row, min(rg.y, rg.x + row + 31));
     const int nt = rt.y - rt.x + 1;
     if (row > 0) __syncwarp();  // the first pass's reads of the stage are done
     if (nt <= 8)
-      leaf_unit<4, KAHAN, POT, false, true>(pos4, rt, U, ax, runs, sW[warp].n, lane, G, eps2, out, partial,
-                                            max_slots, err, fresh, nullptr, nullptr, 1, rg, row);
+      leaf_unit<4, KAHAN, POT, false, true, FRESH>(pos4, rt, U, ax, runs, sW[warp].n, lane, G, eps2, out, partial,
+                                            max_slots, err, nullptr, nullptr, 1, rg, row);
     else if (nt <= 16)
-      leaf_unit<2, KAHAN, POT, false, true>(pos4, rt, U, ax, runs, sW[warp].n, lane, G, eps2, out, partial,
-                                            max_slots, err, fresh, nullptr, nullptr, 1, rg, row);
+      leaf_unit<2, KAHAN, POT, false, true, FRESH>(pos4, rt, U, ax, runs, sW[warp].n, lane, G, eps2, out, partial,
+                                            max_slots, err, nullptr, nullptr, 1, rg, row);
     else
-      leaf_unit_flat<KAHAN, POT>(pos4, rt, U, ax, runs, sW[warp].f, lane, G, eps2, out, partial, max_slots, err, fresh,
-                                 rg, row);
+      leaf_unit_flat<KAHAN, POT, FRESH>(pos4, rt, U, ax, runs, sW[warp].f, lane, G, eps2, out, partial, max_slots, err,
+                                        rg, row);
   }
 }
 
@@ -1924,10 +1931,10 @@ int RunL2LLeaves<P>::run(int num_units, const int* units, const int* anc, const 
 
 template <int P>
 struct RunLeafEval {
-  template <bool K, bool PT>
+  template <bool K, bool PT, bool FR>
   static void go(unsigned nb, cudaStream_t st, const float4* pos4, int num_internal, int num_units, const int4* units,
                  const int2* aux, const int2* runs, const int2* ranges, float G, float eps2, float4* out,
-                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err, bool fresh);
+                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err);
   static int run(int mode, const float* pos4, int num_internal, int num_units, const int* units, const int* aux,
                  const int* runs, const int* ranges, const float* centers, const float* locals, float G, float eps2,
                  float* out, float* partial, int num_split, const int* split, cudaStream_t st,
@@ -1936,26 +1943,26 @@ struct RunLeafEval {
 };
 
 template <int P>
-template <bool K, bool PT>
+template <bool K, bool PT, bool FR>
 void RunLeafEval<P>::go(unsigned nb, cudaStream_t st, const float4* pos4, int num_internal, int num_units, const int4* units,
                  const int2* aux, const int2* runs, const int2* ranges, float G, float eps2, float4* out,
-                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err, bool fresh) {
+                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err) {
   if (rung)
-    k_leaf_units<K, PT, true><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
-                                                                  ranges, G, eps2, out, partial, max_slots, err, fresh,
+    k_leaf_units<K, PT, FR, true><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
+                                                                  ranges, G, eps2, out, partial, max_slots, err,
                                                                   rung, lw, nlw);
   else if (flat) {
     // 23.5 KB of shared memory per block: ask for the carveout that holds
     // the eight blocks per SM the launch bounds allow.
     static const cudaError_t carve = cudaFuncSetAttribute(
-        k_leaf_units_flat<K, PT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        k_leaf_units_flat<K, PT, FR>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     (void)carve;
-    k_leaf_units_flat<K, PT><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
-                                                                 ranges, G, eps2, out, partial, max_slots, err, fresh);
+    k_leaf_units_flat<K, PT, FR><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
+                                                                 ranges, G, eps2, out, partial, max_slots, err);
   }
   else
-    k_leaf_units<K, PT><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs, ranges,
-                                                            G, eps2, out, partial, max_slots, err, fresh);
+    k_leaf_units<K, PT, FR><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs, ranges,
+                                                            G, eps2, out, partial, max_slots, err);
 }
 
 template <int P>
@@ -1986,10 +1993,15 @@ int RunLeafEval<P>::run(int mode, const float* pos4, int num_internal, int num_u
     if (far_only) return JB_OK;
     if (!far_after) {  // FAR_AFTER: the near field is already in out (and partials)
       const bool kahan = (mode & JB_P2P_KAHAN) != 0, pot = (mode & JB_P2P_POTENTIAL) != 0;
-      if (kahan && pot) go<true, true>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err, fresh);
-      else if (kahan) go<true, false>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err, fresh);
-      else if (pot) go<false, true>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err, fresh);
-      else go<false, false>(nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err, fresh);
+      auto kernel = [&](auto k, auto pt_, auto fr) {
+        go<decltype(k)::value, decltype(pt_)::value, decltype(fr)::value>(
+            nb, st, a0, num_internal, num_units, a1, a2, a3, a4, G, eps2, o, pt, rung, lw, nlw, flat, max_slots, err);
+      };
+      constexpr std::true_type yes{};
+      constexpr std::false_type no{};
+      auto with_pot = [&](auto k, auto p_) { fresh ? kernel(k, p_, yes) : kernel(k, p_, no); };
+      auto with_sums = [&](auto k) { pot ? with_pot(k, yes) : with_pot(k, no); };
+      kahan ? with_sums(yes) : with_sums(no);
       rc = launch_status();
       if (rc) return rc;
     }
