@@ -423,10 +423,13 @@ class Pass:
         self.d_leaf_runs = up(self.leaf_sched.runs)
         self.d_leaf_split = up(self.leaf_sched.split)
         self.leaf_partials = torch.empty((max(self.leaf_sched.num_slots, 1) * _lib.JB_MAX_LEAF_OCCUPANCY, 4), device=dev, dtype=torch.float32)
-        # the downward sweep straight to this pass's leaves (jb_l2l_leaves) at
-        # orders <= 8; l2l(cascade=True), and orders 9-10 (where the direct
-        # chain measured slower: 1.07 against 0.88 ms at 4M), run it level by level
-        self.l2l_direct = self.p <= 8
+        # the downward sweep straight to this pass's leaves (jb_l2l_leaves), or
+        # level by level (l2l(cascade=True), and orders 9-10 on large trees): at
+        # order 10 the direct chain spills, and where the levels are wide they
+        # are the cheaper form (clustered 2M, 99k nodes, a step: 20.20 against
+        # 20.51 ms direct; 1M, 48k nodes: 12.38 against 12.19; 200k: the sweep
+        # 368 against 169 us)
+        self.l2l_direct = self.p <= 8 or t.num_internal <= 65536
         if _on_gpu(dt):
             units, anc = l2l_leaf_schedule_device(dt, self.leaf_range)
         else:
@@ -689,7 +692,7 @@ class Pass:
                                "must not be used further")
 
     def l2l(self, stream=None, cascade: bool = False) -> None:
-        """Downward sweep after the M2L.  By default straight to the leaves:
+        """Downward sweep after the M2L.  By default (l2l_direct) straight to the leaves:
         each leaf adds L2L(a -> leaf) of every ancestor a with far pairs
         (jb_l2l_leaves, one launch; the internal nodes keep their own M2L
         sums).  cascade=True: level by level (jb_l2l_level), every node's
