@@ -515,6 +515,13 @@ JB_API int jb_leaf_eval_noalloc(int p, int p2p_mode, const float* pos4, int num_
                                 const float* centers, const float* locals, float G, float eps2, float* out_acc4,
                                 int num_slots, int num_split, const int* split, void* stream);
 
+/* Stream helpers: bytes of dst set to zero, a device-to-device copy (both kernels
+ * that keep the stream's priority; addresses and bytes multiples of 4), and
+ * `stream` made to wait for what `on` holds so far.  All capturable.        */
+JB_API int jb_zero(void* dst, int64_t bytes, void* stream);
+JB_API int jb_copy(void* dst, const void* src, int64_t bytes, void* stream);
+JB_API int jb_stream_wait(void* stream, void* on);
+
 /* Sorted slots of input-order target indices: slots[q] = inv_perm[targets[q]],
  * n particles.  An index outside [0, n) takes slot 0 and sets the flag, which
  * is copied to *bad_host (pinned, so that the copy is asynchronous): record an

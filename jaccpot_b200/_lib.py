@@ -137,6 +137,9 @@ _SIGNATURES = {
     "jb_l2l_level": [_I, _I, _I, _P, _P, _P, _P, _P],
     "jb_leaf_eval": [_I, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _F, _F, _P, _P, _I, _P, _P],
     "jb_leaf_eval_noalloc": [_I, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _F, _F, _P, _I, _I, _P, _P],
+    "jb_zero": [_P, _I64, _P],
+    "jb_copy": [_P, _P, _I64, _P],
+    "jb_stream_wait": [_P, _P],
     "jb_sort_targets": [_I64, _I64, _P, _P, _P, _P, _P, _P],
     "jb_eval_targets": [_I, _P, _I, _P, _P, _P, _P, _P, _P, _I64, _P, _F, _F, _P, _P],
     "jb_adj_near": [_P, _P, _I, _I, _P, _P, _P, _P, _F, _F, _P, _P, _I, _P, _P],

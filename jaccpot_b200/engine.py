@@ -31,13 +31,20 @@ def _ptr(t: torch.Tensor | None) -> int | None:
 
 
 def _zero(t: torch.Tensor, stream: torch.cuda.Stream | None) -> None:
-    """t.zero_() on `stream` (default: torch's current stream), in order with
-    the kernels a stage enqueues there."""
-    if stream is None:
-        t.zero_()
-    else:
-        with torch.cuda.stream(stream):
-            t.zero_()
+    """Zeroes t (contiguous) on `stream` (default: torch's current stream), in
+    order with the kernels a stage enqueues there."""
+    _lib.check(_lib.lib().jb_zero(t.data_ptr(), t.numel() * t.element_size(), _stream_handle(stream)), "jb_zero")
+
+
+def _copy(dst: torch.Tensor, src: torch.Tensor, stream: torch.cuda.Stream | None) -> None:
+    """Copies contiguous src over dst of the same size and type on `stream`."""
+    _lib.check(_lib.lib().jb_copy(dst.data_ptr(), src.data_ptr(), dst.numel() * dst.element_size(),
+                                  _stream_handle(stream)), "jb_copy")
+
+
+def _wait(stream: torch.cuda.Stream | None, on: torch.cuda.Stream | None) -> None:
+    """Makes `stream` wait for the work queued on `on` (None: torch's current stream)."""
+    _lib.check(_lib.lib().jb_stream_wait(_stream_handle(stream), _stream_handle(on)), "jb_stream_wait")
 
 
 def _stream_handle(stream: torch.cuda.Stream | None) -> int:
@@ -600,16 +607,15 @@ class Pass:
     def run_weighted(self, rung_sorted: torch.Tensor, level_weights: torch.Tensor) -> torch.Tensor:
         """run() with every pair scaled by its level's weight: the near field on
         the current stream beside the far-field chain on far_stream()."""
-        main = torch.cuda.current_stream(self.dt.device)
-        far = self.far_stream() if self.overlap else main
-        if far is not main:
-            far.wait_stream(main)
+        main, far = None, self.far_stream() if self.overlap else None
+        if far is not None:
+            _wait(far, main)
         self.evaluate_weighted(rung_sorted, level_weights, main, part="near_first")
         self.upward(far)
         self.m2l_weighted(self.far_level_weights(rung_sorted, level_weights, far), far)
         self.l2l(far)
-        if far is not main:
-            main.wait_stream(far)
+        if far is not None:
+            _wait(main, far)
         return self.evaluate_weighted(rung_sorted, level_weights, main, part="far_after")
 
     def evaluate_weighted(self, rung_sorted: torch.Tensor, level_weights: torch.Tensor, stream=None,
@@ -712,11 +718,7 @@ class Pass:
         own sums at every node -- what the adjoint reads."""
         t, dt, ws, s = self.dt.topo, self.dt, self.ws, _stream_handle(stream)
         rows = self.leaf_rows()
-        if stream is None:
-            rows.copy_(ws.locals[t.num_internal:])
-        else:
-            with torch.cuda.stream(stream):
-                rows.copy_(ws.locals[t.num_internal:])
+        _copy(rows, ws.locals[t.num_internal:], stream)
         _lib.check(self.lib.jb_l2l_leaves_to(self.p, self.num_l2l_units, _ptr(self.d_l2l_units), _ptr(self.d_l2l_anc),
                                              _ptr(ws.centers), _ptr(ws.locals), t.num_internal, _ptr(rows), s),
                    "jb_l2l_leaves_to")
@@ -831,14 +833,13 @@ class Pass:
                 self.upward(stream)
             self.downward(stream, cascade=cascade, own=own)
             return self.evaluate(stream, potential=potential)
-        main = stream if stream is not None else torch.cuda.current_stream(self.dt.device)
-        far = self.far_stream()
-        far.wait_stream(main)  # the particles are loaded
+        main, far = stream, self.far_stream()
+        _wait(far, main)  # the particles are loaded
         self.evaluate(main, potential=potential, part="near_first")
         if upward:
             self.upward(far)
         self.downward(far, cascade=cascade, own=own)
-        main.wait_stream(far)
+        _wait(main, far)
         return self.evaluate(main, potential=potential, part="far_after")
 
     def capture(self, positions: torch.Tensor, masses: torch.Tensor, acc: torch.Tensor,
@@ -929,14 +930,13 @@ class Pass:
             raise ValueError("the adjoint runs on the whole leaf range")
         t, dt, ws, lb = self.dt.topo, self.dt, self.ws, self.lib
         A = self._adj_buffers()
-        main = stream if stream is not None else torch.cuda.current_stream(dt.device)
-        far = self.far_stream() if self.overlap else main
-        s, fs = main.cuda_stream, far.cuda_stream
+        main, far = stream, self.far_stream() if self.overlap else stream
+        s, fs = _stream_handle(main), _stream_handle(far)
         w = w.to(device=dt.device, dtype=torch.float32).contiguous()
         _lib.check(lb.jb_gather_sorted(t.num_particles, _ptr(w), _ptr(A["zeros"]), _ptr(dt.perm), _ptr(A["w4"]), s),
                    "jb_gather_sorted(w)")
         if far is not main:
-            far.wait_stream(main)
+            _wait(far, main)
         sc = A["sched"]
         _lib.check(lb.jb_adj_near(_ptr(ws.pos4), _ptr(A["w4"]), t.num_internal, int(sc.units.shape[0]),
                                   _ptr(A["units"]), _ptr(A["aux"]), _ptr(A["runs"]), _ptr(dt.node_ranges), self.G,
@@ -965,7 +965,7 @@ class Pass:
                                     _ptr(dt.parent), _ptr(ws.centers), _ptr(A["cbar4"]), _ptr(A["mbar"]),
                                     _ptr(A["chain4"]), fs), "jb_adj_leaves")
         if far is not main:
-            main.wait_stream(far)
+            _wait(main, far)
         _lib.check(lb.jb_adj_particles(self.p, _ptr(ws.pos4), t.num_nodes, t.num_internal, _ptr(dt.node_ranges),
                                        _ptr(ws.centers), _ptr(A["mbar"]), _ptr(A["cbar4"]), _ptr(A["chain4"]),
                                        _ptr(A["far4"]), _ptr(A["xm4"]), s), "jb_adj_particles")
