@@ -91,21 +91,31 @@ __global__ void k_force_min_level(int first, int last, const int* __restrict__ l
 // (l+|m|)! doubled for m != 0 in the real no-sqrt2 packing
 // (_adaptive_policy.py:161-214 dehnen_multipole_power_by_degree), in FP64 for
 // l = 0..p (a point mass m at distance r has P_l = m r^l).
-__global__ void k_dehnen_power(int p, int num_nodes, const float* __restrict__ mult, int rs,
-                               double* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= num_nodes) return;
-  const float* M = mult + (size_t)i * rs;
-  for (int l = 0; l <= p; ++l) {
-    double acc = 0.0;
-    for (int m = -l; m <= l; ++m) {
-      const int am = m < 0 ? -m : m;
-      const double w = factd2(l - am) * factd2(l + am) * (m != 0 ? 2.0 : 1.0);
-      const double c = (double)M[l * l + l + m];
-      acc += w * c * c;
-    }
-    out[(size_t)i * (p + 1) + l] = sqrt(acc);
+//
+// Thread per node and degree, the weights formed once a block (a thread per
+// node that built its factorials per coefficient took 308 us at 97k nodes, p = 8).
+__global__ void __launch_bounds__(128) k_dehnen_power(int p, int num_nodes, const float* __restrict__ mult, int rs,
+                                                      double* __restrict__ out) {
+  constexpr int N = JB_MAX_ORDER + 1;
+  __shared__ double w[N][N];
+  for (int k = threadIdx.x; k < N * N; k += 128) {
+    const int l = k / N, am = k % N;
+    double f = am != 0 ? 2.0 : 1.0;  // (l - am)! (l + am)!, doubled: exact in FP64 up to l = 10
+    for (int q = 2; q <= l - am; ++q) f *= (double)q;
+    for (int q = 2; q <= l + am; ++q) f *= (double)q;
+    w[l][am] = f;
   }
+  __syncthreads();
+  const int64_t t = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  const int i = (int)(t / (p + 1)), l = (int)(t % (p + 1));
+  if (i >= num_nodes) return;
+  const float* M = mult + (size_t)i * rs + l * l + l;
+  double acc = 0.0;
+  for (int m = -l; m <= l; ++m) {
+    const double c = (double)M[m];
+    acc += w[l][m < 0 ? -m : m] * c * c;
+  }
+  out[t] = sqrt(acc);
 }
 
 // The 12 features of far pair (t <- s).
@@ -482,7 +492,7 @@ JB_API int jb_node_dehnen_power(int p, int num_nodes, const float* mult, int row
       (num_nodes > 0 && (!mult || !out)))
     return JB_ERR_ARG;
   if (num_nodes == 0) return JB_OK;
-  k_dehnen_power<<<gblocks(num_nodes, 128), 128, 0, GST(stream)>>>(p, num_nodes, mult, row_stride, out);
+  k_dehnen_power<<<gblocks((int64_t)num_nodes * (p + 1), 128), 128, 0, GST(stream)>>>(p, num_nodes, mult, row_stride, out);
   return launch_status();
 }
 

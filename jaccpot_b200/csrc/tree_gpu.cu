@@ -403,13 +403,52 @@ __device__ __forceinline__ int walk_decide(const WalkCtx& w, int a, int b) {
 // Returns the gear index, or -1.  Every step is a separately rounded FP64
 // operation (this file is compiled with -fmad=false), in the order the
 // oracle's restatement (oracle/adaptive_walk.py) uses.
-__device__ int error_gear(const WalkCtx& w, int t, int s, double d, double rt, double rs) {
-  double rtp[kMaxGearOrder + 1], dp[kMaxGearOrder + 3];
-  const int pmax = w.gear_order[w.num_gears - 1];
+//
+// The sum runs unrolled for orders up to 10 (pair_error): powers in registers
+// and the binomials as literals.  With arrays indexed by a run-time order and
+// C(p, l) by a product and a division per term (exact integers either way, so
+// the same bits) the walk's steps at clustered 1M, order 8, took 2.24 ms.
+template <int PP>
+struct Binomials {
+  double c[PP + 1] = {};
+  __host__ __device__ constexpr Binomials() {
+    c[0] = 1.0;
+    for (int l = 1; l <= PP; ++l) c[l] = c[l - 1] * (double)(PP - l + 1) / (double)l;
+  }
+};
+
+// E_p, and d^(p+2) into *dpow.
+template <int PP>
+__device__ __forceinline__ double pair_error(const double* __restrict__ P, int npow, double rt, double d, double* dpow) {
+  constexpr Binomials<PP> C{};
+  double rtp[PP + 1], e = 0.0, dp = 1.0;
   rtp[0] = 1.0;
-  for (int k = 1; k <= pmax; ++k) rtp[k] = rtp[k - 1] * rt;
-  dp[0] = 1.0;
-  for (int k = 1; k <= pmax + 2; ++k) dp[k] = dp[k - 1] * d;
+#pragma unroll
+  for (int k = 1; k <= PP; ++k) rtp[k] = rtp[k - 1] * rt;
+#pragma unroll
+  for (int l = 0; l <= PP; ++l)
+    if (l < npow) e = e + (C.c[l] * P[l]) * rtp[PP - l];
+#pragma unroll
+  for (int k = 1; k <= PP + 2; ++k) dp = dp * d;
+  *dpow = dp;
+  return e;
+}
+
+__device__ __noinline__ double pair_error_any(const double* __restrict__ P, int npow, int p, double rt, double d,
+                                              double* dpow) {
+  double rtp[kMaxGearOrder + 1], e = 0.0, c = 1.0, dp = 1.0;  // c = C(p, l)
+  rtp[0] = 1.0;
+  for (int k = 1; k <= p; ++k) rtp[k] = rtp[k - 1] * rt;
+  for (int l = 0; l <= p && l < npow; ++l) {
+    if (l > 0) c = (c * (double)(p - l + 1)) / (double)l;
+    e = e + (c * P[l]) * rtp[p - l];
+  }
+  for (int k = 1; k <= p + 2; ++k) dp = dp * d;
+  *dpow = dp;
+  return e;
+}
+
+__device__ __forceinline__ int error_gear(const WalkCtx& w, int t, int s, double d, double rt, double rs) {
   const double den = fmax(rs + rt, 1e-24);
   const double imp = (8.0 * fmax(rs, rt)) / den;
   const double thr = fmax(w.eps * (double)w.fscale[t], 1e-24);
@@ -417,13 +456,24 @@ __device__ int error_gear(const WalkCtx& w, int t, int s, double d, double rt, d
   int first = -1;
   bool pass = false;
   for (int g = 0; g < w.num_gears; ++g) {
-    const int p = w.gear_order[g];
-    double e = 0.0, c = 1.0;  // c = C(p, l)
-    for (int l = 0; l <= p && l < w.npow; ++l) {
-      if (l > 0) c = (c * (double)(p - l + 1)) / (double)l;
-      e = e + (c * P[l]) * rtp[p - l];
+    double e, dp;
+    switch (w.gear_order[g]) {  // the same for every pair of a launch
+#define JB_PAIR_ERROR(n) \
+  case n: e = pair_error<n>(P, w.npow, rt, d, &dp); break;
+      JB_PAIR_ERROR(1)
+      JB_PAIR_ERROR(2)
+      JB_PAIR_ERROR(3)
+      JB_PAIR_ERROR(4)
+      JB_PAIR_ERROR(5)
+      JB_PAIR_ERROR(6)
+      JB_PAIR_ERROR(7)
+      JB_PAIR_ERROR(8)
+      JB_PAIR_ERROR(9)
+      JB_PAIR_ERROR(10)
+#undef JB_PAIR_ERROR
+      default: e = pair_error_any(P, w.npow, w.gear_order[g], rt, d, &dp);
     }
-    const double ferr = ((w.G * imp) * e) / dp[p + 2];
+    const double ferr = ((w.G * imp) * e) / dp;
     pass = ferr < thr;
     if (pass && first < 0) first = g;
   }
