@@ -377,10 +377,12 @@ __global__ void __launch_bounds__(128) k_far_level_weights(int num_nodes, const 
 
 static inline unsigned blocks_1d(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
 
-// Fills and copies as kernels: a cudaMemsetAsync or device-to-device
-// cudaMemcpyAsync takes no stream priority, and behind a launch that fills the
-// GPU it held the far-field chain up until that drained (500k, per-pair orders:
-// the step 1139 -> 1195 us with a memset of the locals).
+// Fills and copies as kernels, on the stream given and with its priority: a
+// cudaMemsetAsync or device-to-device cudaMemcpyAsync has none, and the far
+// field's chain starts with one beside a near field that fills the GPU.  Bound
+// by the launch at small passes, by HBM at large ones (16 bytes a thread and
+// step); against a context of tensor streams around a tensor's fill or copy a
+// pass at 2k takes 64 us, not 92.
 __global__ void __launch_bounds__(256) k_fill_words(int* __restrict__ p, int64_t n, int v) {
   const int64_t step = (int64_t)gridDim.x * 256, t = (int64_t)blockIdx.x * 256 + threadIdx.x;
   const bool wide = ((uintptr_t)p & 15) == 0;
