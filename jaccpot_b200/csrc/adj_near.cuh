@@ -1,18 +1,22 @@
 #pragma once
 // Near-field adjoint, warp per leaf unit.  For the pair (k, l), d = x_k - x_l,
-// q = (|d|^2 + eps^2)^-1/2:
-//   dL/dx_k += G [ -m_l q^3 w_k + m_k q^3 w_l + 3 q^5 (m_l (w_k.d) - m_k (w_l.d)) d ]
+// q = (|d|^2 + eps^2)^-1/2, y = m_l w_k - m_k w_l:
+//   dL/dx_k += G q^3 (3 q^2 (y . d) d - y)
 //   dL/dm_k += G q^3 (w_l . d)
 // which needs l in near(k) <=> k in near(l) (the lists are symmetric).
 //
-// Per target the pair sums are S = sum q^3 m_l, V = sum q^3 w_l, A = sum q^5
-// (m_l (w_k.d) - m_k (w_l.d)) d and D = sum q^3 (w_l.d), so w_k and m_k enter
-// once a target: 26 FP32 operations and one rsqrt a pair where the terms
-// written out took 43, and the sources come two to an instruction
-// (f32x2), staged per coordinate as in k_leaf_units_flat.  The kernel is bound
-// by FP32 issue and by the seven 16-byte broadcast loads per four sources.
-// At a Plummer sphere of 1M (leaf 32, 2.0e9 pairs): 4.02 ms with one lane per
-// target and scalar pairs.
+// A close pair's m_l w_k and m_k w_l are each up to a thousand times the result
+// and nearly cancel where the cotangent varies slowly, so y is formed first, as
+// the difference of two rounded products with what the second's rounding left
+// out put back (Kahan): to about an ulp of y itself, whatever the masses, and
+// exactly 0 for w = const and equal masses or for w = m times powers of two.  Summing
+// the terms apart (m_k sum q^3 w_l - w_k sum q^3 m_l + ..., 26 operations a pair)
+// left the rounding of the large sums in the small result.
+//
+// 35 FP32 operations and one rsqrt a pair (a gradient call at a Plummer sphere of
+// 1M, order 6: 7.57 ms, 7.13 with the terms apart, 10.9 with one lane per target
+// and each pair's three terms added in turn); the sources come two to an
+// instruction (f32x2), staged per coordinate as in k_leaf_units_flat.
 #include "fmm_kernels.cuh"
 
 namespace jb {
@@ -21,25 +25,26 @@ constexpr int kAdjChunk = 32;             // sources per chunk (item)
 constexpr int kAdjSlot = kAdjChunk + 4;   // slot stride: the slots one load reads use distinct banks
 
 // Four ring slots of sources per coordinate (x, y, z, m, w), the targets and
-// their sums.
+// their sums (dL/dx, dL/dm)/G.
 struct alignas(16) AdjStage {
   float v[7][4][kAdjSlot];
-  float4 tp[32], tw[32];
-  float4 sv[32], ad[32];  // (S, V) and (A, D)
-};
-
-struct AdjSums {
-  float4 sv, ad;
+  float4 tp[32], tw[32], sum[32];
 };
 
 // One target against NS staged sources (a multiple of 4) at position o of
 // slot sl; SELF: source self_j is the target.
 template <bool SELF>
-__device__ __forceinline__ AdjSums adj_chunk(const AdjStage& st, int sl, int o, int ns, float4 t, float4 w, int self_j,
-                                             float eps2) {
+__device__ __forceinline__ float4 adj_chunk(const AdjStage& st, int sl, int o, int ns, float4 t, float4 w, int self_j,
+                                            float eps2) {
   const f32x2 TX = f2(t.x, t.x), TY = f2(t.y, t.y), TZ = f2(t.z, t.z), E2 = f2(eps2, eps2);
-  const f32x2 WX = f2(w.x, w.x), WY = f2(w.y, w.y), WZ = f2(w.z, w.z), NM = f2(-t.w, -t.w);
-  f32x2 S = f2(0.f, 0.f), VX = S, VY = S, VZ = S, AX = S, AY = S, AZ = S, D = S;
+  const f32x2 NX = f2(-w.x, -w.x), NY = f2(-w.y, -w.y), NZ = f2(-w.z, -w.z);
+  const f32x2 M = f2(t.w, t.w), NM = f2(-t.w, -t.w), M3 = f2(-3.f, -3.f);
+  f32x2 X = f2(0.f, 0.f), Y = X, Z = X, D = X;
+  // -y = m_k w_l - m_l w_k, one component
+  auto minus_y = [&](f32x2 nw, f32x2 sm, f32x2 ws) {
+    const f32x2 p = f2_mul(M, ws);
+    return f2_sub(f2_fma(sm, nw, p), f2_fma(NM, ws, p));
+  };
   auto pair2 = [&](f32x2 sx, f32x2 sy, f32x2 sz, f32x2 sm, f32x2 wx, f32x2 wy, f32x2 wz, int j0) {
     const f32x2 dx = f2_sub(TX, sx), dy = f2_sub(TY, sy), dz = f2_sub(TZ, sz);
     const f32x2 d2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, E2)));
@@ -51,24 +56,19 @@ __device__ __forceinline__ AdjSums adj_chunk(const AdjStage& st, int sl, int o, 
       qb = j0 + 1 == self_j ? 0.f : qb;
     }
     const f32x2 q = f2(qa, qb), q2 = f2_mul(q, q), q3 = f2_mul(q2, q);
-    S = f2_fma(q3, sm, S);
-    VX = f2_fma(q3, wx, VX);
-    VY = f2_fma(q3, wy, VY);
-    VZ = f2_fma(q3, wz, VZ);
-    const f32x2 wkd = f2_fma(WX, dx, f2_fma(WY, dy, f2_mul(WZ, dz)));
-    const f32x2 wld = f2_fma(wx, dx, f2_fma(wy, dy, f2_mul(wz, dz)));
-    const f32x2 c = f2_mul(f2_mul(q3, q2), f2_fma(NM, wld, f2_mul(sm, wkd)));
-    AX = f2_fma(c, dx, AX);
-    AY = f2_fma(c, dy, AY);
-    AZ = f2_fma(c, dz, AZ);
-    D = f2_fma(q3, wld, D);
+    const f32x2 yx = minus_y(NX, sm, wx), yy = minus_y(NY, sm, wy), yz = minus_y(NZ, sm, wz);
+    const f32x2 g = f2_mul(f2_mul(q2, M3), f2_fma(yx, dx, f2_fma(yy, dy, f2_mul(yz, dz))));
+    X = f2_fma(q3, f2_fma(g, dx, yx), X);
+    Y = f2_fma(q3, f2_fma(g, dy, yy), Y);
+    Z = f2_fma(q3, f2_fma(g, dz, yz), Z);
+    D = f2_fma(q3, f2_fma(wx, dx, f2_fma(wy, dy, f2_mul(wz, dz))), D);
   };
-  const ulonglong2* X[7];
+  const ulonglong2* V[7];
 #pragma unroll
-  for (int k = 0; k < 7; ++k) X[k] = reinterpret_cast<const ulonglong2*>(&st.v[k][sl][o]);
+  for (int k = 0; k < 7; ++k) V[k] = reinterpret_cast<const ulonglong2*>(&st.v[k][sl][o]);
 #pragma unroll 4
   for (int i = 0; i < ns / 4; ++i) {
-    const ulonglong2 x = X[0][i], y = X[1][i], z = X[2][i], m = X[3][i], wx = X[4][i], wy = X[5][i], wz = X[6][i];
+    const ulonglong2 x = V[0][i], y = V[1][i], z = V[2][i], m = V[3][i], wx = V[4][i], wy = V[5][i], wz = V[6][i];
     pair2(x.x, y.x, z.x, m.x, wx.x, wy.x, wz.x, 4 * i);
     pair2(x.y, y.y, z.y, m.y, wx.y, wy.y, wz.y, 4 * i + 2);
   }
@@ -77,7 +77,7 @@ __device__ __forceinline__ AdjSums adj_chunk(const AdjStage& st, int sl, int o, 
     f2_split(v, lo, hi);
     return lo + hi;
   };
-  return AdjSums{make_float4(sum(S), sum(VX), sum(VY), sum(VZ)), make_float4(sum(AX), sum(AY), sum(AZ), sum(D))};
+  return make_float4(sum(X), sum(Y), sum(Z), sum(D));
 }
 
 __device__ __forceinline__ float4 add4(float4 a, float4 b) {
@@ -116,20 +116,16 @@ __device__ __forceinline__ void adj_unit(const float4* __restrict__ pos4, const 
   const bool tgt = lane < nt;
   S.tp[lane] = tgt ? pos4[rg.x + lane] : zero4;
   S.tw[lane] = tgt ? w4[rg.x + lane] : zero4;
-  S.sv[lane] = zero4;
-  S.ad[lane] = zero4;
+  S.sum[lane] = zero4;
   __syncwarp();
   // adds the items' sums, G lanes to a target, in lane order
-  auto add_items = [&](AdjSums v, int nl) {
+  auto add_items = [&](float4 v, int nl) {
 #pragma unroll
     for (int h = 1; h < G; ++h) {
-      const float4 a = shfl_down4(v.sv, h), b = shfl_down4(v.ad, h);
-      if (lane % G == 0) v.sv = add4(v.sv, a), v.ad = add4(v.ad, b);
+      const float4 a = shfl_down4(v, h);
+      if (lane % G == 0) v = add4(v, a);
     }
-    if (lane % G == 0 && lane < nl) {
-      S.sv[lane / G] = add4(S.sv[lane / G], v.sv);
-      S.ad[lane / G] = add4(S.ad[lane / G], v.ad);
-    }
+    if (lane % G == 0 && lane < nl) S.sum[lane / G] = add4(S.sum[lane / G], v);
   };
   if (aux.y & 1) {  // the leaf itself, 32 at a time, the diagonal excluded
     for (int b = lr.x; b <= lr.y; b += 32) {
@@ -178,16 +174,12 @@ __device__ __forceinline__ void adj_unit(const float4* __restrict__ pos4, const 
           if (++staged < C) fetch(staged * CH + lane);
         }
         __syncwarp();
-        const AdjSums v = adj_chunk<false>(S, c & 3, 0, CH, S.tp[t], S.tw[t], -1, eps2);
-        const float4 sv2 = shfl_down4(v.sv, nt), ad2 = shfl_down4(v.ad, nt);
+        const float4 v = adj_chunk<false>(S, c & 3, 0, CH, S.tp[t], S.tw[t], -1, eps2);
+        const float4 v2 = shfl_down4(v, nt);
         if (tgt && base + lane < total) {
-          float4 a = add4(S.sv[t], v.sv), b = add4(S.ad[t], v.ad);
-          if (lane + nt < 32 && base + lane + nt < total) {  // lane + nt holds (t, c + 1)
-            a = add4(a, sv2);
-            b = add4(b, ad2);
-          }
-          S.sv[t] = a;
-          S.ad[t] = b;
+          float4 a = add4(S.sum[t], v);
+          if (lane + nt < 32 && base + lane + nt < total) a = add4(a, v2);  // lane + nt holds (t, c + 1)
+          S.sum[t] = a;
         }
         t += 32 - nt;  // item f + 32
         c += 1;
@@ -200,10 +192,8 @@ __device__ __forceinline__ void adj_unit(const float4* __restrict__ pos4, const 
   }
   __syncwarp();
   if (tgt) {
-    const float4 sv = S.sv[lane], ad = S.ad[lane], w = S.tw[lane];
-    const float m = S.tp[lane].w;
-    const float4 res = make_float4(G_ * (m * sv.y - sv.x * w.x + 3.f * ad.x), G_ * (m * sv.z - sv.x * w.y + 3.f * ad.y),
-                                   G_ * (m * sv.w - sv.x * w.z + 3.f * ad.z), G_ * ad.w);
+    const float4 v = S.sum[lane];
+    const float4 res = make_float4(G_ * v.x, G_ * v.y, G_ * v.z, G_ * v.w);
     if (aux.x < 0) out[rg.x + lane] = res;
     else partial[(size_t)aux.x * kMaxLeaf + row + lane] = res;
   }

@@ -119,3 +119,38 @@ def test_sweeps_straight_to_the_leaves_match_the_level_sweeps(kind, n, p, leaf, 
     em = np.abs(gm - wm) / np.maximum(np.abs(wm), 1e-3 * np.abs(wm).max())
     assert np.percentile(ex, 99) <= 1e-4, np.percentile(ex, [50, 99, 100])
     assert np.percentile(em, 99) <= 1e-4, np.percentile(em, [50, 99, 100])
+
+
+@pytest.mark.parametrize("cotangent", ["constant", "position", "mass", "few"])
+@pytest.mark.parametrize("masses", ["equal", "spread"])
+@pytest.mark.parametrize("n,leaf,sources", [(60, 8, 4096), (700, 16, 4096), (700, 25, 4096), (900, 30, 100),
+                                            (1500, 64, 4096)])
+def test_near_field_gradient_cancels_within_the_pair(n, leaf, sources, masses, cotangent):
+    """Cotangents that vary slowly between neighbours, on particles of which half
+    have a neighbour at a thousandth of the usual distance: the pair's m_l w_k -
+    m_k w_l is far below its two terms.  Each component is a sum of n terms of at
+    most 4 q^3 |m_l w_k - m_k w_l|, T_i in all, each with fewer than 85
+    roundings, the differences among them rounded at their own size:
+    |difference| <= (104 + n / 32) 2^-23 T_i.  With a constant cotangent on equal
+    masses, or one proportional to the masses, T_i and the gradient are 0."""
+    rng = np.random.default_rng(5)
+    pos, mass = workloads.plummer(n, 3)
+    pos[n // 2:] = pos[:n - n // 2] + 1e-3 * rng.normal(size=(n - n // 2, 3))
+    pos = pos.astype(np.float32)
+    mass = np.full(n, 1.0 / n) if masses == "equal" else np.exp(2.0 * rng.normal(size=n)) / n
+    mass = mass.astype(np.float32)
+    # halves and doubles are exact, so that "mass" is proportional in FP32 too
+    w = {"constant": np.full((n, 3), 0.7), "position": pos, "mass": mass[:, None] * np.array([0.5, 2.0, 1.0]),
+         "few": np.where(np.arange(n)[:, None] % 20 == 0, rng.normal(size=(n, 3)), 0.0)}[cotangent].astype(np.float32)
+    topo = tree.build_topology(pos, mass, leaf_size=leaf, theta=1e-6, device="cuda")
+    assert topo.num_far_pairs == 0
+    gx, _ = _grad(topo, 4, pos, mass, w, 0.0, leaf_unit_sources=sources)
+    x, m, ww = pos.astype(np.float64), mass.astype(np.float64), w.astype(np.float64)
+    d = x[:, None] - x[None]
+    r2 = (d ** 2).sum(-1)
+    np.fill_diagonal(r2, np.inf)
+    q = 1.0 / np.sqrt(r2)
+    y = m[None, :, None] * ww[:, None] - m[:, None, None] * ww[None]
+    want = ((q ** 3)[..., None] * (3 * (q ** 2 * (y * d).sum(-1))[..., None] * d - y)).sum(1)
+    size = (4 * q ** 3 * np.linalg.norm(y, axis=-1)).sum(1)
+    assert (np.abs(gx - want).max(1) <= (104 + n / 32) * 2.0 ** -23 * size).all()
