@@ -437,11 +437,6 @@ JB_API int jb_l2l_level(int p, int first, int last, const int* left, const int* 
 JB_API int jb_l2l_leaves(int p, int num_units, const int* units, const int* anc, const float* centers,
                          float* locals, void* stream);
 
-/* jb_l2l_leaves with the sums added to leaf_rows (num_leaves rows that hold the
- * leaves' own M2L sums) instead of the leaves' rows of locals.              */
-JB_API int jb_l2l_leaves_to(int p, int num_units, const int* units, const int* anc, const float* centers,
-                            const float* locals, int num_internal, float* leaf_rows, void* stream);
-
 /* Leaf evaluation over work units: L2P of each leaf's local at its particles
  * (runtime/kernels/_evaluate.py:2106-2484, evaluate_local_real_with_grad) plus
  * the near field over the self leaf and the leaf's neighbour list
@@ -564,11 +559,11 @@ JB_API int jb_gather_unsorted(int64_t n, const float* acc4, const int64_t* inv_p
 /*   jb_adj_m2l, jb_adj_m2l_centers, jb_adj_m2m_level (root first),         */
 /*   jb_adj_p2m.  cbar4 (num_nodes float4) and mbar (num_nodes x stride)    */
 /*   start at zero.  Or, in a third of the launches and with a near field    */
-/*   that can run beside the rest, from locals that hold each node's own M2L */
-/*   sum: jb_adj_near; jb_adj_leaf_far (cbar4 NULL, xm4 a buffer of its own, */
-/*   the leaves' complete locals from jb_l2l_leaves_to), jb_adj_l2l_hops,    */
-/*   jb_adj_m2l, jb_adj_far_nodes, jb_adj_leaves; jb_adj_particles.  mbar and */
-/*   chain4 start at zero; w4 is the sorted float4 cotangent (w, 0);         */
+/*   that can run beside the rest, after jb_l2l_leaves and with a copy of the */
+/*   leaves' rows from before it (own M2L sums): jb_adj_near; jb_adj_leaf_far */
+/*   (cbar4 NULL, xm4 a buffer of its own), jb_adj_l2l_hops, jb_adj_m2l,     */
+/*   jb_adj_far_nodes, jb_adj_leaves; jb_adj_particles.  mbar and chain4     */
+/*   start at zero; w4 is the sorted float4 cotangent (w, 0);         */
 /*   xm4[i] = (dL/dx, dL/dy, dL/dz, dL/dm) sorted.  Needs symmetric near and */
 /*   far lists (jb_tree_build emits both directions).  Orders 1..9.         */
 /* ------------------------------------------------------------------------ */
@@ -606,11 +601,12 @@ JB_API int jb_adj_m2m_level(int p, int first, int last, const int* left, const i
 JB_API int jb_adj_l2l_hops(int p, int num_hops, const int64_t* hop_offsets, const int* items, const float* centers,
                            float* lbar, void* stream);
 /* cbar4 of every node (set): the M2L's displacement terms (g4: scratch of
- * num_pairs float4) and Lbar . D L - M . D Mbar with the node's own M2L sums. */
+ * num_pairs float4) and Lbar . D L - M . D Mbar with the node's own M2L sums:
+ * rows of locals, for leaves those of own_rows (num_nodes - num_internal rows). */
 JB_API int jb_adj_far_nodes(int p, int num_nodes, int64_t num_pairs, const int* pair_tgt, const int* far_src,
                             const int64_t* far_off, const int* rev, const float* mult, const float* lbar,
-                            const float* locals, const float* mbar, const float* centers, float* g4, float* cbar4,
-                            void* stream);
+                            const float* locals, int num_internal, const float* own_rows, const float* mbar,
+                            const float* centers, float* g4, float* cbar4, void* stream);
 /* M2M VJP straight to the leaves, over the units of jb_l2l_schedule_device:
  * adds each leaf's ancestors into its mbar row; chain4[leaf] (num_nodes rows)
  * is the chain of the centres of mass.                                      */

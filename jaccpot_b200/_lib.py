@@ -148,10 +148,9 @@ _SIGNATURES = {
     "jb_adj_m2l": [_I, _I, _P, _P, _P, _P, _P, _P, _I, _P, _P],
     "jb_adj_m2l_centers": [_I, _I, _I64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P],
     "jb_adj_l2l_hops": [_I, _I, _P, _P, _P, _P, _P],
-    "jb_adj_far_nodes": [_I, _I, _I64, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P],
+    "jb_adj_far_nodes": [_I, _I, _I64, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _P, _P],
     "jb_adj_leaves": [_I, _I, _P, _P, _P, _P, _P, _P, _P, _P],
     "jb_adj_particles": [_I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P],
-    "jb_l2l_leaves_to": [_I, _I, _P, _P, _P, _P, _I, _P, _P],
     "jb_adj_m2m_level": [_I, _I, _I, _P, _P, _P, _P, _P, _P, _P],
     "jb_adj_p2m": [_I, _P, _I, _I, _P, _P, _P, _P, _P, _P],
     "jb_gear_param_count": [],

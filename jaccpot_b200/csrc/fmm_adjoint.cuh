@@ -298,8 +298,9 @@ template <int P>
 __global__ void __launch_bounds__(128) k_adj_nodes(int num_nodes, const int64_t* __restrict__ far_off,
                                                    const int* __restrict__ rev, const float4* __restrict__ g4,
                                                    const float* __restrict__ mult, const float* __restrict__ lbar,
-                                                   const float* __restrict__ locals, const float* __restrict__ mbar,
-                                                   float4* __restrict__ cbar4) {
+                                                   const float* __restrict__ locals, int num_internal,
+                                                   const float* __restrict__ own_rows,
+                                                   const float* __restrict__ mbar, float4* __restrict__ cbar4) {
   constexpr int C = csize(P), CS = cstride(P);
   const int u = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (u >= num_nodes) return;
@@ -313,10 +314,11 @@ __global__ void __launch_bounds__(128) k_adj_nodes(int num_nodes, const int64_t*
       z += a.z - b.z;
     }
     const size_t o = (size_t)u * CS;
+    const float* F = u < num_internal ? locals + o : own_rows + (size_t)(u - num_internal) * CS;
     for (int k = lane; k < C; k += 32) {
       float wx, wy, wz;
       ladder_col(lbar + o, k, wx, wy, wz);
-      const float f = locals[o + k];
+      const float f = F[k];
       x = fmaf(wx, f, x), y = fmaf(wy, f, y), z = fmaf(wz, f, z);
       ladder_col(mult + o, k, wx, wy, wz);
       const float h = -mbar[o + k];
@@ -502,7 +504,8 @@ struct RunAdj {
   static int m2l_pairs(int64_t num_pairs, const int* pair_tgt, const int* far_src, const float* mult,
                        const float* lbar, const float* centers, float* g4, cudaStream_t st);
   static int nodes(int num_nodes, const int64_t* far_off, const int* rev, const float* g4, const float* mult,
-                   const float* lbar, const float* locals, const float* mbar, float* cbar4, cudaStream_t st);
+                   const float* lbar, const float* locals, int num_internal, const float* own_rows, const float* mbar,
+                   float* cbar4, cudaStream_t st);
   static int l2l_hops(int num_hops, const int64_t* off, const int* items, const float* centers, float* lbar,
                       cudaStream_t st);
   static int leaves(int num_units, const int* units, const int* anc, const int* parent, const float* centers,
@@ -556,9 +559,11 @@ int RunAdj<P>::m2l_pairs(int64_t num_pairs, const int* pair_tgt, const int* far_
 
 template <int P>
 int RunAdj<P>::nodes(int num_nodes, const int64_t* far_off, const int* rev, const float* g4, const float* mult,
-                     const float* lbar, const float* locals, const float* mbar, float* cbar4, cudaStream_t st) {
+                     const float* lbar, const float* locals, int num_internal, const float* own_rows, const float* mbar,
+                     float* cbar4, cudaStream_t st) {
   k_adj_nodes<P><<<blocks_for(num_nodes, 4), 128, 0, st>>>(num_nodes, far_off, rev, reinterpret_cast<const float4*>(g4),
-                                                           mult, lbar, locals, mbar, reinterpret_cast<float4*>(cbar4));
+                                                           mult, lbar, locals, num_internal, own_rows, mbar,
+                                                           reinterpret_cast<float4*>(cbar4));
   return launch_status();
 }
 
@@ -571,7 +576,7 @@ int RunAdj<P>::l2l_hops(int num_hops, const int64_t* off, const int* items, cons
 template <int P>
 int RunAdj<P>::leaves(int num_units, const int* units, const int* anc, const int* parent, const float* centers,
                       const float* cbar4, float* mbar, float* chain4, cudaStream_t st) {
-  return launch_l2l_leaves<P, true>(num_units, units, anc, centers, mbar, mbar, cbar4, chain4, parent, st);
+  return launch_l2l_leaves<P, true>(num_units, units, anc, centers, mbar, cbar4, chain4, parent, st);
 }
 
 template <int P>

@@ -725,18 +725,7 @@ JB_API int jb_m2l_mixed(int p_max, int num_units, const int* units, const int* b
 JB_API int jb_l2l_leaves(int p, int num_units, const int* units, const int* anc, const float* centers,
                          float* locals, void* stream) {
   if (num_units < 0 || (num_units > 0 && (!units || !anc || !centers || !locals))) return JB_ERR_ARG;
-  return dispatch<RunL2LLeaves>(p, num_units, units, anc, centers, locals, locals, ST(stream));
-}
-
-JB_API int jb_l2l_leaves_to(int p, int num_units, const int* units, const int* anc, const float* centers,
-                            const float* locals, int num_internal, float* leaf_rows, void* stream) {
-  if (num_units < 0 || num_internal < 0 ||
-      (num_units > 0 && (!units || !anc || !centers || !locals || !leaf_rows)))
-    return JB_ERR_ARG;
-  const int cs = jb_coeff_stride(p);
-  if (cs <= 0) return JB_ERR_ORDER;
-  return dispatch<RunL2LLeaves>(p, num_units, units, anc, centers, locals, leaf_rows - (ptrdiff_t)num_internal * cs,
-                                ST(stream));
+  return dispatch<RunL2LLeaves>(p, num_units, units, anc, centers, locals, ST(stream));
 }
 
 JB_API int jb_l2l_level(int p, int first, int last, const int* left, const int* right, const float* centers,
@@ -902,14 +891,17 @@ JB_API int jb_adj_l2l_hops(int p, int num_hops, const int64_t* hop_offsets, cons
 
 JB_API int jb_adj_far_nodes(int p, int num_nodes, int64_t num_pairs, const int* pair_tgt, const int* far_src,
                             const int64_t* far_off, const int* rev, const float* mult, const float* lbar,
-                            const float* locals, const float* mbar, const float* centers, float* g4, float* cbar4,
-                            void* stream) {
-  if (num_nodes < 1 || num_pairs < 0 || !far_off || !cbar4 || !mult || !lbar || !locals || !mbar ||
+                            const float* locals, int num_internal, const float* own_rows, const float* mbar,
+                            const float* centers, float* g4, float* cbar4, void* stream) {
+  if (num_nodes < 1 || num_pairs < 0 || num_internal < 0 || num_internal >= num_nodes || !far_off || !cbar4 || !mult ||
+      !lbar || !locals || !own_rows || !mbar ||
       (num_pairs > 0 && (!pair_tgt || !far_src || !rev || !centers || !g4)))
     return JB_ERR_ARG;
   return dispatch_adj(p, [&](auto R) {
     const int rc = decltype(R)::m2l_pairs(num_pairs, pair_tgt, far_src, mult, lbar, centers, g4, ST(stream));
-    return rc ? rc : decltype(R)::nodes(num_nodes, far_off, rev, g4, mult, lbar, locals, mbar, cbar4, ST(stream));
+    return rc ? rc
+              : decltype(R)::nodes(num_nodes, far_off, rev, g4, mult, lbar, locals, num_internal, own_rows, mbar, cbar4,
+                                   ST(stream));
   });
 }
 

@@ -413,17 +413,16 @@ __global__ void __launch_bounds__(kM2LThreads, 4) k_m2l_units_coop(int num_units
 // with every leaf's chain in parallel, where the cascade runs one dependent
 // launch per level.
 //
-// Results go to rows out + leaf * stride, which hold the leaves' own sums
-// before (out = locals: in place).  ADJ is the same sweep of the M2M's
-// adjoint: L2L(c_leaf - c_a) of each ancestor's row, and per leaf the chain of
-// the centres of mass, chain4[leaf] = (sum_a cbar_a / mu_a, sum_a (c_leaf - c_a)
-// . cbar_a / mu_a); below a node without mass, whose centre the masses do not
-// move, that node stands for the leaf in the last sum.
+// ADJ is the same sweep of the M2M's adjoint: L2L(c_leaf - c_a) of each
+// ancestor's row, and per leaf the chain of the centres of mass, chain4[leaf] =
+// (sum_a cbar_a / mu_a, sum_a (c_leaf - c_a) . cbar_a / mu_a); below a node
+// without mass, whose centre the masses do not move, that node stands for the
+// leaf in the last sum.
 template <int P, bool ADJ>
 __global__ void __launch_bounds__(kM2LThreads, 4) k_l2l_leaves(int num_units, const int4* __restrict__ units,
                                                                const int* __restrict__ anc,
                                                                const float4* __restrict__ centers,
-                                                               const float* locals, float* out,
+                                                               float* __restrict__ locals,
                                                                const float4* __restrict__ cbar4,
                                                                float4* __restrict__ chain4,
                                                                const int* __restrict__ parent) {
@@ -496,7 +495,7 @@ __global__ void __launch_bounds__(kM2LThreads, 4) k_l2l_leaves(int num_units, co
   }
   cp_async_wait_all();
   if (!ok || n == 0) return;
-  float* dst = out + (ptrdiff_t)leaf * CS;
+  float* dst = locals + (size_t)leaf * CS;
 #pragma unroll
   for (int k = 0; k < C; ++k) dst[k] += acc[k];
   if (ADJ) chain4[leaf] = chain;
@@ -1906,27 +1905,27 @@ int RunL2L<P>::run(int first, int last, const int* left, const int* right, const
 }
 
 template <int P, bool ADJ>
-int launch_l2l_leaves(int num_units, const int* units, const int* anc, const float* centers, const float* locals,
-                      float* out, const float* cbar4, float* chain4, const int* parent, cudaStream_t st) {
+int launch_l2l_leaves(int num_units, const int* units, const int* anc, const float* centers, float* locals,
+                      const float* cbar4, float* chain4, const int* parent, cudaStream_t st) {
   if (num_units <= 0) return JB_OK;
   const size_t sm = sizeof(float4) * kM2LThreads * row4(P) + sizeof(int) * kM2LThreads;
   cudaFuncSetAttribute(k_l2l_leaves<P, ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_l2l_leaves<P, ADJ><<<blocks_for(num_units, kM2LThreads), kM2LThreads, sm, st>>>(
-      num_units, reinterpret_cast<const int4*>(units), anc, reinterpret_cast<const float4*>(centers), locals, out,
+      num_units, reinterpret_cast<const int4*>(units), anc, reinterpret_cast<const float4*>(centers), locals,
       reinterpret_cast<const float4*>(cbar4), reinterpret_cast<float4*>(chain4), parent);
   return launch_status();
 }
 
 template <int P>
 struct RunL2LLeaves {
-  static int run(int num_units, const int* units, const int* anc, const float* centers, const float* locals, float* out,
+  static int run(int num_units, const int* units, const int* anc, const float* centers, float* locals,
                  cudaStream_t st);
 };
 
 template <int P>
-int RunL2LLeaves<P>::run(int num_units, const int* units, const int* anc, const float* centers, const float* locals,
-                         float* out, cudaStream_t st) {
-  return launch_l2l_leaves<P, false>(num_units, units, anc, centers, locals, out, nullptr, nullptr, nullptr, st);
+int RunL2LLeaves<P>::run(int num_units, const int* units, const int* anc, const float* centers, float* locals,
+                         cudaStream_t st) {
+  return launch_l2l_leaves<P, false>(num_units, units, anc, centers, locals, nullptr, nullptr, nullptr, st);
 }
 
 template <int P>

@@ -399,7 +399,6 @@ class Pass:
         self.m2l_unit_pairs = int(m2l_unit_pairs)
         self.leaf_unit_sources = int(leaf_unit_sources)
         self.ws = Workspace.allocate(dt, self.p)
-        self.own_locals = False  # ws.locals holds the M2L's own sums, leaf_rows() the leaves' complete locals
         self.lib = _lib.lib()
         t = dt.topo
         self.leaf_range = (0, t.num_leaves) if leaf_range is None else (int(leaf_range[0]), int(leaf_range[1]))
@@ -463,9 +462,8 @@ class Pass:
         q.leaf_partials = torch.empty_like(self.leaf_partials)
         if getattr(self, "gear_sched", None) is not None:
             q.gear_partials = torch.empty_like(self.gear_partials)
-        for name in ("_tc", "_tc_status", "_adj", "_far_stream", "_leaf_rows", "_weights"):
+        for name in ("_tc", "_tc_status", "_adj", "_far_stream", "_weights"):
             q.__dict__.pop(name, None)
-        q.own_locals = False
         return q
 
     def near_pair_interactions(self) -> torch.Tensor:
@@ -547,7 +545,6 @@ class Pass:
 
     def m2l(self, stream=None) -> None:
         ws, s, sc = self.ws, _stream_handle(stream), self.m2l_sched
-        self.own_locals = False
         _zero(ws.locals, stream)
         if self.m2l_mode == _lib.JB_M2L_SPLIT_BF16:
             self._m2l_split(s, stream)
@@ -578,7 +575,6 @@ class Pass:
         w = far_w.to(device=self.dt.device, dtype=torch.float32).contiguous()
         if w.numel() != self.dt.topo.num_far_pairs:
             raise ValueError("one weight per far pair is required")
-        self.own_locals = False
         _zero(ws.locals, stream)
         _lib.check(self.lib.jb_m2l_weighted(self.p, int(sc.units.shape[0]), _ptr(self.d_m2l_units), _ptr(ws.mult),
                                             _ptr(ws.centers), _ptr(self.dt.far_src), _ptr(w) if w.numel() else None,
@@ -631,7 +627,7 @@ class Pass:
         _lib.check(self.lib.jb_leaf_eval_weighted(self.p, mode, _ptr(ws.pos4), _ptr(r), int(lw.numel()), _ptr(lw),
                                                   t.num_internal, int(sc.units.shape[0]), _ptr(self.d_leaf_units),
                                                   _ptr(self.d_leaf_aux), _ptr(self.d_leaf_runs),
-                                                  _ptr(dt.node_ranges), _ptr(ws.centers), self._leaf_locals_ptr(),
+                                                  _ptr(dt.node_ranges), _ptr(ws.centers), _ptr(ws.locals),
                                                   self.G, self.eps2, _ptr(ws.acc4), _ptr(self.leaf_partials),
                                                   int(sc.split.shape[0]), _ptr(self.d_leaf_split),
                                                   _stream_handle(stream)), "jb_leaf_eval_weighted")
@@ -701,41 +697,21 @@ class Pass:
         """Downward sweep after the M2L.  By default (l2l_direct) straight to the leaves:
         each leaf adds L2L(a -> leaf) of every ancestor a with far pairs
         (jb_l2l_leaves, one launch; the internal nodes keep their own M2L
-        sums).  cascade=True: level by level (jb_l2l_level), every node's
-        local complete -- what the adjoint reads."""
+        sums, which the adjoint reads).  cascade=True: level by level
+        (jb_l2l_level), every node's local complete."""
         t, dt, ws, s = self.dt.topo, self.dt, self.ws, _stream_handle(stream)
         if self.l2l_direct and not cascade:
-            _lib.check(self.lib.jb_l2l_leaves(self.p, self.num_l2l_units, _ptr(self.d_l2l_units), _ptr(self.d_l2l_anc),
-                                              _ptr(ws.centers), _ptr(ws.locals), s), "jb_l2l_leaves")
+            self._l2l_leaves(stream)
             return
         lo = dt.level_offsets
         for lev in range(dt.l2l_first_level, t.num_levels):
             _lib.check(self.lib.jb_l2l_level(self.p, lo[lev], lo[lev + 1], _ptr(dt.left), _ptr(dt.right),
                                              _ptr(ws.centers), _ptr(ws.locals), s), "jb_l2l_level")
 
-    def l2l_to_rows(self, stream=None) -> None:
-        """The downward sweep into leaf_rows(), with ws.locals left as the M2L's
-        own sums at every node -- what the adjoint reads."""
-        t, dt, ws, s = self.dt.topo, self.dt, self.ws, _stream_handle(stream)
-        rows = self.leaf_rows()
-        _copy(rows, ws.locals[t.num_internal:], stream)
-        _lib.check(self.lib.jb_l2l_leaves_to(self.p, self.num_l2l_units, _ptr(self.d_l2l_units), _ptr(self.d_l2l_anc),
-                                             _ptr(ws.centers), _ptr(ws.locals), t.num_internal, _ptr(rows), s),
-                   "jb_l2l_leaves_to")
-        self.own_locals = True
-
-    def leaf_rows(self) -> torch.Tensor:
-        """(leaves, stride): the leaves' complete locals beside ws.locals."""
-        if getattr(self, "_leaf_rows", None) is None:
-            self._leaf_rows = torch.empty((self.dt.topo.num_leaves, self.ws.stride), device=self.dt.device,
-                                          dtype=torch.float32)
-        return self._leaf_rows
-
-    def _leaf_locals_ptr(self) -> int:
-        """Base address for the kernels that read leaf rows by node id."""
-        if not self.own_locals:
-            return _ptr(self.ws.locals)
-        return _ptr(self.leaf_rows()) - 4 * self.ws.stride * self.dt.topo.num_internal
+    def _l2l_leaves(self, stream) -> None:
+        _lib.check(self.lib.jb_l2l_leaves(self.p, self.num_l2l_units, _ptr(self.d_l2l_units), _ptr(self.d_l2l_anc),
+                                          _ptr(self.ws.centers), _ptr(self.ws.locals), _stream_handle(stream)),
+                   "jb_l2l_leaves")
 
     _PARTS = {"near": _lib.JB_P2P_NEAR_ONLY, "far": _lib.JB_P2P_FAR_ONLY,
               "near_first": _lib.JB_P2P_NEAR_FIRST, "far_after": _lib.JB_P2P_FAR_AFTER}
@@ -756,7 +732,7 @@ class Pass:
             mode |= self._PARTS[part]
         _lib.check(self.lib.jb_leaf_eval(self.p, mode, _ptr(ws.pos4), t.num_internal, int(sc.units.shape[0]),
                                          _ptr(self.d_leaf_units), _ptr(self.d_leaf_aux), _ptr(self.d_leaf_runs),
-                                         _ptr(dt.node_ranges), _ptr(ws.centers), self._leaf_locals_ptr(), self.G,
+                                         _ptr(dt.node_ranges), _ptr(ws.centers), _ptr(ws.locals), self.G,
                                          self.eps2, _ptr(acc4), _ptr(self.leaf_partials),
                                          int(sc.split.shape[0]), _ptr(self.d_leaf_split),
                                          _stream_handle(stream)), "jb_leaf_eval")
@@ -770,7 +746,7 @@ class Pass:
         if out is None:
             out = torch.empty((nt, 4), device=dt.device, dtype=torch.float32)
         _lib.check(self.lib.jb_eval_targets(self.p, _ptr(ws.pos4), t.num_internal, _ptr(dt.node_ranges),
-                                            _ptr(ws.centers), self._leaf_locals_ptr(), _ptr(dt.near_off),
+                                            _ptr(ws.centers), _ptr(ws.locals), _ptr(dt.near_off),
                                             _ptr(dt.near_src), _ptr(dt.leaf_of), nt, _ptr(ts), self.G, self.eps2,
                                             _ptr(out), _stream_handle(stream)), "jb_eval_targets")
         return out
@@ -802,12 +778,25 @@ class Pass:
         _lib.check(self.lib.jb_gather_unsorted(n, _ptr(self.ws.acc4), _ptr(self.dt.inv_perm), _ptr(acc),
                                                _ptr(pot), _stream_handle(stream)), "jb_gather_unsorted")
 
-    def downward(self, stream=None, cascade: bool = False, own: bool = False) -> None:
+    def downward(self, stream=None, cascade: bool = False, own_rows: torch.Tensor | None = None) -> None:
+        """M2L and L2L.  own_rows (leaves, stride), float32: takes the leaves' own
+        M2L sums before the sweep adds their ancestors', for vjp; the sweep then
+        goes straight to the leaves, so the internal nodes keep theirs."""
         self.m2l(stream)
-        if own:
-            self.l2l_to_rows(stream)
-        else:
+        if own_rows is None:
             self.l2l(stream, cascade=cascade)
+            return
+        ws, ni = self.ws, self.dt.topo.num_internal
+        if cascade:
+            raise ValueError("the level-by-level sweep leaves no node's own sums")
+        self._check_own_rows(own_rows)
+        _copy(own_rows, ws.locals[ni:], stream)
+        self._l2l_leaves(stream)
+
+    def _check_own_rows(self, rows: torch.Tensor) -> None:
+        want = (self.dt.topo.num_leaves, self.ws.stride)
+        if tuple(rows.shape) != want or rows.dtype != torch.float32 or not rows.is_contiguous() or not rows.is_cuda:
+            raise ValueError(f"own_rows must be a contiguous float32 device tensor of shape {want}")
 
     def far_stream(self) -> torch.cuda.Stream:
         """The high-priority stream run(overlap=True) puts the far-field chain
@@ -819,11 +808,10 @@ class Pass:
         return self._far_stream
 
     def run(self, stream=None, cascade: bool = False, potential: bool = False,
-            overlap: bool | None = None, own: bool = False, upward: bool = True) -> torch.Tensor:
+            overlap: bool | None = None, own_rows: torch.Tensor | None = None, upward: bool = True) -> torch.Tensor:
         """Whole pass on the particles already in ws.pos4; returns sorted acc4
-        (cascade: the level-by-level downward sweep, see l2l; own: leave every
-        node's own M2L sum in ws.locals, see l2l_to_rows; upward=False: the
-        centres and multipoles are already there).  overlap
+        (cascade: the level-by-level downward sweep, see l2l; own_rows: see
+        downward; upward=False: the centres and multipoles are already there).  overlap
         (default self.overlap): the near field runs on `stream` while the
         upward sweep, M2L and L2L run on far_stream(), joined before the L2P
         and the sum of split leaves; the result has the same bits as the
@@ -831,14 +819,14 @@ class Pass:
         if not (self.overlap if overlap is None else overlap):
             if upward:
                 self.upward(stream)
-            self.downward(stream, cascade=cascade, own=own)
+            self.downward(stream, cascade=cascade, own_rows=own_rows)
             return self.evaluate(stream, potential=potential)
         main, far = stream, self.far_stream()
         _wait(far, main)  # the particles are loaded
         self.evaluate(main, potential=potential, part="near_first")
         if upward:
             self.upward(far)
-        self.downward(far, cascade=cascade, own=own)
+        self.downward(far, cascade=cascade, own_rows=own_rows)
         _wait(main, far)
         return self.evaluate(main, potential=potential, part="far_after")
 
@@ -898,6 +886,7 @@ class Pass:
                 "mbar": torch.empty((t.num_nodes, cs), **f32),
                 "cbar4": torch.empty((t.num_nodes, 4), **f32),
                 "chain4": torch.empty((t.num_nodes, 4), **f32),
+                "own_rows": torch.empty((t.num_leaves, cs), **f32),
                 "g4": torch.empty((max(t.num_far_pairs, 1), 4), **f32),
                 "pair_tgt": dt.far_pair_targets(),
                 "rev": (dt.far_reverse_index() if t.num_far_pairs else torch.zeros(1, dtype=torch.int32, device=dev)),
@@ -916,19 +905,22 @@ class Pass:
         return self._adj
 
     def vjp(self, w: torch.Tensor, grad_pos: torch.Tensor, grad_mass: torch.Tensor, stream=None,
-            recompute: bool = True) -> None:
+            recompute: bool = True, own_rows: torch.Tensor | None = None) -> None:
         """Gradient of sum(w * acc) w.r.t. the input-order positions and masses
         currently loaded (acc = the pass's accelerations, input order), written
         into grad_pos (N,3) and grad_mass (N,).  recompute=True reruns the
         upward and downward sweeps first (multipoles / locals are not kept from
-        the forward call); False reuses the coefficients in the workspace when
-        they are those of run(own=True) (own_locals).  With self.overlap the
-        near field's adjoint runs on `stream` beside the rest on far_stream()."""
+        the forward call); False reuses the workspace's centres and multipoles,
+        and with own_rows, what run(own_rows=...) or downward(own_rows=...) of
+        these particles filled, its locals too.  With self.overlap the near
+        field's adjoint runs on `stream` beside the rest on far_stream()."""
         if self.p > 9:
             raise ValueError("the adjoint is built for expansion orders <= 9")
         if self.leaf_range != (0, self.dt.topo.num_leaves):
             raise ValueError("the adjoint runs on the whole leaf range")
         t, dt, ws, lb = self.dt.topo, self.dt, self.ws, self.lib
+        if own_rows is not None:
+            self._check_own_rows(own_rows)
         A = self._adj_buffers()
         main, far = stream, self.far_stream() if self.overlap else stream
         s, fs = _stream_handle(main), _stream_handle(far)
@@ -942,13 +934,15 @@ class Pass:
                                   _ptr(A["units"]), _ptr(A["aux"]), _ptr(A["runs"]), _ptr(dt.node_ranges), self.G,
                                   self.eps2, _ptr(A["xm4"]), _ptr(A["partials"]), int(sc.split.shape[0]),
                                   _ptr(A["split"]), s), "jb_adj_near")
-        if recompute or not self.own_locals:
+        if recompute:
             self.upward(far)
-            self.downward(far, own=True)
+        if recompute or own_rows is None:
+            own_rows = A["own_rows"]
+            self.downward(far, own_rows=own_rows)
         _zero(A["mbar"], far)
         _zero(A["chain4"], far)
         _lib.check(lb.jb_adj_leaf_far(self.p, _ptr(ws.pos4), _ptr(A["w4"]), t.num_nodes, t.num_internal,
-                                      _ptr(dt.node_ranges), _ptr(ws.centers), self._leaf_locals_ptr(), self.G,
+                                      _ptr(dt.node_ranges), _ptr(ws.centers), _ptr(ws.locals), self.G,
                                       _ptr(A["far4"]), _ptr(A["lbar"]), None, fs), "jb_adj_leaf_far")
         items, offsets = dt.m2m_hops()
         _lib.check(lb.jb_adj_l2l_hops(self.p, len(offsets) - 1, offsets.ctypes.data, _ptr(items), _ptr(ws.centers),
@@ -959,8 +953,8 @@ class Pass:
                                  int(msc.split.shape[0]), _ptr(A["m2l_split"]), fs), "jb_adj_m2l")
         _lib.check(lb.jb_adj_far_nodes(self.p, t.num_nodes, t.num_far_pairs, _ptr(A["pair_tgt"]), _ptr(dt.far_src),
                                        _ptr(dt.far_off), _ptr(A["rev"]), _ptr(ws.mult), _ptr(A["lbar"]),
-                                       _ptr(ws.locals), _ptr(A["mbar"]), _ptr(ws.centers), _ptr(A["g4"]),
-                                       _ptr(A["cbar4"]), fs), "jb_adj_far_nodes")
+                                       _ptr(ws.locals), t.num_internal, _ptr(own_rows), _ptr(A["mbar"]),
+                                       _ptr(ws.centers), _ptr(A["g4"]), _ptr(A["cbar4"]), fs), "jb_adj_far_nodes")
         _lib.check(lb.jb_adj_leaves(self.p, self.num_l2l_units, _ptr(self.d_l2l_units), _ptr(self.d_l2l_anc),
                                     _ptr(dt.parent), _ptr(ws.centers), _ptr(A["cbar4"]), _ptr(A["mbar"]),
                                     _ptr(A["chain4"]), fs), "jb_adj_leaves")
