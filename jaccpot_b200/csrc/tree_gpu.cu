@@ -40,6 +40,7 @@
 #include "../../include/jaccpot_b200.h"
 
 #include "dev_prims.cuh"
+#include "walk_children.h"
 
 namespace jbdev {
 
@@ -355,7 +356,6 @@ __global__ void k_internal_com(int first, int last, const int* __restrict__ left
 // ---------------------------------------------------------------------------
 // 4. Dual walk, breadth-first over node pairs.
 // ---------------------------------------------------------------------------
-enum : int { kNone = 0, kSelf = 1, kFar = 2, kNear = 3, kSplitA = 4, kSplitB = 5 };
 constexpr int kMaxGears = 8;
 constexpr int kMaxGearOrder = 24;
 constexpr int kGearShift = 56;  // far keys of the adaptive walk carry the gear in bits 56..63
@@ -516,7 +516,10 @@ constexpr int kWalkThreads = 256, kWalkBlocks = 148 * 8;
 // steps without looking; with a count, a scan and an emit per step, each
 // behind a read-back, the steps of a clustered walk took 25-30 us each.
 // Nothing is written past a buffer's end, but the counts go on, so that the
-// host sees what the lists need.
+// host sees that a list needs more room.  A frontier holds every one of its
+// places below both the count and the end (walk_children); the pairs past the
+// end are dropped with all that they would open into, so after that the counts
+// are only what the lists need at least.
 template <bool ADAPTIVE>
 __global__ void __launch_bounds__(kWalkThreads) k_walk_step(const int2* __restrict__ fr, int2* __restrict__ next,
                                                             int64_t cap_front, WalkCtx w,
@@ -537,7 +540,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_step(const int2* __restri
     }
     // children (at most 4 a thread), far and near keys (at most 2) as the
     // three fields of one word: 11, 10 and 10 bits hold a block's sums
-    const unsigned ca = d == kSelf ? (ADAPTIVE ? 4 : 3) : (d >= kSplitA ? 2 : 0);
+    const unsigned ca = walk_child_count<ADAPTIVE>(d);
     const unsigned cf = d == kFar ? (ADAPTIVE ? 1 : 2) : 0, cn = d == kNear ? (ADAPTIVE ? 1 : 2) : 0;
     const unsigned mine = ca | cf << 11 | cn << 21;
     unsigned incl = mine;
@@ -562,19 +565,8 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_step(const int2* __restri
     __syncthreads();
     const int64_t oa = (int64_t)room[0] + (before & 2047u), of = (int64_t)room[1] + (before >> 11 & 1023u);
     const int64_t on = (int64_t)room[2] + (before >> 21);
-    if (d == kSelf && oa + ca <= cap_front) {
-      const int l = w.left[a], r = w.right[a];
-      next[oa] = make_int2(l, l);
-      next[oa + 1] = make_int2(r, r);
-      next[oa + 2] = make_int2(l, r);
-      if (ADAPTIVE) next[oa + 3] = make_int2(r, l);
-    } else if (d == kSplitA && oa + 2 <= cap_front) {
-      next[oa] = make_int2(w.left[a], b);
-      next[oa + 1] = make_int2(w.right[a], b);
-    } else if (d == kSplitB && oa + 2 <= cap_front) {
-      next[oa] = make_int2(a, w.left[b]);
-      next[oa + 1] = make_int2(a, w.right[b]);
-    } else if (d == kFar && of + cf <= cap_far) {
+    walk_children<ADAPTIVE>(d, a, b, w.left, w.right, next, oa, cap_front);
+    if (d == kFar && of + cf <= cap_far) {
       far_keys[of] = ((uint64_t)g << kGearShift) | ((uint64_t)a << far_shift) | (uint64_t)b;
       if (!ADAPTIVE) far_keys[of + 1] = ((uint64_t)b << far_shift) | (uint64_t)a;
     } else if (d == kNear && on + cn <= cap_near) {
@@ -665,9 +657,10 @@ int64_t walk_lists(jb_dtree& t, const WalkCtx& w, bool adaptive, int NN, int L, 
   DBuf w0, w1, queue, far_keys, near_keys;
   int64_t n_far = 0, n_near = 0;
   if (NN > 1) {
-    // room for the widest frontier and the lists seen over the configurations
-    // (frontier below 40 pairs a node, far list below 256 a node); a walk that
-    // needs more is counted to its end, then run again with twice the room
+    // room for the widest frontier and the lists of the usual opening angles
+    // (at theta 0.6 below 40 pairs a node in a frontier and 256 in the far list;
+    // uniform, theta 0.2: 100 in a frontier); a walk that needs more runs again
+    // with twice what it counted, until everything has found room
     int64_t cap_front = std::max<int64_t>(1 << 16, 64 * (int64_t)NN);
     int64_t cap_far = std::max<int64_t>(1 << 16, 256 * (int64_t)NN), cap_near = std::max<int64_t>(1 << 16, 256 * (int64_t)L);
     ck(queue.alloc(kWalkWords * 8));
