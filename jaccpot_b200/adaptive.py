@@ -125,7 +125,7 @@ def prepare(positions, masses, *, leaf_size: int, orders, eps: float, theta_max:
     ps = engine.Pass(dt, p_top, G=G, eps2=eps2, m2l_mode=m2l_mode, p2p_mode=p2p_mode, **pass_kw)
     ps.ws.pos4, ps.ws.centers, ps.ws.mult = tree_ws
     if len(orders) > 1 and topo.num_far_pairs:
-        ps.set_gears(topo.device_arrays["far_gears"], orders)
+        ps.set_gears(topo.device_array("far_gears"), orders)
     return AdaptivePrepared(topology=topo, device_topology=dt, pass_=ps, orders=orders, eps=float(eps),
                             theta_max=float(theta_max), prepass_far_pairs=pre_far,
                             prepass_near=pre_near)

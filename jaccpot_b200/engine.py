@@ -62,12 +62,13 @@ class DeviceTopology:
         self.device = dev
         # arrays of a tree built on this device are taken as they are, others
         # are uploaded (a dummy word when empty, so no pointer is null)
-        built = topo.device_array if isinstance(topo, DeviceBuiltTopology) else (lambda name: None)
+        built = topo.device_array if isinstance(topo, DeviceBuiltTopology) else (lambda name, stream: None)
         self.as_built = True  # every array as the device builder left it
         here = torch.device(dev.type, torch.cuda.current_device() if dev.index is None else dev.index)
+        stream = _lib.stream_handle(here)
 
         def up(name, dt, empty=False):
-            t = built(name)
+            t = built(name, stream)
             if t is not None and t.device == here:
                 return t
             self.as_built = False

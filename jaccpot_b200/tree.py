@@ -114,7 +114,11 @@ class DeviceBuiltTopology(Topology):
     read as numpy arrays; from then on the host's array is the field.  An
     evaluation needs only the sizes and the level offsets there: at clustered
     1M the copies down and up again were 35 of the 52 ms that the GPU was busy
-    in a call on new particles, and most of the host's 140 ms."""
+    in a call on new particles, and most of the host's 140 ms.
+
+    The tensors are filled in order on the stream that was current when the
+    object was made; reads on the host, and ``device_array`` under another
+    stream, wait for that."""
 
     m2l_targets = _OnFirstRead()
     far_gears = _OnFirstRead()
@@ -130,9 +134,21 @@ class DeviceBuiltTopology(Topology):
         t.leaf_size, t.theta = int(leaf_size), float(theta)
         t.level_offsets = level_offsets
         t.gear_orders = None if gear_orders is None else tuple(int(o) for o in gear_orders)
-        t.device_arrays = arrays
         t._sizes = _field_sizes(n, info)
+        t._take(arrays, {})
         return t
+
+    def _take(self, arrays: dict, streams: dict) -> None:
+        """The tensors, those without an entry in `streams` (the stream they
+        belong to) being of the current one, and an event behind what fills them."""
+        import torch
+
+        device = next(iter(arrays.values())).device
+        here = _lib.stream_handle(device)
+        self.device_arrays = arrays
+        self._streams = {name: streams.get(name, here) for name in arrays}
+        self._ready = torch.cuda.Event()
+        self._ready.record(torch.cuda.current_stream(device))
 
     @property
     def num_far_pairs(self) -> int:
@@ -142,17 +158,30 @@ class DeviceBuiltTopology(Topology):
     def num_near_pairs(self) -> int:
         return int(self.near_leaves.shape[0]) if "near_leaves" in self.__dict__ else self._sizes["near_leaves"]
 
-    def device_array(self, name: str):
-        """The field's tensor, with at least one element; None when the field has
-        been read on the host, whose array then counts."""
-        return None if name in self.__dict__ else self.__dict__.get("device_arrays", {}).get(name)
+    def device_array(self, name: str, stream: int | None = None):
+        """The field's tensor, with at least one element, for use on the current
+        stream (`stream`: its handle, for callers that have it); None when the
+        field has been read on the host, whose array then counts."""
+        a = None if name in self.__dict__ else self.__dict__.get("device_arrays", {}).get(name)
+        if a is not None and (_lib.stream_handle(a.device) if stream is None else stream) != self._streams[name]:
+            import torch
+
+            here = torch.cuda.current_stream(a.device)
+            here.wait_event(self._ready)
+            a.record_stream(here)  # its memory waits for this use before it serves another
+        return a
 
     def with_geometry(self, centers_f64, radii_f64) -> "DeviceBuiltTopology":
-        """The same tree and lists with other centres and radii (device tensors)."""
+        """The same tree and lists with other centres and radii (device tensors
+        of the current stream)."""
+        import torch
+
         t = copy.copy(self)
-        for name in ("centers_f64", "radii_f64"):
+        moved = {"centers_f64": centers_f64, "radii_f64": radii_f64}
+        for name in moved:
             t.__dict__.pop(name, None)
-        t.device_arrays = dict(self.device_arrays, centers_f64=centers_f64, radii_f64=radii_f64)
+        torch.cuda.current_stream(centers_f64.device).wait_event(self._ready)  # one event for both
+        t._take({**self.device_arrays, **moved}, {k: s for k, s in self._streams.items() if k not in moved})
         return t
 
     def _host(self, name: str):
@@ -163,6 +192,7 @@ class DeviceBuiltTopology(Topology):
             elif name not in d.get("device_arrays", {}):  # far_gears without an error-controlled walk
                 return None
             else:
+                self._ready.synchronize()
                 a = d["device_arrays"][name][:self._sizes[name]].cpu().numpy()
                 d[name] = a.reshape({"node_ranges": (-1, 2), "centers_f64": (-1, 3)}.get(name, (-1,)))
         return d[name]
@@ -318,6 +348,7 @@ class DeviceTree:
         self._lb = _lib.lib()
         self._h = ctypes.c_void_p()
         stream = _lib.stream_handle(pos.device)
+        self._streams = {stream}  # the handle's buffers are freed on these
         _lib.check(self._lb.jb_tree_build_device(n, pos.data_ptr(), mass.data_ptr(), self.leaf_size, self.theta,
                                                  stream, ctypes.byref(self._h)), "jb_tree_build_device")
         self.info = _lib.TreeInfo()
@@ -339,6 +370,7 @@ class DeviceTree:
         if pw.dim() != 2 or pw.shape[0] != self.info.num_nodes or fs.shape != (self.info.num_nodes,):
             raise ValueError("power must be (num_nodes, P+1) and force_scale (num_nodes,)")
         stream = _lib.stream_handle(self.device)
+        self._streams.add(stream)
         _lib.check(self._lb.jb_dtree_adaptive_walk(self._h, int(pw.shape[1]), pw.data_ptr(), fs.data_ptr(),
                                                    float(G), float(eps), float(theta_max), int(orders.size),
                                                    orders.ctypes.data, stream), "jb_dtree_adaptive_walk")
@@ -372,6 +404,8 @@ class DeviceTree:
         for f in names:
             if self.sizes[f] == 0:
                 arrays[f].zero_()
+        for s in self._streams - {stream}:  # the copies are done before a buffer is freed
+            _lib.check(self._lb.jb_stream_wait(s, stream), "jb_stream_wait")
         offsets = np.empty(self.info.num_levels + 1, dtype=np.int32)
         _lib.check(self._lb.jb_dtree_copy(self._h, _lib.DTREE_FIELDS["level_offsets"][0], offsets.ctypes.data),
                    "tree field copy (level_offsets)")
