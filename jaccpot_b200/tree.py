@@ -9,9 +9,8 @@ jaccpot/runtime/fmm_state.py:870-897 for the state that carries them.
 
 from __future__ import annotations
 
-import copy
 import ctypes
-from dataclasses import dataclass, field
+from dataclasses import dataclass, field, fields
 
 import numpy as np
 
@@ -176,13 +175,19 @@ class DeviceBuiltTopology(Topology):
         of the current stream)."""
         import torch
 
-        t = copy.copy(self)
+        t = object.__new__(DeviceBuiltTopology)
+        t.__dict__.update(self.__dict__)
         moved = {"centers_f64": centers_f64, "radii_f64": radii_f64}
         for name in moved:
             t.__dict__.pop(name, None)
         torch.cuda.current_stream(centers_f64.device).wait_event(self._ready)  # one event for both
         t._take({**self.device_arrays, **moved}, {k: s for k, s in self._streams.items() if k not in moved})
         return t
+
+    def __reduce__(self):
+        """Copies and saved files are plain Topologies of host arrays, which a
+        process without a GPU can load."""
+        return Topology, tuple(getattr(self, f.name) for f in fields(Topology))
 
     def _host(self, name: str):
         d = self.__dict__

@@ -5,6 +5,9 @@ the copies out of them are done.  The reference is the host build."""
 
 from __future__ import annotations
 
+import copy
+import pickle
+
 import numpy as np
 import pytest
 
@@ -99,3 +102,21 @@ def test_a_pass_on_another_stream_waits(particles):
     del topo
     ps.load_particles(p, m)
     assert torch.equal(ps.run(), want)
+
+
+@pytest.mark.parametrize("gears", [False, True])
+@pytest.mark.parametrize("again", [lambda t: pickle.loads(pickle.dumps(t)), copy.deepcopy, copy.copy])
+def test_saved_and_copied_topologies_are_host_arrays(particles, again, gears):
+    pos, mass = particles
+    with tree.DeviceTree(pos, mass, leaf_size=16, theta=0.6) as dtree:
+        if gears:
+            nn = dtree.info.num_nodes
+            dtree.adaptive_walk(torch.ones((nn, 4), device="cuda"), torch.ones(nn, device="cuda"), G=1.0, eps=1e-2,
+                                gear_orders=(1, 3))
+        topo = dtree.topology()
+    back = again(topo)
+    assert type(back) is tree.Topology
+    assert all(v is None or isinstance(v, (int, float, tuple, np.ndarray)) for v in vars(back).values())
+    assert (back.theta, back.leaf_size, back.gear_orders) == (topo.theta, topo.leaf_size, topo.gear_orders)
+    assert (back.far_gears is None) == (not gears) and (not gears or np.array_equal(back.far_gears, topo.far_gears))
+    _same(back, topo)
