@@ -193,7 +193,9 @@ JB_API int jb_dtree_adaptive_walk(jb_dtree* t, int num_degrees, const double* po
  * (runtime/kernels/_m2l.py:1667) and near-field schedules
  * (nearfield/_schedules.py:271).  All pointers are DEVICE memory; the handle
  * owns its outputs (pool memory, freed on the build stream).  The calls
- * synchronise the stream.                                                   */
+ * synchronise the stream; the _queued forms leave the last kernels in flight,
+ * so that their inputs and outputs are in order on that stream alone, and so
+ * do jb_l2l_schedule_device and jb_m2m_schedule_device.                     */
 typedef struct jb_dsched jb_dsched;
 typedef struct {
   int64_t num_units, num_split, num_slots, num_runs, num_targets;
@@ -214,6 +216,11 @@ JB_API int jb_m2l_schedule_device(int num_nodes, const int64_t* far_off, int max
                                   const int* targets, void* stream, jb_dsched** out);
 /* Leaves [leaf_lo, leaf_hi); max_sources >= 1. */
 JB_API int jb_leaf_schedule_device(int num_internal, int num_leaves, const int* node_ranges, const int64_t* near_off,
+                                   const int* near_src, int leaf_lo, int leaf_hi, int max_sources, void* stream,
+                                   jb_dsched** out);
+JB_API int jb_m2l_schedule_queued(int num_nodes, const int64_t* far_off, int max_pairs, int num_targets,
+                                  const int* targets, void* stream, jb_dsched** out);
+JB_API int jb_leaf_schedule_queued(int num_internal, int num_leaves, const int* node_ranges, const int64_t* near_off,
                                    const int* near_src, int leaf_lo, int leaf_hi, int max_sources, void* stream,
                                    jb_dsched** out);
 /* gears: int32 per far pair in [0, num_gears) (JB_ERR_INDEX otherwise). */

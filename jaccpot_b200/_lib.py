@@ -113,6 +113,8 @@ _SIGNATURES = {
     "jb_far_level_weights": [_I, _I, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P],
     "jb_leaf_eval_weighted": [_I, _I, _P, _P, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _F, _F, _P, _P, _I, _P, _P],
     "jb_m2l_schedule_device": [_I, _P, _I, _I, _P, _P, ctypes.POINTER(_P)],
+    "jb_m2l_schedule_queued": [_I, _P, _I, _I, _P, _P, ctypes.POINTER(_P)],
+    "jb_leaf_schedule_queued": [_I, _I, _P, _P, _P, _I, _I, _I, _P, ctypes.POINTER(_P)],
     "jb_leaf_schedule_device": [_I, _I, _P, _P, _P, _I, _I, _I, _P, ctypes.POINTER(_P)],
     "jb_gear_schedule_device": [_I, _P, _P, _P, _I, _I, _P, ctypes.POINTER(_P)],
     "jb_gear_mixed_schedule_device": [_I, _P, _P, _P, _I, _P, _I, _I, _P, ctypes.POINTER(_P)],

@@ -1149,11 +1149,22 @@ int run_builder(jb_dsched** out, cudaStream_t st, F&& fn) {
   return JB_OK;
 }
 
+// A builder's result once its stream has reached the end of it.
+int finished(int rc, void* stream, jb_dsched** out) {
+  if (rc != JB_OK) return rc;
+  rc = jb::cuda_status(cudaStreamSynchronize(reinterpret_cast<cudaStream_t>(stream)));
+  if (rc != JB_OK) {
+    delete *out;
+    *out = nullptr;
+  }
+  return rc;
+}
+
 }  // namespace
 
 extern "C" {
 
-JB_API int jb_m2l_schedule_device(int num_nodes, const int64_t* far_off, int max_pairs, int num_targets,
+JB_API int jb_m2l_schedule_queued(int num_nodes, const int64_t* far_off, int max_pairs, int num_targets,
                                   const int* targets, void* stream, jb_dsched** out) {
   if (num_nodes < 0 || !far_off || max_pairs < 1 || (targets && num_targets < 0)) return JB_ERR_ARG;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -1162,7 +1173,12 @@ JB_API int jb_m2l_schedule_device(int num_nodes, const int64_t* far_off, int max
   });
 }
 
-JB_API int jb_leaf_schedule_device(int num_internal, int num_leaves, const int* node_ranges, const int64_t* near_off,
+JB_API int jb_m2l_schedule_device(int num_nodes, const int64_t* far_off, int max_pairs, int num_targets,
+                                  const int* targets, void* stream, jb_dsched** out) {
+  return finished(jb_m2l_schedule_queued(num_nodes, far_off, max_pairs, num_targets, targets, stream, out), stream, out);
+}
+
+JB_API int jb_leaf_schedule_queued(int num_internal, int num_leaves, const int* node_ranges, const int64_t* near_off,
                                    const int* near_src, int leaf_lo, int leaf_hi, int max_sources, void* stream,
                                    jb_dsched** out) {
   if (num_internal < 0 || num_leaves < 0 || !node_ranges || !near_off || !near_src || leaf_lo < 0 ||
@@ -1172,6 +1188,14 @@ JB_API int jb_leaf_schedule_device(int num_internal, int num_leaves, const int* 
   return run_builder(out, st, [&](jb_dsched& d) {
     build_leaf(d, num_internal, node_ranges, near_off, near_src, leaf_lo, leaf_hi, max_sources, st);
   });
+}
+
+JB_API int jb_leaf_schedule_device(int num_internal, int num_leaves, const int* node_ranges, const int64_t* near_off,
+                                   const int* near_src, int leaf_lo, int leaf_hi, int max_sources, void* stream,
+                                   jb_dsched** out) {
+  return finished(jb_leaf_schedule_queued(num_internal, num_leaves, node_ranges, near_off, near_src, leaf_lo, leaf_hi,
+                                          max_sources, stream, out),
+                  stream, out);
 }
 
 JB_API int jb_l2l_schedule_device(int num_internal, int leaf_lo, int leaf_hi, const int* parent, const int64_t* far_off,

@@ -437,7 +437,7 @@ def m2l_schedule_device(dt, max_pairs: int = 64, targets=None) -> M2LSchedule:
     tg = None
     if targets is not None:
         tg = torch.as_tensor(np.asarray(targets, dtype=np.int32)).to(dt.device)
-    info, field, free = _run_device("jb_m2l_schedule_device",
+    info, field, free = _run_device("jb_m2l_schedule_queued",
                                     [t.num_nodes, _ptr(dt.far_off), int(max_pairs),
                                      -1 if tg is None else int(tg.numel()), None if tg is None else _ptr(tg)],
                                     dt.device)
@@ -455,7 +455,7 @@ def leaf_schedule_device(dt, max_sources: int = 4096, leaf_range: tuple[int, int
 
     t = dt.topo
     lo, hi = (0, t.num_leaves) if leaf_range is None else (int(leaf_range[0]), int(leaf_range[1]))
-    info, field, free = _run_device("jb_leaf_schedule_device",
+    info, field, free = _run_device("jb_leaf_schedule_queued",
                                     [t.num_internal, t.num_leaves, _ptr(dt.node_ranges), _ptr(dt.near_off),
                                      _ptr(dt.near_src), lo, hi, int(max_sources)], dt.device)
     try:

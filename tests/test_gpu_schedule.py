@@ -5,6 +5,8 @@ schedule gives bit-identical accelerations."""
 
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -136,3 +138,31 @@ def test_pass_is_identical_through_either_schedule(topo):
     host.load_particles(torch.from_numpy(pos).cuda(), torch.from_numpy(mass).cuda())
     b = host.run()
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("form", ["device", "queued"])
+def test_the_device_forms_of_the_c_abi_have_finished_on_return(topo, form):
+    dt = topo[0]
+    t, lb = dt.topo, _lib.lib()
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    ptr = lambda a: a.data_ptr()
+    calls = {
+        "m2l": lambda h: (t.num_nodes, ptr(dt.far_off), 4, 0, None, stream.cuda_stream, ctypes.byref(h)),
+        "leaf": lambda h: (t.num_internal, t.num_leaves, ptr(dt.node_ranges), ptr(dt.near_off), ptr(dt.near_src), 0,
+                           t.num_leaves, 64, stream.cuda_stream, ctypes.byref(h)),
+    }
+    want = {"m2l": schedule.m2l_schedule(t, max_pairs=4).units,
+            "leaf": schedule.leaf_schedule(t, max_sources=64).units}
+    for name, args in calls.items():
+        h = ctypes.c_void_p()
+        _lib.check(getattr(lb, f"jb_{name}_schedule_{form}")(*args(h)), name)
+        if form == "device":
+            assert stream.query()  # nothing of it is left in flight
+        stream.synchronize()
+        got = np.empty(want[name].shape, np.int32)
+        out = torch.empty(got.shape, dtype=torch.int32, device="cuda")
+        _lib.check(lb.jb_dsched_export(h, _lib.JB_SCHED_UNITS, ptr(out), got.nbytes, stream.cuda_stream), "export")
+        stream.synchronize()
+        assert np.array_equal(out.cpu().numpy(), want[name])
+        lb.jb_dsched_free(h)
