@@ -587,12 +587,28 @@ class Pass:
         nodes' rungs (a node's rung is its particles' finest), the same for both
         directions of a pair (force.py:885, :920 there)."""
         t, dt = self.dt.topo, self.dt
+        rung_sorted, level_weights = self._level_args(rung_sorted, level_weights, stream)
         f = self._weight_buffers()
         _lib.check(self.lib.jb_far_level_weights(t.num_nodes, t.num_internal, _ptr(dt.node_ranges), _ptr(dt.parent),
                                                  _ptr(rung_sorted), _ptr(dt.far_off), _ptr(dt.far_src),
                                                  int(level_weights.numel()), _ptr(level_weights), _ptr(f["scratch"]),
                                                  _ptr(f["far_w"]), _stream_handle(stream)), "jb_far_level_weights")
         return f["far_w"][:t.num_far_pairs]
+
+    def _level_args(self, rung_sorted: torch.Tensor, level_weights: torch.Tensor, stream):
+        """Both as the kernels read them (int32 per particle, float32, contiguous,
+        on the device), in order and alive for a launch on `stream`."""
+        dev = self.dt.device
+        r = rung_sorted.to(device=dev, dtype=torch.int32).reshape(-1).contiguous()
+        lw = level_weights.to(device=dev, dtype=torch.float32).reshape(-1).contiguous()
+        if r.numel() < self.dt.topo.num_particles:
+            raise ValueError("one rung per particle is required")
+        made = [b for a, b in ((rung_sorted, r), (level_weights, lw)) if b.data_ptr() != a.data_ptr()]
+        if made and stream is not None:
+            stream.wait_stream(torch.cuda.current_stream(dev))
+            for b in made:
+                b.record_stream(stream)
+        return r, lw
 
     def _weight_buffers(self) -> dict:
         if getattr(self, "_weights", None) is None:
@@ -604,6 +620,7 @@ class Pass:
     def run_weighted(self, rung_sorted: torch.Tensor, level_weights: torch.Tensor) -> torch.Tensor:
         """run() with every pair scaled by its level's weight: the near field on
         the current stream beside the far-field chain on far_stream()."""
+        rung_sorted, level_weights = self._level_args(rung_sorted, level_weights, None)
         main, far = None, self.far_stream() if self.overlap else None
         if far is not None:
             _wait(far, main)
@@ -620,8 +637,7 @@ class Pass:
         """evaluate() with every near pair scaled by
         level_weights[max(rung_i, rung_j)] (rung per sorted particle)."""
         t, dt, ws, sc = self.dt.topo, self.dt, self.ws, self.leaf_sched
-        r = rung_sorted.to(device=dt.device, dtype=torch.int32).contiguous()
-        lw = level_weights.to(device=dt.device, dtype=torch.float32).contiguous()
+        r, lw = self._level_args(rung_sorted, level_weights, stream)
         mode = self.p2p_mode
         if part is not None:
             mode |= self._PARTS[part]

@@ -31,3 +31,26 @@ def test_weights_equal_numpy(kind, n, leaf, levels):
     node = np.array([max(-1, rung[a:b + 1].max()) for a, b in topo.node_ranges])
     want = lw[np.clip(np.maximum(node[topo.far_pair_targets()], node[topo.far_sources]), 0, levels - 1)]
     assert got.shape == (topo.num_far_pairs,) and np.array_equal(got, want)
+
+
+def test_rungs_and_weights_of_any_type_and_layout():
+    n = 5000
+    pos, mass = workloads.GENERATORS["plummer"](n, 2)
+    topo = tree.build_topology(pos, mass, leaf_size=16, theta=0.7, device="cuda")
+    ps = engine.Pass(engine.DeviceTopology(topo, "cuda"), 3)
+    ps.load_particles(torch.from_numpy(pos).cuda(), torch.from_numpy(mass).cuda())
+    rung = torch.from_numpy(np.random.default_rng(5).integers(0, 4, n).astype(np.int32)).cuda()
+    lw = torch.tensor([1.0, 0.5, 0.25, 0.125], device="cuda")
+    want_w, want = ps.far_level_weights(rung, lw).clone(), ps.run_weighted(rung, lw).clone()
+    odd = (torch.stack([rung, rung - 7], dim=1)[:, 0].long(), torch.stack([lw, lw + 1], dim=1).double()[:, 0])
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for r, w in (odd, (odd[0].cpu(), odd[1].cpu())):
+        assert torch.equal(ps.far_level_weights(r, w), want_w)
+        assert torch.equal(ps.run_weighted(r, w), want)
+        got = ps.far_level_weights(r, w, side)
+        side.synchronize()
+        assert torch.equal(got, want_w)
+    for call in (ps.far_level_weights, ps.run_weighted, ps.evaluate_weighted):
+        with pytest.raises(ValueError, match="one rung per particle"):
+            call(rung[:-1], lw)
