@@ -249,12 +249,14 @@ JB_API int jb_far_reverse_index(int num_nodes, const int64_t* far_off, const int
  * there is none): the sweep by levels starts at its level.                  */
 JB_API int jb_l2l_schedule_device(int num_internal, int leaf_lo, int leaf_hi, const int* parent, const int64_t* far_off,
                                   void* stream, jb_dsched** out);
-/* Items of jb_m2m_hops: JB_SCHED_AUX holds int32[num_units][2] (node, source;
+/* Items of jb_m2m_hops, for a tree of up to JB_M2M_HOPS_MAX_LEVELS levels of
+ * internal nodes (JB_ERR_ARG for one that needs more than JB_MAX_M2M_HOPS): JB_SCHED_AUX holds int32[num_units][2] (node, source;
  * -1 where a place is empty), hop k's in [hop_offsets[k], hop_offsets[k + 1]),
  * both multiples of 32.  The lowest single_levels (0 to 16) heights above the
  * leaves have a hop each, the others one for four.  hop_offsets is host memory
  * for JB_MAX_M2M_HOPS + 1 values, *num_hops the hops used.                  */
 #define JB_MAX_M2M_HOPS 64
+#define JB_M2M_HOPS_MAX_LEVELS 208
 JB_API int jb_m2m_schedule_device(int num_nodes, int num_internal, const int* parent, const int* left,
                                   const int* right, int single_levels, int64_t* hop_offsets, int* num_hops,
                                   void* stream, jb_dsched** out);

@@ -33,6 +33,7 @@ JB_LEAF_EVAL_NOALLOC_MAX_SLOTS = 16384
 JB_MAX_LEAF_OCCUPANCY = 64
 JB_MIXED_GEAR_SEGMENTS = 4
 JB_MAX_M2M_HOPS = 64
+JB_M2M_HOPS_MAX_LEVELS = 208
 JB_LEAF_ERR_OCCUPANCY, JB_LEAF_ERR_SLOT = 1, 2
 (JB_SCHED_UNITS, JB_SCHED_AUX, JB_SCHED_RUNS, JB_SCHED_SPLIT, JB_SCHED_FAR_SOURCES, JB_SCHED_GEAR_OFFSETS,
  JB_SCHED_TARGETS, JB_SCHED_PAIRS_PER_GEAR) = range(8)

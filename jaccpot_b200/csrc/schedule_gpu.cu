@@ -929,7 +929,7 @@ __global__ void k_anc_count(int num_internal, int lo, int hi, const int* __restr
         top = a;  // ids fall towards the root
       }
     cnt[j] = c;
-    key[j] = (uint64_t)(255 - c);  // a tree has fewer than 128 levels
+    key[j] = (uint64_t)(255 - min(c, 255));  // one digit; a built tree has fewer than 128 levels
   }
   const unsigned have = __ballot_sync(kFull, ok && c > 0);
   top = __reduce_min_sync(kFull, top);
@@ -1001,6 +1001,7 @@ void build_l2l(jb_dsched& d, int num_internal, int lo, int hi, const int* parent
 // ---------------------------------------------------------------------------
 constexpr int kHopLevels = 4, kHopMost = 1 << kHopLevels;
 constexpr int kHopClasses = kHopLevels;  // padded sizes kHopMost, ..., 4, 2
+constexpr int kHopKeys = JB_MAX_M2M_HOPS * kHopClasses;
 
 struct HopBands {
   int singles;
@@ -1055,13 +1056,14 @@ __global__ void k_hop_keys(int num_internal, const int* __restrict__ left, const
   hop_sources(i, left, right, height, bands, [&](int) { ++n; });
   int cls = 0;  // padded size kHopMost >> cls
   while ((kHopMost >> (cls + 1)) >= n) ++cls;
-  const int k = bands.hop(height[i]) * kHopClasses + cls;  // heights below 128, at most 16 singles: under 192 keys
+  // a built tree's heights are below 128: with at most 16 singles under 192
+  // keys; a deeper one is counted past them and refused
+  const int k = min(bands.hop(height[i]) * kHopClasses + cls, kHopKeys);
   key[i] = (uint64_t)k;
   idx[i] = i;
   atomicAdd(bins + k, 1);
 }
 
-constexpr int kHopKeys = 256;
 struct HopLayout {
   int first[kHopKeys];  // place of the key's first node in key order
   int item[kHopKeys];   // its first item
@@ -1088,22 +1090,23 @@ void build_m2m(jb_dsched& d, int num_nodes, int num_internal, const int* parent,
   Scratch s;
   DBuf height, arrived, k0, k1, v0, v1;
   ck(height.alloc((size_t)num_nodes * 4));
-  ck(arrived.alloc(((size_t)num_internal + kHopKeys) * 4));  // and the key counts
+  ck(arrived.alloc(((size_t)num_internal + kHopKeys + 1) * 4));  // and the key counts
   int* bins = arrived.as<int>() + num_internal;
   for (DBuf* b : {&k0, &k1}) ck(b->alloc((size_t)num_internal * 8));
   for (DBuf* b : {&v0, &v1}) ck(b->alloc((size_t)num_internal * 4));
   ck(cudaMemsetAsync(height.p, 0, (size_t)num_nodes * 4, st));
-  ck(cudaMemsetAsync(arrived.p, 0, ((size_t)num_internal + kHopKeys) * 4, st));
+  ck(cudaMemsetAsync(arrived.p, 0, ((size_t)num_internal + kHopKeys + 1) * 4, st));
   k_node_heights<<<nblocks(num_nodes - num_internal, 128), 128, 0, st>>>(num_internal, num_nodes, parent,
                                                                          height.as<int>(), arrived.as<int>());
   ck_launch();
   k_hop_keys<<<nblocks(num_internal, 128), 128, 0, st>>>(num_internal, left, right, height.as<int>(), bands,
-                                                         k0.as<uint64_t>(),                                                         v0.as<int>(), bins);
+                                                         k0.as<uint64_t>(), v0.as<int>(), bins);
   ck_launch();
-  int count[kHopKeys];
+  int count[kHopKeys + 1];
   ck(cudaMemcpyAsync(count, bins, sizeof(count), cudaMemcpyDeviceToHost, st));
   radix_sort(k0.as<uint64_t>(), v0.as<int>(), k1.as<uint64_t>(), v1.as<int>(), num_internal, 8, s, st);
   ck(cudaStreamSynchronize(st));
+  if (count[kHopKeys] > 0) throw Fail{JB_ERR_ARG};
   HopLayout h{};
   int nodes = 0, hops = 0;
   int64_t items = 0;

@@ -445,7 +445,8 @@ class Pass:
         self.d_l2l_units = up(units)
         self.d_l2l_anc = up(anc)
         # the M2M by hops of several levels, or level by level on a large tree
-        self.m2m_hops = _on_gpu(dt) and t.num_internal <= M2M_HOPS_MAX_INTERNAL
+        self.m2m_hops = (_on_gpu(dt) and t.num_internal <= M2M_HOPS_MAX_INTERNAL
+                         and t.num_levels <= _lib.JB_M2M_HOPS_MAX_LEVELS)
         if self.m2m_hops:
             dt.m2m_hops()
         # run(): the near field on the caller's stream while the upward sweep,
@@ -935,6 +936,8 @@ class Pass:
             raise ValueError("the adjoint is built for expansion orders <= 9")
         if self.leaf_range != (0, self.dt.topo.num_leaves):
             raise ValueError("the adjoint runs on the whole leaf range")
+        if self.dt.topo.num_levels > _lib.JB_M2M_HOPS_MAX_LEVELS:  # no built tree has 128
+            raise ValueError(f"the adjoint is built for trees of up to {_lib.JB_M2M_HOPS_MAX_LEVELS} levels")
         t, dt, ws, lb = self.dt.topo, self.dt, self.ws, self.lib
         if own_rows is not None:
             self._check_own_rows(own_rows)
