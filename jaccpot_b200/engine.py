@@ -987,18 +987,19 @@ class Pass:
                                          _ptr(grad_mass), s), "jb_gather_unsorted(grad)")
 
     def launches_per_run(self) -> int:
-        """This library's kernel launches in one run(): P2M, one M2M per hop or level,
-        the M2L (one launch per non-empty gear with gears) and its split
-        reduce, one L2L per level from the first with a non-zero local, the
-        leaf L2P + P2P and their split reduce."""
+        """This library's kernel launches in one run() with the FP32 M2L: P2M, one
+        M2M per hop or level, the fill that zeroes the locals, the M2L (one launch
+        per non-empty gear with gears by gear) and its split reduce, the L2L (one
+        launch straight to the leaves, or one per level from the first with a
+        non-zero local), the near field, the L2P and the sum of split leaves."""
         t = self.dt.topo
         gs = getattr(self, "gear_sched", None)
-        if isinstance(gs, MixedGearM2LSchedule):
-            m2l = int(gs.units.shape[0] > 0) + int(gs.split.shape[0] > 0)
-        elif gs is not None and self.m2l_mode == _lib.JB_M2L_FP32:
-            m2l = int((np.diff(np.asarray(gs.gear_offsets)) > 0).sum()) + int(gs.split.shape[0] > 0)
+        sc = self.m2l_sched if gs is None or self.m2l_mode != _lib.JB_M2L_FP32 else gs
+        if hasattr(sc, "gear_offsets"):
+            m2l = int((np.diff(np.asarray(sc.gear_offsets)) > 0).sum())
         else:
-            m2l = 1 + int(self.m2l_sched.split.shape[0] > 0)
-        l2l = t.num_levels - self.dt.l2l_first_level
+            m2l = int(sc.units.shape[0] > 0)
+        m2l += int(sc.split.shape[0] > 0)
+        l2l = int(self.num_l2l_units > 0) if self.l2l_direct else t.num_levels - self.dt.l2l_first_level
         m2m = int((np.diff(self.dt.m2m_hops()[1]) > 0).sum()) if self.m2m_hops else t.num_levels
-        return (1 + m2m + m2l + l2l + 2 + int(self.leaf_sched.split.shape[0] > 0))
+        return 1 + m2m + 1 + m2l + l2l + 2 + int(self.leaf_sched.split.shape[0] > 0)
