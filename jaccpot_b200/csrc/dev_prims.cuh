@@ -102,29 +102,6 @@ inline unsigned nblocks(int64_t n, int per) { return (unsigned)std::max<int64_t>
 // ---------------------------------------------------------------------------
 constexpr int kScanThreads = 1024, kScanItems = 4, kScanTile = kScanThreads * kScanItems;
 
-// Three counters scanned together (the dual walk's children / far / near).
-struct I3 {
-  int a, b, c;
-};
-__device__ __forceinline__ I3 operator+(I3 x, I3 y) { return I3{x.a + y.a, x.b + y.b, x.c + y.c}; }
-__device__ __forceinline__ I3 operator-(I3 x, I3 y) { return I3{x.a - y.a, x.b - y.b, x.c - y.c}; }
-template <typename T>
-__device__ __forceinline__ T zero() {
-  return T(0);
-}
-template <>
-__device__ __forceinline__ I3 zero<I3>() {
-  return I3{0, 0, 0};
-}
-template <typename T>
-__device__ __forceinline__ T shfl_up(T v, int o) {
-  return __shfl_up_sync(kFull, v, o);
-}
-template <>
-__device__ __forceinline__ I3 shfl_up<I3>(I3 v, int o) {
-  return I3{__shfl_up_sync(kFull, v.a, o), __shfl_up_sync(kFull, v.b, o), __shfl_up_sync(kFull, v.c, o)};
-}
-
 // Exclusive scan of one tile per block; the tile's sum goes to tile_sums
 // (and to *total when the whole input is one tile).
 template <typename T>
@@ -135,16 +112,16 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const T* __restrict
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
   T v[kScanItems];
-  T s = zero<T>();
+  T s = T(0);
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
-    v[i] = (base + i < n) ? in[base + i] : zero<T>();
+    v[i] = (base + i < n) ? in[base + i] : T(0);
     s = s + v[i];
   }
   T incl = s;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const T y = shfl_up<T>(incl, o);
+    const T y = __shfl_up_sync(kFull, incl, o);
     if (lane >= o) incl = incl + y;
   }
   if (lane == 31) warp_sums[warp] = incl;
@@ -154,7 +131,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const T* __restrict
     T wi = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const T y = shfl_up<T>(wi, o);
+      const T y = __shfl_up_sync(kFull, wi, o);
       if (lane >= o) wi = wi + y;
     }
     warp_sums[lane] = wi - w;

@@ -25,7 +25,8 @@
 // in between carry no derivative, and a node without far pairs none at all.
 // The sweeps level by level (jb_adj_l2l_level, jb_adj_m2m_level, jb_adj_p2m with
 // a leaf-far stage that fills cbar4) give the same gradients from complete
-// locals at every node, with a launch per level.
+// locals at every node, with a launch per level: the C ABI's plain sequence,
+// which Pass.vjp does not take and the tests check the other against.
 // Transposes come for free: the real M2L matrix is symmetric and
 // M2M(d)^T = L2L(d) for the same displacement (both checked in the tests).
 // Every output element has one writer per launch (no atomics).
@@ -33,6 +34,8 @@
 // cbar4[node] = (dL/dc_x, dL/dc_y, dL/dc_z, dL/dmu) accumulates over stages;
 // xm4[i] = (dL/dx, dL/dy, dL/dz, dL/dm) per sorted particle.
 #include "fmm_kernels.cuh"
+
+#include <algorithm>
 
 namespace jb {
 
@@ -521,8 +524,8 @@ struct RunAdj {
 
 template <int P>
 int RunAdj<P>::leaf_far(const float* pos4, const float* w4, int num_nodes, int num_internal, const int* ranges,
-                      const float* centers, const float* locals, float G, float* xm4, float* lbar, float* cbar4,
-                      cudaStream_t st) {
+                        const float* centers, const float* locals, float G, float* xm4, float* lbar, float* cbar4,
+                        cudaStream_t st) {
   const int L = num_nodes - num_internal;
   if (L <= 0) return JB_OK;
   const size_t sm = sizeof(float) * kWarpsPerBlock * (32 * (csize(P) + 1) + cstride(P));
@@ -536,7 +539,7 @@ int RunAdj<P>::leaf_far(const float* pos4, const float* w4, int num_nodes, int n
 
 template <int P>
 int RunAdj<P>::l2l_level(int first, int last, const int* left, const int* right, const float* centers,
-                       const float* locals, float* lbar, float* cbar4, cudaStream_t st) {
+                         const float* locals, float* lbar, float* cbar4, cudaStream_t st) {
   if (last <= first) return JB_OK;
   k_adj_l2l_level<P><<<blocks_for(last - first, 128), 128, 0, st>>>(
       first, last, left, right, reinterpret_cast<const float4*>(centers), locals, lbar,
@@ -546,11 +549,10 @@ int RunAdj<P>::l2l_level(int first, int last, const int* left, const int* right,
 
 template <int P>
 int RunAdj<P>::m2l_pairs(int64_t num_pairs, const int* pair_tgt, const int* far_src, const float* mult,
-                       const float* lbar, const float* centers, float* g4, cudaStream_t st) {
+                         const float* lbar, const float* centers, float* g4, cudaStream_t st) {
   if (num_pairs <= 0) return JB_OK;
   cudaFuncSetAttribute(k_adj_m2l_pairs<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_pairs_smem<P>());
-  const int64_t resident = 148 * 4 * kM2LThreads;
-  const int rounds = (int)(num_pairs >= kAdjPairs * resident ? kAdjPairs : 1 + num_pairs / resident);
+  const int rounds = (int)std::min<int64_t>(kAdjPairs, 1 + num_pairs / kM2LResident);
   k_adj_m2l_pairs<P><<<blocks_for(num_pairs, kM2LThreads * rounds), kM2LThreads, adj_pairs_smem<P>(), st>>>(
       num_pairs, pair_tgt, far_src, mult, lbar, reinterpret_cast<const float4*>(centers),
       reinterpret_cast<float4*>(g4), rounds);
@@ -594,7 +596,7 @@ int RunAdj<P>::particles(const float* pos4, int num_nodes, int num_internal, con
 
 template <int P>
 int RunAdj<P>::m2m_level(int first, int last, const int* left, const int* right, const float* centers,
-                       const float* mult, float* mbar, float* cbar4, cudaStream_t st) {
+                         const float* mult, float* mbar, float* cbar4, cudaStream_t st) {
   if (last <= first) return JB_OK;
   k_adj_m2m_level<P><<<blocks_for(last - first, 128), 128, 0, st>>>(
       first, last, left, right, reinterpret_cast<const float4*>(centers), mult, mbar,
@@ -604,7 +606,7 @@ int RunAdj<P>::m2m_level(int first, int last, const int* left, const int* right,
 
 template <int P>
 int RunAdj<P>::p2m(const float* pos4, int num_nodes, int num_internal, const int* ranges, const float* centers,
-                 const float* mbar, const float* cbar4, float* xm4, cudaStream_t st) {
+                   const float* mbar, const float* cbar4, float* xm4, cudaStream_t st) {
   const int L = num_nodes - num_internal;
   if (L <= 0) return JB_OK;
   k_adj_p2m<P><<<blocks_for(L, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, st>>>(

@@ -213,6 +213,7 @@ __global__ void __launch_bounds__(128) k_m2m_level(int first, int last, const in
 // registers (255 per thread, 8 warps per SM).
 // ---------------------------------------------------------------------------
 constexpr int kM2LThreads = 64;
+constexpr int64_t kM2LResident = 148 * 4 * kM2LThreads;  // threads of 4 blocks on each of 148 SMs (M2L_RESIDENT_THREADS)
 
 __host__ __device__ constexpr int row4(int p) { return (cstride(p) / 4) | 1; }  // float4 per smem row (odd)
 
@@ -1781,7 +1782,7 @@ struct RunP2M {
 
 template <int P>
 int RunP2M<P>::run(const float* pos4, int num_nodes, int num_internal, const int* ranges, float* centers, float* mult,
-                 cudaStream_t st) {
+                   cudaStream_t st) {
   const int L = num_nodes - num_internal;
   if (L <= 0) return JB_OK;
   const size_t sm = sizeof(float) * kWarpsPerBlock * 32 * (csize(P) + 1);
@@ -1800,7 +1801,7 @@ struct RunM2M {
 
 template <int P>
 int RunM2M<P>::run(int first, int last, const int* left, const int* right, const int* ranges, float* centers,
-                 float* mult, cudaStream_t st) {
+                   float* mult, cudaStream_t st) {
   if (last <= first) return JB_OK;
   if (last - first <= g_split_max_parents[0]) {
     k_m2m_level_split<P><<<blocks_for(2 * (int64_t)(last - first), kSplitItems), 128, 0, st>>>(
@@ -1833,8 +1834,8 @@ struct RunM2L {
 
 template <int P>
 int RunM2L<P>::run(int num_units, const int* units, const float* mult, const float* centers, const int* far_src,
-                 float* locals, float* partials, int num_split, const int* split, cudaStream_t st, bool neg,
-                 int rs, const float* far_w) {
+                   float* locals, float* partials, int num_split, const int* split, cudaStream_t st, bool neg, int rs,
+                   const float* far_w) {
   if (rs <= 0) rs = cstride(P);
   if (num_units > 0) {
     const bool coop = g_m2l_coop != 0;
@@ -1865,7 +1866,8 @@ struct RunM2LMixed {
 
 template <int P>
 int RunM2LMixed<P>::run(int num_units, const int* units, const int* bounds, const float* mult, const float* centers,
-                 const int* far_src, float* locals, float* partials, int num_split, const int* split, cudaStream_t st) {
+                        const int* far_src, float* locals, float* partials, int num_split, const int* split,
+                        cudaStream_t st) {
   const int rs = cstride(P);
   if (num_units > 0) {
     const size_t sm = sizeof(float4) * kM2LThreads * row4(P);
@@ -1892,7 +1894,7 @@ struct RunL2L {
 
 template <int P>
 int RunL2L<P>::run(int first, int last, const int* left, const int* right, const float* centers, float* locals,
-                 cudaStream_t st) {
+                   cudaStream_t st) {
   if (last <= first) return JB_OK;
   if (last - first <= g_split_max_parents[1]) {
     k_l2l_level_split<P><<<blocks_for(2 * (int64_t)(last - first), kSplitItems), 128, 0, st>>>(
@@ -1943,9 +1945,10 @@ struct RunLeafEval {
 
 template <int P>
 template <bool K, bool PT, bool FR>
-void RunLeafEval<P>::go(unsigned nb, cudaStream_t st, const float4* pos4, int num_internal, int num_units, const int4* units,
-                 const int2* aux, const int2* runs, const int2* ranges, float G, float eps2, float4* out,
-                 float4* partial, const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err) {
+void RunLeafEval<P>::go(unsigned nb, cudaStream_t st, const float4* pos4, int num_internal, int num_units,
+                        const int4* units, const int2* aux, const int2* runs, const int2* ranges, float G, float eps2,
+                        float4* out, float4* partial, const int* rung, const float* lw, int nlw, bool flat,
+                        int max_slots, int* err) {
   if (rung)
     k_leaf_units<K, PT, FR, true><<<nb, 32 * kWarpsPerBlock, 0, st>>>(pos4, num_internal, num_units, units, aux, runs,
                                                                   ranges, G, eps2, out, partial, max_slots, err,
@@ -1966,10 +1969,9 @@ void RunLeafEval<P>::go(unsigned nb, cudaStream_t st, const float4* pos4, int nu
 
 template <int P>
 int RunLeafEval<P>::run(int mode, const float* pos4, int num_internal, int num_units, const int* units, const int* aux,
-                 const int* runs, const int* ranges, const float* centers, const float* locals, float G, float eps2,
-                 float* out, float* partial, int num_split, const int* split, cudaStream_t st,
-                 const int* rung, const float* lw, int nlw, bool flat,
-                 int max_slots, int* err) {
+                        const int* runs, const int* ranges, const float* centers, const float* locals, float G,
+                        float eps2, float* out, float* partial, int num_split, const int* split, cudaStream_t st,
+                        const int* rung, const float* lw, int nlw, bool flat, int max_slots, int* err) {
   if (num_units > 0) {
     const unsigned nb = blocks_for(num_units, kWarpsPerBlock);
     auto a0 = reinterpret_cast<const float4*>(pos4);
@@ -2022,9 +2024,9 @@ struct RunTargets {
 };
 
 template <int P>
-int RunTargets<P>::run(const float* pos4, int num_internal, const int* ranges, const float* centers, const float* locals,
-                 const int64_t* near_off, const int* near_src, const int* leaf_of, int64_t nt, const int* ts, float G,
-                 float eps2, float* out, cudaStream_t st) {
+int RunTargets<P>::run(const float* pos4, int num_internal, const int* ranges, const float* centers,
+                       const float* locals, const int64_t* near_off, const int* near_src, const int* leaf_of,
+                       int64_t nt, const int* ts, float G, float eps2, float* out, cudaStream_t st) {
   if (nt <= 0) return JB_OK;
   k_targets_far<P><<<blocks_for(nt, 128), 128, 0, st>>>(
       reinterpret_cast<const float4*>(pos4), num_internal, reinterpret_cast<const float4*>(centers), locals,

@@ -48,7 +48,8 @@ def _slots(n_per: np.ndarray) -> tuple[np.ndarray, np.ndarray]:
     return slot, slot[first]
 
 
-# Threads of the M2L kernels resident on a B200: 148 SMs x 4 blocks x 64.
+# Threads of the M2L kernels resident on a B200: 148 SMs x 4 blocks x 64
+# (kM2LResident).
 M2L_RESIDENT_THREADS = 148 * 4 * 64
 
 
