@@ -1691,11 +1691,12 @@ __global__ void __launch_bounds__(128) k_targets_far(const float4* __restrict__ 
 // leaves that follow one another in memory join into runs, whose particle
 // counts are summed up in shared memory.  The warp then walks the group's
 // particles 32 at a time, each lane finding its particle's run with a cursor
-// that only advances, four particles in flight per lane.  The kernel is bound
-// by issue (70% of the slots).  A call with 65,536 targets of a Plummer sphere
-// of 1M (order 6, leaf 32, 1,900 sources each): a leaf per lane, 32 cache lines
-// to a load, 387 us of kernel; runs read in turn, one load in flight, 378 us the
-// whole call; a cursor over the leaves themselves 330; over the runs 262.
+// that only advances, four particles in flight per lane.  Bound by issue while an
+// SM works (72% of the slots), which is half of the kernel's time: a few targets
+// have many times the others' sources.  A call with 65,536 targets of a Plummer
+// sphere of 1M (order 6, leaf 32, 1,900 sources each): a leaf per lane, 32 cache
+// lines to a load, 387 us of kernel; runs read in turn, one load in flight, 378 us
+// the whole call; a cursor over the leaves themselves 330; over the runs 262.
 constexpr int kTargetWarps = 8;
 static __global__ void __launch_bounds__(32 * kTargetWarps) k_targets_near(
     const float4* __restrict__ pos4, int num_internal, const int2* __restrict__ ranges,
