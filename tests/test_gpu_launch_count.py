@@ -23,7 +23,10 @@ def _kernels(ps):
     with profile(activities=[ProfilerActivity.CUDA]) as p:
         ps.run()
         torch.cuda.synchronize()
-    return sum(1 for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA and "k_" in e.name)
+    names = [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    if not names:
+        pytest.skip("the profiler has no kernel records on this machine")
+    return sum("k_" in name for name in names)
 
 
 @pytest.mark.parametrize("form", ["direct", "hops off", "cascade", "split leaves and targets", "mixed", "per_gear",
